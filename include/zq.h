@@ -84,10 +84,10 @@ typedef enum zq_type {
  *               (inside the path's 1e-3 bar), and it NEEDS the workspace of
  *               zq_matmul_workspace_bytes(); without one the call returns ZQ_ERR_BAD_ARG (it is
  *               not served by the slower small-batch kernel behind the caller's back).
- *               17 to 48 rows: zq_matmul_workspace_bytes() is non-zero for matrices of 12 288 rows
- *               and more, and a call that brings that workspace runs the weight-streaming
- *               tensor-core form (fp16 operands, 3e-4, 2-3 x faster); a call without workspace,
- *               or on a smaller matrix, runs passes of the 16-row kernel (1e-7).
+ *               17 to 48 rows: a call that brings the workspace of zq_matmul_workspace_bytes() runs
+ *               one product in place of passes of the 16-row kernel (a call without): on matrices
+ *               of 12 288 rows and more the weight-streaming tensor-core form (fp16 operands,
+ *               3e-4), on smaller ones a form that keeps 22 mantissa bits (1e-7).
  *   ZQ_ACT_Q8 : each activation row is first quantised to 32-wide int8 blocks and
  *               the dots are exact int8 x int8 -> int32 — the Gemma-3 path
  *               (src/gguf/thread_pool.zig:96-160 -> src/gguf/simd_dot.zig:25-152).

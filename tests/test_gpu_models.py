@@ -45,6 +45,16 @@ def test_gpt2_tiny_parity(zq, oracle):
     assert max(errs) <= 1e-5, max(errs)  # f32 activations: no quantiser in the loop
 
 
+@pytest.mark.parametrize("tokens", [17, 70, 600])
+def test_gpt2_prompt_through_the_split_product(zq, oracle, tokens):
+    """Prompts of one and of two chunks; 600 tokens give every tile shape of the product work."""
+    host = hostmodel.Gpt2Host.synthetic(dict(hostmodel.GPT2_SMALL, vocab=1000, layer=1), qtype=ggml.Q4_1, seed=42, device="cuda")
+    prompt = np.random.default_rng(46).integers(0, 1000, size=tokens)
+    gt, ct, errs = run_parity(zq.Gpt2(host.randomize_small_params()), oracle.Gpt2(host, 8), prompt, 2)
+    assert gt == ct
+    assert max(errs) <= 1e-5, max(errs)
+
+
 @pytest.mark.parametrize("qtypes", [(ggml.Q8_0, ggml.Q8_0, ggml.Q8_0), (ggml.Q4_0, ggml.Q8_0, ggml.Q4_1),
                                     (ggml.Q4_1, ggml.Q4_1, ggml.Q4_1)])
 def test_gemma3_tiny_parity(zq, oracle, qtypes):

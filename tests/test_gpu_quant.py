@@ -107,6 +107,22 @@ def test_matmul_small_batches_f32(zq, oracle, qtype, m):
     assert rel_l2(got, want) <= REL_L2_GUARD
 
 
+@pytest.mark.parametrize("qtype", TYPES)
+@pytest.mark.parametrize("m,n,k", [(17, 33, 32), (45, 520, 1184), (48, 5003, 96), (24, 96, 6912)])
+def test_split_product_keeps_f32_accuracy(zq, oracle, qtype, m, n, k):
+    raw = make_weight(oracle, qtype, n, k)
+    x = make_x(m, k)
+    x[3] = 0.0
+    x[4] *= 1e20
+    bias = make_x(1, n)[0]
+    res = make_x(m, n)
+    got = zq.quant_matmul_no_grad(torch.from_numpy(x).cuda(), zq.QuantWeight(raw, qtype, n, k), zq.ACT_F32,
+                                  bias=torch.from_numpy(bias).cuda(), residual=torch.from_numpy(res).cuda()).cpu().numpy()
+    want = x.astype(np.float64) @ oracle.dequantize(qtype, raw, n * k).reshape(n, k).astype(np.float64).T + bias + res
+    for r in range(m):  # 22 bits of every activation, f32 sums of up to 216 blocks: below 2^-24 * (4 + sqrt(216)) of a row
+        assert rel_l2(got[r], want[r]) <= 1.2e-6, r
+
+
 REL_L2_GEMM_GUARD = 6e-4  # fp16 operands (weights and activations each rounded once, <= 2^-12 relative)
 
 

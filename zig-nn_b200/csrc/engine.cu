@@ -72,6 +72,7 @@ struct zq_gpt2 {
     std::vector<float*> k, v;  // per layer [ctx][embed]
     float *x = nullptr, *ln = nullptr, *qkv = nullptr, *att = nullptr, *hid = nullptr, *logits = nullptr;
     float* scores = nullptr;  // [head][ctx] attention scratch
+    void* split = nullptr;    // a prefill chunk's activations in two fp16 parts
     uint32_t* d_state = nullptr;
     int32_t* d_tokens = nullptr;   // token ids of a prefill chunk
     uint32_t max_rows = 1;         // rows the activation buffers hold (prefill chunk size)
@@ -92,7 +93,8 @@ struct zq_gpt2 {
 };
 
 // y[T][out] = W . (ln ? LayerNorm(x) : x)[T][in] + bias [gelu] [+ residual[T][out]]. Quantised weights run
-// in passes of up to 16 rows through the decode kernel (every row keeps the arithmetic of a decode step);
+// through the decode kernel up to 16 rows and through the split product (the same parts of the activations and
+// f32 sums over blocks) from 17 rows on;
 // f32 weights (the .f32 branch of linear_forward_q, gpt2.zig:652-671) row by row with a separate epilogue.
 // The norm runs as its own small launch: folded into the GEMV prologue every CTA repeats its two
 // block-wide reductions before it can start, which measured 12% slower per step.
@@ -105,6 +107,7 @@ static int gpt2_linear(zq_gpt2* m, const Linear& L, const float* x, float* y, co
     }
     zq_epilogue ep{bias, gelu, nullptr, residual};
     if (L.qw) {
+        if (T >= kSplitMinRows) return launch_gemm_split(L.qw, x, y, T, &ep, m->split, st);
         rc = launch_gemv_mma_passes_f32(L.qw, x, y, T, &ep, st);
         if (rc == ZQ_ERR_LIMIT) rc = launch_gemv_f32(L.qw, x, y, T, &ep, st);
         return rc;
@@ -263,8 +266,8 @@ int zq_gpt2_create(const zq_gpt2_config* cfg, const zq_gpt2_weights* w, zq_strea
         cudaMemsetAsync(m->k[l], 0, (size_t)cfg->ctx * E * sizeof(float), st);
         cudaMemsetAsync(m->v[l], 0, (size_t)cfg->ctx * E * sizeof(float), st);
     }
-    // activation buffers hold a prefill chunk of up to 128 tokens (a decode step uses row 0)
-    m->max_rows = cfg->ctx < 128 ? cfg->ctx : 128;
+    // activation buffers hold a prefill chunk of up to 512 tokens (a decode step uses row 0)
+    m->max_rows = cfg->ctx < 512 ? cfg->ctx : 512;
     const size_t R = m->max_rows;
     TRY(m->arena.alloc_n(&m->x, R * E));
     TRY(m->arena.alloc_n(&m->ln, R * (E > F ? E : F)));
@@ -273,6 +276,11 @@ int zq_gpt2_create(const zq_gpt2_config* cfg, const zq_gpt2_weights* w, zq_strea
     TRY(m->arena.alloc_n(&m->hid, R * F));
     TRY(m->arena.alloc_n(&m->logits, cfg->vocab));
     TRY(m->arena.alloc_n(&m->scores, R * cfg->head * cfg->ctx));
+    size_t split = 0;
+    for (const zq_gpt2::Block& b : m->blocks)
+        for (const Linear* L : {&b.qkv, &b.proj, &b.fc, &b.mproj})
+            if (L->qw) split = std::max(split, gemm_split_workspace_bytes(L->qw, m->max_rows));
+    TRY(m->arena.alloc(&m->split, split));
     TRY(m->arena.alloc_n(&m->d_tokens, R));
     TRY(m->arena.alloc_n(&m->d_state, 4));
     TRY(m->arena.alloc_n(&m->d_arg, 1));

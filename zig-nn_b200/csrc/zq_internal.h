@@ -172,6 +172,12 @@ bool gemm_trans_pair_takes(const zq_weight* w, uint32_t m_rows);
 size_t gemm_trans_pair_workspace_bytes(const zq_weight* w, uint32_t m_rows);
 int launch_gemm_trans_pair(const zq_weight* w, const float* grad_out, float* grad_x, uint32_t m_rows, int accumulate,
                            void* workspace, cudaStream_t st);
+// f32-accurate product for more rows than a pass of the decode kernel (gemm_split.cu); `workspace` holds
+// gemm_split_workspace_bytes() bytes, 256-byte aligned; x 16-byte aligned.
+int launch_gemm_split(const zq_weight* w, const float* x, float* y, uint32_t m_rows, const zq_epilogue* ep, void* workspace,
+                      cudaStream_t st);
+size_t gemm_split_workspace_bytes(const zq_weight* w, uint32_t m_rows);
+constexpr uint32_t kSplitMinRows = 17;
 constexpr uint32_t kStreamMinRowsF32 = 17;  // f32-activation calls from this many rows on take it when they bring a workspace
 
 // ---- fused decode-step launchers (ops.cu). `state` is device memory: state[0] = current token,
