@@ -139,6 +139,27 @@ def test_gpt2_small_full_size_greedy_64(zq, oracle):
     assert max(errs) <= 1e-3, max(errs)
 
 
+@pytest.mark.parametrize("head,kv,dim", [(4, 1, 32), (2, 1, 64), (4, 2, 64), (3, 1, 128), (2, 1, 256), (40, 1, 256)])
+def test_gemma3_prompt_attention_bit_exact(zq, oracle, head, kv, dim):
+    """Prompts through attention_prefill.cu at every head dimension that it has: row groups and tiles with remainders,
+    windows that start inside a tile, a second chunk, one more token; many heads for 16 rows per CTA. The CPU path has one
+    key head; with two, the prompt token by token is the reference."""
+    cfg = dict(GEMMA_TINY, head=head, head_kv=kv, head_dim=dim, ctx=700, sliding_window=90, layer=2, global_every=2)
+    host = hostmodel.Gemma3Host.synthetic(cfg, qtype=ggml.Q8_0, seed=42, std=0.08).randomize_small_params()
+    eng = zq.Gemma3(host)
+    for n in (2, 65, 200, 600):
+        prompt = np.random.default_rng(n).integers(0, GEMMA_TINY["vocab"], size=n)
+        if kv == 1:
+            ref = oracle.Gemma3(host, 8)
+            want = ref.prefill(prompt), ref.decode_next(5)
+        else:
+            eng.prefill(prompt[:1])
+            steps = [eng.decode_next(int(t)).cpu().numpy() for t in [*prompt[1:], 5]]
+            want = steps[-2:]
+        assert np.array_equal(eng.prefill(prompt).cpu().numpy(), want[0]), n
+        assert np.array_equal(eng.decode_next(5).cpu().numpy(), want[1]), n
+
+
 def test_gemma3_1b_full_size_greedy_64(zq, oracle):
     """Gemma-3-1B shape, Q8_0, seed 42, 16-token prompt, first 64 greedy tokens identical."""
     host = hostmodel.Gemma3Host.synthetic(hostmodel.GEMMA3_1B, qtype=ggml.Q8_0, seed=42, std=0.02, device="cuda")

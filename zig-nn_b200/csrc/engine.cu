@@ -52,6 +52,11 @@ __global__ void greedy_feed_kernel(uint32_t* state, const int32_t* arg, uint32_t
     state[2] += 1;
 }
 
+// Tokens of a prefill chunk: kPrefillChunkRows where attention runs row by row and keeps every row's scores in memory. The
+// products cover the GPU better the more rows they have (GPT-2, 900 tokens, 16-token attention in both: 13.0 ms in chunks of
+// 128, 6.7 in chunks of 512).
+constexpr uint32_t kPrefillChunk = 512, kPrefillChunkRows = 128;
+
 }  // namespace
 }  // namespace zq
 
@@ -76,6 +81,7 @@ struct zq_gpt2 {
     uint32_t* d_state = nullptr;
     int32_t* d_tokens = nullptr;   // token ids of a prefill chunk
     uint32_t max_rows = 1;         // rows the activation buffers hold (prefill chunk size)
+    bool prefill_attention = false;  // chunks take attention_prefill.cu; otherwise the decode step's kernels, row by row
     int32_t* d_arg = nullptr;
     uint32_t* d_record = nullptr;  // ctx entries for greedy decoding
     uint32_t seq_len = 0;
@@ -126,9 +132,9 @@ static int gpt2_linear(zq_gpt2* m, const Linear& L, const float* x, float* y, co
 
 // Forward pass over T consecutive tokens starting at position m->d_state[1] (gpt2.zig:423-509). T == 1 is a
 // decode step (token in m->d_state[0]); T > 1 a batched prefill chunk (tokens in m->d_tokens). Eight
-// launches per layer when decoding: ln1 | qkv | cache write + scores | softmax.V | proj + residual | ln2 |
+// launches per layer when decoding (pos0 is the host's copy of the position, for a chunk): ln1 | qkv | cache write + scores | softmax.V | proj + residual | ln2 |
 // fc + gelu | mproj + residual. Logits are those of the last row.
-static int gpt2_forward(zq_gpt2* m, uint32_t T, int variant, cudaStream_t st) {
+static int gpt2_forward(zq_gpt2* m, uint32_t T, int variant, cudaStream_t st, uint32_t pos0 = 0) {
     const zq_gpt2_config& C = m->c;
     const uint32_t E = C.embed, hd = E / C.head;
     if (T == 0 || T > m->max_rows) return ZQ_ERR_BAD_ARG;
@@ -143,7 +149,11 @@ static int gpt2_forward(zq_gpt2* m, uint32_t T, int variant, cudaStream_t st) {
             if ((rc = launch_write_kv_step(k_new, v_new, m->k[l], m->v[l], m->d_state, E, T, 3 * E, st))) return rc;
             k_new = v_new = nullptr;
         }
-        if ((rc = launch_attention_step(m->qkv, m->k[l], m->v[l], k_new, v_new, m->att, nullptr, nullptr, nullptr,
+        if (T > 1 && m->prefill_attention) {
+            if ((rc = launch_attention_prefill(m->qkv, m->k[l], m->v[l], m->att, nullptr, nullptr, nullptr, C.head, C.head,
+                                               hd, m->d_state, 0, pos0 + T, ZQ_ATTN_GPT2_SOFTMAX, T, 3 * E, st)))
+                return rc;
+        } else if ((rc = launch_attention_step(m->qkv, m->k[l], m->v[l], k_new, v_new, m->att, nullptr, nullptr, nullptr,
                                         m->scores, C.head, C.head, hd, m->d_state, 0, C.ctx, ZQ_ATTN_GPT2_SOFTMAX, T,
                                         3 * E, nullptr, 0, nullptr, nullptr, nullptr, 0.0f, st)))
             return rc;
@@ -266,8 +276,10 @@ int zq_gpt2_create(const zq_gpt2_config* cfg, const zq_gpt2_weights* w, zq_strea
         cudaMemsetAsync(m->k[l], 0, (size_t)cfg->ctx * E * sizeof(float), st);
         cudaMemsetAsync(m->v[l], 0, (size_t)cfg->ctx * E * sizeof(float), st);
     }
-    // activation buffers hold a prefill chunk of up to 512 tokens (a decode step uses row 0)
-    m->max_rows = cfg->ctx < 512 ? cfg->ctx : 512;
+    // activation buffers hold a prefill chunk (a decode step uses row 0). Row-by-row attention keeps every row's scores
+    // in memory, so its chunks are shorter.
+    m->prefill_attention = attention_prefill_takes(E / cfg->head, cfg->ctx);
+    m->max_rows = std::min(cfg->ctx, m->prefill_attention ? kPrefillChunk : kPrefillChunkRows);
     const size_t R = m->max_rows;
     TRY(m->arena.alloc_n(&m->x, R * E));
     TRY(m->arena.alloc_n(&m->ln, R * (E > F ? E : F)));
@@ -275,7 +287,7 @@ int zq_gpt2_create(const zq_gpt2_config* cfg, const zq_gpt2_weights* w, zq_strea
     TRY(m->arena.alloc_n(&m->att, R * E));
     TRY(m->arena.alloc_n(&m->hid, R * F));
     TRY(m->arena.alloc_n(&m->logits, cfg->vocab));
-    TRY(m->arena.alloc_n(&m->scores, R * cfg->head * cfg->ctx));
+    TRY(m->arena.alloc_n(&m->scores, (m->prefill_attention ? 1 : R) * cfg->head * cfg->ctx));
     size_t split = 0;
     for (const zq_gpt2::Block& b : m->blocks)
         for (const Linear* L : {&b.qkv, &b.proj, &b.fc, &b.mproj})
@@ -344,7 +356,7 @@ int zq_gpt2_prefill(zq_gpt2* m, const uint32_t* h_tokens, uint32_t n, zq_stream 
             rc = gpt2_run(m, last ? STEP_LOGITS : STEP_CACHE_ONLY, st);
         } else {
             ZQ_CUDA(cudaMemcpyAsync(m->d_tokens, h_tokens + t0, T * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-            rc = gpt2_forward(m, T, last ? STEP_LOGITS : STEP_CACHE_ONLY, st);
+            rc = gpt2_forward(m, T, last ? STEP_LOGITS : STEP_CACHE_ONLY, st, t0);
             ZQ_CUDA(cudaStreamSynchronize(st));  // h_tokens is the caller's memory
         }
         if (rc != ZQ_OK) return rc;
@@ -421,6 +433,8 @@ struct zq_gemma3 {
     uint32_t* d_state = nullptr;
     int32_t* d_tokens = nullptr;  // token ids of a prefill chunk / of a batched decode step
     uint32_t max_rows = 1;        // rows the activation buffers hold (prefill chunk size, >= n_seq)
+    uint32_t chunk = 1;           // tokens of a prefill chunk
+    bool prefill_attention = false;  // as in zq_gpt2
     int32_t* d_arg = nullptr;
     uint32_t* d_record = nullptr;
     uint32_t seq_len = 0;
@@ -470,8 +484,9 @@ static int gemma_linear(zq_gemma3* m, const zq_weight* w, float* y, uint32_t y_s
 // Logits (and the argmax of a greedy step) are those of the last row.
 // batch == false: the T rows are consecutive tokens of sequence `seq` (its cache slot). batch == true: row r
 // is the next token of sequence r, at position m->d_pos[r], and every row's logits go to m->logits_batch.
+// pos0: the host's copy of a chunk's first position.
 static int gemma3_forward(zq_gemma3* m, uint32_t T, int variant, cudaStream_t st, uint32_t seq = 0,
-                          bool batch = false) {
+                          bool batch = false, uint32_t pos0 = 0) {
     const zq_gemma3_config& C = m->c;
     const uint32_t E = C.embed, D = C.head_dim, QD = C.head * D, KD = C.head_kv * D, F = C.ffn;
     const uint32_t QKV = QD + 2 * KD;
@@ -508,7 +523,11 @@ static int gemma3_forward(zq_gemma3* m, uint32_t T, int variant, cudaStream_t st
                                              cache_stride, st)))
                 return rc;
         }
-        if ((rc = launch_attention_step(m->qkv, m->k[l] + slot, m->v[l] + slot, fused_qk ? m->qkv + QD : nullptr,
+        if (!fused_qk && m->prefill_attention) {
+            if ((rc = launch_attention_prefill(m->qkv, m->k[l] + slot, m->v[l] + slot, nullptr, m->xq, m->xscale, m->xsum,
+                                               C.head, C.head_kv, D, m->d_state, window, pos0 + T, 0, T, QKV, st)))
+                return rc;
+        } else if ((rc = launch_attention_step(m->qkv, m->k[l] + slot, m->v[l] + slot, fused_qk ? m->qkv + QD : nullptr,
                                         fused_qk ? m->qkv + QD + KD : nullptr, nullptr, m->xq, m->xscale, m->xsum,
                                         m->scores, C.head, C.head_kv, D, m->d_state, window, max_len, 0, T, QKV, row_pos,
                                         cache_stride, fused_qk ? b.q_norm_w : nullptr, b.k_norm_w, m->freqs, C.rms_eps,
@@ -729,9 +748,10 @@ int zq_gemma3_create_batch(const zq_gemma3_config* cfg, const zq_gemma3_weights*
             return cuda_fail(e);
         }
     }
-    // activation buffers hold a prefill chunk of up to 128 tokens (a decode step uses row 0)
-    m->max_rows = C.ctx < 128 ? C.ctx : 128;
-    if (m->max_rows < n_seq) m->max_rows = n_seq;
+    // activation buffers hold a prefill chunk (a decode step uses row 0)
+    m->prefill_attention = attention_prefill_takes(D, C.ctx);
+    m->chunk = std::min(C.ctx, m->prefill_attention ? kPrefillChunk : kPrefillChunkRows);
+    m->max_rows = std::max(m->chunk, n_seq);
     const size_t R = m->max_rows;
     TRY(m->arena.alloc_n(&m->d_pos, n_seq));
     if (n_seq > 1) TRY(m->arena.alloc_n(&m->logits_batch, (size_t)n_seq * C.vocab));
@@ -741,7 +761,7 @@ int zq_gemma3_create_batch(const zq_gemma3_config* cfg, const zq_gemma3_weights*
     TRY(m->arena.alloc_n(&m->gu, R * 2 * (size_t)F));
     TRY(m->arena.alloc_n(&m->ffn, R * E));
     TRY(m->arena.alloc_n(&m->logits, C.vocab));
-    TRY(m->arena.alloc_n(&m->scores, R * C.head * C.ctx));
+    TRY(m->arena.alloc_n(&m->scores, (m->prefill_attention ? n_seq : R) * C.head * C.ctx));
     TRY(m->arena.alloc_n(&m->xq, R * max_dim));
     TRY(m->arena.alloc_n(&m->xscale, R * (max_dim / 32)));
     TRY(m->arena.alloc_n(&m->xsum, R * (max_dim / 32)));
@@ -821,8 +841,8 @@ int zq_gemma3_prefill_seq(zq_gemma3* m, uint32_t seq, const uint32_t* h_tokens, 
     cudaStream_t st = as_stream(stream);
     m->seq_lens[seq] = 0;
     if (seq == 0) m->seq_len = 0;
-    // chunks of up to max_rows tokens, each a batched forward pass (every row = the arithmetic of a decode step)
-    const uint32_t chunk = m->c.ctx < 128 ? m->c.ctx : 128;
+    // chunks, each a batched forward pass (every row = the arithmetic of a decode step)
+    const uint32_t chunk = m->chunk;
     for (uint32_t t0 = 0; t0 < n; t0 += chunk) {
         const uint32_t T = n - t0 < chunk ? n - t0 : chunk;
         const bool last = t0 + T == n;
@@ -835,7 +855,7 @@ int zq_gemma3_prefill_seq(zq_gemma3* m, uint32_t seq, const uint32_t* h_tokens, 
             rc = gemma3_forward(m, 1, last ? STEP_LOGITS : STEP_CACHE_ONLY, st, seq);
         } else {
             ZQ_CUDA(cudaMemcpyAsync(m->d_tokens, h_tokens + t0, T * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-            rc = gemma3_forward(m, T, last ? STEP_LOGITS : STEP_CACHE_ONLY, st, seq);
+            rc = gemma3_forward(m, T, last ? STEP_LOGITS : STEP_CACHE_ONLY, st, seq, false, t0);
             ZQ_CUDA(cudaStreamSynchronize(st));  // h_tokens is the caller's memory
         }
         if (rc != ZQ_OK) return rc;

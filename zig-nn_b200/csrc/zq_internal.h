@@ -209,6 +209,14 @@ int launch_attention_step(const float* q, float* kc, float* vc, const float* k_n
                           uint32_t max_len, int flags, uint32_t rows, uint32_t q_stride, const uint32_t* row_pos,
                           size_t cache_stride, const float* q_norm_w, const float* k_norm_w, const float* freqs,
                           float norm_eps, cudaStream_t st);
+// The same for a prompt's tokens, several rows at once, whose keys and values are in the caches (attention_prefill.cu);
+// `end`: an upper bound of the last token's position + 1. q (normalised and rotated) and the caches start on 16-byte
+// boundaries. attention_prefill_takes: whether head_dim has such a kernel and the scores of rows over `ctx` positions fit
+// its shared memory (ZQ_ERR_LIMIT otherwise).
+bool attention_prefill_takes(uint32_t head_dim, uint32_t ctx);
+int launch_attention_prefill(const float* q, const float* kc, const float* vc, float* out, int8_t* oq, float* oscale,
+                             int32_t* osum, uint32_t n_head, uint32_t n_kv_head, uint32_t head_dim, const uint32_t* state,
+                             uint32_t window, uint32_t end, int flags, uint32_t rows, uint32_t q_stride, cudaStream_t st);
 // f32 matvec (GPT-2 vocabulary head) with an optional LayerNorm of x in the prologue (gemv.cu).
 int launch_matvec_ln_f32(const float* w, const float* x, float* y, uint32_t out_dim, uint32_t in_dim,
                          const float* ln_gamma, const float* ln_beta, float ln_eps, cudaStream_t st);
