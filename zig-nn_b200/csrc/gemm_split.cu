@@ -9,9 +9,9 @@
 // scaled before it is added: with the scale folded into 19-bit weights the sum over all of K would stay inside the tensor
 // core, whose accumulation is coarser than the f32 sum over blocks. The activations are split once per call into an image
 // in fragment order (split_rows_kernel), so the loop loads them with 128-bit accesses free of bank conflicts; a warp owns
-// MT x 16 weight rows and unpacks a weight word once for all NT x 8 activation rows.
-// Measured (B200, graph-timed, split_rows included, passes of the decode kernel before): 3072 <- 768 at 45 rows 30.8 -> 14.7
-// us, 1152 <- 6912 at 45 rows 135 -> 39 us; GPT-2's 900-token prompt, chunks of 128 -> 512 tokens, 55.5 -> 13 ms.
+// 16 weight rows and unpacks a weight word once for all NT x 8 activation rows.
+// Measured (B200, graph-timed, split_rows included; passes of the decode kernel, this product tile by tile in its MMAs, as it
+// is): 3072 <- 768 at 48 rows 31, 15.2, 12.9 us and at 512 rows -, 79, 36.5; 1152 <- 6912 at 48 rows 137, 40, 31 us.
 #include "zq_internal.h"
 
 namespace zq {
@@ -130,7 +130,7 @@ __device__ __forceinline__ uint2 lds64(uint32_t addr) {
     return v;
 }
 __device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
@@ -169,9 +169,10 @@ __device__ __forceinline__ void unpack_q4(uint32_t q, uint32_t& lo02, uint32_t& 
     hi13 = hfma2((s & 0x00F000F0u) | 0x64006400u, k16th, kAdd);
 }
 
-// A stage of the ring holds KS quads (4 blocks each): per quad the activations of NT tiles (4 KB each, q4_1: and their
-// sums), and per warp the packed words and scales of its own quad and MT x 16 rows, each lane's pieces in its own slots.
-template <int TYPE, int WR, int KS, int MT, int NT>
+// A CTA has WR x KS warps: WR x 16 weight rows, NT x 8 activation rows, and KS parts of K. A stage of the ring holds KS quads
+// (4 blocks each): per quad the activations of NT tiles (4 KB each, q4_1: and their sums), and per warp the packed words and
+// scales of its own quad and 16 rows, each lane's pieces in its own slots.
+template <int TYPE, int WR, int KS, int NT>
 struct SplitStage {
     static constexpr uint32_t kSums = TYPE == ZQ_TYPE_Q4_1 ? 128 : 0;
     static constexpr uint32_t kTile = 4096 + kSums;
@@ -179,51 +180,46 @@ struct SplitStage {
     static constexpr uint32_t kWq = TYPE == ZQ_TYPE_Q8_0 ? 2048 : 1024;
     static constexpr uint32_t kWsHalf = TYPE == ZQ_TYPE_Q4_1 ? 512 : 256;
     static constexpr uint32_t kWTile = kWq + 2 * kWsHalf;
-    static constexpr uint32_t kBytes = kAct + WR * KS * MT * kWTile;
+    static constexpr uint32_t kBytes = kAct + WR * KS * kWTile;
 };
 
-template <int TYPE, int WR, int KS, int MT, int NT, int D>
+template <int TYPE, int WR, int KS, int NT, int D>
 __global__ void __launch_bounds__(WR * KS * 32)
 gemm_split_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc, SplitImage im, float* __restrict__ y,
                   uint32_t N, uint32_t M, uint32_t nbp, uint32_t scp, SplitEpilogue ep) {
     constexpr bool Q8 = TYPE == ZQ_TYPE_Q8_0, Q41 = TYPE == ZQ_TYPE_Q4_1;
     constexpr uint32_t QB = Q8 ? 32 : 16, QUAD = 4 * QB, SB = Q41 ? 4 : 2, THREADS = WR * KS * 32;
-    using S = SplitStage<TYPE, WR, KS, MT, NT>;
+    using S = SplitStage<TYPE, WR, KS, NT>;
     extern __shared__ __align__(128) unsigned char smem[];
     const uint32_t smem32 = (uint32_t)__cvta_generic_to_shared(smem);
     const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
     const uint32_t wr = warp % WR, ks = warp / WR;
     const uint32_t nq = nbp / 4, steps = (nq + KS - 1) / KS;
-    const uint32_t n0 = blockIdx.x * (WR * MT * 16) + wr * MT * 16, tile0 = blockIdx.y * NT, tiles = (M + 7) / 8;
-
+    const uint32_t n0 = blockIdx.x * (WR * 16) + wr * 16, tile0 = blockIdx.y * NT, tiles = (M + 7) / 8;
     const uint32_t nt = min((uint32_t)NT, tiles - tile0);  // tiles that exist
-    const uint8_t* pw[MT][2];
-    const uint8_t* ps[MT][2];
+
+    const uint8_t* pw[2];
+    const uint8_t* ps[2];
 #pragma unroll
-    for (int i = 0; i < MT; ++i)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t row = min(n0 + i * 16 + h * 8 + g, N - 1);
-            pw[i][h] = qs + (size_t)row * nbp * QB + 16 * t;
-            ps[i][h] = sc + (size_t)row * scp * SB;
-        }
-    const uint32_t wslot = smem32 + S::kAct + warp * MT * S::kWTile;
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t row = min(n0 + h * 8 + g, N - 1);
+        pw[h] = qs + (size_t)row * nbp * QB + 16 * t;
+        ps[h] = sc + (size_t)row * scp * SB;
+    }
+    const uint32_t wslot = smem32 + S::kAct + warp * S::kWTile;
 
     auto issue_weights = [&](uint32_t stage, uint32_t step) {
         const uint32_t q = step * KS + ks;
         if (q >= nq) return;
+        const uint32_t wb = wslot + stage * S::kBytes;
 #pragma unroll
-        for (int i = 0; i < MT; ++i) {
-            const uint32_t wb = wslot + stage * S::kBytes + i * S::kWTile;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                cp_async16(wb + h * 512 + lane * 16, pw[i][h] + (size_t)q * QUAD);
-                if (Q8) cp_async16(wb + 1024 + h * 512 + lane * 16, pw[i][h] + (size_t)q * QUAD + 64);
-                if (Q41)
-                    cp_async16(wb + S::kWq + h * S::kWsHalf + lane * 16, ps[i][h] + (size_t)q * 16);
-                else
-                    cp_async8(wb + S::kWq + h * S::kWsHalf + lane * 8, ps[i][h] + (size_t)q * 8);
-            }
+        for (int h = 0; h < 2; ++h) {
+            cp_async16(wb + h * 512 + lane * 16, pw[h] + (size_t)q * QUAD);
+            if (Q8) cp_async16(wb + 1024 + h * 512 + lane * 16, pw[h] + (size_t)q * QUAD + 64);
+            if (Q41)
+                cp_async16(wb + S::kWq + h * S::kWsHalf + lane * 16, ps[h] + (size_t)q * 16);
+            else
+                cp_async8(wb + S::kWq + h * S::kWsHalf + lane * 8, ps[h] + (size_t)q * 8);
         }
     };
     auto issue_acts = [&](uint32_t stage, uint32_t step) {
@@ -249,23 +245,19 @@ gemm_split_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc
     // Sums in two levels, kFlush quads below and those above: the f32 chain over K stays as short as that of the
     // decode kernel, which cuts K into up to eight parts (in one level the error at 216 blocks was 1.6e-7 against 1.2e-7).
     constexpr uint32_t kFlush = 4;
-    float acc[MT][NT][4], sum[MT][NT][4];
+    float acc[NT][4], sum[NT][4];
 #pragma unroll
-    for (int i = 0; i < MT; ++i)
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[j][c] = sum[j][c] = 0.0f;
+    auto flush = [&] {
 #pragma unroll
         for (int j = 0; j < NT; ++j)
 #pragma unroll
-            for (int c = 0; c < 4; ++c) acc[i][j][c] = sum[i][j][c] = 0.0f;
-    auto flush = [&] {
-#pragma unroll
-        for (int i = 0; i < MT; ++i)
-#pragma unroll
-            for (int j = 0; j < NT; ++j)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) {
-                    sum[i][j][c] += acc[i][j][c];
-                    acc[i][j][c] = 0.0f;
-                }
+            for (int c = 0; c < 4; ++c) {
+                sum[j][c] += acc[j][c];
+                acc[j][c] = 0.0f;
+            }
     };
 
     pdl_launch_dependents();
@@ -291,74 +283,70 @@ gemm_split_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc
         p_stage = p_stage + 1 == (uint32_t)D ? 0 : p_stage + 1;
 
         if (s * KS + ks < nq) {
-            const uint32_t act = smem32 + stage * S::kBytes + ks * NT * S::kTile;
-            uint4 wlo[MT][2], whi[MT][2], ws[MT][2];
+            const uint32_t act = smem32 + stage * S::kBytes + ks * NT * S::kTile, wb = wslot + stage * S::kBytes;
+            uint4 wlo[2], whi[2], ws[2];
 #pragma unroll
-            for (int i = 0; i < MT; ++i) {
-                const uint32_t wb = wslot + stage * S::kBytes + i * S::kWTile;
-#pragma unroll
-                for (int h = 0; h < 2; ++h) {
-                    wlo[i][h] = lds128(wb + h * 512 + lane * 16);
-                    if (Q8) whi[i][h] = lds128(wb + 1024 + h * 512 + lane * 16);
-                    if (Q41) {
-                        ws[i][h] = lds128(wb + S::kWq + h * S::kWsHalf + lane * 16);
-                    } else {
-                        const uint2 v = lds64(wb + S::kWq + h * S::kWsHalf + lane * 8);
-                        ws[i][h].x = v.x;
-                        ws[i][h].y = v.y;
-                    }
+            for (int h = 0; h < 2; ++h) {
+                wlo[h] = lds128(wb + h * 512 + lane * 16);
+                if (Q8) whi[h] = lds128(wb + 1024 + h * 512 + lane * 16);
+                if (Q41) {
+                    ws[h] = lds128(wb + S::kWq + h * S::kWsHalf + lane * 16);
+                } else {
+                    const uint2 v = lds64(wb + S::kWq + h * S::kWsHalf + lane * 8);
+                    ws[h].x = v.x;
+                    ws[h].y = v.y;
                 }
             }
 #pragma unroll 1  // unrolled, the compiler unpacks all four blocks ahead and spills; the words rotate instead
             for (int b = 0; b < 4; ++b) {
-                uint32_t aL[MT][4], aH[MT][4];
-                float d[MT][2], mn[MT][2];
+                uint32_t aL[4], aH[4];
+                float d[2], mn[2];
 #pragma unroll
-                for (int i = 0; i < MT; ++i) {
-#pragma unroll
-                    for (int h = 0; h < 2; ++h) {
-                        if (Q8) {
-                            unpack_q8(wlo[i][h].x, aL[i][h], aL[i][2 + h]);
-                            unpack_q8(whi[i][h].x, aH[i][h], aH[i][2 + h]);
-                        } else {
-                            unpack_q4<!Q41>(wlo[i][h].x, aL[i][h], aL[i][2 + h], aH[i][h], aH[i][2 + h]);
-                        }
-                        const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&ws[i][h].x));
-                        d[i][h] = f.x;
-                        mn[i][h] = f.y;  // q4_1; otherwise the next block's scale
-                        rotate(wlo[i][h]);
-                        if (Q8) rotate(whi[i][h]);
-                        if (Q41) {
-                            rotate(ws[i][h]);
-                        } else {
-                            ws[i][h].x = b & 1 ? ws[i][h].y : ws[i][h].x >> 16;
-                        }
+                for (int h = 0; h < 2; ++h) {
+                    if (Q8) {
+                        unpack_q8(wlo[h].x, aL[h], aL[2 + h]);
+                        unpack_q8(whi[h].x, aH[h], aH[2 + h]);
+                        rotate(whi[h]);
+                    } else {
+                        unpack_q4<!Q41>(wlo[h].x, aL[h], aL[2 + h], aH[h], aH[2 + h]);
+                    }
+                    rotate(wlo[h]);
+                    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&ws[h].x));
+                    d[h] = f.x;
+                    mn[h] = f.y;  // q4_1; otherwise the next block's scale
+                    if (Q41) {
+                        rotate(ws[h]);
+                    } else {
+                        ws[h].x = b & 1 ? ws[h].y : ws[h].x >> 16;
                     }
                 }
+                // One of the four MMAs after the other over all tiles: a tile's MMAs depend on one another (28 cycles each),
+                // and taken tile by tile a warp waits out the latency of each.
+                uint4 hi[NT], lo[NT];
+                float p[NT][4];
 #pragma unroll
-                for (int j = 0; j < NT; ++j) {
-                    if (j >= nt) break;
-                    const uint32_t at = act + j * S::kTile;
-                    const uint4 hi = lds128(at + b * 1024 + lane * 16), lo = lds128(at + b * 1024 + 512 + lane * 16);
-                    float2 xs = make_float2(0.0f, 0.0f);
-                    if (Q41) {
-                        const uint2 v = lds64(at + 4096 + b * 32 + t * 8);
-                        xs = make_float2(__uint_as_float(v.x), __uint_as_float(v.y));
+                for (int j = 0; j < NT; ++j) {  // tiles past the last: what the stage happens to hold, stored nowhere
+                    const uint32_t at = act + j * S::kTile + b * 1024 + lane * 16;
+                    lo[j] = lds128(at + 512);
+                    hi[j] = lds128(at);
+                    p[j][0] = p[j][1] = p[j][2] = p[j][3] = 0.0f;
+                }
+#pragma unroll
+                for (int ph = 0; ph < 4; ++ph)
+#pragma unroll
+                    for (int j = 0; j < NT; ++j) {
+                        const uint4& v = ph < 2 ? lo[j] : hi[j];
+                        mma_f16(p[j], ph & 1 ? aH : aL, ph & 1 ? v.z : v.x, ph & 1 ? v.w : v.y);
                     }
 #pragma unroll
-                    for (int i = 0; i < MT; ++i) {
-                        float p[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-                        mma_f16(p, aL[i], lo.x, lo.y);
-                        mma_f16(p, aH[i], lo.z, lo.w);
-                        mma_f16(p, aL[i], hi.x, hi.y);
-                        mma_f16(p, aH[i], hi.z, hi.w);
+                for (int j = 0; j < NT; ++j) {
 #pragma unroll
-                        for (int c = 0; c < 4; ++c) acc[i][j][c] = fmaf(p[c], d[i][c >> 1], acc[i][j][c]);
-                        if (Q41) {
+                    for (int c = 0; c < 4; ++c) acc[j][c] = fmaf(p[j][c], d[c >> 1], acc[j][c]);
+                    if (Q41) {
+                        const uint2 v = lds64(act + j * S::kTile + 4096 + b * 32 + t * 8);
+                        const float xs[2] = {__uint_as_float(v.x), __uint_as_float(v.y)};
 #pragma unroll
-                            for (int c = 0; c < 4; ++c)
-                                acc[i][j][c] = fmaf(mn[i][c >> 1], c & 1 ? xs.y : xs.x, acc[i][j][c]);
-                        }
+                        for (int c = 0; c < 4; ++c) acc[j][c] = fmaf(mn[c >> 1], xs[c & 1], acc[j][c]);
                     }
                 }
             }
@@ -372,64 +360,57 @@ gemm_split_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc
     flush();
     // sums of the K parts, in their order, through shared memory
     if (KS > 1) {
-        float* red = reinterpret_cast<float*>(smem);  // [ks - 1][wr][MT * NT * 4][32]
+        float* red = reinterpret_cast<float*>(smem);  // [ks - 1][wr][NT * 4][32]
         if (ks > 0) {
-            float* to = red + (size_t)((ks - 1) * WR + wr) * (MT * NT * 4 * 32) + lane;
+            float* to = red + (size_t)((ks - 1) * WR + wr) * (NT * 4 * 32) + lane;
 #pragma unroll
-            for (int i = 0; i < MT; ++i)
+            for (int j = 0; j < NT; ++j)
 #pragma unroll
-                for (int j = 0; j < NT; ++j)
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) to[((i * NT + j) * 4 + c) * 32] = sum[i][j][c];
+                for (int c = 0; c < 4; ++c) to[(j * 4 + c) * 32] = sum[j][c];
         }
         __syncthreads();
         if (ks > 0) return;
 #pragma unroll
         for (int k = 1; k < KS; ++k) {
-            const float* from = red + (size_t)((k - 1) * WR + wr) * (MT * NT * 4 * 32) + lane;
+            const float* from = red + (size_t)((k - 1) * WR + wr) * (NT * 4 * 32) + lane;
 #pragma unroll
-            for (int i = 0; i < MT; ++i)
+            for (int j = 0; j < NT; ++j)
 #pragma unroll
-                for (int j = 0; j < NT; ++j)
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) sum[i][j][c] += from[((i * NT + j) * 4 + c) * 32];
+                for (int c = 0; c < 4; ++c) sum[j][c] += from[(j * 4 + c) * 32];
         }
     }
 #pragma unroll
-    for (int i = 0; i < MT; ++i) {
+    for (int h = 0; h < 2; ++h) {
+        const uint32_t n = n0 + h * 8 + g;
+        if (n >= N) continue;
+        const float bias = ep.bias ? ep.bias[n] : 0.0f;
 #pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t n = n0 + i * 16 + h * 8 + g;
-            if (n >= N) continue;
-            const float bias = ep.bias ? ep.bias[n] : 0.0f;
+        for (int j = 0; j < NT; ++j) {
 #pragma unroll
-            for (int j = 0; j < NT; ++j) {
-#pragma unroll
-                for (int c = 0; c < 2; ++c) {
-                    const uint32_t m = (tile0 + j) * 8 + 2 * t + c;
-                    if (m >= M) continue;
-                    const size_t o = (size_t)m * N + n;
-                    float v = sum[i][j][h * 2 + c] * im.post[m];
-                    if (ep.bias) v = __fadd_rn(v, bias);
-                    if (ep.gelu) v = gelu_tanh(v);
-                    if (ep.mul) v = __fmul_rn(v, ep.mul[o]);
-                    if (ep.residual) v = __fadd_rn(ep.residual[o], v);
-                    y[o] = v;
-                }
+            for (int c = 0; c < 2; ++c) {
+                const uint32_t m = (tile0 + j) * 8 + 2 * t + c;
+                if (m >= M) continue;
+                const size_t o = (size_t)m * N + n;
+                float v = sum[j][h * 2 + c] * im.post[m];
+                if (ep.bias) v = __fadd_rn(v, bias);
+                if (ep.gelu) v = gelu_tanh(v);
+                if (ep.mul) v = __fmul_rn(v, ep.mul[o]);
+                if (ep.residual) v = __fadd_rn(ep.residual[o], v);
+                y[o] = v;
             }
         }
     }
 }
 
-template <int TYPE, int WR, int KS, int MT, int NT, int D>
+template <int TYPE, int WR, int KS, int NT, int D>
 int launch_cfg(const zq_weight* w, const SplitImage& im, float* y, uint32_t M, const SplitEpilogue& ep, cudaStream_t st) {
-    const dim3 grid((w->out_dim + WR * MT * 16 - 1) / (WR * MT * 16), (M + NT * 8 - 1) / (NT * 8));
+    const dim3 grid((w->out_dim + WR * 16 - 1) / (WR * 16), (M + NT * 8 - 1) / (NT * 8));
     if (grid.y > 65535u) return ZQ_ERR_LIMIT;
-    constexpr size_t ring = (size_t)D * SplitStage<TYPE, WR, KS, MT, NT>::kBytes;
-    constexpr size_t red = (size_t)(KS - 1) * WR * MT * NT * 512;
+    constexpr size_t ring = (size_t)D * SplitStage<TYPE, WR, KS, NT>::kBytes;
+    constexpr size_t red = (size_t)(KS - 1) * WR * NT * 512;
     constexpr size_t smem = ring > red ? ring : red;
     static_assert(smem <= 227 * 1024, "a CTA's shared memory");
-    auto kern = gemm_split_kernel<TYPE, WR, KS, MT, NT, D>;
+    auto kern = gemm_split_kernel<TYPE, WR, KS, NT, D>;
     ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     ZQ_CUDA(launch_pdl(kern, grid, dim3(WR * KS * 32), smem, st, w->qs, static_cast<const uint8_t*>(w->sc), im, y,
                        w->out_dim, M, w->nbp, w->scp, ep));
@@ -442,9 +423,14 @@ int launch_type(const zq_weight* w, const SplitImage& im, float* y, uint32_t M, 
     auto ctas = [&](uint32_t rows, uint32_t cols) {
         return (uint64_t)((w->out_dim + rows - 1) / rows) * ((M + cols - 1) / cols);
     };
-    if (ctas(128, 64) >= sms) return launch_cfg<TYPE, 4, 1, 2, 8, 2>(w, im, y, M, ep, st);
-    if (ctas(64, 64) >= sms / 2) return launch_cfg<TYPE, 4, 2, 1, 8, 2>(w, im, y, M, ep, st);
-    return launch_cfg<TYPE, 2, 4, 1, 4, 2>(w, im, y, M, ep, st);
+    // The smallest tile whose CTAs run all at once, its K cut over the warps; past that the tile that reads the least
+    // per MMA (us with the split, in the order of the lines, the tile taken in brackets: 768 <- 3072 at 32 rows [13.3], 15.9,
+    // 20.6, 31.2; 2304 <- 768 at 17 rows 9.8, [7.2], 9.0, 11.2; 2304 <- 768 at 48 rows 14.1, 11.5, [9.6], 13.1;
+    // 3072 <- 768 at 48 rows 18.0, 12.3, 15.2, [12.9] and at 512 rows 160, 105, 78, [36.5]).
+    if (ctas(16, 16) <= sms) return launch_cfg<TYPE, 1, 8, 2, 2>(w, im, y, M, ep, st);
+    if (ctas(32, 16) <= sms) return launch_cfg<TYPE, 2, 4, 2, 3>(w, im, y, M, ep, st);
+    if (ctas(32, 32) <= sms) return launch_cfg<TYPE, 2, 4, 4, 2>(w, im, y, M, ep, st);
+    return launch_cfg<TYPE, 4, 2, 4, 2>(w, im, y, M, ep, st);
 }
 
 }  // namespace
