@@ -108,7 +108,7 @@ def test_matmul_small_batches_f32(zq, oracle, qtype, m):
 
 
 @pytest.mark.parametrize("qtype", TYPES)
-@pytest.mark.parametrize("m,n,k", [(17, 33, 32), (45, 520, 1184), (48, 5003, 96), (24, 96, 6912)])
+@pytest.mark.parametrize("m,n,k", [(17, 33, 32), (45, 520, 1184), (48, 5003, 96), (24, 96, 6912), (48, 2304, 768), (17, 2304, 288)])
 def test_split_product_keeps_f32_accuracy(zq, oracle, qtype, m, n, k):
     raw = make_weight(oracle, qtype, n, k)
     x = make_x(m, k)
@@ -189,6 +189,18 @@ def test_matmul_small_batches_q8_bit_exact(zq, oracle, m):
     got = zq.quant_matmul_no_grad(torch.from_numpy(x).cuda(), qw, zq.ACT_Q8).cpu().numpy()
     want = oracle.linear(ggml.Q4_1, raw, x, n, k, act_mode=1, n_threads=4)
     assert np.array_equal(got, want)
+
+
+@pytest.mark.parametrize("qtype", TYPES)
+@pytest.mark.parametrize("m,n,k", [(2, 7, 32), (8, 1601, 1184), (9, 33, 16384), (45, 521, 6912)])
+def test_matmul_q8_with_k_over_the_warps_bit_exact(zq, oracle, qtype, m, n, k):
+    """The four forms of the product that leaves its terms in shared memory: one and two weight tiles per CTA, up to 8 and
+    up to 16 rows; one block, a part of a quad, several rounds over K."""
+    raw = make_weight(oracle, qtype, n, k)
+    x = make_x(m, k)
+    x[1] *= 100.0
+    got = zq.quant_matmul_no_grad(torch.from_numpy(x).cuda(), zq.QuantWeight(raw, qtype, n, k), zq.ACT_Q8).cpu().numpy()
+    assert np.array_equal(got, oracle.linear(qtype, raw, x, n, k, act_mode=1, n_threads=8))
 
 
 @pytest.mark.parametrize("qtype", TYPES)

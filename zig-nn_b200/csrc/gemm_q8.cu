@@ -277,6 +277,184 @@ gemm_q8_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc, c
     }
 }
 
+// ---- the same for products that leave the GPU idle: K split over the warps of a CTA -------------------
+// The terms of an output have to be added in block order, but they need not be computed in that order. A CTA owns 16
+// activation rows x NTL * 8 weight rows; its eight warps take the quads of K in turn, compute the block terms (activations
+// as the A operand of the MMA, weights as B) and leave them in shared memory, and one thread per output then adds them in
+// order. Nothing waits for anything until all terms of a round are there, so a launch costs the latency of a few loads and
+// one chain of nb adds, where the kernel above walks over all of K with one quad per step. What bounds it: that chain (4
+// cycles a block) and the terms' way through shared memory; the products that fill the GPU stay with the kernel above,
+// whose sums never leave their registers.
+constexpr int kTermWarps = 8;
+
+template <int TYPE>
+struct TermQuad {         // what one lane needs of one quad of the activations
+    uint32_t a[4][4];     // words t and 4 + t of rows g and g + 8
+    float s[2][4];        // their scales
+    int32_t qs[2][4];     // and sums (4-bit types)
+};
+
+template <int TYPE, int NTL, bool WIDE>
+__global__ void __launch_bounds__(kTermWarps * 32)
+gemm_q8_terms_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc, const int8_t* __restrict__ xq,
+                     const float* __restrict__ xscale, const int32_t* __restrict__ xqsum, float* __restrict__ y,
+                     uint32_t N, uint32_t K, uint32_t M, uint32_t nb, uint32_t scp, uint32_t round_blocks, QgEpilogue ep) {
+    constexpr bool Q8 = TYPE == ZQ_TYPE_Q8_0, Q41 = TYPE == ZQ_TYPE_Q4_1;
+    constexpr uint32_t QB = Q8 ? 32 : 16, SB = Q41 ? 4 : 2;
+    constexpr uint32_t H = WIDE ? 2 : 1;                // WIDE: more than 8 activation rows
+    constexpr uint32_t OUTS = 64 * H * NTL;             // outputs of the CTA
+    extern __shared__ __align__(16) float terms[];      // [blocks of a round][NTL][row][8 weight rows]
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    const uint32_t nbp = (nb + 3u) & ~3u, n0 = blockIdx.x * (8 * NTL), m0 = blockIdx.y * 16;
+
+    const uint8_t* pw[NTL];
+    const uint8_t* ps[NTL][2];
+#pragma unroll
+    for (int i = 0; i < NTL; ++i) {
+        pw[i] = qs + (size_t)min(n0 + i * 8 + g, N - 1) * nbp * QB + 16 * t;
+        ps[i][0] = sc + (size_t)min(n0 + i * 8 + 2 * t, N - 1) * scp * SB;
+        ps[i][1] = sc + (size_t)min(n0 + i * 8 + 2 * t + 1, N - 1) * scp * SB;
+    }
+    const uint32_t row_a = min(m0 + g, M - 1), row_b = min(m0 + g + 8, M - 1);
+    pdl_launch_dependents();
+    // the weight rows on their way into L2 while the kernel before this one still runs
+    if (tid < 8 * NTL && n0 + tid < N) {
+        const uint8_t* row = qs + (size_t)(n0 + tid) * nbp * QB;
+        for (uint32_t o = 0; o < nbp * QB; o += 16384) prefetch_l2_bulk(row + o, min(nbp * QB - o, 16384u));
+    }
+    pdl_wait();
+
+    TermQuad<TYPE> x;
+    uint4 w[NTL][2];
+    uint4 ws[NTL][2];
+    auto load = [&](uint32_t q) {
+#pragma unroll
+        for (int i = 0; i < NTL; ++i) {
+            w[i][0] = __ldg(reinterpret_cast<const uint4*>(pw[i] + (size_t)q * 4 * QB));
+            if (Q8) w[i][1] = __ldg(reinterpret_cast<const uint4*>(pw[i] + (size_t)q * 4 * QB + 64));
+#pragma unroll
+            for (int h = 0; h < 2; ++h) {
+                if (Q41) {
+                    ws[i][h] = __ldg(reinterpret_cast<const uint4*>(ps[i][h]) + q);
+                } else {
+                    const uint2 v = __ldg(reinterpret_cast<const uint2*>(ps[i][h]) + q);
+                    ws[i][h].x = v.x;
+                    ws[i][h].y = v.y;
+                }
+            }
+        }
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            const uint32_t blk = min(q * 4 + b, nb - 1);  // terms of blocks that do not exist are not stored
+#pragma unroll
+            for (uint32_t h = 0; h < H; ++h) {
+                const uint32_t row = h ? row_b : row_a;
+                const uint32_t* p = reinterpret_cast<const uint32_t*>(xq + (size_t)row * K + (size_t)blk * 32) + t;
+                x.a[b][h] = p[0];
+                x.a[b][2 + h] = p[4];
+                x.s[h][b] = xscale[(size_t)row * nb + blk];
+                if (!Q8) x.qs[h][b] = xqsum[(size_t)row * nb + blk];
+            }
+            if (!WIDE) x.a[b][1] = x.a[b][3] = 0;
+        }
+    };
+    auto compute = [&](uint32_t q, uint32_t round0) {
+#pragma unroll
+        for (int b = 0; b < 4; ++b) {
+            if (q * 4 + b >= nb) break;
+            float* to = terms + (size_t)(q * 4 + b - round0) * OUTS + g * 8 + 2 * t;
+#pragma unroll
+            for (int i = 0; i < NTL; ++i) {
+                uint32_t b0, b1;
+                if (Q8) {
+                    b0 = pick4(w[i][0], b);
+                    b1 = pick4(w[i][1], b);
+                } else {
+                    const uint32_t u = pick4(w[i][0], b);
+                    b0 = u & 0x0F0F0F0Fu;
+                    b1 = (u >> 4) & 0x0F0F0F0Fu;
+                }
+                int d[4];
+                mma_s8(d, x.a[b][0], x.a[b][1], x.a[b][2], x.a[b][3], b0, b1);
+                float dw[2], mw[2];
+#pragma unroll
+                for (int c = 0; c < 2; ++c) {
+                    const uint32_t u = Q41 ? pick4(ws[i][c], b) : (b < 2 ? ws[i][c].x : ws[i][c].y);
+                    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&u));
+                    dw[c] = !Q41 && (b & 1) ? f.y : f.x;
+                    mw[c] = f.y;
+                }
+#pragma unroll
+                for (uint32_t h = 0; h < H; ++h) {
+                    float v[2];
+#pragma unroll
+                    for (int c = 0; c < 2; ++c) {
+                        int dot = d[h * 2 + c];
+                        if (TYPE == ZQ_TYPE_Q4_0) dot -= 8 * x.qs[h][b];
+                        v[c] = __fmul_rn(__fmul_rn(dw[c], x.s[h][b]), (float)dot);
+                        if (Q41) v[c] = __fadd_rn(v[c], __fmul_rn(__fmul_rn(mw[c], x.s[h][b]), (float)x.qs[h][b]));
+                    }
+                    *reinterpret_cast<float2*>(to + (i * H + h) * 64) = make_float2(v[0], v[1]);
+                }
+            }
+        }
+    };
+
+    float run = 0.0f;
+#pragma unroll 1
+    for (uint32_t r0 = 0; r0 < nb; r0 += round_blocks) {
+        const uint32_t end = min(r0 + round_blocks, nb);
+#pragma unroll 2
+        for (uint32_t q = r0 / 4 + warp; q * 4 < end; q += kTermWarps) {
+            load(q);
+            compute(q, r0);
+        }
+        __syncthreads();
+        if (tid < OUTS) {
+            const float* from = terms + tid;
+            uint32_t b = 0;
+            const uint32_t n = end - r0;
+            for (; b + 16 <= n; b += 16) {
+                float v[16];
+#pragma unroll
+                for (int u = 0; u < 16; ++u) v[u] = from[(size_t)(b + u) * OUTS];
+#pragma unroll
+                for (int u = 0; u < 16; ++u) run = __fadd_rn(run, v[u]);
+            }
+            for (; b < n; ++b) run = __fadd_rn(run, from[(size_t)b * OUTS]);
+        }
+        __syncthreads();
+    }
+    if (tid < OUTS) {
+        const uint32_t n = n0 + tid / (64 * H) * 8 + (tid & 7u), m = m0 + ((tid >> 3) & 7u) + (tid / 64 % H) * 8;
+        if (n < N && m < M) {
+            const size_t o = (size_t)m * N + n;
+            float v = run;
+            if (ep.bias) v = __fadd_rn(v, ep.bias[n]);
+            if (ep.gelu) v = gelu_tanh(v);
+            if (ep.mul) v = __fmul_rn(v, ep.mul[o]);
+            if (ep.residual) v = __fadd_rn(ep.residual[o], v);
+            y[o] = v;
+        }
+    }
+}
+
+template <int TYPE, int NTL, bool WIDE>
+int launch_terms(const zq_weight* w, const int8_t* xq, const float* xs, const int32_t* xsum, float* y, uint32_t M,
+                 QgEpilogue ep, cudaStream_t st) {
+    constexpr uint32_t kBlockBytes = (WIDE ? 128 : 64) * NTL * 4;
+    constexpr uint32_t kMost = 112 * 1024 / kBlockBytes / 4 * 4;  // two CTAs share an SM
+    const uint32_t rounds = (w->nb + kMost - 1) / kMost, per = ((w->nb + rounds - 1) / rounds + 3) / 4 * 4;
+    const dim3 grid((w->out_dim + 8 * NTL - 1) / (8 * NTL), (M + 15) / 16);
+    if (grid.y > 65535u) return ZQ_ERR_LIMIT;
+    auto kern = gemm_q8_terms_kernel<TYPE, NTL, WIDE>;
+    const size_t smem = (size_t)per * kBlockBytes;
+    ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ZQ_CUDA(launch_pdl(kern, grid, dim3(kTermWarps * 32), smem, st, w->qs, static_cast<const uint8_t*>(w->sc), xq, xs, xsum,
+                       y, w->out_dim, w->in_dim, M, w->nb, w->scp, per, ep));
+    return ZQ_OK;
+}
+
 template <int TYPE, int W, int NT, int D>
 int launch_cfg(const zq_weight* w, const int8_t* xq, const float* xs, const int32_t* xsum, float* y, uint32_t M,
                QgEpilogue ep, cudaStream_t st) {
@@ -301,6 +479,17 @@ int launch_cfg(const zq_weight* w, const int8_t* xq, const float* xs, const int3
 template <int TYPE>
 int launch_one(const zq_weight* w, const int8_t* xq, const float* xs, const int32_t* xsum, float* y, uint32_t M,
                QgEpilogue ep, cudaStream_t st) {
+    // Few tiles of 8 weight rows x 16 activation rows: K split over the warps (B200, graph-timed with the quantiser,
+    // the kernel above and then this form: 1152 <- 6912 8_0 at 8 rows 25.4 and 10.9 us, 4_1 at 48 rows 28.5 and 26.9;
+    // 1152 <- 1024 at 16 rows 6.7 and 5.1; 5003 <- 1184 at 8 rows 7.7 and 6.5; beyond, 13824 <- 1152 at 8 rows 8.9 and
+    // 10.9). Two weight tiles per CTA once one would give more CTAs than the GPU holds at a time.
+    const uint64_t tiles = (uint64_t)((w->out_dim + 7) / 8) * ((M + 15) / 16);
+    if (tiles <= 640 && M <= 8)
+        return tiles <= 192 ? launch_terms<TYPE, 1, false>(w, xq, xs, xsum, y, M, ep, st)
+                            : launch_terms<TYPE, 2, false>(w, xq, xs, xsum, y, M, ep, st);
+    if (tiles <= 480)
+        return tiles <= 192 ? launch_terms<TYPE, 1, true>(w, xq, xs, xsum, y, M, ep, st)
+                            : launch_terms<TYPE, 2, true>(w, xq, xs, xsum, y, M, ep, st);
     const uint64_t rt = (w->out_dim + 15) / 16, mt8 = (M + 7) / 8;
     uint32_t nt_cap = 1, nt_min = 1;
     while (nt_cap < 8 && nt_cap < mt8) nt_cap *= 2;
