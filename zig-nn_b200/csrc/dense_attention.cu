@@ -512,7 +512,7 @@ int plain_rows(const GqaShape& s, const void* q, const void* kc, const void* vc,
 uint32_t decode_splits(const GqaShape& s, uint32_t rows) {
     const uint32_t R = s.heads / s.kv_heads, ctas = rows * s.kv_heads * ((R + 15) / 16);
     const uint32_t least = std::min(32u, std::max(1u, (s.ctx + 255) / 256)), most = std::min(32u, (s.ctx + kTile - 1) / kTile);
-    return std::max(least, std::min(most, 148 / ctas));
+    return std::max(least, std::min(most, 148 / std::max(1u, ctas)));
 }
 
 template <int D>
