@@ -52,6 +52,17 @@ def test_linear_any_number_of_rows(zq, f32, rows_k):
         close(w.linear(zq.dense_rows(torch.tensor(x), f32)), x @ W.T, 3e-6, "T=%d" % T)
 
 
+@pytest.mark.parametrize("rows_k", [(37889, 72), (18945, 130), (9500, 328), (33, 64)])
+def test_linear_few_rows_on_the_tensor_cores(zq, rows_k):
+    """One, two, four and eight warps to a tile's K; a last tile of one row."""
+    rng = np.random.default_rng(7)
+    W, bits = bf16(rng.standard_normal(rows_k))
+    w = zq.DenseWeight(bits)
+    for T in (3, 8):
+        x = held(rng.standard_normal((T, rows_k[1])), False)
+        close(w.linear(zq.dense_rows(torch.tensor(x))), x @ W.T, 3e-6, "T=%d" % T)
+
+
 def test_linear_many_tiles(zq):
     """More tiles than CTAs, so that the accumulators take turns, with ragged edges on both sides."""
     rng = np.random.default_rng(2)

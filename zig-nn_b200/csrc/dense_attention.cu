@@ -403,10 +403,13 @@ gqa_combine_kernel(const __grid_constant__ AttnArgs a) {
     bf16* out = a.out + (size_t)r * a.out_pitch;
     for (uint32_t d = threadIdx.x; d < pad32(s.vdim); d += blockDim.x) {
         float acc = 0.0f;
-#pragma unroll 8
-        for (uint32_t i = 0; i < n; ++i) {
-            const float v = d < s.vdim ? a.part[(row0 + (size_t)i * s.heads) * s.vdimp + d] : 0.0f;
-            acc = fmaf(__shfl_sync(0xFFFFFFFFu, f, i), v, acc);
+        for (uint32_t i0 = 0; i0 < n; i0 += 8) {  // eight ranges requested together, the last of them too
+            float v[8];
+#pragma unroll
+            for (uint32_t u = 0; u < 8; ++u)
+                v[u] = d < s.vdim && i0 + u < n ? a.part[(row0 + (size_t)(i0 + u) * s.heads) * s.vdimp + d] : 0.0f;
+#pragma unroll
+            for (uint32_t u = 0; u < 8; ++u) acc = fmaf(__shfl_sync(0xFFFFFFFFu, f, i0 + u), v[u], acc);
         }
         if (d < s.vdim) out[(size_t)h * s.vdim + d] = __float2bfloat16_rn(acc * inv);
     }
