@@ -103,7 +103,8 @@ attention_prefill_kernel(PrefillArgs a) {
 
     for (uint32_t i = tid; i < kRows * (HD / 4); i += T) {
         const uint32_t r = min(i / (HD / 4), n - 1), c = i % (HD / 4);
-        reinterpret_cast<float4*>(qs)[i] = *reinterpret_cast<const float4*>(a.q + (size_t)(t0 + r) * a.q_stride + (size_t)h * HD + c * 4);
+        const float* from = a.q + (size_t)(t0 + r) * a.q_stride + (size_t)h * HD + c * 4;
+        reinterpret_cast<float4*>(qs)[i] = *reinterpret_cast<const float4*>(from);
     }
     // ---- dots: 16 lane sums over the dimensions (dimension mod 16), added in order
     const uint32_t n_key_tiles = (hi - lo + kKeys - 1) / kKeys * S::kParts;
@@ -146,7 +147,8 @@ attention_prefill_kernel(PrefillArgs a) {
                 for (int c = 0; c < 4; ++c) {
                     float4 kv[KL], qv[RW];
 #pragma unroll
-                    for (uint32_t k = 0; k < KL; ++k) kv[k] = *reinterpret_cast<const float4*>(k0 + k * 32 * S::kPitch + d + 4 * c);
+                    for (uint32_t k = 0; k < KL; ++k)
+                        kv[k] = *reinterpret_cast<const float4*>(k0 + k * 32 * S::kPitch + d + 4 * c);
 #pragma unroll
                     for (uint32_t r = 0; r < RW; ++r) qv[r] = *reinterpret_cast<const float4*>(q0 + r * HD + d + 4 * c);
 #pragma unroll

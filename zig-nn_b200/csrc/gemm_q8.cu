@@ -454,7 +454,7 @@ gemm_q8_terms_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__
 
 template <int TYPE, int NTL, bool WIDE>
 int launch_terms(const zq_weight* w, const int8_t* xq, const float* xs, const int32_t* xsum, float* y, uint32_t M,
-                 QgEpilogue ep, cudaStream_t st) {
+                 QgEpilogue ep, bool split, cudaStream_t st) {
     constexpr uint32_t kBlockBytes = (WIDE ? 128 : 64) * NTL * 4;
     constexpr uint32_t kMost = 112 * 1024 / kBlockBytes / 4 * 4;  // two CTAs share an SM
     const uint32_t rounds = (w->nb + kMost - 1) / kMost, per = ((w->nb + rounds - 1) / rounds + 3) / 4 * 4;
@@ -463,22 +463,22 @@ int launch_terms(const zq_weight* w, const int8_t* xq, const float* xs, const in
     auto kern = gemm_q8_terms_kernel<TYPE, NTL, WIDE>;
     const size_t smem = (size_t)per * kBlockBytes;
     ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    ZQ_CUDA(launch_pdl(kern, grid, dim3(kTermWarps * 32), smem, st, w->qs, static_cast<const uint8_t*>(w->sc), xq, xs, xsum,
-                       y, w->out_dim, w->in_dim, M, w->nb, w->scp, per, ep));
+    ZQ_CUDA(launch_pdl_split(split, kern, grid, dim3(kTermWarps * 32), smem, st, w->qs,
+                       static_cast<const uint8_t*>(w->sc), xq, xs, xsum, y, w->out_dim, w->in_dim, M, w->nb, w->scp, per, ep));
     return ZQ_OK;
 }
 
 template <int TYPE, int W, int NT, int D>
 int launch_cfg(const zq_weight* w, const int8_t* xq, const float* xs, const int32_t* xsum, float* y, uint32_t M,
-               QgEpilogue ep, cudaStream_t st) {
+               QgEpilogue ep, bool split, cudaStream_t st) {
     const dim3 grid((w->out_dim + W * 16 - 1) / (W * 16), (M + NT * 8 - 1) / (NT * 8));
     if (grid.y > 65535u) return ZQ_ERR_LIMIT;
     const size_t smem = (size_t)D * QgStage<TYPE, W, NT>::kBytes;
     auto kern = gemm_q8_kernel<TYPE, W, NT, D>;
     if (smem > 48 * 1024)
         ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    ZQ_CUDA(launch_pdl(kern, grid, dim3(W * 32), smem, st, w->qs, static_cast<const uint8_t*>(w->sc), xq, xs, xsum,
-                       y, w->out_dim, w->in_dim, M, w->nb, w->scp, ep));
+    ZQ_CUDA(launch_pdl_split(split, kern, grid, dim3(W * 32), smem, st, w->qs,
+                       static_cast<const uint8_t*>(w->sc), xq, xs, xsum, y, w->out_dim, w->in_dim, M, w->nb, w->scp, ep));
     return ZQ_OK;
 }
 
@@ -491,18 +491,18 @@ int launch_cfg(const zq_weight* w, const int8_t* xq, const float* xs, const int3
 // one-warp CTAs; 1152->13824 at 64 rows: 21 us with NT = 4, 25 us with NT = 8.)
 template <int TYPE>
 int launch_one(const zq_weight* w, const int8_t* xq, const float* xs, const int32_t* xsum, float* y, uint32_t M,
-               QgEpilogue ep, cudaStream_t st) {
+               QgEpilogue ep, bool split, cudaStream_t st) {
     // Few tiles of 8 weight rows x 16 activation rows: K split over the warps (B200, graph-timed with the quantiser,
     // the kernel above and then this form: 1152 <- 6912 8_0 at 8 rows 25.4 and 10.9 us, 4_1 at 48 rows 28.5 and 26.9;
     // 1152 <- 1024 at 16 rows 6.7 and 5.1; 5003 <- 1184 at 8 rows 7.7 and 6.5; beyond, 13824 <- 1152 at 8 rows 8.9 and
     // 10.9). Two weight tiles per CTA once one would give more CTAs than the GPU holds at a time.
     const uint64_t tiles = (uint64_t)((w->out_dim + 7) / 8) * ((M + 15) / 16);
     if (tiles <= 640 && M <= 8)
-        return tiles <= 192 ? launch_terms<TYPE, 1, false>(w, xq, xs, xsum, y, M, ep, st)
-                            : launch_terms<TYPE, 2, false>(w, xq, xs, xsum, y, M, ep, st);
+        return tiles <= 192 ? launch_terms<TYPE, 1, false>(w, xq, xs, xsum, y, M, ep, split, st)
+                            : launch_terms<TYPE, 2, false>(w, xq, xs, xsum, y, M, ep, split, st);
     if (tiles <= 480)
-        return tiles <= 192 ? launch_terms<TYPE, 1, true>(w, xq, xs, xsum, y, M, ep, st)
-                            : launch_terms<TYPE, 2, true>(w, xq, xs, xsum, y, M, ep, st);
+        return tiles <= 192 ? launch_terms<TYPE, 1, true>(w, xq, xs, xsum, y, M, ep, split, st)
+                            : launch_terms<TYPE, 2, true>(w, xq, xs, xsum, y, M, ep, split, st);
     const uint64_t rt = (w->out_dim + 15) / 16, mt8 = (M + 7) / 8;
     uint32_t nt_cap = 1, nt_min = 1;
     while (nt_cap < 8 && nt_cap < mt8) nt_cap *= 2;
@@ -514,17 +514,18 @@ int launch_one(const zq_weight* w, const int8_t* xq, const float* xs, const int3
             break;
         }
     switch (nt) {
-        case 8: return launch_cfg<TYPE, 8, 8, 3>(w, xq, xs, xsum, y, M, ep, st);
-        case 4: return launch_cfg<TYPE, 4, 4, 4>(w, xq, xs, xsum, y, M, ep, st);
-        case 2: return launch_cfg<TYPE, 4, 2, 6>(w, xq, xs, xsum, y, M, ep, st);
-        default: return launch_cfg<TYPE, 4, 1, 8>(w, xq, xs, xsum, y, M, ep, st);
+        case 8: return launch_cfg<TYPE, 8, 8, 3>(w, xq, xs, xsum, y, M, ep, split, st);
+        case 4: return launch_cfg<TYPE, 4, 4, 4>(w, xq, xs, xsum, y, M, ep, split, st);
+        case 2: return launch_cfg<TYPE, 4, 2, 6>(w, xq, xs, xsum, y, M, ep, split, st);
+        default: return launch_cfg<TYPE, 4, 1, 8>(w, xq, xs, xsum, y, M, ep, split, st);
     }
 }
 
 }  // namespace
 
 int launch_gemm_q8(const zq_weight* w, const int8_t* xq, const float* xscale, const int32_t* xsum, float* y,
-                   uint32_t m_rows, const zq_epilogue* ep, cudaStream_t st) {
+                   uint32_t m_rows, const zq_epilogue* ep, cudaStream_t st, bool shared_split) {
+    const bool split = shared_split && m_rows <= kSharedSplitRows;
     QgEpilogue a{nullptr, nullptr, nullptr, 0};
     if (ep) {
         a.bias = ep->d_bias;
@@ -533,9 +534,9 @@ int launch_gemm_q8(const zq_weight* w, const int8_t* xq, const float* xscale, co
         a.residual = ep->d_residual;
     }
     switch (w->type) {
-        case ZQ_TYPE_Q4_0: return launch_one<ZQ_TYPE_Q4_0>(w, xq, xscale, xsum, y, m_rows, a, st);
-        case ZQ_TYPE_Q4_1: return launch_one<ZQ_TYPE_Q4_1>(w, xq, xscale, xsum, y, m_rows, a, st);
-        case ZQ_TYPE_Q8_0: return launch_one<ZQ_TYPE_Q8_0>(w, xq, xscale, xsum, y, m_rows, a, st);
+        case ZQ_TYPE_Q4_0: return launch_one<ZQ_TYPE_Q4_0>(w, xq, xscale, xsum, y, m_rows, a, split, st);
+        case ZQ_TYPE_Q4_1: return launch_one<ZQ_TYPE_Q4_1>(w, xq, xscale, xsum, y, m_rows, a, split, st);
+        case ZQ_TYPE_Q8_0: return launch_one<ZQ_TYPE_Q8_0>(w, xq, xscale, xsum, y, m_rows, a, split, st);
         default: return ZQ_ERR_UNSUPPORTED;
     }
 }

@@ -805,10 +805,11 @@ int launch_norm_quant(const float* src, const float* w1, float* res, const float
     const size_t smem = dim * sizeof(float);
     cudaError_t e;
     if (dim <= 256 * 5) {
-        e = res ? launch_pdl(norm_quant_kernel<true, 5>, dim3(rows), dim3(256), smem, st, src, w1, res, w2, dim, eps, q,
-                             scale, sum, src_stride)
-                : launch_pdl(norm_quant_kernel<false, 5>, dim3(rows), dim3(256), smem, st, src, w1, nullptr, nullptr,
-                             dim, eps, q, scale, sum, src_stride);
+        const bool split = rows <= kSharedSplitRows;
+        e = res ? launch_pdl_split(split, norm_quant_kernel<true, 5>, dim3(rows), dim3(256), smem, st, src, w1, res, w2, dim,
+                                   eps, q, scale, sum, src_stride)
+                : launch_pdl_split(split, norm_quant_kernel<false, 5>, dim3(rows), dim3(256), smem, st, src, w1, nullptr,
+                                   nullptr, dim, eps, q, scale, sum, src_stride);
     } else {
         e = res ? launch_pdl(norm_quant_kernel<true, 0>, dim3(rows), dim3(256), smem, st, src, w1, res, w2, dim, eps, q,
                              scale, sum, src_stride)
@@ -836,8 +837,8 @@ int launch_gelu_mul_quant(const float* gate, const float* up, uint32_t n, int8_t
     if (n % 32) return ZQ_ERR_BAD_ARG;
     if (rows == 0) return ZQ_OK;
     const size_t total = (size_t)rows * n;
-    ZQ_CUDA(launch_pdl(gelu_mul_quant_kernel, dim3(grid1d(total, 256)), dim3(256), 0, st, gate, up,
-                       (uint32_t)(total / 32), q, scale, sum, n / 32, in_stride));
+    ZQ_CUDA(launch_pdl_split(rows <= kSharedSplitRows, gelu_mul_quant_kernel, dim3(grid1d(total, 256)), dim3(256), 0, st, gate,
+                             up, (uint32_t)(total / 32), q, scale, sum, n / 32, in_stride));
     return ZQ_OK;
 }
 
@@ -867,7 +868,8 @@ int launch_attention_step(const float* q, float* kc, float* vc, const float* k_n
     uint32_t tiles_x = (max_len + 15) / 16;
     const bool loop = rows >= 16 && tiles_x > 8;
     if (loop) tiles_x = 8;
-    ZQ_CUDA(launch_pdl(loop ? attention_scores_step_kernel<true> : attention_scores_step_kernel<false>,
+    const bool split = rows <= kSharedSplitRows;
+    ZQ_CUDA(launch_pdl_split(split, loop ? attention_scores_step_kernel<true> : attention_scores_step_kernel<false>,
                        dim3(tiles_x, n_head, rows), dim3(256), smem_scores, st, q, kc, vc, k_new, v_new, scores, n_head,
                        n_kv_head, head_dim, state, window, q_stride, scores_stride, row_pos, cache_stride, nr));
     const dim3 grid(n_head, (head_dim + kAttnDims - 1) / kAttnDims, rows);
@@ -875,14 +877,14 @@ int launch_attention_step(const float* q, float* kc, float* vc, const float* k_n
         auto kern = attention_softmax_v_step_kernel<true>;
         if (smem > 24 * 1024)  // the kernel also holds a 16 KB static tile
             ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        ZQ_CUDA(launch_pdl(kern, grid, dim3(256), smem, st, static_cast<const float*>(scores),
+        ZQ_CUDA(launch_pdl_split(split, kern, grid, dim3(256), smem, st, static_cast<const float*>(scores),
                            static_cast<const float*>(vc), out, oq, oscale, osum, n_head, n_kv_head, head_dim, state,
                            window, tail, scores_stride, row_pos, cache_stride));
     } else {
         auto kern = attention_softmax_v_step_kernel<false>;
         if (smem > 24 * 1024)
             ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        ZQ_CUDA(launch_pdl(kern, grid, dim3(256), smem, st, static_cast<const float*>(scores),
+        ZQ_CUDA(launch_pdl_split(split, kern, grid, dim3(256), smem, st, static_cast<const float*>(scores),
                            static_cast<const float*>(vc), out, nullptr, nullptr, nullptr, n_head, n_kv_head, head_dim,
                            state, window, tail, scores_stride, row_pos, cache_stride));
     }

@@ -84,22 +84,40 @@ __device__ __forceinline__ void prefetch_l2_line(const void* p) {
 // streams has other predecessors than the one kernel that it could overlap with).
 inline thread_local bool whole_dependency = false;
 
+// shared_split: ask for the split of an SM's memory that leaves most to shared memory. A kernel that wants another split than
+// the one before it starts only when the SM has drained; a streaming kernel, on the other hand, needs L1 for its loads in
+// flight, so only launches of few rows ask for it.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
-                              Args... args) {
+inline cudaError_t launch_pdl_split(bool shared_split, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                    cudaStream_t st, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = grid;
     cfg.blockDim = block;
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchAttribute attr[2];
+    uint32_t n = 0;
+    if (!whole_dependency) {
+        attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[n++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (shared_split) {
+        attr[n].id = cudaLaunchAttributePreferredSharedMemoryCarveout;
+        attr[n++].val.sharedMemCarveout = cudaSharedmemCarveoutMaxShared;
+    }
     cfg.attrs = attr;
-    cfg.numAttrs = whole_dependency ? 0 : 1;
+    cfg.numAttrs = n;
     whole_dependency = false;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
 }
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                              Args... args) {
+    return launch_pdl_split(false, kernel, grid, block, smem, st, args...);
+}
+// Rows of a launch up to which the kernels of a Gemma-3 step ask for the split of the exact int8 products among them (eight
+// sequences and short prompts 35.8 -> 34.0 ms; with 512 rows it costs the streaming ones 1 % of a prompt).
+constexpr uint32_t kSharedSplitRows = 64;
 #endif
 
 // Exponent e of the power-of-two row scale 2^-e that brings a row's largest magnitude `amax` just under 2^14
@@ -153,8 +171,9 @@ int launch_gemv_q8(const zq_weight* w, const int8_t* xq, const float* xscale, co
 int launch_quantize_rows_q8(const float* x, uint32_t m_rows, uint32_t in_dim, int8_t* q,
                             float* scale, int32_t* sum, cudaStream_t st);
 // Exact int8 tensor-core GEMM for many Q8-quantised activation rows; bit-identical to launch_gemv_q8 (gemm_q8.cu).
+// shared_split: see launch_pdl_split; not for a product alone (16 rows of 1152 <- 6912 with their quantiser 13.4 us, 14.2 so).
 int launch_gemm_q8(const zq_weight* w, const int8_t* xq, const float* xscale, const int32_t* xsum, float* y,
-                   uint32_t m_rows, const zq_epilogue* ep, cudaStream_t st);
+                   uint32_t m_rows, const zq_epilogue* ep, cudaStream_t st, bool shared_split = false);
 constexpr uint32_t kGemmMinRows = 49;  // below this, passes of the 16-row decode kernel are faster
 // x16[m][k] = fp16(x[m][k] * 2^-e_m), post[m] = 2^e_m (gemm.cu).
 int launch_convert_rows_f16(const float* x, __half* x16, float* post, uint32_t m_rows, uint32_t in_dim,
