@@ -53,14 +53,28 @@ def test_linear_any_number_of_rows(zq, f32, rows_k):
 
 
 @pytest.mark.parametrize("rows_k", [(37889, 72), (18945, 130), (9500, 328), (33, 64)])
-def test_linear_few_rows_on_the_tensor_cores(zq, rows_k):
-    """One, two, four and eight warps to a tile's K; a last tile of one row."""
+def test_linear_few_rows(zq, rows_k):
+    """Two weight rows to a warp, the last warp with one; one row to a warp."""
     rng = np.random.default_rng(7)
     W, bits = bf16(rng.standard_normal(rows_k))
     w = zq.DenseWeight(bits)
     for T in (3, 8):
         x = held(rng.standard_normal((T, rows_k[1])), False)
         close(w.linear(zq.dense_rows(torch.tensor(x))), x @ W.T, 3e-6, "T=%d" % T)
+
+
+@pytest.mark.parametrize("f32", PRECISIONS)
+@pytest.mark.parametrize("rows_k", [(37889, 72), (5000, 200), (130, 1100), (515, 328)])
+def test_rows_do_not_depend_on_each_other(zq, f32, rows_k):
+    """Up to eight rows share one order of the sum over K (two rows to a warp, one, and one to four warps): a sequence's bits
+    stay the same when others join its step or leave it."""
+    rng = np.random.default_rng(8)
+    bits = [bf16(rng.standard_normal(rows_k))[1] for _ in range(2)]
+    x = zq.dense_rows(torch.tensor(held(rng.standard_normal((8, rows_k[1])), f32)), f32)
+    for call in (zq.DenseWeight(bits[0]).linear, zq.DenseWeight(*bits).glu):
+        alone = torch.cat([call(x[r:r + 1]) for r in range(8)])
+        for T in range(2, 9):
+            assert torch.equal(call(x[:T]), alone[:T]), T
 
 
 def test_linear_many_tiles(zq):

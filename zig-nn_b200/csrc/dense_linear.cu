@@ -208,155 +208,8 @@ int gemv_shape(GemvParams p, uint32_t rows, uint32_t kp, uint32_t gy, uint32_t g
     return ZQ_OK;
 }
 
-// ---- up to 8 bf16 activation rows on the tensor cores -------------------------------------------------
-// mma.sync.m16n8k16 with 16 weight rows as A and the activation rows as the 8 columns of B. Any permutation of K serves as
-// long as both operands use it, so a lane takes 16 contiguous bytes of its weight rows and of its activation row per 32 K and
-// they are the fragments of two MMAs as they lie: no shared memory, no unpacking, and one load of x for 16 weight rows. The
-// kernel above, which multiplies in f32, spends 8 multiply-adds and an unpacked copy of x on every weight from several rows
-// on; here the weights' way from memory is what is left. The tensor core sums 16 products and the sums over K are added in
-// f32 outside of it, whose rounding it does not keep (50304 <- 768, error against 64 bits: 4e-7 with all of K inside, 8e-8
-// so; f32 multiply-adds 7e-8; a result is rounded to bf16, 2e-3, before it is multiplied again). KW warps share a tile's K (64 of it in turn) and meet in shared
-// memory; enough of them that about 16 warps per SM are at work.
-// Measured (B200, graph-timed, the kernel above and this one, 8 rows): 50304 <- 768 34.6 and 13.0 us (77 MB: 11.8 at the copy
-// rate), gated 2 x 6912 <- 1152 16.5 and 5.6, 1152 <- 6912 13.5 and 6.5, 768 <- 768 4.1 and 2.0.
-constexpr int kRowsWarps = 8;
-
-__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
-                                         uint32_t b1) {
-    asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%10,%10,%10};"
-        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
-        : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "f"(0.0f));
-}
-
-template <bool GLU, int KW>
-__global__ void __launch_bounds__(kRowsWarps * 32)
-dense_rows_kernel(const __grid_constant__ GemvParams p) {
-    constexpr int WR = kRowsWarps / KW, P = GLU ? 2 : 1;  // tiles of the CTA; matrices of 16 rows per tile (gate, up)
-    constexpr int U = GLU ? 1 : 2;                        // runs of 64 K held ahead
-    __shared__ float red[KW > 1 ? kRowsWarps * P * 128 : 1];
-    pdl_launch_dependents();
-    const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
-    const uint32_t wr = warp % WR, ks = warp / WR;
-    const LinGroup G = p.groups.g[blockIdx.y];
-    const uint32_t j0 = (blockIdx.x * WR + wr) * 16;
-    const bool real = j0 < G.rows;
-    const bf16* w[P][2];
-#pragma unroll
-    for (int m = 0; m < P; ++m)
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const uint32_t j = min(j0 + h * 8 + g, G.rows - 1);
-            w[m][h] = p.w + (size_t)(G.w_row + (GLU ? glu_row(j, m) : j)) * p.kp + 8 * t;
-        }
-    if (p.prefetch && real && ks == 0 && lane < 16) {
-        const uint32_t j = min(j0 + lane, G.rows - 1);
-#pragma unroll
-        for (int m = 0; m < P; ++m) prefetch_l2_bulk(p.w + (size_t)(G.w_row + (GLU ? glu_row(j, m) : j)) * p.kp, p.kp * 2);
-    }
-    const uint32_t runs = p.kp / 64;
-    uint4 cur[U][P][2][2];  // [run ahead][matrix][row half][32 K]
-    auto load = [&](uint4 (&to)[P][2][2], uint32_t u) {
-#pragma unroll
-        for (int m = 0; m < P; ++m)
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-                for (int c = 0; c < 2; ++c)
-                    to[m][h][c] = u < runs ? __ldg(reinterpret_cast<const uint4*>(w[m][h] + u * 64 + c * 32)) : make_uint4(0, 0, 0, 0);
-    };
-#pragma unroll
-    for (int i = 0; i < U; ++i) load(cur[i], ks + i * KW);
-    float acc[P][2][4];  // [matrix][32 K of a run]
-#pragma unroll
-    for (int m = 0; m < P; ++m)
-#pragma unroll
-        for (int c = 0; c < 2; ++c) acc[m][c][0] = acc[m][c][1] = acc[m][c][2] = acc[m][c][3] = 0.0f;
-    pdl_wait();
-    const bf16* x = static_cast<const bf16*>(p.x) + (size_t)(G.x_row + min(g, p.T - 1)) * p.kp + 8 * t;
-    for (uint32_t u = ks; u < runs; u += U * KW) {
-        uint4 nxt[U][P][2][2];
-#pragma unroll
-        for (int i = 0; i < U; ++i) load(nxt[i], u + (U + i) * KW);
-#pragma unroll
-        for (int i = 0; i < U; ++i) {
-            if (u + i * KW >= runs) break;
-#pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                const uint4 xv = *reinterpret_cast<const uint4*>(x + (u + i * KW) * 64 + c * 32);
-#pragma unroll
-                for (int m = 0; m < P; ++m) {
-                    const uint4 &a = cur[i][m][0][c], &b = cur[i][m][1][c];
-                    float d0[4], d1[4];
-                    mma_bf16(d0, a.x, b.x, a.y, b.y, xv.x, xv.y);
-                    mma_bf16(d1, a.z, b.z, a.w, b.w, xv.z, xv.w);
-#pragma unroll
-                    for (int e = 0; e < 4; ++e) acc[m][c][e] += d0[e] + d1[e];
-                }
-            }
-        }
-#pragma unroll
-        for (int i = 0; i < U; ++i)
-#pragma unroll
-            for (int m = 0; m < P; ++m)
-#pragma unroll
-                for (int h = 0; h < 2; ++h)
-#pragma unroll
-                    for (int c = 0; c < 2; ++c) cur[i][m][h][c] = nxt[i][m][h][c];
-    }
-#pragma unroll
-    for (int m = 0; m < P; ++m)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) acc[m][0][e] += acc[m][1][e];
-    if (KW > 1) {
-#pragma unroll
-        for (int m = 0; m < P; ++m)
-            *reinterpret_cast<float4*>(red + ((warp * P + m) * 32 + lane) * 4) =
-                make_float4(acc[m][0][0], acc[m][0][1], acc[m][0][2], acc[m][0][3]);
-        __syncthreads();
-        if (ks > 0) return;
-#pragma unroll
-        for (int k = 1; k < KW; ++k)
-#pragma unroll
-            for (int m = 0; m < P; ++m) {
-                const float4 v = *reinterpret_cast<const float4*>(red + (((k * WR + wr) * P + m) * 32 + lane) * 4);
-                acc[m][0][0] += v.x;
-                acc[m][0][1] += v.y;
-                acc[m][0][2] += v.z;
-                acc[m][0][3] += v.w;
-            }
-    }
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-        const uint32_t j = j0 + g + (e >> 1) * 8, r = 2 * t + (e & 1);
-        if (j >= G.rows || r >= p.T) continue;
-        const size_t o = (size_t)r * p.y_stride + G.y_col + j;
-        if (GLU)
-            static_cast<bf16*>(p.y)[o] = to_act<bf16>(glu_value(acc[0][0][e], acc[P - 1][0][e], p.glu.kind, p.glu.limit));
-        else
-            static_cast<float*>(p.y)[o] = acc[0][0][e];
-    }
-}
-
-template <bool GLU>
-int tensor_rows(GemvParams p, uint32_t rows, uint32_t n_groups, cudaStream_t st) {
-    p.prefetch = (uint64_t)rows * (GLU ? 2 : 1) * n_groups * p.kp * 2 <= (64u << 20);  // a part of L2 at most
-    const uint64_t tiles = (uint64_t)((rows + 15) / 16) * n_groups, want = (uint64_t)sm_count() * 16;
-    auto go = [&](auto kern, uint32_t kw) {
-        const uint32_t wr = kRowsWarps / kw;
-        const cudaError_t e = launch_pdl(kern, dim3(((rows + 15) / 16 + wr - 1) / wr, n_groups), dim3(kRowsWarps * 32), 0, st, p);
-        return e != cudaSuccess ? cuda_fail(e) : ZQ_OK;
-    };
-    if (tiles >= want) return go(dense_rows_kernel<GLU, 1>, 1);
-    if (tiles * 2 >= want) return go(dense_rows_kernel<GLU, 2>, 2);
-    if (tiles * 4 >= want) return go(dense_rows_kernel<GLU, 4>, 4);
-    return go(dense_rows_kernel<GLU, 8>, 8);
-}
-
 template <typename TX, bool GLU>
 int gemv_rows(const GemvParams& p, uint32_t rows, uint32_t n_groups, cudaStream_t st) {
-    // From three rows on the tensor cores; with two the f32 kernel is level or ahead on narrow deep matrices (768 <- 3072: 2.8
-    // and 3.4 us), with one ahead.
-    if (sizeof(TX) == 2 && p.T >= 3 && p.T <= 8) return tensor_rows<GLU>(p, rows, n_groups, st);
     if (p.T == 1) return gemv_shape<TX, 1, GLU, false>(p, rows, p.kp, n_groups, 1, st);
     if (p.T == 2) return gemv_shape<TX, 2, GLU, false>(p, rows, p.kp, n_groups, 1, st);
     if (p.T <= 4) return gemv_shape<TX, 4, GLU, false>(p, rows, p.kp, n_groups, 1, st);
