@@ -190,6 +190,27 @@ def test_attention_prefill_and_decode(zq, f32, shape):
 
 
 @pytest.mark.parametrize("f32", PRECISIONS)
+@pytest.mark.parametrize("ctx,shape", [(1100, (4, 4, 64, 64)), (256, (8, 8, 40, 24)), (2048, (4, 1, 256, 256))])
+def test_attention_rows_do_not_depend_on_each_other(zq, f32, ctx, shape):
+    """Sixteen sequences in a step: each has the bits that it has alone, and the values, at the borders of tiles and ranges
+    (four tiles to a range, one range over several tiles, more ranges than a short row has tiles)."""
+    rng = np.random.default_rng(9)
+    H, G, d, e = shape
+    n, scale = 16, d ** -0.5
+    c, k, v = fill_cache(zq, rng, shape, ctx, n, f32, scale)
+    pos = np.array([0, 1, 62, 63, 64, 127, 128, 191, 192, 193, 254, 255, ctx // 2, ctx - 65, ctx - 2, ctx - 1])
+    slots = list(rng.permutation(n))
+    q = held(rng.standard_normal((n, H, d)), f32)
+    x = queries(c, q)
+    alone = torch.cat([c.attend(x[r:r + 1], pos[r:r + 1], slots[r:r + 1], False) for r in range(n)])
+    close(alone[:, :H * e], attend_rows(q, [k[s] for s in slots], [v[s] for s in slots], pos, scale), 1e-5 if f32 else 8e-3)
+    for T in (2, 3, 8, 16):
+        for r0 in range(0, n, T):
+            r = slice(r0, min(r0 + T, n))
+            assert torch.equal(c.attend(x[r], pos[r], slots[r], False), alone[r]), (T, r0)
+
+
+@pytest.mark.parametrize("f32", PRECISIONS)
 def test_attention_finds_one_key_among_many(zq, f32):
     """One key answers the query (its score stands out by far); it is put at tile borders, at the first token, at the
     row's own place and one place behind it, where it must not be seen."""

@@ -7,8 +7,6 @@
 //     mixing and the cache write of the new token happen in the same kernel;
 //   * f32, and heads beyond 256 dimensions: one warp-parallel online softmax per (row, head), plain multiply-adds.
 // A weight is rounded to bf16 for its product with the values; the sum it is divided by adds the same rounded weights.
-#include <algorithm>
-
 #include "dense.h"
 #include "tile_common.cuh"
 
@@ -228,8 +226,9 @@ gqa_prefill_kernel(const __grid_constant__ AttnArgs a) {
         for (uint32_t t = m0 / R; t <= last / R; ++t) zero_pad(a.out + (size_t)t * a.out_pitch, s.heads * s.vdim, a.out_pitch);
 }
 
-// STAGES: tiles of the ring; 1: the range is one tile.
-template <int D, uint32_t STAGES>
+constexpr uint32_t kDecodeStages = 3;
+
+template <int D>
 __global__ void __launch_bounds__(128)
 gqa_decode_kernel(const __grid_constant__ AttnArgs a) {
     constexpr int S = D / 16;
@@ -255,7 +254,7 @@ gqa_decode_kernel(const __grid_constant__ AttnArgs a) {
     }
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm);
     const uint32_t kbytes = kTile * (s.dimp + 8) * 2, vbytes = kTile * (s.vdimp + 8) * 2;
-    auto ktile = [&](uint32_t b) { return base + (b % STAGES) * (kbytes + vbytes); };
+    auto ktile = [&](uint32_t b) { return base + (b % kDecodeStages) * (kbytes + vbytes); };
     auto vtile = [&](uint32_t b) { return ktile(b) + kbytes; };
     const size_t slot = (size_t)(uint32_t)a.slots[r] * s.ctx;
     const bf16* kc = a.kc + slot * s.kv_heads * s.dimp;
@@ -266,14 +265,14 @@ gqa_decode_kernel(const __grid_constant__ AttnArgs a) {
     const bool fused = a.pre.qkv != nullptr, own = fused && k_end == len;
     const uint32_t c_end = own ? k_end - 1 : k_end;
 #pragma unroll
-    for (uint32_t t = 0; t == 0 || t + 1 < STAGES; ++t) {
+    for (uint32_t t = 0; t + 1 < kDecodeStages; ++t) {
         if (t < n_tiles) {
             load_tile(ktile(t), kc, s.kv_heads, g, s.dimp, k_begin + t * kTile, c_end);
             load_tile(vtile(t), vc, s.kv_heads, g, s.vdimp, k_begin + t * kTile, c_end);
         }
         copy_commit();
     }
-    bf16* own_q = reinterpret_cast<bf16*>(sm + STAGES * (kbytes + vbytes));  // [16][dimp], then own key and value
+    bf16* own_q = reinterpret_cast<bf16*>(sm + kDecodeStages * (kbytes + vbytes));  // [16][dimp], then own key and value
     bf16 *own_k = own_q + 16 * s.dimp, *own_v = own_k + s.dimp;
     if (fused) {
         const QkvPostArgs& f = a.pre;
@@ -308,18 +307,18 @@ gqa_decode_kernel(const __grid_constant__ AttnArgs a) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[v][e] = 0.0f;
     for (uint32_t t = 0; t < n_tiles; ++t) {
-        const uint32_t ahead = t + STAGES - 1;
-        if (STAGES > 1 && ahead < n_tiles) {
+        const uint32_t ahead = t + kDecodeStages - 1;
+        if (ahead < n_tiles) {
             load_tile(ktile(ahead), kc, s.kv_heads, g, s.dimp, k_begin + ahead * kTile, c_end);
             load_tile(vtile(ahead), vc, s.kv_heads, g, s.vdimp, k_begin + ahead * kTile, c_end);
         }
         copy_commit();
-        copy_wait<STAGES - 1>();
+        copy_wait<kDecodeStages - 1>();
         __syncthreads();
         if (own && t + 1 == n_tiles) {  // the place behind the copied keys
             const uint32_t at = k_end - 1 - (k_begin + t * kTile);
-            unsigned char* kt = sm + (t % STAGES) * (kbytes + vbytes) + at * (s.dimp + 8) * 2;
-            unsigned char* vt = sm + (t % STAGES) * (kbytes + vbytes) + kbytes + at * (s.vdimp + 8) * 2;
+            unsigned char* kt = sm + (t % kDecodeStages) * (kbytes + vbytes) + at * (s.dimp + 8) * 2;
+            unsigned char* vt = sm + (t % kDecodeStages) * (kbytes + vbytes) + kbytes + at * (s.vdimp + 8) * 2;
             for (uint32_t e = threadIdx.x; e < s.dimp; e += blockDim.x) reinterpret_cast<bf16*>(kt)[e] = own_k[e];
             for (uint32_t e = threadIdx.x; e < s.vdimp; e += blockDim.x) reinterpret_cast<bf16*>(vt)[e] = own_v[e];
             __syncthreads();
@@ -508,13 +507,11 @@ int plain_rows(const GqaShape& s, const void* q, const void* kc, const void* vc,
     return go(gqa_plain_kernel<TA, 32>, 32);
 }
 
-// Ranges of the keys of a decode step: of 256 keys, and down to a tile each while rows and heads leave SMs without a CTA (4
-// heads over one key head of 256, one row at 1500 keys: eight CTAs took 21 us; with 24, a step of six such layers is 30 us
-// shorter).
-uint32_t decode_splits(const GqaShape& s, uint32_t rows) {
-    const uint32_t R = s.heads / s.kv_heads, ctas = rows * s.kv_heads * ((R + 15) / 16);
-    const uint32_t least = std::min(32u, std::max(1u, (s.ctx + 255) / 256)), most = std::min(32u, (s.ctx + kTile - 1) / kTile);
-    return std::max(least, std::min(most, 148 / std::max(1u, ctas)));
+// Ranges of a row's keys, by the cache's capacity alone (256 keys each when it is full): a row's ranges, and with them its
+// bits, do not depend on the other rows of its step.
+uint32_t decode_splits(const GqaShape& s) {
+    const uint32_t n = (s.ctx + 255) / 256;
+    return n < 1 ? 1 : n > 32 ? 32 : n;
 }
 
 template <int D>
@@ -531,17 +528,12 @@ int tiles_launch(AttnArgs& a, bool one_sequence, cudaStream_t st) {
         ZQ_CUDA(cudaFuncSetAttribute(gqa_prefill_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * tile));
         return done(launch_pdl(gqa_prefill_kernel<D>, dim3((a.rows * R + 63) / 64, s.kv_heads), dim3(128), 2 * tile, st, a));
     }
-    a.splits = decode_splits(s, a.rows);
-    // Ranges of one tile need no ring, and a CTA of 75 KB in place of 209 KB (head_dim 256) can wait on its SM for the
-    // kernel ahead of it to end (Lenisun, 1500-token prompt and 24 steps of six such layers: 13.79 ms with the ring, 13.36
-    // without).
-    const uint32_t stages = (s.ctx + a.splits - 1) / a.splits <= kTile ? 1 : 3;
-    uint32_t smem = stages * tile + (17 * s.dimp + s.vdimp) * 2;
+    uint32_t smem = kDecodeStages * tile + (17 * s.dimp + s.vdimp) * 2;
     const uint32_t meet = (4 * 16 * 2 + 4 * 16 * s.vdimp) * 4;
     if (smem < meet) smem = meet;
-    auto kern = stages == 1 ? gqa_decode_kernel<D, 1> : gqa_decode_kernel<D, 3>;
-    ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    int rc = done(launch_pdl(kern, dim3(a.splits, s.kv_heads * ((R + 15) / 16), a.rows), dim3(128), smem, st, a));
+    a.splits = decode_splits(s);
+    ZQ_CUDA(cudaFuncSetAttribute(gqa_decode_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    int rc = done(launch_pdl(gqa_decode_kernel<D>, dim3(a.splits, s.kv_heads * ((R + 15) / 16), a.rows), dim3(128), smem, st, a));
     if (rc != ZQ_OK || a.splits == 1) return rc;
     return done(launch_pdl(gqa_combine_kernel, dim3(s.heads, a.rows), dim3(s.vdim >= 256 ? 256 : pad_to(s.vdim, 32)), 0, st, a));
 }
@@ -549,9 +541,8 @@ int tiles_launch(AttnArgs& a, bool one_sequence, cudaStream_t st) {
 }  // namespace
 
 size_t gqa_work_bytes(const GqaShape& s, uint32_t max_rows) {
-    size_t n = (size_t)max_rows * decode_splits(s, max_rows);
-    for (uint32_t r = 1; r < max_rows && r <= 148; ++r) n = std::max(n, (size_t)r * decode_splits(s, r));  // fewer rows, more ranges
-    return n * s.heads * (s.vdimp + 2) * sizeof(float);
+    const size_t n = decode_splits(s);
+    return (size_t)max_rows * n * s.heads * (s.vdimp + 2) * sizeof(float);
 }
 
 static bool tiled(const GqaShape& s) { return s.dimp <= 256 && s.vdimp <= 256; }
