@@ -200,9 +200,10 @@ size_t zq_matmul_transposed_workspace_bytes(const zq_weight* w, uint32_t m_rows)
  * out_dim must be a multiple of 8 (ZQ_ERR_UNSUPPORTED otherwise).
  * d_workspace: zq_matmul_transposed_workspace_bytes() bytes, 256-byte aligned.
  * Tensor-core product of fp16 copies (one rounding each for weights and gradients), f32 accumulation:
- * about 3e-4 relative L2 against the f32 statement. On small shapes the sums over the weight rows may be split
- * over CTAs and meet through atomic adds, so the last bits depend on the schedule there; more than 256 rows on a
- * matrix of 1024 weight rows and more run the tcgen05 GEMM on W^T (deterministic). */
+ * about 3e-4 relative L2 against the f32 statement. Where the tiles of 128 x 128 outputs do not give every
+ * multiprocessor two of them and out_dim is above 896, the sums over the weight rows may be split over CTAs and meet
+ * through atomic adds, so the last bits depend on the schedule; all other calls give the same bits on every run. More
+ * than 256 rows on a matrix of 1024 weight rows and more run the tcgen05 GEMM on W^T (the same bits too). */
 int zq_matmul_transposed(const zq_weight* w, const float* d_grad_out, float* d_grad_x, uint32_t m_rows,
                          int accumulate, void* d_workspace, size_t workspace_bytes, zq_stream stream);
 

@@ -394,6 +394,19 @@ def test_matmul_transposed_accumulates_like_the_reference_kernels(zq, oracle):
     assert rel_l2(gx2.cpu().numpy(), want2) <= REL_L2_TRANS
 
 
+def test_matmul_transposed_in_one_part_adds_its_whole_sum(zq):
+    """Output tiles that give every SM two CTAs: the weight rows stay in one part, so a tile is stored or added as a whole
+    and no schedule of partial sums is in the bits."""
+    out_dim, in_dim, m = 6912, 1152, 4200
+    g = torch.Generator(device="cuda").manual_seed(12)
+    raw = ggml.quantize(ggml.Q8_0, torch.randn(out_dim, in_dim, generator=g, device="cuda") * 0.02)
+    qw = zq.QuantWeight(raw, ggml.Q8_0, out_dim, in_dim)
+    go = torch.randn(m, out_dim, generator=g, device="cuda") * 1e-3
+    base = torch.randn(m, in_dim, generator=g, device="cuda")
+    got = zq.quant_matmul_transposed(go, qw)
+    assert torch.equal(zq.quant_matmul_transposed(go, qw, grad_x=base.clone(), accumulate=True), base + got)
+
+
 def test_quant_matmul_backward_to_activations(zq, oracle):
     """quant_matmul_no_grad on an input that requires grad carries the backward to x (the weight stays
     frozen): d/dx sum(y * c) = c . W."""

@@ -174,14 +174,16 @@ int launch_trans(const zq_weight* w, const __half* g16, const float* post, float
     ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     const uint32_t quads = (w->in_dim + TK - 1) / TK, mt = (M + TM - 1) / TM;
     const uint32_t n_chunks = (w->out_dim + TJ - 1) / TJ;
-    // Split the weight rows so that the waves of CTAs (one per SM) take the fewest stages, kStart of them for a CTA's start
-    // and its store, at least four stages per CTA. (Doubling the parts until the grid covered the
-    // GPU twice, then so, us with the conversion of the gradients: 6912 x 1152, 512 gradients, eight parts of 7 stages and
-    // four of 14: 51.2, 40.9; 50000 x 512, 512 gradients, 328, 153.)
+    // Tiles that give every SM two CTAs keep all weight rows in one part, which stores its tile: the same bits on every
+    // run. Fewer tiles: as many parts as make the waves of CTAs (one per SM) take the fewest stages, kStart of them for a
+    // CTA's start and its store, at least four stages per CTA. (Parts doubled until the grid covered the GPU twice, then
+    // so, us with the conversion of the gradients: 6912 x 1152, 512 gradients, eight parts of 7 stages and four of 14:
+    // 51.2, 40.9; 50000 x 512, 512 gradients, 328, 153.)
     constexpr uint32_t kStart = 4;
+    const bool may_split = quads * mt < (uint32_t)sm_count() * 2 && n_chunks >= 8;
     uint32_t splits = 1;
     uint64_t best = ~0ull;
-    for (uint32_t s = 1; s <= 64 && (s == 1 || n_chunks / s >= 4); ++s) {
+    for (uint32_t s = 1; may_split && s <= 64 && n_chunks / s >= 4; ++s) {
         const uint64_t waves = ((uint64_t)quads * mt * s + sm_count() - 1) / sm_count();
         const uint64_t cost = waves * ((n_chunks + s - 1) / s + kStart);
         if (cost < best) {
