@@ -407,6 +407,21 @@ def test_matmul_transposed_in_one_part_adds_its_whole_sum(zq):
     assert torch.equal(zq.quant_matmul_transposed(go, qw, grad_x=base.clone(), accumulate=True), base + got)
 
 
+@pytest.mark.parametrize("out_dim,in_dim,m", [(50000, 512, 512), (20000, 1024, 256), (6912, 1152, 512), (4104, 64, 40)])
+def test_matmul_transposed_in_parts_sums_in_f32(zq, out_dim, in_dim, m):
+    """Weights and gradients that fp16 holds exactly: what is left is the summation. Chains of 32 MMAs (512 products, each
+    MMA cut to 2^-23 of the sum at most), added in f32: below 32 * 2^-23 = 3.8e-6."""
+    g = torch.Generator(device="cuda").manual_seed(13)
+    q = torch.randint(-127, 128, (out_dim * in_dim // 32, 32), generator=g, device="cuda", dtype=torch.int8)
+    scale = torch.full((q.shape[0], 1), 2.0 ** -10, dtype=torch.float16, device="cuda")
+    raw = torch.cat([scale.view(torch.uint8), q.view(torch.uint8)], dim=1).reshape(-1)
+    qw = zq.QuantWeight(raw, ggml.Q8_0, out_dim, in_dim)
+    go = torch.randn(m, out_dim, generator=g, device="cuda").half().float()
+    want = go.double() @ (q.reshape(out_dim, in_dim).double() * 2.0 ** -10)
+    got = zq.quant_matmul_transposed(go, qw).double()
+    assert float((got - want).norm() / want.norm()) <= 3.8e-6
+
+
 def test_quant_matmul_backward_to_activations(zq, oracle):
     """quant_matmul_no_grad on an input that requires grad carries the backward to x (the weight stays
     frozen): d/dx sum(y * c) = c . W."""

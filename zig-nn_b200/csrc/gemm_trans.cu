@@ -11,7 +11,9 @@
 // Weights and gradients are each rounded once to fp16: about 3e-4 relative L2 against the f32 statement.
 //
 // A matrix with few 128-column tiles (K = 1152 has nine) would leave most SMs idle, so the weight rows
-// can be split over blockIdx.z; the partial tiles then meet in grad_x through red.global.add.f32.
+// can be split over blockIdx.z; the partial tiles then meet in grad_x through red.global.add.f32. The sums inside the
+// MMA accumulators are coarser than f32 additions, so a product whose rows may be split adds them up in f32 every
+// kChain stages: as short a chain as the finest split leaves, whatever the split.
 #include "gemm_common.cuh"
 
 namespace zq {
@@ -24,6 +26,7 @@ constexpr int TK = 128;       // output columns per CTA: one quad of blocks
 constexpr int TJ = 128;       // weight rows (contraction) per stage
 constexpr int STAGES = 3;
 constexpr int THREADS = 256;
+constexpr uint32_t kChain = 4;    // stages whose sum stays inside the accumulators of a product that may be split
 constexpr uint32_t STAGE_BYTES = 4 * HALF_TILE;  // W tile (k halves 0 / 1), grad_out tile (j halves 0 / 1)
 
 enum StoreMode { STORE = 0, ADD = 1, ATOMIC_ADD = 2 };
@@ -36,7 +39,7 @@ template <int TYPE>
 __global__ void __launch_bounds__(THREADS, 1)
 gemm_trans_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc, const __half* __restrict__ g16,
                   const float* __restrict__ post, float* __restrict__ gx, uint32_t N, uint32_t K, uint32_t M,
-                  uint32_t nbp, uint32_t scp, uint32_t chunks_per_split, int mode) {
+                  uint32_t nbp, uint32_t scp, uint32_t chunks_per_split, int mode, bool fold) {
     constexpr bool Q8 = TYPE == ZQ_TYPE_Q8_0;
     constexpr bool Q41 = TYPE == ZQ_TYPE_Q4_1;
     constexpr uint32_t QB = Q8 ? 32 : 16;
@@ -79,11 +82,24 @@ gemm_trans_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc
 
     // consumer role: warp grid 4 (m) x 2 (k); warp tile 32 x 64
     const uint32_t wm = warp & 3, wk = warp >> 2;
-    float acc[2][8][4];
+    float acc[2][8][4], sum[2][8][4];
 #pragma unroll
     for (int i = 0; i < 2; ++i)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) acc[i][j][0] = acc[i][j][1] = acc[i][j][2] = acc[i][j][3] = 0.0f;
+        for (int j = 0; j < 8; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[i][j][e] = sum[i][j][e] = 0.0f;
+    auto fold_sums = [&] {
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) {
+                    sum[i][j][e] += acc[i][j][e];
+                    acc[i][j][e] = 0.0f;
+                }
+    };
 
     // A (grad_out) matrices: (rows 0-7 | 8-15) x (j 0-7 | 8-15). B (weights, transposed on load): matrices
     // (j 0-7, k 0-7), (j 8-15, k 0-7), (j 0-7, k 8-15), (j 8-15, k 8-15): lane l supplies row l % 16 of the
@@ -132,7 +148,17 @@ gemm_trans_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc
                 }
             }
         }
+        if (fold && s % kChain == kChain - 1) fold_sums();
         __syncthreads();  // this stage may be overwritten by the stores / copies of the next iteration
+    }
+    if (fold) {
+        fold_sums();
+#pragma unroll
+        for (int i = 0; i < 2; ++i)
+#pragma unroll
+            for (int j = 0; j < 8; ++j)
+#pragma unroll
+                for (int e = 0; e < 4; ++e) acc[i][j][e] = sum[i][j][e];
     }
 
     // acc[i][j]: rows m (g, g + 8), columns k (2t, 2t + 1)
@@ -199,7 +225,7 @@ int launch_trans(const zq_weight* w, const __half* g16, const float* post, float
         if (!accumulate) ZQ_CUDA(cudaMemsetAsync(gx, 0, (size_t)M * w->in_dim * sizeof(float), st));
     }
     kern<<<dim3(quads, mt, splits), THREADS, smem, st>>>(w->qs, static_cast<const uint8_t*>(w->sc), g16, post, gx,
-                                                          w->out_dim, w->in_dim, M, w->nbp, w->scp, per, mode);
+                                                          w->out_dim, w->in_dim, M, w->nbp, w->scp, per, mode, may_split);
     ZQ_LAUNCH_CHECK();
     return ZQ_OK;
 }
