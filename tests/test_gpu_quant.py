@@ -3,6 +3,8 @@
 Bars: dequantised weights bit-exact; Q8-activation outputs bit-exact; f32-activation outputs
 rel-L2 <= 1e-3 (the stated bar) — and <= 2e-6 as an implementation guard, since both sides
 compute in f32."""
+import threading
+
 import numpy as np
 import pytest
 import torch
@@ -121,6 +123,35 @@ def test_split_product_keeps_f32_accuracy(zq, oracle, qtype, m, n, k):
     want = x.astype(np.float64) @ oracle.dequantize(qtype, raw, n * k).reshape(n, k).astype(np.float64).T + bias + res
     for r in range(m):  # 22 bits of every activation, f32 sums of up to 216 blocks: below 2^-24 * (4 + sqrt(216)) of a row
         assert rel_l2(got[r], want[r]) <= 1.2e-6, r
+
+
+def test_weights_of_different_depth_on_two_threads(zq):
+    """A kernel's limit of shared memory is the process's: a shallow weight's call on one thread must not lower it under a
+    deep weight's launch on another."""
+    from zignn_b200 import _lib
+    lib, failed = _lib.load(), []
+
+    def calls(k):
+        stream = torch.cuda.Stream()
+        with torch.cuda.stream(stream):
+            qw = zq.QuantWeight(ggml.quantize(ggml.Q8_0, torch.ones(64, k)).numpy(), ggml.Q8_0, 64, k)
+            x, y = torch.ones(16, k, device="cuda"), torch.empty(16, 64, device="cuda")
+            need = qw.workspace_bytes(16, zq.ACT_Q8)
+            ws = torch.empty(need, dtype=torch.uint8, device="cuda")
+        args = (qw.handle, x.data_ptr(), y.data_ptr(), 16, zq.ACT_Q8, None, ws.data_ptr(), need, stream.cuda_stream)
+        for _ in range(30000):
+            status = lib.zq_matmul(*args)
+            if status:
+                failed.append((k, status, lib.zq_last_cuda_error()))
+                break
+        stream.synchronize()
+
+    threads = [threading.Thread(target=calls, args=(k,)) for k in (1152, 6912)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not failed, failed
 
 
 REL_L2_GEMM_GUARD = 6e-4  # fp16 operands (weights and activations each rounded once, <= 2^-12 relative)

@@ -275,6 +275,8 @@ attention_prefill_kernel(PrefillArgs a) {
     }
 }
 
+constexpr size_t kMostSmem = 227 * 1024;  // of a CTA
+
 uint32_t pitch_of(uint32_t span) { return (span + kKeys - 1) / kKeys * kKeys + 4; }
 
 template <int HD, int ROWS>
@@ -287,9 +289,10 @@ int launch_rows(PrefillArgs a, uint32_t end, cudaStream_t st) {
     const uint32_t span = a.window && end > a.window + ROWS ? a.window + ROWS : end;  // positions that a CTA may see
     a.pitch = pitch_of(span);
     const size_t smem = prefill_smem<HD, ROWS>(a.pitch);
-    if (smem > 227 * 1024) return ZQ_ERR_LIMIT;
+    if (smem > kMostSmem) return ZQ_ERR_LIMIT;
     auto kern = attention_prefill_kernel<HD, ROWS>;
-    ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // the most that any prompt asks for: the limit is the process's, and another thread may be about to launch a longer one
+    ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMostSmem));
     ZQ_CUDA(launch_pdl(kern, dim3((a.rows + ROWS - 1) / ROWS, a.n_head), dim3(PrefillShape<HD, ROWS>::kThreads), smem, st, a));
     return ZQ_OK;
 }
@@ -308,10 +311,10 @@ int launch_hd(const PrefillArgs& a, uint32_t end, cudaStream_t st) {
 bool attention_prefill_takes(uint32_t head_dim, uint32_t ctx) {
     const uint32_t pitch = pitch_of(ctx);
     switch (head_dim) {
-        case 32: return prefill_smem<32, 16>(pitch) <= 227 * 1024;
-        case 64: return prefill_smem<64, 16>(pitch) <= 227 * 1024;
-        case 128: return prefill_smem<128, 16>(pitch) <= 227 * 1024;
-        case 256: return prefill_smem<256, 16>(pitch) <= 227 * 1024;
+        case 32: return prefill_smem<32, 16>(pitch) <= kMostSmem;
+        case 64: return prefill_smem<64, 16>(pitch) <= kMostSmem;
+        case 128: return prefill_smem<128, 16>(pitch) <= kMostSmem;
+        case 256: return prefill_smem<256, 16>(pitch) <= kMostSmem;
         default: return false;
     }
 }

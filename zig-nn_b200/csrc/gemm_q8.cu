@@ -462,7 +462,8 @@ int launch_terms(const zq_weight* w, const int8_t* xq, const float* xs, const in
     if (grid.y > 65535u) return ZQ_ERR_LIMIT;
     auto kern = gemm_q8_terms_kernel<TYPE, NTL, WIDE>;
     const size_t smem = (size_t)per * kBlockBytes;
-    ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    // the most that any call asks for: the limit is the process's, and another thread may be about to launch a deeper matrix
+    ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kMost * kBlockBytes)));
     ZQ_CUDA(launch_pdl_split(split, kern, grid, dim3(kTermWarps * 32), smem, st, w->qs,
                        static_cast<const uint8_t*>(w->sc), xq, xs, xsum, y, w->out_dim, w->in_dim, M, w->nb, w->scp, per, ep));
     return ZQ_OK;
