@@ -358,6 +358,27 @@ def test_gpt2_persistent_decode_kernel_against_the_launch_sequence(zq, qtype):
     assert _lib.device_error(clear=False) == 0
 
 
+@pytest.mark.parametrize("kind", ["gpt2", "gemma3"])
+def test_engines_of_different_sizes_side_by_side(zq, kind):
+    """A smaller model's engine must not lower the persistent kernel's limit of shared memory under a larger one's steps."""
+    if kind == "gpt2":
+        make = lambda cfg: zq.Gpt2(hostmodel.Gpt2Host.synthetic(cfg, qtype=ggml.Q4_0, seed=5).randomize_small_params())
+        tiny, big = GPT2_TINY, dict(hostmodel.GPT2_SMALL, vocab=1000, layer=1)
+    else:
+        make = lambda cfg: zq.Gemma3(hostmodel.Gemma3Host.synthetic(cfg, qtype=ggml.Q8_0, seed=5).randomize_small_params())
+        tiny, big = GEMMA_TINY, dict(hostmodel.GEMMA3_1B, vocab=2048, layer=1)
+    for first, second in ((big, tiny), (tiny, big)):
+        a = make(first)
+        assert a.decode_mode == zq.DECODE_PERSISTENT
+        a.prefill([1, 2, 3])
+        want = a.decode_next(4)
+        b = make(second)
+        b.prefill([1, 2, 3])
+        b.decode_next(4)
+        a.prefill([1, 2, 3])
+        assert torch.equal(a.decode_next(4), want)
+
+
 def test_gpt2_persistent_decode_kernel_full_size_greedy(zq):
     """GPT-2 small, Q4_0: 128 greedy tokens from the on-device loop of the persistent kernel equal those of the
     launch sequence (the workload of the decode benchmark)."""

@@ -1518,7 +1518,7 @@ int gemma_decoder_create(const GemmaDecoderDesc& desc, GemmaDecoder** out) {
     d->smem = off + (size_t)n_slots * slot_bytes;
 
     d->grid = grid;
-    cudaError_t e = cudaFuncSetAttribute(gemma3_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d->smem);
+    cudaError_t e = cudaFuncSetAttribute(gemma3_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
     int per_sm = 0;
     if (e == cudaSuccess)
         e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gemma3_decode_kernel, kThreads, d->smem);

@@ -1047,7 +1047,7 @@ int gpt_decoder_create(const GptDecoderDesc& desc, GptDecoder** out) {
     p.slot_bytes = slot_bytes;
     d->smem = off + (size_t)n_slots * slot_bytes;
     d->grid = grid;
-    cudaError_t e = cudaFuncSetAttribute(gpt2_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)d->smem);
+    cudaError_t e = cudaFuncSetAttribute(gpt2_decode_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)budget);
     int per_sm = 0;
     if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, gpt2_decode_kernel, kThreads, d->smem);
     if (e != cudaSuccess || per_sm < 1) {

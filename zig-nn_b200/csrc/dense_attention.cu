@@ -519,20 +519,22 @@ int tiles_launch(AttnArgs& a, bool one_sequence, cudaStream_t st) {
     const GqaShape& s = a.s;
     const uint32_t R = s.heads / s.kv_heads;
     const uint32_t tile = kTile * (s.dimp + 8 + s.vdimp + 8) * 2;
+    constexpr uint32_t kMostTile = kTile * (256 + 8 + 256 + 8) * 2;
     if (one_sequence && a.rows > 1) {
         // more than one of the small kernel's tiles: the tensor cores (their copies want 128-byte cache rows)
         if (a.rows * R > 64 && s.kv_heads * s.dimp >= 64 && s.kv_heads * s.vdimp >= 64) {
             const int rc = launch_gqa_prefill_tc(s, a.q, a.kc, a.vc, a.out, a.out_pitch, a.scale2, a.slots, a.rows, a.pos0, st);
             if (rc != ZQ_ERR_UNSUPPORTED) return rc;
         }
-        ZQ_CUDA(cudaFuncSetAttribute(gqa_prefill_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * tile));
+        ZQ_CUDA(cudaFuncSetAttribute(gqa_prefill_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kMostTile));
         return done(launch_pdl(gqa_prefill_kernel<D>, dim3((a.rows * R + 63) / 64, s.kv_heads), dim3(128), 2 * tile, st, a));
     }
     uint32_t smem = kDecodeStages * tile + (17 * s.dimp + s.vdimp) * 2;
     const uint32_t meet = (4 * 16 * 2 + 4 * 16 * s.vdimp) * 4;
     if (smem < meet) smem = meet;
     a.splits = decode_splits(s);
-    ZQ_CUDA(cudaFuncSetAttribute(gqa_decode_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    ZQ_CUDA(cudaFuncSetAttribute(gqa_decode_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 kDecodeStages * kMostTile + 18 * 256 * 2));
     int rc = done(launch_pdl(gqa_decode_kernel<D>, dim3(a.splits, s.kv_heads * ((R + 15) / 16), a.rows), dim3(128), smem, st, a));
     if (rc != ZQ_OK || a.splits == 1) return rc;
     return done(launch_pdl(gqa_combine_kernel, dim3(s.heads, a.rows), dim3(s.vdim >= 256 ? 256 : pad_to(s.vdim, 32)), 0, st, a));

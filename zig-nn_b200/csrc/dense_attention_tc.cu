@@ -360,7 +360,8 @@ int launch_gqa_prefill_tc(const GqaShape& s, const bf16* q, const bf16* kc, cons
     if ((rc = tensor_map_2d(kc, (uint64_t)s.kv_heads * s.dimp * 2, cache_rows, 128, AT_KEYS, 128, &mk)) != ZQ_OK) return rc;
     if ((rc = tensor_map_2d(vc, (uint64_t)s.kv_heads * s.vdimp * 2, cache_rows, 128, AT_KEYS, 128, &mv)) != ZQ_OK) return rc;
     const uint32_t smem = p.dk * AT_QATOM + 2 * (p.dk + p.dv) * AT_ATOM + 2 * AT_QATOM + 1024;
-    ZQ_CUDA(cudaFuncSetAttribute(gqa_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ZQ_CUDA(cudaFuncSetAttribute(gqa_prefill_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 4 * AT_QATOM + 2 * (4 + 4) * AT_ATOM + 2 * AT_QATOM + 1024));
     const uint32_t R = s.heads / s.kv_heads;
     const cudaError_t e = launch_pdl(gqa_prefill_tc_kernel, dim3((rows * R + 127) / 128, s.kv_heads), dim3(AT_THREADS), smem, st,
                                      mk, mv, p);

@@ -372,14 +372,15 @@ __device__ __forceinline__ void put_split_pair(unsigned char* image, uint32_t at
 }
 inline int chunk_scan_launch(ChunkParams p, bool delta, cudaStream_t st) {
     const uint32_t stage = p.image_bytes + kValueBytes;
-    p.stages = 224 * 1024 / stage;
+    constexpr uint32_t kMost = 224 * 1024;
+    p.stages = kMost / stage;
     if (p.stages > kChunkStages) p.stages = kChunkStages;
     if (p.stages < 2) return ZQ_ERR_LIMIT;
     const uint32_t smem = p.stages * stage;
     int rc = device_error_word(&p.err);
     if (rc != ZQ_OK) return rc;
     auto go = [&](auto kern) {
-        ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
         const cudaError_t e = launch_pdl(kern, dim3(p.heads, p.blocks), dim3(160), smem, st, p);
         return e == cudaSuccess ? ZQ_OK : cuda_fail(e);
     };

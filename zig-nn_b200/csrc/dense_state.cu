@@ -978,8 +978,9 @@ int done(cudaError_t e) { return e == cudaSuccess ? ZQ_OK : cuda_fail(e); }
 
 template <typename K>
 int allow_smem(K kern, size_t smem) {
-    if (smem > 220 * 1024) return ZQ_ERR_LIMIT;
-    if (smem > 48 * 1024) ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr size_t kMost = 220 * 1024;
+    if (smem > kMost) return ZQ_ERR_LIMIT;
+    if (smem > 48 * 1024) ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
     return ZQ_OK;
 }
 

@@ -377,8 +377,9 @@ int done(cudaError_t e) { return e == cudaSuccess ? ZQ_OK : cuda_fail(e); }
 
 template <typename K>
 int wkv_smem(K kern, size_t smem) {
-    if (smem > 220 * 1024) return ZQ_ERR_LIMIT;
-    if (smem > 48 * 1024) ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr size_t kMost = 220 * 1024;
+    if (smem > kMost) return ZQ_ERR_LIMIT;
+    if (smem > 48 * 1024) ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
     return ZQ_OK;
 }
 
@@ -439,9 +440,10 @@ int launch_wkv(const WkvArgs& a, uint32_t rows, bool one_sequence, bool f32, cud
     p.n_chunks = (rows + p.chunk_len - 1) / p.chunk_len;
     if (!p.per_row) {
         const size_t smem = (kDecayTokens + 65) * (size_t)a.rank * sizeof(float);
-        if (smem > 200 * 1024) return ZQ_ERR_LIMIT;
+        constexpr size_t kMost = 200 * 1024;
+        if (smem > kMost) return ZQ_ERR_LIMIT;
         if (smem > 48 * 1024)
-            ZQ_CUDA(cudaFuncSetAttribute(wkv_decay_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            ZQ_CUDA(cudaFuncSetAttribute(wkv_decay_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
         const dim3 grid((a.heads * a.dim + 63) / 64, (rows + kDecayTokens - 1) / kDecayTokens);
         int rc = done(launch_pdl(wkv_decay_kernel, grid, dim3(256), smem, st, p));
         if (rc != ZQ_OK) return rc;

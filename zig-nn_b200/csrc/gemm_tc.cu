@@ -1207,7 +1207,7 @@ int launch_stream_tn(const zq_weight* w, const __half* xt, const float* post, fl
         if (n_chunk_ring > (uint32_t)TS_MAX_CHUNKS) n_chunk_ring = TS_MAX_CHUNKS;
     }
     const size_t smem = (size_t)n_ring * W_STAGE + bring_bytes + (size_t)n_chunk_ring * CHUNK_BYTES + 1024;
-    ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(budget + 1024u)));
     const uint32_t row_tiles = (w->out_dim + TN - 1) / TN;
     const uint64_t tiles_total = (uint64_t)row_tiles * m_tiles;
     const uint32_t sms = (uint32_t)sm_count();
@@ -1264,7 +1264,7 @@ int launch_stream_pair(const zq_weight* w, const __half* xt, const float* post, 
     if (n_ring < 2) return ZQ_ERR_UNSUPPORTED;
     const uint32_t n_bring = 2u * n_ring;
     const size_t smem = (size_t)n_ring * W_STAGE + (size_t)n_bring * btile_bytes + (size_t)n_chunk_ring * CHUNK_BYTES + 1024;
-    ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(budget + 1024u)));
     const uint64_t tiles_whole = (uint64_t)((w->out_dim + 255u) / 256u) * m_tiles;
     if (tiles_whole > 0x7FFFFFFFu) return ZQ_ERR_LIMIT;
     const uint32_t pairs_max = (uint32_t)sm_count() / 2u;
@@ -1493,7 +1493,7 @@ int launch_trans_pair(const zq_weight* w, const float* grad_out, float* grad_x, 
     if (n_ring < 2) return ZQ_ERR_UNSUPPORTED;
     const uint32_t n_bring = 2u * n_ring;
     const size_t smem = (size_t)n_ring * W_STAGE + (size_t)n_bring * btile_bytes + 1024;
-    ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(budget + 1024u)));
     const uint64_t tiles_whole = (uint64_t)(rows_pad / 256u) * m_tiles;
     if (tiles_whole > 0x7FFFFFFFu) return ZQ_ERR_LIMIT;
     const uint32_t pairs_max = (uint32_t)sm_count() / 2u;

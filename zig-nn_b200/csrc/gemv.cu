@@ -369,18 +369,16 @@ EpilogueArgs make_ep(const zq_epilogue* ep, size_t row_offset_elems) {
 }
 
 template <typename K>
-int set_smem(K kernel, size_t bytes) {
-    if (bytes > 48 * 1024) {
-        if (bytes > 227 * 1024) return ZQ_ERR_LIMIT;
-        ZQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
-    }
+int set_smem(K kernel, size_t bytes, size_t most) {
+    if (bytes > most) return ZQ_ERR_LIMIT;
+    if (bytes > 48 * 1024) ZQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)most));
     return ZQ_OK;
 }
 
 template <int TYPE, int G, int R>
 int launch_f32_one(const zq_weight* w, const float* x, float* y, EpilogueArgs ep, cudaStream_t st) {
     const size_t smem = ((size_t)w->nb * XPAD + w->nb) * sizeof(float);
-    int rc = set_smem(gemv_f32_kernel<TYPE, G, R>, smem);
+    int rc = set_smem(gemv_f32_kernel<TYPE, G, R>, smem, 227 * 1024);
     if (rc != ZQ_OK) return rc;
     const uint32_t rows_per_cta = kWarps * (32 / G) * R;
     const uint64_t tiles = ((uint64_t)w->out_dim + rows_per_cta - 1) / rows_per_cta;
@@ -445,7 +443,7 @@ int launch_quantize_rows_q8(const float* x, uint32_t m_rows, uint32_t in_dim, in
 int launch_matvec_ln_f32(const float* w, const float* x, float* y, uint32_t out_dim, uint32_t in_dim,
                          const float* ln_gamma, const float* ln_beta, float ln_eps, cudaStream_t st) {
     const size_t smem = (size_t)in_dim * sizeof(float);
-    int rc = set_smem(matvec_f32_kernel, smem);
+    int rc = set_smem(matvec_f32_kernel, smem, 227 * 1024 - 10 * sizeof(float));  // and its static array
     if (rc != ZQ_OK) return rc;
     const uint64_t tiles = ((uint64_t)out_dim + 7) / 8;
     const uint64_t cap = (uint64_t)sm_count() * 8;

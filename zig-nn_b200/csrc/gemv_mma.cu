@@ -1129,10 +1129,11 @@ int launch_rows1_cfg(const zq_weight* w, const float* x, float* y, EpilogueArgs 
     smem = (smem + 127) & ~(size_t)127;
     const uint32_t ring_off = (uint32_t)smem;
     smem += (size_t)W * D * (Q8 ? 2048 : 1024);
-    if (smem > (size_t)(227 * 1024) / CTAS - 1024) return ZQ_ERR_LIMIT;  // CTAS CTAs per SM must fit
+    constexpr size_t kMost = (size_t)(227 * 1024) / CTAS - 1024;  // CTAS CTAs per SM must fit
+    if (smem > kMost) return ZQ_ERR_LIMIT;
     auto kern = gemv_mma1_kernel<TYPE, D, CTAS, W, ARGMAX>;
     if (smem > 48 * 1024)
-        ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
     const uint32_t cta_tiles = (w->out_dim + W * 16 - 1) / (W * 16);
     const uint32_t cap = sms * CTAS;
     ZQ_CUDA(launch_pdl(kern, dim3(cta_tiles < cap ? cta_tiles : cap), dim3(W * 32), smem, st, w->qs,
@@ -1173,6 +1174,8 @@ int launch_rows1_any(const zq_weight* w, const float* x, float* y, EpilogueArgs 
     }
 }
 
+constexpr size_t kPlanMostSmem = 200 * 1024;
+
 struct Plan {
     uint32_t WR, KS, grid, ring_off, warps;
     size_t smem;
@@ -1210,7 +1213,7 @@ Plan make_plan(const zq_weight* w, uint32_t M, int ns, bool use_ring, bool with_
     const size_t depth = q8 ? Ring<true, false>::kDepth : Ring<false, false>::kDepth;
     if (use_ring) smem += (size_t)p.WR * ks * depth * stage;
     p.smem = smem;
-    p.fits = smem <= 200 * 1024;
+    p.fits = smem <= kPlanMostSmem;
     const uint32_t cta_tiles = (tiles + p.WR - 1) / p.WR;
     uint32_t per_sm = (uint32_t)((224 * 1024) / (smem + 1024));
     if (per_sm > (uint32_t)kCtasPerSm) per_sm = kCtasPerSm;  // register budget set by the launch bounds
@@ -1226,7 +1229,7 @@ int launch_kernel(const zq_weight* w, const float* x, float* y, uint32_t M, Epil
     if (!p.fits) return ZQ_ERR_LIMIT;
     auto kern = gemv_mma_kernel<TYPE, NS, USE_RING>;
     if (p.smem > 48 * 1024)
-        ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)p.smem));
+        ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPlanMostSmem));
     ZQ_CUDA(launch_pdl(kern, dim3(p.grid), dim3(p.warps * 32), p.smem, st, w->qs,
                        static_cast<const uint8_t*>(w->sc), x, y, w->out_dim, w->in_dim, w->nb, w->scp, M, p.WR, p.KS,
                        p.ring_off, ep));

@@ -435,10 +435,11 @@ int launch_rows(const zq_weight* w, const int8_t* xq, const float* xs, const int
     smem = (smem + 127) & ~(size_t)127;
     const uint32_t ring_off = (uint32_t)smem;
     smem += (size_t)kRowsWarps * kRowsDepth * (Q8 ? 2048 : 1024);
-    if (smem > (size_t)(227 * 1024) / 2 - 1024) return ZQ_ERR_LIMIT;  // two CTAs per SM
+    constexpr size_t kMost = (size_t)(227 * 1024) / 2 - 1024;  // two CTAs per SM
+    if (smem > kMost) return ZQ_ERR_LIMIT;
     auto kern = gemv_q8_rows_kernel<TYPE>;
     if (smem > 48 * 1024)
-        ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
     const uint32_t cta_tiles = (w->out_dim + kRowsWarps * 16 - 1) / (kRowsWarps * 16);
     const uint32_t cap = sms * 2;
     ZQ_CUDA(launch_pdl(kern, dim3(cta_tiles < cap ? cta_tiles : cap), dim3(kRowsWarps * 32), smem, st, w->qs,
@@ -468,10 +469,11 @@ int launch_one(const zq_weight* w, const int8_t* xq, const float* xs, const int3
     auto smem_for = [&](uint32_t r) { return fixed + (size_t)r * 16 * (w->nbp + 1) * sizeof(float); };
     while (wr > 1 && smem_for(wr) > 96 * 1024) wr /= 2;
     const size_t smem = smem_for(wr);
-    if (smem > 200 * 1024) return ZQ_ERR_LIMIT;
+    constexpr size_t kMost = 200 * 1024;
+    if (smem > kMost) return ZQ_ERR_LIMIT;
     auto kern = gemv_q8_kernel<TYPE>;
     if (smem > 48 * 1024)
-        ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
     const uint32_t cta_tiles = (tiles + wr - 1) / wr;
     uint32_t per_sm = (uint32_t)((200 * 1024) / (smem + 1024));
     if (per_sm > 4) per_sm = 4;

@@ -848,7 +848,8 @@ int launch_attention_step(const float* q, float* kc, float* vc, const float* k_n
                           uint32_t max_len, int flags, uint32_t rows, uint32_t q_stride, const uint32_t* row_pos,
                           size_t cache_stride, const float* q_norm_w, const float* k_norm_w, const float* freqs,
                           float norm_eps, cudaStream_t st) {
-    if (max_len == 0 || max_len > 180 * 1024 / 4) return ZQ_ERR_LIMIT;
+    constexpr size_t kMostScores = 180 * 1024;
+    if (max_len == 0 || max_len > kMostScores / 4) return ZQ_ERR_LIMIT;
     if (oq && head_dim % 32) return ZQ_ERR_BAD_ARG;
     if (rows == 0) return ZQ_OK;
     // new keys are taken from the caller's rows only when no row needs another row's key: one row, or
@@ -876,14 +877,14 @@ int launch_attention_step(const float* q, float* kc, float* vc, const float* k_n
     if (oq) {
         auto kern = attention_softmax_v_step_kernel<true>;
         if (smem > 24 * 1024)  // the kernel also holds a 16 KB static tile
-            ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMostScores));
         ZQ_CUDA(launch_pdl_split(split, kern, grid, dim3(256), smem, st, static_cast<const float*>(scores),
                            static_cast<const float*>(vc), out, oq, oscale, osum, n_head, n_kv_head, head_dim, state,
                            window, tail, scores_stride, row_pos, cache_stride));
     } else {
         auto kern = attention_softmax_v_step_kernel<false>;
         if (smem > 24 * 1024)
-            ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+            ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMostScores));
         ZQ_CUDA(launch_pdl_split(split, kern, grid, dim3(256), smem, st, static_cast<const float*>(scores),
                            static_cast<const float*>(vc), out, nullptr, nullptr, nullptr, n_head, n_kv_head, head_dim,
                            state, window, tail, scores_stride, row_pos, cache_stride));
