@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 import torch
 
-from zignn_b200 import ggml
+from zignn_b200 import ggml, hostmodel
 
 pytestmark = pytest.mark.gpu
 
@@ -260,6 +260,17 @@ def test_many_rows_without_workspace_is_refused(zq, oracle):
     rc = lib.zq_matmul(qw.handle, C.c_void_p(x.data_ptr()), C.c_void_p(y.data_ptr()), 48, zq.ACT_F32, C.byref(ep), None, 0,
                        stream())
     assert rc == 0
+
+
+def test_refused_allocation_is_not_reported_again(zq):
+    """An engine whose caches do not fit is refused; the next call must not report that error as its own."""
+    cfg = dict(vocab=64, embed=64, head=4, head_kv=4, head_dim=512, layer=1, ctx=46080, ffn=64, rope_base=1e4, sliding_window=16,
+               rms_eps=1e-6, global_every=1)
+    host = hostmodel.Gemma3Host.synthetic(cfg, qtype=ggml.Q8_0, seed=1).randomize_small_params()
+    with pytest.raises(RuntimeError, match="NO_MEM"):
+        zq.Gemma3Batch(host, 1024)  # 386 GB to a cache
+    qw = zq.QuantWeight(ggml.quantize(ggml.Q4_0, torch.ones(64, 64)).numpy(), ggml.Q4_0, 64, 64)
+    assert bool((zq.quant_matmul_transposed(torch.ones(2, 64, device="cuda"), qw) == 64.0).all())
 
 
 @pytest.mark.parametrize("m", [1, 64])

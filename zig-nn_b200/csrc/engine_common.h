@@ -18,10 +18,7 @@ struct DeviceArena {
     }
     int alloc(void** out, size_t bytes) {
         cudaError_t e = cudaMalloc(out, bytes ? bytes : 4);
-        if (e != cudaSuccess) {
-            g_last_cuda_error = (int)e;
-            return e == cudaErrorMemoryAllocation ? ZQ_ERR_NO_MEM : ZQ_ERR_CUDA;
-        }
+        if (e != cudaSuccess) return alloc_fail(e);
         ptrs.push_back(*out);
         total += bytes;
         return ZQ_OK;

@@ -156,8 +156,7 @@ int make_weight(int type, uint32_t out_dim, uint32_t in_dim, zq_weight** out) {
     cudaError_t e = cudaMalloc(&w->base, w->bytes);
     if (e != cudaSuccess) {
         delete w;
-        g_last_cuda_error = (int)e;
-        return e == cudaErrorMemoryAllocation ? ZQ_ERR_NO_MEM : ZQ_ERR_CUDA;
+        return alloc_fail(e);
     }
     w->qs = static_cast<uint8_t*>(w->base);
     w->sc = w->qs + qs_pad;
@@ -278,10 +277,7 @@ int zq_weight_upload(const void* h_raw, int type, uint32_t out_dim, uint32_t in_
     const size_t raw_bytes = zq_tensor_bytes(type, (size_t)out_dim * in_dim);
     void* staging = nullptr;
     cudaError_t e = cudaMalloc(&staging, raw_bytes);
-    if (e != cudaSuccess) {
-        g_last_cuda_error = (int)e;
-        return e == cudaErrorMemoryAllocation ? ZQ_ERR_NO_MEM : ZQ_ERR_CUDA;
-    }
+    if (e != cudaSuccess) return alloc_fail(e);
     cudaStream_t st = as_stream(stream);
     int rc = ZQ_OK;
     e = cudaMemcpyAsync(staging, h_raw, raw_bytes, cudaMemcpyHostToDevice, st);

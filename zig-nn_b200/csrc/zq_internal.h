@@ -39,9 +39,15 @@ namespace zq {
 
 extern thread_local int g_last_cuda_error;
 
+// Takes the error from the runtime too: left there, the launch check of the next call would report it again.
 inline int cuda_fail(cudaError_t e) {
     g_last_cuda_error = (int)e;
+    cudaGetLastError();
     return ZQ_ERR_CUDA;
+}
+inline int alloc_fail(cudaError_t e) {
+    const int rc = cuda_fail(e);
+    return e == cudaErrorMemoryAllocation ? ZQ_ERR_NO_MEM : rc;
 }
 
 #define ZQ_CUDA(call)                                   \
