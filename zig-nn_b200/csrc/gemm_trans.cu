@@ -107,6 +107,7 @@ gemm_trans_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc
     const uint32_t a_row = wm * 32 + (lane & 15), a_chunk = lane >> 4;
     const uint32_t b_row = lane & 15, b_chunk = lane >> 4;
 
+    fold = fold && nst > kChain;
     load_w(c_lo);
     issue_g(0, c_lo);
     asm volatile("cp.async.commit_group;" ::: "memory");
@@ -204,8 +205,9 @@ int launch_trans(const zq_weight* w, const __half* g16, const float* post, float
     // run. Fewer tiles: as many parts as make the waves of CTAs (one per SM) take the fewest stages, kStart of them for a
     // CTA's start and its store, at least four stages per CTA. (Parts doubled until the grid covered the GPU twice, then
     // so, us with the conversion of the gradients: 6912 x 1152, 512 gradients, eight parts of 7 stages and four of 14:
-    // 51.2, 40.9; 50000 x 512, 512 gradients, 328, 153.)
-    constexpr uint32_t kStart = 4;
+    // 51.2, 40.9; 50000 x 512, 512 gradients, 328, 153. With kStart = 4 a wave that left a quarter of the SMs idle was
+    // taken over three full ones: 5000 x 6912, 16 gradients, two parts 52, eight 47.)
+    constexpr uint32_t kStart = 1;
     const bool may_split = quads * mt < (uint32_t)sm_count() * 2 && n_chunks >= 8;
     uint32_t splits = 1;
     uint64_t best = ~0ull;
