@@ -285,7 +285,7 @@ size_t prefill_smem(uint32_t pitch) {
 }
 
 template <int HD, int ROWS>
-int launch_rows(PrefillArgs a, uint32_t end, cudaStream_t st) {
+int launch_rows(PrefillArgs a, uint32_t end, bool shared_split, cudaStream_t st) {
     const uint32_t span = a.window && end > a.window + ROWS ? a.window + ROWS : end;  // positions that a CTA may see
     a.pitch = pitch_of(span);
     const size_t smem = prefill_smem<HD, ROWS>(a.pitch);
@@ -293,17 +293,18 @@ int launch_rows(PrefillArgs a, uint32_t end, cudaStream_t st) {
     auto kern = attention_prefill_kernel<HD, ROWS>;
     // the most that any prompt asks for: the limit is the process's, and another thread may be about to launch a longer one
     ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMostSmem));
-    ZQ_CUDA(launch_pdl(kern, dim3((a.rows + ROWS - 1) / ROWS, a.n_head), dim3(PrefillShape<HD, ROWS>::kThreads), smem, st, a));
+    ZQ_CUDA(launch_pdl_split(shared_split, kern, dim3((a.rows + ROWS - 1) / ROWS, a.n_head),
+                             dim3(PrefillShape<HD, ROWS>::kThreads), smem, st, a));
     return ZQ_OK;
 }
 
 // Four tokens per CTA while sixteen would leave half of the GPU without one (head_dim 256, 40 tokens of 4 heads: 19.9 us
 // with sixteen, 9.9 us with four).
 template <int HD>
-int launch_hd(const PrefillArgs& a, uint32_t end, cudaStream_t st) {
+int launch_hd(const PrefillArgs& a, uint32_t end, bool shared_split, cudaStream_t st) {
     constexpr int kFew = HD >= 64 ? 4 : 16;
-    if ((a.rows + 15) / 16 * a.n_head * 2 < (uint32_t)sm_count()) return launch_rows<HD, kFew>(a, end, st);
-    return launch_rows<HD, 16>(a, end, st);
+    if ((a.rows + 15) / 16 * a.n_head * 2 < (uint32_t)sm_count()) return launch_rows<HD, kFew>(a, end, shared_split, st);
+    return launch_rows<HD, 16>(a, end, shared_split, st);
 }
 
 }  // namespace
@@ -321,17 +322,18 @@ bool attention_prefill_takes(uint32_t head_dim, uint32_t ctx) {
 
 int launch_attention_prefill(const float* q, const float* kc, const float* vc, float* out, int8_t* oq, float* oscale,
                              int32_t* osum, uint32_t n_head, uint32_t n_kv_head, uint32_t head_dim, const uint32_t* state,
-                             uint32_t window, uint32_t end, int flags, uint32_t rows, uint32_t q_stride, cudaStream_t st) {
+                             uint32_t window, uint32_t end, int flags, uint32_t rows, uint32_t q_stride, cudaStream_t st,
+                             bool shared_split) {
     if (rows == 0) return ZQ_OK;
     const uint32_t kv_dim = n_kv_head * head_dim;
     if (((uintptr_t)q | (uintptr_t)kc | (uintptr_t)vc) & 15 || q_stride % 4 || n_head > 65535u) return ZQ_ERR_LIMIT;
     PrefillArgs a{q, kc, vc, out, oq, oscale, osum, state, n_head, n_head / n_kv_head, kv_dim, rows, window, q_stride, 0,
                   (flags & ZQ_ATTN_GPT2_SOFTMAX) ? 1 : 0};
     switch (head_dim) {
-        case 32: return launch_hd<32>(a, end, st);
-        case 64: return launch_hd<64>(a, end, st);
-        case 128: return launch_hd<128>(a, end, st);
-        case 256: return launch_hd<256>(a, end, st);
+        case 32: return launch_hd<32>(a, end, shared_split, st);
+        case 64: return launch_hd<64>(a, end, shared_split, st);
+        case 128: return launch_hd<128>(a, end, shared_split, st);
+        case 256: return launch_hd<256>(a, end, shared_split, st);
         default: return ZQ_ERR_LIMIT;
     }
 }

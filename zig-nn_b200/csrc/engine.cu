@@ -435,6 +435,7 @@ struct zq_gemma3 {
     uint32_t max_rows = 1;        // rows the activation buffers hold (prefill chunk size, >= n_seq)
     uint32_t chunk = 1;           // tokens of a prefill chunk
     bool prefill_attention = false;  // as in zq_gpt2
+    bool whole_products = true;      // every block has q | k | v and gate | up as one matrix each: a step of several rows has no GEMV
     int32_t* d_arg = nullptr;
     uint32_t* d_record = nullptr;
     uint32_t seq_len = 0;
@@ -447,6 +448,7 @@ struct zq_gemma3 {
     // (decode_gemma.cu); otherwise, and for prefill chunks and batched sequences, as the launch sequence.
     GemmaDecoder* decoder = nullptr;
     int decode_mode = ZQ_DECODE_AUTO;
+    bool shares_split(uint32_t rows) const { return whole_products && step_shares_split(rows); }
     ~zq_gemma3() {
         gemma_decoder_free(decoder);
         zq_weight_free(token_embd);
@@ -467,7 +469,7 @@ struct zq_gemma3 {
 // Activation rows are quantised once (thread_pool.zig:111-114); any number of weights consume them.
 // T rows: one exact GEMV per row, or from five rows up the exact int8 GEMM (identical results).
 static int gemma_linear(zq_gemma3* m, const zq_weight* w, float* y, uint32_t y_stride, uint32_t T, cudaStream_t st) {
-    if (T >= 2 && y_stride == w->out_dim) return launch_gemm_q8(w, m->xq, m->xscale, m->xsum, y, T, nullptr, st, true);
+    if (T >= 2 && y_stride == w->out_dim) return launch_gemm_q8(w, m->xq, m->xscale, m->xsum, y, T, nullptr, st, m->shares_split(T));
     for (uint32_t r = 0; r < T; ++r) {
         int rc = launch_gemv_q8(w, m->xq + (size_t)r * w->in_dim, m->xscale + (size_t)r * w->nb,
                                 m->xsum + (size_t)r * w->nb, y + (size_t)r * y_stride, 1, nullptr, st);
@@ -494,11 +496,12 @@ static int gemma3_forward(zq_gemma3* m, uint32_t T, int variant, cudaStream_t st
     const size_t cache_stride = (size_t)C.ctx * KD;
     const uint32_t* row_pos = batch ? m->d_pos : nullptr;
     const size_t slot = batch ? 0 : seq * cache_stride;
+    const bool split = m->shares_split(T);
     int rc;
     const int32_t* ids = (T == 1 && !batch) ? reinterpret_cast<const int32_t*>(m->d_state) : m->d_tokens;
     if ((rc = zq_dequant_rows_scaled(m->token_embd, ids, T, sqrtf((float)E), m->x, st))) return rc;
     if ((rc = launch_norm_quant(m->x, m->blocks[0].attn_norm_w, nullptr, nullptr, E, C.rms_eps, m->xq,
-                                m->xscale, m->xsum, T, E, st)))
+                                m->xscale, m->xsum, T, E, st, split)))
         return rc;
     for (uint32_t l = 0; l < C.layer; ++l) {
         const zq_gemma3::Block& b = m->blocks[l];
@@ -520,22 +523,22 @@ static int gemma3_forward(zq_gemma3* m, uint32_t T, int variant, cudaStream_t st
         if (!fused_qk) {
             if ((rc = launch_qk_norm_rope_kv(m->qkv, b.q_norm_w, b.k_norm_w, m->freqs, m->k[l] + slot, m->v[l] + slot,
                                              m->d_state, C.head, C.head_kv, D, C.rms_eps, T, QKV, row_pos,
-                                             cache_stride, st)))
+                                             cache_stride, st, split)))
                 return rc;
         }
         if (!fused_qk && m->prefill_attention) {
             if ((rc = launch_attention_prefill(m->qkv, m->k[l] + slot, m->v[l] + slot, nullptr, m->xq, m->xscale, m->xsum,
-                                               C.head, C.head_kv, D, m->d_state, window, pos0 + T, 0, T, QKV, st)))
+                                               C.head, C.head_kv, D, m->d_state, window, pos0 + T, 0, T, QKV, st, split)))
                 return rc;
         } else if ((rc = launch_attention_step(m->qkv, m->k[l] + slot, m->v[l] + slot, fused_qk ? m->qkv + QD : nullptr,
                                         fused_qk ? m->qkv + QD + KD : nullptr, nullptr, m->xq, m->xscale, m->xsum,
                                         m->scores, C.head, C.head_kv, D, m->d_state, window, max_len, 0, T, QKV, row_pos,
                                         cache_stride, fused_qk ? b.q_norm_w : nullptr, b.k_norm_w, m->freqs, C.rms_eps,
-                                        st)))
+                                        st, split)))
             return rc;
         if ((rc = gemma_linear(m, b.o, m->proj, E, T, st))) return rc;
         if ((rc = launch_norm_quant(m->proj, b.post_attn_norm_w, m->x, b.ffn_norm_w, E, C.rms_eps, m->xq,
-                                    m->xscale, m->xsum, T, E, st)))
+                                    m->xscale, m->xsum, T, E, st, split)))
             return rc;
         // FFN block (gemma3.zig:734-773)
         if (b.gate_up) {
@@ -544,13 +547,13 @@ static int gemma3_forward(zq_gemma3* m, uint32_t T, int variant, cudaStream_t st
             if ((rc = gemma_linear(m, b.gate, m->gu, 2 * F, T, st))) return rc;
             if ((rc = gemma_linear(m, b.up, m->gu + F, 2 * F, T, st))) return rc;
         }
-        if ((rc = launch_gelu_mul_quant(m->gu, m->gu + F, F, m->xq, m->xscale, m->xsum, T, 2 * F, st))) return rc;
+        if ((rc = launch_gelu_mul_quant(m->gu, m->gu + F, F, m->xq, m->xscale, m->xsum, T, 2 * F, st, split))) return rc;
         if ((rc = gemma_linear(m, b.down, m->ffn, E, T, st))) return rc;
         const float* next_norm = l + 1 < C.layer ? m->blocks[l + 1].attn_norm_w
                                  : (variant != STEP_CACHE_ONLY ? m->output_norm_w : nullptr);
         if (next_norm) {
             if ((rc = launch_norm_quant(m->ffn, b.post_ffw_norm_w, m->x, next_norm, E, C.rms_eps, m->xq, m->xscale,
-                                        m->xsum, T, E, st)))
+                                        m->xsum, T, E, st, split)))
                 return rc;
         } else if ((rc = zq_rms_norm_residual(m->ffn, b.post_ffw_norm_w, m->x, E, T, C.rms_eps, st))) {
             return rc;
@@ -730,6 +733,7 @@ int zq_gemma3_create_batch(const zq_gemma3_config* cfg, const zq_gemma3_weights*
             TRY(up_q(&b.gate, s.ffn_gate_weight, F, E));
             TRY(up_q(&b.up, s.ffn_up_weight, F, E));
         }
+        m->whole_products = m->whole_products && b.qkv && b.gate_up;
         TRY(up_q(&b.down, s.ffn_down_weight, E, F));
         TRY(m->arena.alloc_n(&m->k[l], (size_t)n_seq * C.ctx * KD));  // one cache slot per sequence
         TRY(m->arena.alloc_n(&m->v[l], (size_t)n_seq * C.ctx * KD));

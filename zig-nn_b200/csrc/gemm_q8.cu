@@ -526,7 +526,6 @@ int launch_one(const zq_weight* w, const int8_t* xq, const float* xs, const int3
 
 int launch_gemm_q8(const zq_weight* w, const int8_t* xq, const float* xscale, const int32_t* xsum, float* y,
                    uint32_t m_rows, const zq_epilogue* ep, cudaStream_t st, bool shared_split) {
-    const bool split = shared_split && m_rows <= kSharedSplitRows;
     QgEpilogue a{nullptr, nullptr, nullptr, 0};
     if (ep) {
         a.bias = ep->d_bias;
@@ -535,9 +534,9 @@ int launch_gemm_q8(const zq_weight* w, const int8_t* xq, const float* xscale, co
         a.residual = ep->d_residual;
     }
     switch (w->type) {
-        case ZQ_TYPE_Q4_0: return launch_one<ZQ_TYPE_Q4_0>(w, xq, xscale, xsum, y, m_rows, a, split, st);
-        case ZQ_TYPE_Q4_1: return launch_one<ZQ_TYPE_Q4_1>(w, xq, xscale, xsum, y, m_rows, a, split, st);
-        case ZQ_TYPE_Q8_0: return launch_one<ZQ_TYPE_Q8_0>(w, xq, xscale, xsum, y, m_rows, a, split, st);
+        case ZQ_TYPE_Q4_0: return launch_one<ZQ_TYPE_Q4_0>(w, xq, xscale, xsum, y, m_rows, a, shared_split, st);
+        case ZQ_TYPE_Q4_1: return launch_one<ZQ_TYPE_Q4_1>(w, xq, xscale, xsum, y, m_rows, a, shared_split, st);
+        case ZQ_TYPE_Q8_0: return launch_one<ZQ_TYPE_Q8_0>(w, xq, xscale, xsum, y, m_rows, a, shared_split, st);
         default: return ZQ_ERR_UNSUPPORTED;
     }
 }

@@ -799,22 +799,22 @@ inline unsigned grid1d(size_t n, unsigned threads) { return (unsigned)((n + thre
 // ---- launchers used by the engines (declared in zq_internal.h) ----------------------------
 
 int launch_norm_quant(const float* src, const float* w1, float* res, const float* w2, uint32_t dim, float eps,
-                      int8_t* q, float* scale, int32_t* sum, uint32_t rows, uint32_t src_stride, cudaStream_t st) {
+                      int8_t* q, float* scale, int32_t* sum, uint32_t rows, uint32_t src_stride, cudaStream_t st,
+                      bool shared_split) {
     if (dim == 0 || dim % 32 || dim > 48 * 1024 / 4) return ZQ_ERR_LIMIT;
     if (rows == 0) return ZQ_OK;
     const size_t smem = dim * sizeof(float);
     cudaError_t e;
     if (dim <= 256 * 5) {
-        const bool split = rows <= kSharedSplitRows;
-        e = res ? launch_pdl_split(split, norm_quant_kernel<true, 5>, dim3(rows), dim3(256), smem, st, src, w1, res, w2, dim,
-                                   eps, q, scale, sum, src_stride)
-                : launch_pdl_split(split, norm_quant_kernel<false, 5>, dim3(rows), dim3(256), smem, st, src, w1, nullptr,
-                                   nullptr, dim, eps, q, scale, sum, src_stride);
+        e = res ? launch_pdl_split(shared_split, norm_quant_kernel<true, 5>, dim3(rows), dim3(256), smem, st, src, w1, res, w2,
+                                   dim, eps, q, scale, sum, src_stride)
+                : launch_pdl_split(shared_split, norm_quant_kernel<false, 5>, dim3(rows), dim3(256), smem, st, src, w1,
+                                   nullptr, nullptr, dim, eps, q, scale, sum, src_stride);
     } else {
-        e = res ? launch_pdl(norm_quant_kernel<true, 0>, dim3(rows), dim3(256), smem, st, src, w1, res, w2, dim, eps, q,
-                             scale, sum, src_stride)
-                : launch_pdl(norm_quant_kernel<false, 0>, dim3(rows), dim3(256), smem, st, src, w1, nullptr, nullptr,
-                             dim, eps, q, scale, sum, src_stride);
+        e = res ? launch_pdl_split(shared_split, norm_quant_kernel<true, 0>, dim3(rows), dim3(256), smem, st, src, w1, res, w2,
+                                   dim, eps, q, scale, sum, src_stride)
+                : launch_pdl_split(shared_split, norm_quant_kernel<false, 0>, dim3(rows), dim3(256), smem, st, src, w1,
+                                   nullptr, nullptr, dim, eps, q, scale, sum, src_stride);
     }
     ZQ_CUDA(e);
     return ZQ_OK;
@@ -823,22 +823,22 @@ int launch_norm_quant(const float* src, const float* w1, float* res, const float
 int launch_qk_norm_rope_kv(float* qkv, const float* q_norm_w, const float* k_norm_w, const float* freqs,
                            float* kc, float* vc, const uint32_t* state, uint32_t n_head, uint32_t n_kv_head,
                            uint32_t head_dim, float eps, uint32_t rows, uint32_t qkv_stride, const uint32_t* row_pos,
-                           size_t cache_stride, cudaStream_t st) {
+                           size_t cache_stride, cudaStream_t st, bool shared_split) {
     if (head_dim % 2 || head_dim > 48 * 1024 / 4) return ZQ_ERR_LIMIT;
     if (rows == 0) return ZQ_OK;
-    ZQ_CUDA(launch_pdl(qk_norm_rope_kv_kernel, dim3(n_head + 2 * n_kv_head, rows), dim3(128), head_dim * sizeof(float),
-                       st, qkv, q_norm_w, k_norm_w, freqs, kc, vc, state, n_head, n_kv_head, head_dim, eps,
-                       qkv_stride, row_pos, cache_stride));
+    ZQ_CUDA(launch_pdl_split(shared_split, qk_norm_rope_kv_kernel, dim3(n_head + 2 * n_kv_head, rows), dim3(128),
+                             head_dim * sizeof(float), st, qkv, q_norm_w, k_norm_w, freqs, kc, vc, state, n_head, n_kv_head,
+                             head_dim, eps, qkv_stride, row_pos, cache_stride));
     return ZQ_OK;
 }
 
 int launch_gelu_mul_quant(const float* gate, const float* up, uint32_t n, int8_t* q, float* scale,
-                          int32_t* sum, uint32_t rows, uint32_t in_stride, cudaStream_t st) {
+                          int32_t* sum, uint32_t rows, uint32_t in_stride, cudaStream_t st, bool shared_split) {
     if (n % 32) return ZQ_ERR_BAD_ARG;
     if (rows == 0) return ZQ_OK;
     const size_t total = (size_t)rows * n;
-    ZQ_CUDA(launch_pdl_split(rows <= kSharedSplitRows, gelu_mul_quant_kernel, dim3(grid1d(total, 256)), dim3(256), 0, st, gate,
-                             up, (uint32_t)(total / 32), q, scale, sum, n / 32, in_stride));
+    ZQ_CUDA(launch_pdl_split(shared_split, gelu_mul_quant_kernel, dim3(grid1d(total, 256)), dim3(256), 0, st, gate, up,
+                             (uint32_t)(total / 32), q, scale, sum, n / 32, in_stride));
     return ZQ_OK;
 }
 
@@ -847,7 +847,7 @@ int launch_attention_step(const float* q, float* kc, float* vc, const float* k_n
                           uint32_t n_kv_head, uint32_t head_dim, const uint32_t* state, uint32_t window,
                           uint32_t max_len, int flags, uint32_t rows, uint32_t q_stride, const uint32_t* row_pos,
                           size_t cache_stride, const float* q_norm_w, const float* k_norm_w, const float* freqs,
-                          float norm_eps, cudaStream_t st) {
+                          float norm_eps, cudaStream_t st, bool shared_split) {
     constexpr size_t kMostScores = 180 * 1024;
     if (max_len == 0 || max_len > kMostScores / 4) return ZQ_ERR_LIMIT;
     if (oq && head_dim % 32) return ZQ_ERR_BAD_ARG;
@@ -869,8 +869,7 @@ int launch_attention_step(const float* q, float* kc, float* vc, const float* k_n
     uint32_t tiles_x = (max_len + 15) / 16;
     const bool loop = rows >= 16 && tiles_x > 8;
     if (loop) tiles_x = 8;
-    const bool split = rows <= kSharedSplitRows;
-    ZQ_CUDA(launch_pdl_split(split, loop ? attention_scores_step_kernel<true> : attention_scores_step_kernel<false>,
+    ZQ_CUDA(launch_pdl_split(shared_split, loop ? attention_scores_step_kernel<true> : attention_scores_step_kernel<false>,
                        dim3(tiles_x, n_head, rows), dim3(256), smem_scores, st, q, kc, vc, k_new, v_new, scores, n_head,
                        n_kv_head, head_dim, state, window, q_stride, scores_stride, row_pos, cache_stride, nr));
     const dim3 grid(n_head, (head_dim + kAttnDims - 1) / kAttnDims, rows);
@@ -878,14 +877,14 @@ int launch_attention_step(const float* q, float* kc, float* vc, const float* k_n
         auto kern = attention_softmax_v_step_kernel<true>;
         if (smem > 24 * 1024)  // the kernel also holds a 16 KB static tile
             ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMostScores));
-        ZQ_CUDA(launch_pdl_split(split, kern, grid, dim3(256), smem, st, static_cast<const float*>(scores),
+        ZQ_CUDA(launch_pdl_split(shared_split, kern, grid, dim3(256), smem, st, static_cast<const float*>(scores),
                            static_cast<const float*>(vc), out, oq, oscale, osum, n_head, n_kv_head, head_dim, state,
                            window, tail, scores_stride, row_pos, cache_stride));
     } else {
         auto kern = attention_softmax_v_step_kernel<false>;
         if (smem > 24 * 1024)
             ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMostScores));
-        ZQ_CUDA(launch_pdl_split(split, kern, grid, dim3(256), smem, st, static_cast<const float*>(scores),
+        ZQ_CUDA(launch_pdl_split(shared_split, kern, grid, dim3(256), smem, st, static_cast<const float*>(scores),
                            static_cast<const float*>(vc), out, nullptr, nullptr, nullptr, n_head, n_kv_head, head_dim,
                            state, window, tail, scores_stride, row_pos, cache_stride));
     }

@@ -121,9 +121,12 @@ inline cudaError_t launch_pdl(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
                               Args... args) {
     return launch_pdl_split(false, kernel, grid, block, smem, st, args...);
 }
-// Rows of a launch up to which the kernels of a Gemma-3 step ask for the split of the exact int8 products among them (eight
-// sequences and short prompts 35.8 -> 34.0 ms; with 512 rows it costs the streaming ones 1 % of a prompt).
-constexpr uint32_t kSharedSplitRows = 64;
+// Whether the kernels of a Gemma-3 step or prompt of `rows` rows ask for the split of the exact int8 products among them. From
+// two rows on: one row goes to the GEMV, which wants L1, and kernels that ask beside it cost a step of the launch sequence up to
+// 7 % (Gemma-3-1B, 8_0, context 16: 1.105 and 1.186 ms). Up to 64: a step of 64 sequences is 3.02 ms without and 2.75 with it
+// for 4_0 weights, 2.51 and 2.55 for 8_0; with 512 rows the streaming kernels lose 1 % of a prompt.
+constexpr bool step_shares_split(uint32_t rows) { return rows >= 2 && rows <= 64; }
+static_assert(!step_shares_split(1) && !step_shares_split(65), "steps whose products do not ask for the split");
 #endif
 
 // Exponent e of the power-of-two row scale 2^-e that brings a row's largest magnitude `amax` just under 2^14
@@ -215,14 +218,15 @@ constexpr uint32_t kStreamMinRowsF32 = 17;  // f32-activation calls from this ma
 // res == nullptr: quantise rms_norm(src, w1).  Otherwise res += rms_norm(src, w1) and quantise
 // rms_norm(res, w2).
 int launch_norm_quant(const float* src, const float* w1, float* res, const float* w2, uint32_t dim, float eps,
-                      int8_t* q, float* scale, int32_t* sum, uint32_t rows, uint32_t src_stride, cudaStream_t st);
+                      int8_t* q, float* scale, int32_t* sum, uint32_t rows, uint32_t src_stride, cudaStream_t st,
+                      bool shared_split = false);
 // qkv = [q heads | k heads | v heads]; q is normalised and rotated in place, k and v go to the caches.
 int launch_qk_norm_rope_kv(float* qkv, const float* q_norm_w, const float* k_norm_w, const float* freqs,
                            float* kc, float* vc, const uint32_t* state, uint32_t n_head, uint32_t n_kv_head,
                            uint32_t head_dim, float eps, uint32_t rows, uint32_t qkv_stride, const uint32_t* row_pos,
-                           size_t cache_stride, cudaStream_t st);
+                           size_t cache_stride, cudaStream_t st, bool shared_split = false);
 int launch_gelu_mul_quant(const float* gate, const float* up, uint32_t n, int8_t* q, float* scale,
-                          int32_t* sum, uint32_t rows, uint32_t in_stride, cudaStream_t st);
+                          int32_t* sum, uint32_t rows, uint32_t in_stride, cudaStream_t st, bool shared_split = false);
 // Single-query attention over positions [max(0, pos + 1 - window), pos] (window 0 = all); max_len is the
 // largest window any step can have. k_new / v_new (optional, rows == 1): this step's key / value rows,
 // stored into row `pos` of the caches by the same launch. `out` (f32) and `oq/oscale/osum` (quantised)
@@ -233,7 +237,7 @@ int launch_attention_step(const float* q, float* kc, float* vc, const float* k_n
                           uint32_t n_kv_head, uint32_t head_dim, const uint32_t* state, uint32_t window,
                           uint32_t max_len, int flags, uint32_t rows, uint32_t q_stride, const uint32_t* row_pos,
                           size_t cache_stride, const float* q_norm_w, const float* k_norm_w, const float* freqs,
-                          float norm_eps, cudaStream_t st);
+                          float norm_eps, cudaStream_t st, bool shared_split = false);
 // The same for a prompt's tokens, several rows at once, whose keys and values are in the caches (attention_prefill.cu);
 // `end`: an upper bound of the last token's position + 1. q (normalised and rotated) and the caches start on 16-byte
 // boundaries. attention_prefill_takes: whether head_dim has such a kernel and the scores of rows over `ctx` positions fit
@@ -241,7 +245,8 @@ int launch_attention_step(const float* q, float* kc, float* vc, const float* k_n
 bool attention_prefill_takes(uint32_t head_dim, uint32_t ctx);
 int launch_attention_prefill(const float* q, const float* kc, const float* vc, float* out, int8_t* oq, float* oscale,
                              int32_t* osum, uint32_t n_head, uint32_t n_kv_head, uint32_t head_dim, const uint32_t* state,
-                             uint32_t window, uint32_t end, int flags, uint32_t rows, uint32_t q_stride, cudaStream_t st);
+                             uint32_t window, uint32_t end, int flags, uint32_t rows, uint32_t q_stride, cudaStream_t st,
+                             bool shared_split = false);
 // f32 matvec (GPT-2 vocabulary head) with an optional LayerNorm of x in the prologue (gemv.cu).
 int launch_matvec_ln_f32(const float* w, const float* x, float* y, uint32_t out_dim, uint32_t in_dim,
                          const float* ln_gamma, const float* ln_beta, float ln_eps, cudaStream_t st);
