@@ -87,7 +87,8 @@ typedef enum zq_type {
  *               17 to 48 rows: a call that brings the workspace of zq_matmul_workspace_bytes() runs
  *               one product in place of passes of the 16-row kernel (a call without): on matrices
  *               of 12 288 rows and more the weight-streaming tensor-core form (fp16 operands,
- *               3e-4), on smaller ones a form that keeps 22 mantissa bits (1e-7).
+ *               3e-4), on smaller ones a form that keeps 22 mantissa bits (1e-7). Where the passes
+ *               are faster (some matrices at up to 20 rows) zq_matmul_workspace_bytes() is 0.
  *   ZQ_ACT_Q8 : each activation row is first quantised to 32-wide int8 blocks and
  *               the dots are exact int8 x int8 -> int32 — the Gemma-3 path
  *               (src/gguf/thread_pool.zig:96-160 -> src/gguf/simd_dot.zig:25-152).

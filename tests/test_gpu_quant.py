@@ -125,6 +125,20 @@ def test_split_product_keeps_f32_accuracy(zq, oracle, qtype, m, n, k):
         assert rel_l2(got[r], want[r]) <= 1.2e-6, r
 
 
+@pytest.mark.parametrize("qtype,m,n,k,split", [(ggml.Q8_0, 20, 4752, 96, False), (ggml.Q8_0, 21, 4752, 96, True),
+                                               (ggml.Q4_1, 17, 4736, 96, True), (ggml.Q4_0, 17, 4752, 12256, False),
+                                               (ggml.Q4_0, 17, 4752, 12288, True), (ggml.Q8_0, 16, 768, 768, False)])
+def test_rows_in_passes_or_in_one_product(zq, qtype, m, n, k, split):
+    """Both sides of the rule between passes and the split product; the accuracy is that of f32 on either."""
+    g = torch.Generator(device="cuda").manual_seed(15)
+    qw = zq.QuantWeight(ggml.quantize(qtype, torch.randn(n, k, generator=g, device="cuda") * 0.02), qtype, n, k)
+    assert (qw.workspace_bytes(m, zq.ACT_F32) > 0) == split
+    x = torch.randn(m, k, generator=g, device="cuda")
+    want = x.double() @ qw.dequantize().double().T
+    err = (zq.quant_matmul_no_grad(x, qw).double() - want).norm(dim=1) / want.norm(dim=1)
+    assert float(err.max()) <= 1.4e-6  # 22 bits of every activation, f32 sums of 384 blocks: 2^-24 * (4 + sqrt(384))
+
+
 def test_weights_of_different_depth_on_two_threads(zq):
     """A kernel's limit of shared memory is the process's: a shallow weight's call on one thread must not lower it under a
     deep weight's launch on another."""

@@ -100,7 +100,7 @@ struct zq_gpt2 {
 
 // y[T][out] = W . (ln ? LayerNorm(x) : x)[T][in] + bias [gelu] [+ residual[T][out]]. Quantised weights run
 // through the decode kernel up to 16 rows and through the split product (the same parts of the activations and
-// f32 sums over blocks) from 17 rows on;
+// f32 sums over blocks) from 17 rows on, wherever that is faster;
 // f32 weights (the .f32 branch of linear_forward_q, gpt2.zig:652-671) row by row with a separate epilogue.
 // The norm runs as its own small launch: folded into the GEMV prologue every CTA repeats its two
 // block-wide reductions before it can start, which measured 12% slower per step.
@@ -113,7 +113,7 @@ static int gpt2_linear(zq_gpt2* m, const Linear& L, const float* x, float* y, co
     }
     zq_epilogue ep{bias, gelu, nullptr, residual};
     if (L.qw) {
-        if (T >= kSplitMinRows) return launch_gemm_split(L.qw, x, y, T, &ep, m->split, st);
+        if (gemm_split_takes(L.qw, T)) return launch_gemm_split(L.qw, x, y, T, &ep, m->split, st);
         rc = launch_gemv_mma_passes_f32(L.qw, x, y, T, &ep, st);
         if (rc == ZQ_ERR_LIMIT) rc = launch_gemv_f32(L.qw, x, y, T, &ep, st);
         return rc;

@@ -435,6 +435,17 @@ int launch_type(const zq_weight* w, const SplitImage& im, float* y, uint32_t M, 
 
 }  // namespace
 
+// Up to 20 rows the last pass has at most four and costs the least, while the product pads to 24 rows or 32. On matrices whose
+// tiles of 32 x 32 do not run all at once the passes stay ahead, unless K is so deep that a pass holds two rows or the
+// matrix so large that its passes take the ring (B200, us in passes and split, 17 rows: 5760 <- 6144 8_0 62.8 and 78.9, 9472 <-
+// 5120 4_1 57.1 and 69.4; 4096 <- 6144 8_0 as 0.65; 6912 <- 14336 4_0 as 0.63; 8192 <- 8192 8_0 as 0.42; 24 rows of 5760 <- 6144
+// 8_0 level, 25 as 0.88).
+bool gemm_split_takes(const zq_weight* w, uint32_t m_rows) {
+    if (m_rows < 17) return false;
+    const bool ring = w->type != ZQ_TYPE_Q4_1 && (size_t)w->out_dim * w->nbp * w->qb >= ((size_t)64 << 20);
+    return m_rows > 20 || (w->out_dim + 31) / 32 <= (uint32_t)sm_count() || w->in_dim >= 12288 || ring;
+}
+
 size_t gemm_split_workspace_bytes(const zq_weight* w, uint32_t m_rows) {
     const size_t tiles = (m_rows + 7) / 8;
     return align256(tiles * w->nbp * 1024) + align256(tiles * w->nbp * 32) + align256(tiles * 8 * sizeof(float));

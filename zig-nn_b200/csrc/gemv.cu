@@ -471,7 +471,7 @@ size_t zq_matmul_workspace_bytes(const zq_weight* w, uint32_t m_rows, int act_mo
     }
     if (act_mode == ZQ_ACT_F32 && m_rows >= kStreamMinRowsF32 && gemm_stream_takes(w, m_rows))
         return gemm_tc_workspace_bytes(w, m_rows);
-    if (act_mode == ZQ_ACT_F32 && m_rows >= kSplitMinRows) return gemm_split_workspace_bytes(w, m_rows);
+    if (act_mode == ZQ_ACT_F32 && gemm_split_takes(w, m_rows)) return gemm_split_workspace_bytes(w, m_rows);
     return 0;
 }
 
@@ -504,9 +504,9 @@ int zq_matmul(const zq_weight* w, const float* d_x, float* d_y, uint32_t m_rows,
         if (m_rows >= kStreamMinRowsF32 && gemm_stream_takes(w, m_rows) && d_workspace &&
             ((uintptr_t)d_workspace & 255) == 0 && workspace_bytes >= gemm_tc_workspace_bytes(w, m_rows))
             return launch_gemm_tc(w, d_x, d_y, m_rows, epilogue, d_workspace, st);
-        // other calls of 17-48 rows: one f32-accurate product in place of two or three passes (3072 <- 768 at 24
-        // rows 17 us in passes, 8.6 us split; 1152 <- 6912 at 45 rows 135 and 39 us; up to 16 rows one pass is faster)
-        if (m_rows >= kSplitMinRows && d_workspace && ((uintptr_t)d_workspace & 255) == 0 &&
+        // other calls of 17-48 rows: one f32-accurate product in place of two and more passes, where it is faster (3072 <- 768
+        // at 24 rows 17 us in passes, 8.6 split; 1152 <- 6912 at 48 rows 137 and 31; up to 16 rows one pass is faster)
+        if (gemm_split_takes(w, m_rows) && d_workspace && ((uintptr_t)d_workspace & 255) == 0 &&
             workspace_bytes >= gemm_split_workspace_bytes(w, m_rows))
             return launch_gemm_split(w, d_x, d_y, m_rows, epilogue, d_workspace, st);
         // passes of up to 16 activation rows over the weights
