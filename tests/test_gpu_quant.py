@@ -237,10 +237,14 @@ def test_matmul_small_batches_q8_bit_exact(zq, oracle, m):
 
 
 @pytest.mark.parametrize("qtype", TYPES)
-@pytest.mark.parametrize("m,n,k", [(2, 7, 32), (8, 1601, 1184), (9, 33, 16384), (45, 521, 6912)])
+@pytest.mark.parametrize("m,n,k", [(2, 7, 32), (8, 1601, 1184), (9, 33, 16384), (45, 521, 6912), (2, 7, 544), (8, 1184, 16384),
+                                   (5, 1185, 512), (8, 4736, 1536), (8, 4737, 1536), (16, 1184, 512), (17, 600, 768), (33, 1184, 2048),
+                                   (41, 1184, 2048), (17, 776, 768), (17, 776, 736), (49, 1184, 2048),
+                                   (2, 40, 480), (3, 1185, 480), (700, 20, 544)])
 def test_matmul_q8_with_k_over_the_warps_bit_exact(zq, oracle, qtype, m, n, k):
     """The four forms of the product that leaves its terms in shared memory: one and two weight tiles per CTA, up to 8 and
-    up to 16 rows; one block, a part of a quad, several rounds over K."""
+    up to 16 rows; a part of a quad, several rounds over K. Both sides of every line of its rule, the kernel that takes what is
+    left among them (few blocks; more tiles than CTAs at a time)."""
     raw = make_weight(oracle, qtype, n, k)
     x = make_x(m, k)
     x[1] *= 100.0

@@ -493,15 +493,24 @@ int launch_cfg(const zq_weight* w, const int8_t* xq, const float* xs, const int3
 template <int TYPE>
 int launch_one(const zq_weight* w, const int8_t* xq, const float* xs, const int32_t* xsum, float* y, uint32_t M,
                QgEpilogue ep, bool split, cudaStream_t st) {
-    // Few tiles of 8 weight rows x 16 activation rows: K split over the warps (B200, graph-timed with the quantiser,
-    // the kernel above and then this form: 1152 <- 6912 8_0 at 8 rows 25.4 and 10.9 us, 4_1 at 48 rows 28.5 and 26.9;
-    // 1152 <- 1024 at 16 rows 6.7 and 5.1; 5003 <- 1184 at 8 rows 7.7 and 6.5; beyond, 13824 <- 1152 at 8 rows 8.9 and
-    // 10.9). Two weight tiles per CTA once one would give more CTAs than the GPU holds at a time.
-    const uint64_t tiles = (uint64_t)((w->out_dim + 7) / 8) * ((M + 15) / 16);
-    if (tiles <= 640 && M <= 8)
-        return tiles <= 192 ? launch_terms<TYPE, 1, false>(w, xq, xs, xsum, y, M, ep, split, st)
+    // Few tiles of 8 weight rows x 16 activation rows: K split over the warps. How many tiles it may be depends on K, whose
+    // blocks are what the warps share (below 16 to 24 of them the kernel above is ahead), and on how many CTAs run at once: two
+    // per SM, up to 8 rows with one weight tile or with 4_1 weights one. More pay where the kernel above pads an odd number of
+    // 8-row tiles to an even one, or unpacks 4_1; fewer where it reads whole bytes, a ring of which is on its way from HBM
+    // before the kernel ahead has ended. Two weight tiles per CTA once one would give more CTAs than run at once.
+    // (B200, the kernel above and then this form. Graph-timed with the quantiser, us: 1152 <- 6912 8_0 at 8 rows 25.4 and 10.9,
+    // 1152 <- 1024 at 16 rows 6.7 and 5.1, 4736 <- 1152 8_0 at 8 rows 7.5 and 6.2; left to the kernel above: 1536 <- 256 at 8
+    // rows 4.3 and 5.8, 3072 <- 768 4_1 at 8 rows 6.4 and 6.8. Whole Gemma-3-1B steps, ms: 40 sequences of 8_0 2.59 and 2.29, of
+    // 4_1 3.02 and 2.65; left to the kernel above: 32 sequences of 8_0 2.09 and 2.14, 48 of 8_0 2.31 and 2.43.)
+    const uint64_t tiles = (uint64_t)((w->out_dim + 7) / 8) * ((M + 15) / 16), sms = (uint64_t)sm_count();
+    const uint32_t nb = w->nb;
+    constexpr bool Q41 = TYPE == ZQ_TYPE_Q4_1, Q8 = TYPE == ZQ_TYPE_Q8_0;
+    if (M <= 8 && (tiles <= 2 * sms ? nb >= 16 : tiles <= 4 * sms && nb >= (Q41 ? 48 : 20)))
+        return tiles <= sms ? launch_terms<TYPE, 1, false>(w, xq, xs, xsum, y, M, ep, split, st)
                             : launch_terms<TYPE, 2, false>(w, xq, xs, xsum, y, M, ep, split, st);
-    if (tiles <= 480)
+    const bool padded = (M + 7) / 8 & 1u;
+    const uint64_t most = Q41 || padded ? 480 : Q8 && M > 16 ? 192 : 2 * sms;
+    if (M > 8 && (tiles <= sms ? nb >= 16 : tiles <= most && nb >= 24))
         return tiles <= 192 ? launch_terms<TYPE, 1, true>(w, xq, xs, xsum, y, M, ep, split, st)
                             : launch_terms<TYPE, 2, true>(w, xq, xs, xsum, y, M, ep, split, st);
     const uint64_t rt = (w->out_dim + 15) / 16, mt8 = (M + 7) / 8;
