@@ -47,7 +47,8 @@ def test_gpt2_tiny_parity(zq, oracle):
 
 @pytest.mark.parametrize("tokens", [17, 70, 600])
 def test_gpt2_prompt_through_the_split_product(zq, oracle, tokens):
-    """Prompts of one and of two chunks; 600 tokens give every tile shape of the product work."""
+    """Prompts of one chunk and of two (512 and 88 tokens); between them 17, 70, 88 and 512 rows reach every tile shape of the
+    product on these four matrices."""
     host = hostmodel.Gpt2Host.synthetic(dict(hostmodel.GPT2_SMALL, vocab=1000, layer=1), qtype=ggml.Q4_1, seed=42, device="cuda")
     prompt = np.random.default_rng(46).integers(0, 1000, size=tokens)
     gt, ct, errs = run_parity(zq.Gpt2(host.randomize_small_params()), oracle.Gpt2(host, 8), prompt, 2)
@@ -158,6 +159,28 @@ def test_gemma3_prompt_attention_bit_exact(zq, oracle, head, kv, dim):
             want = steps[-2:]
         assert np.array_equal(eng.prefill(prompt).cpu().numpy(), want[0]), n
         assert np.array_equal(eng.decode_next(5).cpu().numpy(), want[1]), n
+
+
+@pytest.mark.parametrize("dim,ctx", [(96, 300), (256, 2305)])
+def test_gemma3_prompt_attention_row_by_row_bit_exact(zq, oracle, dim, ctx):
+    """What attention_prefill.cu does not take: a head dimension without a kernel, scores beyond its shared memory. Chunks of
+    128 tokens, the last with one."""
+    cfg = dict(GEMMA_TINY, head=2, head_dim=dim, ctx=ctx, sliding_window=90, layer=2, global_every=2)
+    host = hostmodel.Gemma3Host.synthetic(cfg, qtype=ggml.Q8_0, seed=42, std=0.08).randomize_small_params()
+    eng, ref = zq.Gemma3(host), oracle.Gemma3(host, 8)
+    for n in (2, 128, 257):
+        prompt = np.random.default_rng(n).integers(0, GEMMA_TINY["vocab"], size=n)
+        assert np.array_equal(eng.prefill(prompt).cpu().numpy(), ref.prefill(prompt)), n
+        assert np.array_equal(eng.decode_next(5).cpu().numpy(), ref.decode_next(5)), n
+
+
+def test_gpt2_prompt_attention_row_by_row(zq, oracle):
+    """A head dimension without a prompt kernel: chunks of 128 tokens, row by row, between the products of many rows."""
+    host = hostmodel.Gpt2Host.synthetic(dict(GPT2_TINY, embed=96, head=1, ctx=300, ffn=384), seed=42, std=0.08)
+    prompt = np.random.default_rng(44).integers(0, GPT2_TINY["vocab"], size=257)
+    gt, ct, errs = run_parity(zq.Gpt2(host.randomize_small_params()), oracle.Gpt2(host, 8), prompt, 4)
+    assert gt == ct
+    assert max(errs) <= 1e-5, max(errs)
 
 
 def test_gemma3_1b_full_size_greedy_64(zq, oracle):

@@ -200,6 +200,17 @@ def test_matmul_many_rows_tensor_core_gemm(zq, oracle, qtype, m, n, k):
     assert rel_l2(got2, want + bias + res) <= REL_L2_GEMM_GUARD
 
 
+def test_many_rows_off_a_16_byte_boundary(zq):
+    """The conversion element by element gives the bits of the one in 16-byte accesses, on rows longer than what that one
+    keeps in registers too."""
+    for m, n, k in ((60, 256, 768), (300, 512, 8224)):
+        qw = zq.QuantWeight(ggml.quantize(ggml.Q4_0, torch.randn(n, k, device="cuda") * 0.02), ggml.Q4_0, n, k)
+        flat = torch.randn(m * k + 1, device="cuda")
+        x = flat[1:].reshape(m, k)
+        assert x.data_ptr() % 16
+        assert torch.equal(zq.quant_matmul_no_grad(x, qw, zq.ACT_F16), zq.quant_matmul_no_grad(x.clone(), qw, zq.ACT_F16))
+
+
 @pytest.mark.parametrize("qtype", TYPES)
 @pytest.mark.parametrize("m", [1, 5, 33])
 def test_f16_activation_mode_any_row_count(zq, oracle, qtype, m):
@@ -469,6 +480,23 @@ def test_matmul_transposed_in_parts_sums_in_f32(zq, out_dim, in_dim, m):
     want = go.double() @ (q.reshape(out_dim, in_dim).double() * 2.0 ** -10)
     got = zq.quant_matmul_transposed(go, qw).double()
     assert float((got - want).norm() / want.norm()) <= 3.8e-6
+
+
+@pytest.mark.parametrize("out_dim,in_dim,m", [(9000, 64, 5), (20008, 96, 130)])
+def test_matmul_transposed_long_and_unaligned_gradient_rows(zq, oracle, out_dim, in_dim, m):
+    """Rows of more than 8192 gradients, and gradients that start off a 16-byte boundary: read element by element."""
+    g = torch.Generator().manual_seed(14)
+    raw = ggml.quantize(ggml.Q4_1, torch.randn(out_dim, in_dim, generator=g) * 0.02).numpy()
+    qw = zq.QuantWeight(raw, ggml.Q4_1, out_dim, in_dim)
+    flat = torch.randn(m * out_dim + 1, generator=g) * 1e-3
+    flat[out_dim - 1] = 3.0  # the largest of row 0 lies behind the first 8192
+    dev = torch.empty(m * out_dim + 1, device="cuda")
+    want = oracle.matmul_transposed(ggml.Q4_1, raw, flat[:-1].reshape(m, out_dim).numpy(), out_dim, in_dim, n_threads=8)
+    for shift in (0, 1):
+        go = dev[shift:shift + m * out_dim].reshape(m, out_dim)
+        go.copy_(flat[:-1].reshape(m, out_dim))
+        got = zq.quant_matmul_transposed(go, qw).cpu().numpy()
+        assert rel_l2(got, want) <= REL_L2_TRANS, shift
 
 
 def test_quant_matmul_backward_to_activations(zq, oracle):
