@@ -131,9 +131,9 @@ static int gpt2_linear(zq_gpt2* m, const Linear& L, const float* x, float* y, co
 }
 
 // Forward pass over T consecutive tokens starting at position m->d_state[1] (gpt2.zig:423-509). T == 1 is a
-// decode step (token in m->d_state[0]); T > 1 a batched prefill chunk (tokens in m->d_tokens). Eight
-// launches per layer when decoding (pos0 is the host's copy of the position, for a chunk): ln1 | qkv | cache write + scores | softmax.V | proj + residual | ln2 |
-// fc + gelu | mproj + residual. Logits are those of the last row.
+// decode step (token in m->d_state[0]); T > 1 a batched prefill chunk (tokens in m->d_tokens; pos0 is the host's
+// copy of its first position). Eight launches per layer when decoding: ln1 | qkv | cache write + scores |
+// softmax.V | proj + residual | ln2 | fc + gelu | mproj + residual. Logits are those of the last row.
 static int gpt2_forward(zq_gpt2* m, uint32_t T, int variant, cudaStream_t st, uint32_t pos0 = 0) {
     const zq_gpt2_config& C = m->c;
     const uint32_t E = C.embed, hd = E / C.head;

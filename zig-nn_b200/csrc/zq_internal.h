@@ -183,7 +183,7 @@ int launch_quantize_rows_q8(const float* x, uint32_t m_rows, uint32_t in_dim, in
 // shared_split: see launch_pdl_split; not for a product alone (16 rows of 1152 <- 6912 with their quantiser 13.4 us, 14.2 so).
 int launch_gemm_q8(const zq_weight* w, const int8_t* xq, const float* xscale, const int32_t* xsum, float* y,
                    uint32_t m_rows, const zq_epilogue* ep, cudaStream_t st, bool shared_split = false);
-constexpr uint32_t kGemmMinRows = 49;  // below this, passes of the 16-row decode kernel are faster
+constexpr uint32_t kGemmMinRows = 49;  // f32-activation calls from here on round to fp16 and need a workspace
 // x16[m][k] = fp16(x[m][k] * 2^-e_m), post[m] = 2^e_m (gemm.cu).
 int launch_convert_rows_f16(const float* x, __half* x16, float* post, uint32_t m_rows, uint32_t in_dim,
                             cudaStream_t st);
