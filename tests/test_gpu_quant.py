@@ -299,6 +299,18 @@ def test_quantize_rows_q8_bit_exact(zq, oracle):
     assert scale[0, 0].item() == 1.0 and q[1, 32].item() == -127 and q[1, 48].item() == 0
 
 
+@pytest.mark.parametrize("qtype", TYPES)
+@pytest.mark.parametrize("n,k,m", [(2003, 96, 509), (1147, 160, 505), (1531, 64, 500), (5003, 64, 45), (700, 32, 30), (17, 480, 9)])
+def test_q8_product_in_every_cta_shape(zq, oracle, qtype, n, k, m):
+    """One call per CTA shape of gemm_q8.cu (the last two take the smallest), with rows, columns and blocks that fill no tile."""
+    raw = make_weight(oracle, qtype, n, k, seed=n)
+    x = make_x(m, k, seed=m)
+    x[m // 2] = 0.0
+    got = zq.quant_matmul_no_grad(torch.from_numpy(x).cuda(), zq.QuantWeight(raw, qtype, n, k), zq.ACT_Q8).cpu().numpy()
+    want = oracle.linear(qtype, raw, x, n, k, act_mode=1, n_threads=8)
+    assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
+
+
 @pytest.mark.parametrize("act", [0, 1])
 def test_epilogue_bias_gelu_mul_residual(zq, oracle, act):
     n, k = 384, 256

@@ -8,21 +8,26 @@
 // rows instead of once per row, and each (weight row, activation row) pair keeps its running f32 sum in
 // a register, so the result is bit-identical to running the decode kernel row by row.
 //
-// Tile: 128 weight rows (8 warps x 16) x 64 activation rows per CTA; K advances by one quad of blocks
+// Tile: W warps x MT x 16 weight rows, NT x 8 activation rows per CTA; K advances by one quad of blocks
 // (128 values). Everything a quad needs travels through a ring of D shared-memory stages filled with
-// cp.async, D - 1 quads ahead of the multiplications: the quantised activations (64 rows x 128 bytes, their
-// scales and sums; 16-byte halves of a (row, block) entry are swapped for rows with bit 2 set so that the
-// fragment loads are free of bank conflicts) and, per lane, the packed weight words and scales of its two
-// rows. The small CTA shapes used for matrices with few rows have only a few warps per SM, so the depth of
-// this ring — not occupancy — is what hides the memory latency there.
+// cp.async, D - 1 quads ahead of the multiplications: the quantised activations (128 bytes per row and their
+// scales; 4_1: and sums) and, per warp, the packed weight words and scales of its rows. The small CTA shapes used
+// for matrices with few rows have only a few warps per SM, so the depth of this ring - not occupancy - is what
+// hides the memory latency there.
+//
+// What bounds it: issue slots and their latencies around the scaling. Per MMA tile of 16 x 8 that is four conversions and, two
+// columns at a time (f32x2), two multiplies and an add for each of its pairs; 4_0 weights are centred before the product, so
+// that no sum of activations is needed. Against one column at a time and sums subtracted behind the product (B200, us with the
+// quantiser and weights from HBM, before and after): 14336 <- 4096 4_0 at 8, 64 and 140 rows 27.4, 91.8, 180 and 22.3, 56.2, 101; 262144 <-
+// 1152 4_1 at 8 rows 86.3 and 58.4; 13824 <- 1152 8_0 at 16, 88 and 512 rows 15.5, 32.4, 91.2 and 11.8, 26.2, 89.2; 1152 <- 6912 8_0 at 512
+// rows 112 and 70.6 (its shape, cheapest_shape). Two weight tiles per warp (MT) share the activation fragments, which costs registers:
+// only shape 1 gains. (The same on tcgen05.mma.kind::i8, a block per MMA of K = 32 and the scaling behind tcgen05.ld, came to 76 and 54
+// us for the two 512-row products, and was slower than this form at all smaller ones: about 8 cycles of an SM for a column of
+// 128 weight rows and a block, where its three f32 operations need 3.)
 #include "zq_internal.h"
 
 namespace zq {
 namespace {
-
-// CTA shape: W warps x 16 weight rows, NT x 8 activation rows. The large shape (8 warps, 64 rows) reads
-// the weights once per 64 activation rows; matrices with few rows take smaller CTAs so that the grid
-// still covers the GPU.
 
 struct QgEpilogue {
     const float* bias;
@@ -48,12 +53,29 @@ __device__ __forceinline__ uint32_t lds32(uint32_t addr) {
     asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr));
     return v;
 }
+__device__ __forceinline__ __half lds_half(uint32_t addr) {
+    unsigned short v;
+    asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(addr));
+    return __ushort_as_half(v);
+}
+__device__ __forceinline__ unsigned long long lds_pair(uint32_t addr) {
+    unsigned long long v;
+    asm volatile("ld.shared.u64 %0, [%1];" : "=l"(v) : "r"(addr));
+    return v;
+}
 __device__ __forceinline__ void mma_s8(int (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0,
                                        uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
                  "{%10,%10,%10,%10};"
                  : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
                  : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1), "r"(0));
+}
+// The same with the four zeros in registers of the caller's.
+__device__ __forceinline__ void mma_s8(int (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, const int (&zero)[4]) {
+    asm volatile("mma.sync.aligned.m16n8k32.row.col.s32.s8.s8.s32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, "
+                 "{%10,%11,%12,%13};"
+                 : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
+                 : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "r"(zero[0]), "r"(zero[1]), "r"(zero[2]), "r"(zero[3]));
 }
 __device__ __forceinline__ uint32_t pick4(const uint4& v, int j) {
     return j == 0 ? v.x : j == 1 ? v.y : j == 2 ? v.z : v.w;
@@ -76,30 +98,55 @@ __device__ __forceinline__ uint2 lds64(uint32_t addr) {
     return v;
 }
 
-// Bytes of one ring stage: activations of the CTA, then per warp the packed words (512 bytes per array:
-// rows g, rows g + 8, and for q8_0 their second halves) and the scales (rows g, rows g + 8).
-template <int TYPE, int W, int NT>
+typedef unsigned long long f32x2;
+__device__ __forceinline__ f32x2 pack2(float a, float b) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(a), "f"(b));
+    return d;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b) {
+    f32x2 d;
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+    return d;
+}
+// a + b. The assembler makes one fused operation of a packed multiply and the packed add behind it, although both say .rn (seen
+// on this toolkit: a * b + c of two such instructions has the bits of fmaf); as a multiply-add whose factor `one` it cannot know to
+// be 1, the sum keeps its own rounding.
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b, f32x2 one) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(b), "l"(one), "l"(a));
+    return d;
+}
+// Nibbles n of a word as signed bytes n - 8.
+__device__ __forceinline__ uint32_t centred(uint32_t n) {
+    const uint32_t s = n ^ 0x08080808u;
+    return s | ((s & 0x08080808u) * 0x1Eu);
+}
+
+// Bytes of one ring stage: activations of the CTA, then per warp the packed words (512 bytes per array of 16 bytes per lane)
+// and the scales of its rows.
+template <int TYPE, int W, int MT, int NT>
 struct QgStage {
     static constexpr uint32_t kXq = 4 * NT * 8 * 32;   // 4 blocks x BM rows x 32 int8
-    static constexpr uint32_t kSc = 4 * NT * 8 * 4;    // 4 blocks x BM rows x f32 (and the same for the sums)
-    static constexpr uint32_t kAct = kXq + 2 * kSc;
-    static constexpr uint32_t kWq = TYPE == ZQ_TYPE_Q8_0 ? 2048 : 1024;
-    static constexpr uint32_t kWsHalf = TYPE == ZQ_TYPE_Q4_1 ? 512 : 256;
-    static constexpr uint32_t kWarp = kWq + 2 * kWsHalf;
+    static constexpr uint32_t kSc = 4 * NT * 8 * 4;    // 4 blocks x BM rows x f32 (4_1: and the same for the sums)
+    static constexpr uint32_t kAct = kXq + (TYPE == ZQ_TYPE_Q4_1 ? 2 : 1) * kSc;
+    static constexpr uint32_t kWq = MT * (TYPE == ZQ_TYPE_Q8_0 ? 2048 : 1024);
+    static constexpr uint32_t kRowScales = TYPE == ZQ_TYPE_Q4_1 ? 16 : 8;
+    static constexpr uint32_t kWarp = kWq + MT * 16 * kRowScales;
     static constexpr uint32_t kBytes = (kAct + W * kWarp + 127u) & ~127u;
 };
 
-template <int TYPE, int W, int NT, int D>
+template <int TYPE, int W, int MT, int NT, int D>
 __global__ void __launch_bounds__(W * 32)
 gemm_q8_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc, const int8_t* __restrict__ xq,
                const float* __restrict__ xscale, const int32_t* __restrict__ xqsum, float* __restrict__ y,
-               uint32_t N, uint32_t K, uint32_t M, uint32_t nb, uint32_t scp, QgEpilogue ep) {
+               uint32_t N, uint32_t K, uint32_t M, uint32_t nb, uint32_t scp, float one, QgEpilogue ep) {
     constexpr bool Q8 = TYPE == ZQ_TYPE_Q8_0;
     constexpr bool Q41 = TYPE == ZQ_TYPE_Q4_1;
     constexpr uint32_t QB = Q8 ? 32 : 16;
     constexpr uint32_t QUAD = 4 * QB;
-    using S = QgStage<TYPE, W, NT>;
-    constexpr int QG_BN = W * 16, QG_BM = NT * 8, QG_NT = NT;
+    using S = QgStage<TYPE, W, MT, NT>;
+    constexpr int QG_BN = W * MT * 16, QG_BM = NT * 8, T = W * 32;
     constexpr uint32_t QG_XQ_BYTES = S::kXq, QG_SC_BYTES = S::kSc, QG_STAGE = S::kBytes;
     extern __shared__ __align__(128) unsigned char smem[];
     const uint32_t smem32 = (uint32_t)__cvta_generic_to_shared(smem);
@@ -107,60 +154,76 @@ gemm_q8_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc, c
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int g = lane >> 2, t = lane & 3;
     const uint32_t nbp = (nb + 3u) & ~3u, nq = nbp / 4;
-    const uint32_t n0 = blockIdx.x * QG_BN + warp * 16, m0 = blockIdx.y * QG_BM;
-
-    const uint32_t row_a = min(n0 + g, N - 1), row_b = min(n0 + g + 8, N - 1);
-    const uint8_t* pa = qs + (size_t)row_a * nbp * QB + 16 * t;
-    const uint8_t* pb = qs + (size_t)row_b * nbp * QB + 16 * t;
-    const uint8_t* sa = sc + (size_t)row_a * scp * (Q41 ? 4 : 2);
-    const uint8_t* sb = sc + (size_t)row_b * scp * (Q41 ? 4 : 2);
+    const uint32_t n0 = blockIdx.x * QG_BN + warp * (MT * 16), m0 = blockIdx.y * QG_BM;
     const uint32_t wring = smem32 + S::kAct + warp * S::kWarp;  // this warp's part of stage 0
 
-    // Quad q -> stage. Activations: xq entries [blk][row][32 bytes] (16-byte halves swapped when row & 4),
-    // scales [blk][row], sums [blk][row]; rows >= M and blocks >= nb are zero-filled (never used for output).
-    // Weights: every lane copies the 16-byte pieces and the scales of its own two rows and reads the same
-    // slots back later, so they need no synchronisation beyond cp.async.wait_group.
+    // Sources of this thread's copies of quad 0; a quad further they lie a constant number of bytes on.
+    // Weights: the words of its own rows g and g + 8 of each tile. 8_0: words 2t and 2t + 1 of the four blocks are 32 contiguous
+    // bytes; 4-bit: word t, whose low nibbles are the block's word t and whose high ones its word 4 + t.
+    // Scales: a lane per row of the warp. Activations: xq entries [blk][row][32 bytes], scales [blk][row], sums [blk][row]; rows
+    // >= M and blocks >= nb are zero-filled (never used for output).
+    uint32_t w_off[MT * 2];
+#pragma unroll
+    for (int r = 0; r < MT * 2; ++r) w_off[r] = min(n0 + r * 8 + g, N - 1) - min(n0, N - 1);
+    const uint8_t* w_base = qs + (size_t)min(n0, N - 1) * nbp * QB + 16 * t;
+    const uint8_t* s_src = sc + (size_t)min(n0 + (uint32_t)lane % (MT * 16), N - 1) * scp * (Q41 ? 4 : 2);
+    constexpr int XP = (8 * QG_BM + T - 1) / T, SP = (4 * QG_BM + T - 1) / T;  // pieces of a thread
     auto issue = [&](uint32_t stage, uint32_t q) {
         const uint32_t base = smem32 + stage * QG_STAGE;
-        for (uint32_t idx = tid; idx < 8u * QG_BM; idx += W * 32) {  // (blk, row, half)
-            const uint32_t b = idx / (2u * QG_BM), r = (idx >> 1) % QG_BM, h = idx & 1u;
-            const uint32_t blk = q * 4 + b, m = m0 + r;
-            const bool ok = m < M && blk < nb;
-            const int8_t* src = xq + (size_t)(ok ? m : 0) * K + (size_t)(ok ? blk : 0) * 32 + h * 16;
-            cp_async16_zfill(base + ((b * QG_BM + r) * 2 + (h ^ ((r >> 2) & 1u))) * 16, src, ok ? 16u : 0u);
+#pragma unroll
+        for (int i = 0; i < XP; ++i) {  // (row, blk, half): a row's 128 bytes by eight neighbouring threads
+            const uint32_t idx = tid + i * T;
+            if (8 * QG_BM % T == 0 || idx < 8u * QG_BM) {
+                const uint32_t r = idx >> 3, b = (idx >> 1) & 3u, h = idx & 1u, m = m0 + r;
+                const bool ok = m < M && q * 4 + b < nb;
+                // 4-bit: the halves of rows with bit 2 set change places, or the fragment loads would meet in a bank
+                const uint32_t to = ((b * QG_BM + r) * 2 + (Q8 ? h : h ^ ((r >> 2) & 1u))) * 16;
+                cp_async16_zfill(base + to, xq + (ok ? (size_t)m * K + q * 128 + (idx & 7u) * 16 : 0), ok ? 16u : 0u);
+            }
         }
-        for (uint32_t idx = tid; idx < 4u * QG_BM; idx += W * 32) {  // (blk, row)
-            const uint32_t b = idx / QG_BM, r = idx % QG_BM;
-            const uint32_t blk = q * 4 + b, m = m0 + r;
-            const bool ok = m < M && blk < nb;
-            const size_t o = (size_t)(ok ? m : 0) * nb + (ok ? blk : 0);
-            cp_async4_zfill(base + QG_XQ_BYTES + (b * QG_BM + r) * 4, xscale + o, ok ? 4u : 0u);
-            cp_async4_zfill(base + QG_XQ_BYTES + QG_SC_BYTES + (b * QG_BM + r) * 4, xqsum + o, ok ? 4u : 0u);
+#pragma unroll
+        for (int i = 0; i < SP; ++i) {  // (row, blk)
+            const uint32_t idx = tid + i * T;
+            if (4 * QG_BM % T == 0 || idx < 4u * QG_BM) {
+                const uint32_t r = idx >> 2, b = idx & 3u, m = m0 + r;
+                const bool ok = m < M && q * 4 + b < nb;
+                const size_t o = ok ? (size_t)m * nb + q * 4 + b : 0;
+                cp_async4_zfill(base + QG_XQ_BYTES + (b * QG_BM + r) * 4, xscale + o, ok ? 4u : 0u);
+                if (Q41) cp_async4_zfill(base + QG_XQ_BYTES + QG_SC_BYTES + (b * QG_BM + r) * 4, xqsum + o, ok ? 4u : 0u);
+            }
         }
         const uint32_t wb = wring + stage * QG_STAGE;
-        cp_async16(wb + lane * 16, pa + (size_t)q * QUAD);
-        cp_async16(wb + 512 + lane * 16, pb + (size_t)q * QUAD);
-        if (Q8) {
-            cp_async16(wb + 1024 + lane * 16, pa + (size_t)q * QUAD + 64);
-            cp_async16(wb + 1536 + lane * 16, pb + (size_t)q * QUAD + 64);
+#pragma unroll
+        for (int r = 0; r < MT * 2; ++r) {
+            const uint8_t* from = w_base + (size_t)w_off[r] * nbp * QB + (size_t)q * QUAD;
+            if (Q8) {  // piece w of a row at w ^ (row & 1): the lanes of a fragment load meet in no bank
+                const uint32_t to = wb + (r * 8 + g) * 128 + ((t ^ (g & 1)) << 4);
+                cp_async16(to, from);
+                cp_async16(to + 64, from + 64);
+            } else {
+                cp_async16(wb + r * 512 + lane * 16, from);
+            }
         }
-        if (Q41) {
-            cp_async16(wb + S::kWq + lane * 16, reinterpret_cast<const uint4*>(sa) + q);
-            cp_async16(wb + S::kWq + S::kWsHalf + lane * 16, reinterpret_cast<const uint4*>(sb) + q);
-        } else {
-            cp_async8(wb + S::kWq + lane * 8, reinterpret_cast<const uint2*>(sa) + q);
-            cp_async8(wb + S::kWq + S::kWsHalf + lane * 8, reinterpret_cast<const uint2*>(sb) + q);
+        if (MT == 2 || lane < 16) {
+            const uint32_t to = wb + S::kWq + lane * S::kRowScales;
+            if (Q41) cp_async16(to, s_src + (size_t)q * 16);
+            else cp_async8(to, s_src + (size_t)q * 8);
         }
     };
 
-    float run[QG_NT][4];
+    const f32x2 one2 = pack2(one, one);
+    int zero[4];
+    asm volatile("mov.b32 %0, 0; mov.b32 %1, 0; mov.b32 %2, 0; mov.b32 %3, 0;" : "=r"(zero[0]), "=r"(zero[1]), "=r"(zero[2]), "=r"(zero[3]));
+    f32x2 run[MT][NT][2];  // [tile][column tile][row g, row g + 8]: columns 2t and 2t + 1
 #pragma unroll
-    for (int j = 0; j < QG_NT; ++j) run[j][0] = run[j][1] = run[j][2] = run[j][3] = 0.0f;
+    for (int i = 0; i < MT; ++i)
+#pragma unroll
+        for (int j = 0; j < NT; ++j) run[i][j][0] = run[i][j][1] = 0;
 
-    // fragment addressing inside a stage: entry (blk, row = 8j + g), word t (and 4 + t), halves swapped by row bit 2
+    // fragment addressing inside a stage: entry (blk, row = 8j + g). 8_0: words 2t and 2t + 1; 4-bit: t and 4 + t, halves swapped
     const uint32_t swap = ((uint32_t)g >> 2) & 1u;
-    const uint32_t frag_lo = ((uint32_t)g * 2 + (0u ^ swap)) * 16 + t * 4;   // word t
-    const uint32_t frag_hi = ((uint32_t)g * 2 + (1u ^ swap)) * 16 + t * 4;   // word 4 + t
+    const uint32_t frag_lo = Q8 ? (uint32_t)lane * 8 : ((uint32_t)g * 2 + swap) * 16 + t * 4;
+    const uint32_t frag_hi = ((uint32_t)g * 2 + (1u ^ swap)) * 16 + t * 4;
 
     // the quantised activations come from the kernel before this one
     pdl_launch_dependents();
@@ -183,74 +246,73 @@ gemm_q8_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc, c
 
         const uint32_t base = smem32 + stage * QG_STAGE;
         const uint32_t wb = wring + stage * QG_STAGE;
-        const uint4 wa = lds128(wb + lane * 16), wbv = lds128(wb + 512 + lane * 16);
-        uint4 wa2 = wa, wb2 = wbv;
-        if (Q8) {
-            wa2 = lds128(wb + 1024 + lane * 16);
-            wb2 = lds128(wb + 1536 + lane * 16);
-        }
-        float da[4], db[4], ma[4], mb[4];
-        if (Q41) {
-            const uint4 sa4 = lds128(wb + S::kWq + lane * 16), sb4 = lds128(wb + S::kWq + S::kWsHalf + lane * 16);
+        const uint32_t blocks = min(4u, nb - q * 4);  // row padding: no term is added for blocks that do not exist
+        uint4 w[MT * 2][Q8 ? 2 : 1];
 #pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                const uint32_t ua = pick4(sa4, b), ub = pick4(sb4, b);
-                const float2 fa = __half22float2(*reinterpret_cast<const __half2*>(&ua));
-                const float2 fb = __half22float2(*reinterpret_cast<const __half2*>(&ub));
-                da[b] = fa.x; ma[b] = fa.y;
-                db[b] = fb.x; mb[b] = fb.y;
-            }
-        } else {
-            const uint2 sa2 = lds64(wb + S::kWq + lane * 8), sb2 = lds64(wb + S::kWq + S::kWsHalf + lane * 8);
-            const float2 a01 = __half22float2(*reinterpret_cast<const __half2*>(&sa2.x));
-            const float2 a23 = __half22float2(*reinterpret_cast<const __half2*>(&sa2.y));
-            const float2 b01 = __half22float2(*reinterpret_cast<const __half2*>(&sb2.x));
-            const float2 b23 = __half22float2(*reinterpret_cast<const __half2*>(&sb2.y));
-            da[0] = a01.x; da[1] = a01.y; da[2] = a23.x; da[3] = a23.y;
-            db[0] = b01.x; db[1] = b01.y; db[2] = b23.x; db[3] = b23.y;
-#pragma unroll
-            for (int b = 0; b < 4; ++b) ma[b] = mb[b] = 0.0f;
+        for (int r = 0; r < MT * 2; ++r) {
+            const uint32_t at = wb + (Q8 ? (r * 8 + g) * 128 + (((2 * t) ^ (g & 1)) << 4) : r * 512 + lane * 16);
+            w[r][0] = lds128(at);
+            if (Q8) w[r][Q8 ? 1 : 0] = lds128(at ^ 16u);
         }
 #pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            if (q * 4 + b >= nb) break;  // row padding: no term is added for blocks that do not exist
-            uint32_t a0, a1, a2, a3;
-            if (Q8) {
-                a0 = pick4(wa, b); a1 = pick4(wbv, b); a2 = pick4(wa2, b); a3 = pick4(wb2, b);
-            } else {
-                const uint32_t ua = pick4(wa, b), ub = pick4(wbv, b);
-                a0 = ua & 0x0F0F0F0Fu; a1 = ub & 0x0F0F0F0Fu;
-                a2 = (ua >> 4) & 0x0F0F0F0Fu; a3 = (ub >> 4) & 0x0F0F0F0Fu;
-            }
-            const uint32_t xb = base + b * (QG_BM * 32), sbase = base + QG_XQ_BYTES + b * (QG_BM * 4);
+        for (uint32_t b = 0; b < 4; ++b) {
+            if (b >= blocks) break;
+            uint32_t a[MT][4];
+            f32x2 dd[MT * 2], mm[MT * 2];
 #pragma unroll
-            for (int j = 0; j < QG_NT; ++j) {
-                const uint32_t b0 = lds32(xb + j * 256 + frag_lo), b1 = lds32(xb + j * 256 + frag_hi);
-                int d[4];
-                mma_s8(d, a0, a1, a2, a3, b0, b1);
-                // columns of this lane: activation rows 8j + 2t and 8j + 2t + 1
-                const uint32_t so = sbase + (j * 8 + 2 * t) * 4;
-                float s0, s1;
-                asm volatile("ld.shared.v2.f32 {%0,%1}, [%2];" : "=f"(s0), "=f"(s1) : "r"(so));
-                int qs0 = 0, qs1 = 0;
-                if (!Q8) asm volatile("ld.shared.v2.s32 {%0,%1}, [%2];" : "=r"(qs0), "=r"(qs1) : "r"(so + QG_SC_BYTES));
-                if (TYPE == ZQ_TYPE_Q4_0) {  // sum((n - 8) * q) = sum(n * q) - 8 * sum(q), exact
-                    d[0] -= 8 * qs0; d[1] -= 8 * qs1; d[2] -= 8 * qs0; d[3] -= 8 * qs1;
+            for (int r = 0; r < MT * 2; ++r) {
+                uint32_t lo = pick4(w[r][0], b), hi = Q8 ? pick4(w[r][Q8 ? 1 : 0], b) : lo >> 4;
+                if (!Q8) {
+                    lo &= 0x0F0F0F0Fu;
+                    hi &= 0x0F0F0F0Fu;
                 }
-                float t0 = __fmul_rn(__fmul_rn(da[b], s0), (float)d[0]);
-                float t1 = __fmul_rn(__fmul_rn(da[b], s1), (float)d[1]);
-                float t2 = __fmul_rn(__fmul_rn(db[b], s0), (float)d[2]);
-                float t3 = __fmul_rn(__fmul_rn(db[b], s1), (float)d[3]);
+                if (TYPE == ZQ_TYPE_Q4_0) {
+                    lo = centred(lo);
+                    hi = centred(hi);
+                }
+                a[r >> 1][r & 1] = lo;
+                a[r >> 1][2 + (r & 1)] = hi;
+                const uint32_t at = wb + S::kWq + (r * 8 + g) * S::kRowScales + b * (Q41 ? 4 : 2);
                 if (Q41) {
-                    t0 = __fadd_rn(t0, __fmul_rn(__fmul_rn(ma[b], s0), (float)qs0));
-                    t1 = __fadd_rn(t1, __fmul_rn(__fmul_rn(ma[b], s1), (float)qs1));
-                    t2 = __fadd_rn(t2, __fmul_rn(__fmul_rn(mb[b], s0), (float)qs0));
-                    t3 = __fadd_rn(t3, __fmul_rn(__fmul_rn(mb[b], s1), (float)qs1));
+                    const uint32_t u = lds32(at);
+                    const float2 f = __half22float2(*reinterpret_cast<const __half2*>(&u));
+                    dd[r] = pack2(f.x, f.x);
+                    mm[r] = pack2(f.y, f.y);
+                } else {
+                    const float f = __half2float(lds_half(at));
+                    dd[r] = pack2(f, f);
                 }
-                run[j][0] = __fadd_rn(run[j][0], t0);
-                run[j][1] = __fadd_rn(run[j][1], t1);
-                run[j][2] = __fadd_rn(run[j][2], t2);
-                run[j][3] = __fadd_rn(run[j][3], t3);
+            }
+            const uint32_t xb = base + b * (QG_BM * 32), sbase = base + QG_XQ_BYTES + b * (QG_BM * 4) + t * 8;
+#pragma unroll
+            for (int j = 0; j < NT; ++j) {
+                uint2 xw;
+                if (Q8) {
+                    xw = lds64(xb + j * 256 + frag_lo);
+                } else {
+                    xw.x = lds32(xb + j * 256 + frag_lo);
+                    xw.y = lds32(xb + j * 256 + frag_hi);
+                }
+                const f32x2 s = lds_pair(sbase + j * 32);  // scales of activation rows 8j + 2t and 8j + 2t + 1
+                f32x2 qsum = 0;
+                if (Q41) {
+                    const uint2 u = lds64(sbase + j * 32 + QG_SC_BYTES);
+                    qsum = pack2((float)(int)u.x, (float)(int)u.y);
+                }
+#pragma unroll
+                for (int i = 0; i < MT; ++i) {
+                    int d[4];
+                    if (Q8) mma_s8(d, a[i], xw.x, xw.y, zero);
+                    else mma_s8(d, a[i][0], a[i][1], a[i][2], a[i][3], xw.x, xw.y);
+                    f32x2 t0 = mul2(mul2(dd[2 * i], s), pack2((float)d[0], (float)d[1]));
+                    f32x2 t1 = mul2(mul2(dd[2 * i + 1], s), pack2((float)d[2], (float)d[3]));
+                    if (Q41) {
+                        t0 = add2(t0, mul2(mul2(mm[2 * i], s), qsum), one2);
+                        t1 = add2(t1, mul2(mul2(mm[2 * i + 1], s), qsum), one2);
+                    }
+                    run[i][j][0] = add2(run[i][j][0], t0, one2);
+                    run[i][j][1] = add2(run[i][j][1], t1, one2);
+                }
             }
         }
         __syncthreads();  // this stage is overwritten by the copies issued in the next iteration
@@ -259,22 +321,23 @@ gemm_q8_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc, c
     asm volatile("cp.async.wait_all;" ::: "memory");
 
 #pragma unroll
-    for (int j = 0; j < QG_NT; ++j) {
+    for (int i = 0; i < MT; ++i)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const uint32_t n = n0 + g + (e >> 1) * 8;
-            const uint32_t m = m0 + j * 8 + 2 * t + (e & 1);
-            if (n < N && m < M) {
-                const size_t o = (size_t)m * N + n;
-                float v = run[j][e];
-                if (ep.bias) v = __fadd_rn(v, ep.bias[n]);
-                if (ep.gelu) v = gelu_tanh(v);
-                if (ep.mul) v = __fmul_rn(v, ep.mul[o]);
-                if (ep.residual) v = __fadd_rn(ep.residual[o], v);
-                y[o] = v;
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const uint32_t n = n0 + i * 16 + g + (e >> 1) * 8;
+                const uint32_t m = m0 + j * 8 + 2 * t + (e & 1);
+                if (n < N && m < M) {
+                    const size_t o = (size_t)m * N + n;
+                    float v = __uint_as_float((uint32_t)(e & 1 ? run[i][j][e >> 1] >> 32 : run[i][j][e >> 1]));
+                    if (ep.bias) v = __fadd_rn(v, ep.bias[n]);
+                    if (ep.gelu) v = gelu_tanh(v);
+                    if (ep.mul) v = __fmul_rn(v, ep.mul[o]);
+                    if (ep.residual) v = __fadd_rn(ep.residual[o], v);
+                    y[o] = v;
+                }
             }
-        }
-    }
 }
 
 // ---- the same for products that leave the GPU idle: K split over the warps of a CTA -------------------
@@ -452,6 +515,17 @@ gemm_q8_terms_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__
     }
 }
 
+// Shared memory that a grid asks for: `need`, or as much as leaves no SM room for more than its share of the CTAs, up to `most`.
+// Under programmatic launches the CTAs of a grid are placed while those of the kernels before it still sit on the SMs, and
+// small ones are then stacked on a few of them. (B200, prompts and steps of several sequences, ms without and with it, products
+// of this file only: eight sequences of 4_1 weights 33.4 and 31.4, six of 4_0 17.2 and 15.6, four of 8_0 21.7 and 20.6; a prompt of 600
+// tokens and 17 steps of 8_0 30.9 and 29.9.)
+uint32_t spread_smem(uint64_t ctas, uint32_t need, uint32_t most) {
+    const uint64_t sms = (uint64_t)sm_count(), share = (ctas + sms - 1) / sms;
+    const uint64_t spread = (227 * 1024 / (share + 1) + 128) & ~(uint64_t)127;
+    return spread < need ? need : spread > most ? most : (uint32_t)spread;
+}
+
 template <int TYPE, int NTL, bool WIDE>
 int launch_terms(const zq_weight* w, const int8_t* xq, const float* xs, const int32_t* xsum, float* y, uint32_t M,
                  QgEpilogue ep, bool split, cudaStream_t st) {
@@ -461,7 +535,7 @@ int launch_terms(const zq_weight* w, const int8_t* xq, const float* xs, const in
     const dim3 grid((w->out_dim + 8 * NTL - 1) / (8 * NTL), (M + 15) / 16);
     if (grid.y > 65535u) return ZQ_ERR_LIMIT;
     auto kern = gemm_q8_terms_kernel<TYPE, NTL, WIDE>;
-    const size_t smem = (size_t)per * kBlockBytes;
+    const uint32_t smem = spread_smem((uint64_t)grid.x * grid.y, per * kBlockBytes, kMost * kBlockBytes);
     // the most that any call asks for: the limit is the process's, and another thread may be about to launch a deeper matrix
     ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kMost * kBlockBytes)));
     ZQ_CUDA(launch_pdl_split(split, kern, grid, dim3(kTermWarps * 32), smem, st, w->qs,
@@ -469,27 +543,48 @@ int launch_terms(const zq_weight* w, const int8_t* xq, const float* xs, const in
     return ZQ_OK;
 }
 
-template <int TYPE, int W, int NT, int D>
+template <int TYPE, int W, int MT, int NT, int D>
 int launch_cfg(const zq_weight* w, const int8_t* xq, const float* xs, const int32_t* xsum, float* y, uint32_t M,
                QgEpilogue ep, bool split, cudaStream_t st) {
-    const dim3 grid((w->out_dim + W * 16 - 1) / (W * 16), (M + NT * 8 - 1) / (NT * 8));
+    const dim3 grid((w->out_dim + W * MT * 16 - 1) / (W * MT * 16), (M + NT * 8 - 1) / (NT * 8));
     if (grid.y > 65535u) return ZQ_ERR_LIMIT;
-    const size_t smem = (size_t)D * QgStage<TYPE, W, NT>::kBytes;
-    auto kern = gemm_q8_kernel<TYPE, W, NT, D>;
-    if (smem > 48 * 1024)
-        ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    constexpr uint32_t kRing = D * QgStage<TYPE, W, MT, NT>::kBytes, kMost = 115 * 1024;
+    static_assert(kRing <= kMost, "ring");
+    const uint32_t smem = spread_smem((uint64_t)grid.x * grid.y, kRing, kMost);
+    auto kern = gemm_q8_kernel<TYPE, W, MT, NT, D>;
+    // the most that any call asks for: the limit is the process's, and another thread may be about to launch a larger grid
+    ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
     ZQ_CUDA(launch_pdl_split(split, kern, grid, dim3(W * 32), smem, st, w->qs,
-                       static_cast<const uint8_t*>(w->sc), xq, xs, xsum, y, w->out_dim, w->in_dim, M, w->nb, w->scp, ep));
+                       static_cast<const uint8_t*>(w->sc), xq, xs, xsum, y, w->out_dim, w->in_dim, M, w->nb, w->scp, 1.0f, ep));
     return ZQ_OK;
 }
 
-// CTA shape by measurement on the Gemma-3 layer shapes (64 and 128 activation rows): a warp owns 16 weight
-// rows x NT column tiles of 8 activation rows. Few column tiles per warp mean more warps (the running sums
-// are a serial chain over K per output, so only more, smaller warp tiles shorten a launch that cannot fill
-// the GPU) but also more passes over the weights through L2; so: the largest NT that still gives about
-// 1000 warps, never so small that a weight is read more than 8 times, and the smallest such NT when no
-// choice reaches 1000 warps. (6912->1152 at 128 rows: 35 us with NT = 2, 41 us with NT = 1, 60 us with
-// one-warp CTAs; 1152->13824 at 64 rows: 21 us with NT = 4, 25 us with NT = 8.)
+// CTA shape: the one whose busiest SM is through a block of K first, by a count of cycles. A CTA holds W * MT * NT MMA tiles; an SM
+// that is full takes `per_tile` cycles for one (more tiles per warp share the fragments of a block), and no warp is through its own
+// tiles before `least`. Measured on a B200 with the quantiser, weights from HBM, us for shapes 0 to 4: 13824 <- 1152 8_0 at 24 rows 20.3,
+// 17.5, 15.0, 14.3, 20.7, at 88 rows 31.9, 30.0, 28.0, 32.0, 53, at 512 rows 89.7, 105, 105, 136, 264; 1152 <- 6912 8_0 at 512 rows
+// 103, 75, 72, 97, 127; 5003 <- 1184 4_0 at 45 rows 20.7, 17.6, 14.0, 10.8, 13.0. The count takes the best of the five or one within
+// 7 % of it for the three types, 1152 to 262144 weight rows and 2 to 512 activation rows.
+int cheapest_shape(uint32_t n, uint32_t m, uint32_t sms) {
+    struct Shape {
+        uint32_t rows, cols, tiles, per_tile, least;  // per_tile in tenths of a cycle
+    };
+    constexpr Shape shapes[5] = {{128, 64, 64, 113, 740}, {128, 32, 32, 130, 560}, {64, 32, 16, 135, 370}, {64, 16, 8, 175, 255}, {64, 8, 4, 340, 215}};
+    int best = 0;
+    uint64_t least = ~0ull;
+    for (int i = 0; i < 5; ++i) {
+        const Shape& s = shapes[i];
+        const uint64_t ctas = (uint64_t)((n + s.rows - 1) / s.rows) * ((m + s.cols - 1) / s.cols);
+        uint64_t cost = (ctas + sms - 1) / sms * s.tiles * s.per_tile;
+        if (cost < s.least * 10ull) cost = s.least * 10ull;
+        if (cost < least) {
+            least = cost;
+            best = i;
+        }
+    }
+    return best;
+}
+
 template <int TYPE>
 int launch_one(const zq_weight* w, const int8_t* xq, const float* xs, const int32_t* xsum, float* y, uint32_t M,
                QgEpilogue ep, bool split, cudaStream_t st) {
@@ -513,21 +608,12 @@ int launch_one(const zq_weight* w, const int8_t* xq, const float* xs, const int3
     if (M > 8 && (tiles <= sms ? nb >= 16 : tiles <= most && nb >= 24))
         return tiles <= 192 ? launch_terms<TYPE, 1, true>(w, xq, xs, xsum, y, M, ep, split, st)
                             : launch_terms<TYPE, 2, true>(w, xq, xs, xsum, y, M, ep, split, st);
-    const uint64_t rt = (w->out_dim + 15) / 16, mt8 = (M + 7) / 8;
-    uint32_t nt_cap = 1, nt_min = 1;
-    while (nt_cap < 8 && nt_cap < mt8) nt_cap *= 2;
-    while (nt_min < nt_cap && (mt8 + nt_min - 1) / nt_min > 8) nt_min *= 2;
-    uint32_t nt = nt_min;
-    for (uint32_t c = nt_cap; c >= nt_min; c /= 2)
-        if (rt * ((mt8 + c - 1) / c) >= 1000) {
-            nt = c;
-            break;
-        }
-    switch (nt) {
-        case 8: return launch_cfg<TYPE, 8, 8, 3>(w, xq, xs, xsum, y, M, ep, split, st);
-        case 4: return launch_cfg<TYPE, 4, 4, 4>(w, xq, xs, xsum, y, M, ep, split, st);
-        case 2: return launch_cfg<TYPE, 4, 2, 6>(w, xq, xs, xsum, y, M, ep, split, st);
-        default: return launch_cfg<TYPE, 4, 1, 8>(w, xq, xs, xsum, y, M, ep, split, st);
+    switch (cheapest_shape(w->out_dim, M, (uint32_t)sms)) {
+        case 0: return launch_cfg<TYPE, 8, 1, 8, 3>(w, xq, xs, xsum, y, M, ep, split, st);
+        case 1: return launch_cfg<TYPE, 4, 2, 4, 3>(w, xq, xs, xsum, y, M, ep, split, st);
+        case 2: return launch_cfg<TYPE, 4, 1, 4, 3>(w, xq, xs, xsum, y, M, ep, split, st);
+        case 3: return launch_cfg<TYPE, 4, 1, 2, 4>(w, xq, xs, xsum, y, M, ep, split, st);
+        default: return launch_cfg<TYPE, 4, 1, 1, 6>(w, xq, xs, xsum, y, M, ep, split, st);
     }
 }
 
