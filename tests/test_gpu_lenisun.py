@@ -210,6 +210,22 @@ def test_attention_rows_do_not_depend_on_each_other(zq, f32, ctx, shape):
             assert torch.equal(c.attend(x[r], pos[r], slots[r], False), alone[r]), (T, r0)
 
 
+@pytest.mark.parametrize("ctx", [2048, 2049, 4100, 6300])
+def test_decode_attention_at_the_borders_of_its_ranges(zq, ctx):
+    """Ranges of one, two, three and four tiles (a ring of one, two and three), rows that end a range, begin one and lie between."""
+    rng = np.random.default_rng(ctx)
+    H, G, d, e = 5, 1, 64, 48
+    per = -(-ctx // 64)
+    tiles = -(-per // 32)
+    c, k, v = fill_cache(zq, rng, (H, G, d, e), ctx, 2, False, d ** -0.5)
+    pos = sorted({0, 63, 64, 64 * tiles - 1, 64 * tiles, 64 * tiles + 1, 1000, ctx - 64, ctx - 1})
+    q = held(rng.standard_normal((len(pos), H, d)), False)
+    x = queries(c, q)
+    for r, p in enumerate(pos):
+        out = c.attend(x[r:r + 1], np.array([p]), [1], False)
+        close(out[:, :H * e], attend_rows(q[r:r + 1], k[1], v[1], np.array([p]), d ** -0.5), 8e-3, "position %d of %d" % (p, ctx))
+
+
 @pytest.mark.parametrize("f32", PRECISIONS)
 def test_attention_finds_one_key_among_many(zq, f32):
     """One key answers the query (its score stands out by far); it is put at tile borders, at the first token, at the

@@ -21,15 +21,23 @@ __device__ __forceinline__ void load_tile(uint32_t dst, const bf16* cache, uint3
     const uint32_t cpr = dp / 8, pitch = (dp + 8) * 2;
     const uint32_t dr = blockDim.x / cpr, dc = blockDim.x % cpr;
     uint32_t row = threadIdx.x / cpr, c = threadIdx.x % cpr;
+    const size_t key_step = (size_t)kv_heads * dp;
+    const bf16* first = cache + (size_t)k0 * key_step + (size_t)g * dp;  // what a copy of zeros names
+    const bf16* from = first + row * key_step + c * 8;
+    uint32_t to = dst + row * pitch + c * 16;
+    const size_t step = dr * key_step + dc * 8, back = key_step - dp;  // a row further, a row's chunks back
     while (row < kTile) {
-        const uint32_t key = k0 + row;
-        const bool ok = key < k_end;
-        copy16(dst + row * pitch + c * 16, cache + ((size_t)(ok ? key : k0) * kv_heads + g) * dp + c * 8, ok);
+        const bool ok = k0 + row < k_end;
+        copy16(to, ok ? from : first, ok);
         row += dr;
         c += dc;
+        from += step;
+        to += dr * pitch + dc * 16;
         if (c >= cpr) {
             c -= cpr;
             ++row;
+            from += back;
+            to += pitch - cpr * 16;
         }
     }
 }
@@ -140,6 +148,7 @@ struct AttnArgs {
     float scale2;  // scale * log2(e)
     const int32_t *pos, *slots;
     uint32_t rows, pos0, splits;
+    uint32_t stages;  // decode: tiles of the ring
     float* part;  // decode: [rows][splits][heads][vdimp] values, then [rows][splits][heads][2] maximum and sum
     // decode with the steps ahead of it (null qkv: q and the row's own key and value are there already)
     QkvPostArgs pre;
@@ -228,24 +237,33 @@ gqa_prefill_kernel(const __grid_constant__ AttnArgs a) {
 
 constexpr uint32_t kDecodeStages = 3;
 
+// What bounds it: latency, of a chain position -> tiles -> query -> scores -> values -> ranges with one warp at work per scheduler. At 1500
+// keys of one key head of 256 a step's call took 18.8 us behind its predecessor with ranges of 256 keys (four tiles, one behind
+// the other) and a ring of 203 KB; 13.4 with ranges of one tile, requested ahead of the wait, and the ring that these need; 11.5 with
+// the warps' sums met row by row (no divisions per element, only the rows that are heads). The second kernel takes 3.0 instead of 2.2.
 template <int D>
 __global__ void __launch_bounds__(128)
 gqa_decode_kernel(const __grid_constant__ AttnArgs a) {
     constexpr int S = D / 16;
     extern __shared__ __align__(16) unsigned char sm[];
     pdl_launch_dependents();
-    pdl_wait();
+    // With `pre`, the row's own key and value are made here, by the CTA whose range ends with them: its copies stop
+    // ahead of them. Its position and the keys and values ahead of its own are then those of earlier steps, which no kernel
+    // of this one writes, and are requested before the wait; without, the kernel ahead may have written any of them.
+    const bool fused = a.pre.qkv != nullptr;
+    if (!fused) pdl_wait();
     const GqaShape& s = a.s;
     const uint32_t R = s.heads / s.kv_heads, m_tiles = (R + 15) / 16;
     const uint32_t split = blockIdx.x, g = blockIdx.y / m_tiles, h0 = (blockIdx.y % m_tiles) * 16, r = blockIdx.z;
     const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t len = (uint32_t)a.pos[r] + 1;
+    const uint32_t len = (uint32_t)__ldcg(a.pos + r) + 1;
     const uint32_t per = ((len + a.splits - 1) / a.splits + kTile - 1) / kTile * kTile;
     const uint32_t k_begin = split * per, k_end = min(len, k_begin + per);
     const uint32_t nh = min(16u, R - h0);  // heads of this CTA
     float* part_ml = a.part + (size_t)a.rows * a.splits * s.heads * s.vdimp;
     const size_t prow = ((size_t)r * a.splits + split) * s.heads + g * R + h0;
     if (k_begin >= k_end) {
+        if (fused) pdl_wait();
         for (uint32_t i = threadIdx.x; i < nh; i += blockDim.x) {
             part_ml[(prow + i) * 2] = -INFINITY;
             part_ml[(prow + i) * 2 + 1] = 0.0f;
@@ -254,25 +272,24 @@ gqa_decode_kernel(const __grid_constant__ AttnArgs a) {
     }
     const uint32_t base = (uint32_t)__cvta_generic_to_shared(sm);
     const uint32_t kbytes = kTile * (s.dimp + 8) * 2, vbytes = kTile * (s.vdimp + 8) * 2;
-    auto ktile = [&](uint32_t b) { return base + (b % kDecodeStages) * (kbytes + vbytes); };
+    auto ktile = [&](uint32_t b) { return base + (b % a.stages) * (kbytes + vbytes); };
     auto vtile = [&](uint32_t b) { return ktile(b) + kbytes; };
-    const size_t slot = (size_t)(uint32_t)a.slots[r] * s.ctx;
+    const size_t slot = (size_t)(uint32_t)__ldcg(a.slots + r) * s.ctx;
     const bf16* kc = a.kc + slot * s.kv_heads * s.dimp;
     const bf16* vc = a.vc + slot * s.kv_heads * s.vdimp;
     const uint32_t n_tiles = (k_end - k_begin + kTile - 1) / kTile;
-    // With `pre`, the row's own key and value are made here, by the CTA whose range ends with them: its copies stop
-    // ahead of them.
-    const bool fused = a.pre.qkv != nullptr, own = fused && k_end == len;
+    const bool own = fused && k_end == len;
     const uint32_t c_end = own ? k_end - 1 : k_end;
-#pragma unroll
-    for (uint32_t t = 0; t + 1 < kDecodeStages; ++t) {
+    const uint32_t early = a.stages == 1 ? 1 : a.stages - 1;  // tiles requested here; one stage: the longest range is one tile
+    for (uint32_t t = 0; t < early; ++t) {
         if (t < n_tiles) {
             load_tile(ktile(t), kc, s.kv_heads, g, s.dimp, k_begin + t * kTile, c_end);
             load_tile(vtile(t), vc, s.kv_heads, g, s.vdimp, k_begin + t * kTile, c_end);
         }
         copy_commit();
     }
-    bf16* own_q = reinterpret_cast<bf16*>(sm + kDecodeStages * (kbytes + vbytes));  // [16][dimp], then own key and value
+    if (fused) pdl_wait();
+    bf16* own_q = reinterpret_cast<bf16*>(sm + a.stages * (kbytes + vbytes));  // [16][dimp], then own key and value
     bf16 *own_k = own_q + 16 * s.dimp, *own_v = own_k + s.dimp;
     if (fused) {
         const QkvPostArgs& f = a.pre;
@@ -307,18 +324,19 @@ gqa_decode_kernel(const __grid_constant__ AttnArgs a) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) o[v][e] = 0.0f;
     for (uint32_t t = 0; t < n_tiles; ++t) {
-        const uint32_t ahead = t + kDecodeStages - 1;
+        const uint32_t ahead = t + early;
         if (ahead < n_tiles) {
             load_tile(ktile(ahead), kc, s.kv_heads, g, s.dimp, k_begin + ahead * kTile, c_end);
             load_tile(vtile(ahead), vc, s.kv_heads, g, s.vdimp, k_begin + ahead * kTile, c_end);
         }
         copy_commit();
-        copy_wait<kDecodeStages - 1>();
+        if (early == 2) copy_wait<2>();
+        else copy_wait<1>();
         __syncthreads();
         if (own && t + 1 == n_tiles) {  // the place behind the copied keys
             const uint32_t at = k_end - 1 - (k_begin + t * kTile);
-            unsigned char* kt = sm + (t % kDecodeStages) * (kbytes + vbytes) + at * (s.dimp + 8) * 2;
-            unsigned char* vt = sm + (t % kDecodeStages) * (kbytes + vbytes) + kbytes + at * (s.vdimp + 8) * 2;
+            unsigned char* kt = sm + (t % a.stages) * (kbytes + vbytes) + at * (s.dimp + 8) * 2;
+            unsigned char* vt = sm + (t % a.stages) * (kbytes + vbytes) + kbytes + at * (s.vdimp + 8) * 2;
             for (uint32_t e = threadIdx.x; e < s.dimp; e += blockDim.x) reinterpret_cast<bf16*>(kt)[e] = own_k[e];
             for (uint32_t e = threadIdx.x; e < s.vdimp; e += blockDim.x) reinterpret_cast<bf16*>(vt)[e] = own_v[e];
             __syncthreads();
@@ -336,10 +354,12 @@ gqa_decode_kernel(const __grid_constant__ AttnArgs a) {
     copy_wait<0>();
     __syncthreads();
     float* ml = reinterpret_cast<float*>(sm);          // [4 warps][16 rows][2]
-    float* ov = ml + 4 * 16 * 2;                       // [4 warps][16 rows][vdimp]
+    const uint32_t vpitch = s.vdimp + 8;               // rows eight banks apart
+    float* ov = ml + 4 * 16 * 2;                       // [4 warps][16 rows][vpitch]
 #pragma unroll
     for (int hf = 0; hf < 2; ++hf) {
         const uint32_t row = (lane >> 2) + hf * 8;
+        if (row >= nh) continue;
         if ((lane & 3) == 0) {
             ml[(warp * 16 + row) * 2] = m[hf];
             ml[(warp * 16 + row) * 2 + 1] = l[hf];
@@ -348,32 +368,35 @@ gqa_decode_kernel(const __grid_constant__ AttnArgs a) {
         for (int v = 0; v < S * 2; ++v) {
             const uint32_t col = v * 8 + (lane & 3) * 2;
             if (col < s.vdimp)
-                *reinterpret_cast<float2*>(ov + (size_t)(warp * 16 + row) * s.vdimp + col) =
+                *reinterpret_cast<float2*>(ov + (size_t)(warp * 16 + row) * vpitch + col) =
                     make_float2(o[v][hf * 2], o[v][hf * 2 + 1]);
         }
     }
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < nh * s.vdimp; i += blockDim.x) {
-        const uint32_t row = i / s.vdimp, col = i % s.vdimp;
-        float mx = -INFINITY;
+#pragma unroll 1
+    for (uint32_t row = 0; row < nh; ++row) {
+        float mx = -INFINITY, sum = 0.0f, f[4];
 #pragma unroll
         for (uint32_t w = 0; w < 4; ++w) mx = fmaxf(mx, ml[(w * 16 + row) * 2]);
-        float sum = 0.0f, acc = 0.0f;
 #pragma unroll
         for (uint32_t w = 0; w < 4; ++w) {
-            const float f = exp2f(ml[(w * 16 + row) * 2] - mx);
-            sum += f * ml[(w * 16 + row) * 2 + 1];
-            acc += f * ov[(size_t)(w * 16 + row) * s.vdimp + col];
+            f[w] = exp2f(ml[(w * 16 + row) * 2] - mx);
+            sum += f[w] * ml[(w * 16 + row) * 2 + 1];
         }
-        if (a.splits == 1) {
-            if (col < s.vdim)
-                a.out[(size_t)r * a.out_pitch + (size_t)(g * R + h0 + row) * s.vdim + col] = __float2bfloat16_rn(acc / sum);
-        } else {
-            a.part[(prow + row) * s.vdimp + col] = acc;
-            if (col == 0) {
-                part_ml[(prow + row) * 2] = mx;
-                part_ml[(prow + row) * 2 + 1] = sum;
+        for (uint32_t col = threadIdx.x; col < s.vdimp; col += blockDim.x) {
+            float acc = 0.0f;
+#pragma unroll
+            for (uint32_t w = 0; w < 4; ++w) acc += f[w] * ov[(size_t)(w * 16 + row) * vpitch + col];
+            if (a.splits == 1) {
+                if (col < s.vdim)
+                    a.out[(size_t)r * a.out_pitch + (size_t)(g * R + h0 + row) * s.vdim + col] = __float2bfloat16_rn(acc / sum);
+            } else {
+                a.part[(prow + row) * s.vdimp + col] = acc;
             }
+        }
+        if (a.splits > 1 && threadIdx.x == 0) {
+            part_ml[(prow + row) * 2] = mx;
+            part_ml[(prow + row) * 2 + 1] = sum;
         }
     }
     if (a.splits == 1 && blockIdx.y == 0) zero_pad(a.out + (size_t)r * a.out_pitch, s.heads * s.vdim, a.out_pitch);
@@ -507,10 +530,11 @@ int plain_rows(const GqaShape& s, const void* q, const void* kc, const void* vc,
     return go(gqa_plain_kernel<TA, 32>, 32);
 }
 
-// Ranges of a row's keys, by the cache's capacity alone (256 keys each when it is full): a row's ranges, and with them its
-// bits, do not depend on the other rows of its step.
+// Ranges of a row's keys, by the cache's capacity alone (a tile each when it is full, longer ones beyond 32 of them): a row's
+// ranges, and with them its bits, do not depend on the other rows of its step. (Prompts of 1500 tokens and 24 steps, Lenisun of width
+// 1152: 14.3 ms with ranges of 256 keys, 13.2 so; six of 200 tokens together 27.6 and 27.2.)
 uint32_t decode_splits(const GqaShape& s) {
-    const uint32_t n = (s.ctx + 255) / 256;
+    const uint32_t n = (s.ctx + kTile - 1) / kTile;
     return n < 1 ? 1 : n > 32 ? 32 : n;
 }
 
@@ -529,10 +553,12 @@ int tiles_launch(AttnArgs& a, bool one_sequence, cudaStream_t st) {
         ZQ_CUDA(cudaFuncSetAttribute(gqa_prefill_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, 2 * kMostTile));
         return done(launch_pdl(gqa_prefill_kernel<D>, dim3((a.rows * R + 63) / 64, s.kv_heads), dim3(128), 2 * tile, st, a));
     }
-    uint32_t smem = kDecodeStages * tile + (17 * s.dimp + s.vdimp) * 2;
-    const uint32_t meet = (4 * 16 * 2 + 4 * 16 * s.vdimp) * 4;
-    if (smem < meet) smem = meet;
     a.splits = decode_splits(s);
+    const uint32_t longest = ((s.ctx + a.splits - 1) / a.splits + kTile - 1) / kTile;  // tiles of a range
+    a.stages = longest < kDecodeStages ? longest : kDecodeStages;
+    uint32_t smem = a.stages * tile + (17 * s.dimp + s.vdimp) * 2;
+    const uint32_t meet = (4 * 16 * 2 + 4 * 16 * (s.vdimp + 8)) * 4;
+    if (smem < meet) smem = meet;
     ZQ_CUDA(cudaFuncSetAttribute(gqa_decode_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  kDecodeStages * kMostTile + 18 * 256 * 2));
     int rc = done(launch_pdl(gqa_decode_kernel<D>, dim3(a.splits, s.kv_heads * ((R + 15) / 16), a.rows), dim3(128), smem, st, a));
