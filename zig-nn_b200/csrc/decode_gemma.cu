@@ -293,20 +293,30 @@ __device__ __forceinline__ XImage ximage(unsigned char* scratch, uint32_t nbp_ma
     return x;
 }
 
-// quantize_row_q8 (simd_dot.zig:25-64) of the 32 values held one per lane, written into the image.
-__device__ __forceinline__ void quant_block_to_image(float v, uint32_t b, int lane, const XImage& x) {
-    // |v| as an unsigned integer orders like the float: one warp-wide integer maximum gives max(abs(v))
-    const float amax = __uint_as_float(__reduce_max_sync(0xFFFFFFFFu, __float_as_uint(fabsf(v))));
+// quantize_row_q8 (simd_dot.zig:25-64) of a vector whose group `gi` of four values each thread holds (eight neighbouring lanes: one
+// block), written into the image; `ok` is the same for the eight. Four values a lane share a block's two divisions and its
+// reductions among eight lanes instead of 32: the quantiser is bound by its instructions, every CTA runs it over the whole vector
+// (Gemma-3-1B, 216 blocks of the feed-forward vector: 14 passes a warp with a value per lane, 4 so).
+__device__ __forceinline__ void quant_group_to_image(float4 v, uint32_t gi, bool ok, const XImage& x) {
+    // |v| as an unsigned integer orders like the float
+    auto bits = [](float f) { return __float_as_uint(fabsf(f)); };
+    uint32_t m = max(max(bits(v.x), bits(v.y)), max(bits(v.z), bits(v.w)));
+#pragma unroll
+    for (int off = 1; off <= 4; off <<= 1) m = max(m, __shfl_xor_sync(0xFFFFFFFFu, m, off));
+    const float amax = __uint_as_float(m);
     const float s = amax > 0.0f ? __fdiv_rn(amax, 127.0f) : 1.0f;
     const float inv = __fdiv_rn(1.0f, s);
-    float r = roundf(__fmul_rn(v, inv));
-    r = fminf(127.0f, fmaxf(-127.0f, r));
-    const int qi = (int)r;
-    const int acc = __reduce_add_sync(0xFFFFFFFFu, qi);
-    const uint32_t w = (uint32_t)lane >> 2;
-    unsigned char* dst = reinterpret_cast<unsigned char*>(w < 4 ? x.xl : x.xh);
-    dst[((((b >> 2) * 4 + (w & 3u)) * 4 + (b & 3u)) << 2) + ((uint32_t)lane & 3u)] = (unsigned char)(signed char)qi;
-    if (lane == 0) {
+    auto quant = [&](float f) { return (int)fminf(127.0f, fmaxf(-127.0f, roundf(__fmul_rn(f, inv)))); };
+    const int q0 = quant(v.x), q1 = quant(v.y), q2 = quant(v.z), q3 = quant(v.w);
+    int acc = (q0 + q1) + (q2 + q3);
+#pragma unroll
+    for (int off = 1; off <= 4; off <<= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, off);
+    if (!ok) return;
+    const uint32_t b = gi >> 3, w = gi & 7u;
+    uint32_t* dst = reinterpret_cast<uint32_t*>(w < 4 ? x.xl : x.xh);
+    dst[((b >> 2) * 4 + (w & 3u)) * 4 + (b & 3u)] =
+        __byte_perm(__byte_perm((uint32_t)q0, (uint32_t)q1, 0x0040), __byte_perm((uint32_t)q2, (uint32_t)q3, 0x0040), 0x5410);
+    if (w == 0) {
         x.xsc[b] = s;
         x.xsum[b] = acc;
     }
@@ -327,9 +337,9 @@ __device__ __forceinline__ void image_padding(const Cta& c, const XImage& x, uin
 }
 
 // An exchanged f32 vector (dim % 32 == 0), quantised into the image. 16 words per thread and pass, all in
-// flight at once: one round trip for up to 8192 elements. The values are parked in `stage` (16 * 512 floats,
-// each thread reads back only what it wrote) so that the quantiser exists once, in a rolled loop: the kernel
-// runs every phase once per layer, and code size, not arithmetic, is what instruction fetch pays for.
+// flight at once: one round trip for up to 8192 elements. The values pass through `stage` (16 * 512 floats) to the lanes that
+// quantise them, in a rolled loop: the kernel runs every phase once per layer, and code size, not arithmetic, is what
+// instruction fetch pays for.
 __device__ __noinline__ void quantise_exchanged(const unsigned long long* buf,
                                                 uint32_t dim, uint32_t epoch, float* stage) {
     const Cta c = make_cta();
@@ -338,16 +348,16 @@ __device__ __noinline__ void quantise_exchanged(const unsigned long long* buf,
     for (uint32_t base = 0; base < dim; base += kConsumers * 16) {
         {
             float v[16];
+            if (base) cbar();  // the pass before has read the stage
             xload_batch<16>(c, p, buf, base + c.tid, kConsumers, dim, epoch, v);
 #pragma unroll
             for (int u = 0; u < 16; ++u) stage[u * kConsumers + c.tid] = v[u];
         }
+        cbar();
+        const uint32_t groups = min(dim - base, (uint32_t)kConsumers * 16) >> 2;
 #pragma unroll 1
-        for (uint32_t u = 0; u < 16; ++u) {
-            const uint32_t i = base + u * kConsumers + c.tid;
-            if (i - c.lane >= dim) break;  // whole warps
-            quant_block_to_image(stage[u * kConsumers + c.tid], i >> 5, c.lane, x);
-        }
+        for (uint32_t g = c.tid; g - c.lane < groups; g += kConsumers)  // whole warps
+            quant_group_to_image(reinterpret_cast<const float4*>(stage)[g], (base >> 2) + g, g < groups, x);
     }
     image_padding(c, x, dim >> 5, (dim / 32 + 3u) & ~3u);
 }
@@ -396,9 +406,18 @@ __device__ __noinline__ void norm_quant(const unsigned long long* src, uint32_t 
     cbar();
     const float ss = sumsq_lanes16(c, xres, dim);
     const float inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)dim), eps)));
+    const uint32_t groups = dim >> 2;
 #pragma unroll 1
-    for (uint32_t i = c.tid; i < dim; i += kConsumers)
-        quant_block_to_image(__fmul_rn(__fmul_rn(xres[i], inv), w2s[i]), i >> 5, c.lane, x);
+    for (uint32_t g = c.tid; g - c.lane < groups; g += kConsumers) {  // whole warps
+        const uint32_t gc = min(g, groups - 1);
+        float4 v = reinterpret_cast<const float4*>(xres)[gc];
+        const float4 w = reinterpret_cast<const float4*>(w2s)[gc];
+        v.x = __fmul_rn(__fmul_rn(v.x, inv), w.x);
+        v.y = __fmul_rn(__fmul_rn(v.y, inv), w.y);
+        v.z = __fmul_rn(__fmul_rn(v.z, inv), w.z);
+        v.w = __fmul_rn(__fmul_rn(v.w, inv), w.w);
+        quant_group_to_image(v, g, g < groups, x);
+    }
     image_padding(c, x, dim >> 5, (dim / 32 + 3u) & ~3u);
 }
 

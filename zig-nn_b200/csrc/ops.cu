@@ -374,6 +374,28 @@ __device__ __forceinline__ void quantize_block_warp(float v, size_t blk, int lan
     }
 }
 
+// The same of a row whose group `g` of four values each thread holds (eight neighbouring lanes: one block; `ok` is the same for the
+// eight). The whole warp calls it.
+__device__ __forceinline__ void quantize_group_warp(float4 v, uint32_t g, bool ok, int8_t* __restrict__ q, float* __restrict__ scale,
+                                                    int32_t* __restrict__ sum) {
+    float amax = fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w)));
+#pragma unroll
+    for (int off = 1; off <= 4; off <<= 1) amax = fmaxf(amax, __shfl_xor_sync(0xFFFFFFFFu, amax, off));
+    const float s = amax > 0.0f ? __fdiv_rn(amax, 127.0f) : 1.0f;
+    const float inv = __fdiv_rn(1.0f, s);
+    auto quant = [&](float f) { return (int)fminf(127.0f, fmaxf(-127.0f, roundf(__fmul_rn(f, inv)))); };
+    const int q0 = quant(v.x), q1 = quant(v.y), q2 = quant(v.z), q3 = quant(v.w);
+    int acc = (q0 + q1) + (q2 + q3);
+#pragma unroll
+    for (int off = 1; off <= 4; off <<= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, off);
+    if (!ok) return;
+    reinterpret_cast<char4*>(q)[g] = make_char4((signed char)q0, (signed char)q1, (signed char)q2, (signed char)q3);
+    if ((g & 7u) == 0) {
+        scale[g >> 3] = s;
+        sum[g >> 3] = acc;
+    }
+}
+
 // RES = false:  h = rms_norm(src, w1)                               -> quantised
 // RES = true:   res += rms_norm(src, w1);  h = rms_norm(res, w2)     -> quantised
 // (gemma3.zig:662-666, 725-737, 768-773: post-norm + residual, then the next block's pre-norm.)
@@ -454,19 +476,21 @@ norm_quant_kernel(const float* __restrict__ src, const float* __restrict__ w1, f
         ss = sumsq_lanes16(xs, dim, part, &bc);
         inv = __fdiv_rn(1.0f, __fsqrt_rn(__fadd_rn(__fdiv_rn(ss, (float)dim), eps)));
     }
-    const int lane = threadIdx.x & 31;
+    // the normalised row, each thread its own elements, then four neighbouring ones a thread to the quantiser
     if (PER > 0) {
 #pragma unroll
         for (int u = 0; u < P; ++u) {
             const uint32_t i = threadIdx.x + u * 256;
-            if (i < dim)  // dim is a multiple of 32: whole warps
-                quantize_block_warp(__fmul_rn(__fmul_rn(xs[i], inv), RES ? rw2[u] : rw1[u]), i >> 5, lane, q, scale, sum);
+            if (i < dim) xs[i] = __fmul_rn(__fmul_rn(xs[i], inv), RES ? rw2[u] : rw1[u]);
         }
     } else {
         const float* wq = RES ? w2 : w1;
-        for (uint32_t i = threadIdx.x; i < dim; i += blockDim.x)
-            quantize_block_warp(__fmul_rn(__fmul_rn(xs[i], inv), wq[i]), i >> 5, lane, q, scale, sum);
+        for (uint32_t i = threadIdx.x; i < dim; i += blockDim.x) xs[i] = __fmul_rn(__fmul_rn(xs[i], inv), wq[i]);
     }
+    __syncthreads();
+    const uint32_t groups = dim >> 2;
+    for (uint32_t g = threadIdx.x; g - (threadIdx.x & 31u) < groups; g += blockDim.x)  // whole warps
+        quantize_group_warp(reinterpret_cast<const float4*>(xs)[min(g, groups - 1)], g, g < groups, q, scale, sum);
 }
 
 // Per-head work between the QKV projection and attention (gemma3.zig:689-716): q and k heads get
