@@ -293,6 +293,23 @@ def test_persistent_decode_kernel_equals_the_launch_sequence(zq, qtypes):
     assert _lib.device_error(clear=False) == 0
 
 
+@pytest.mark.parametrize("embed,ffn", [(32, 96), (96, 8224), (2080, 64)])
+def test_decode_quantisers_of_odd_widths(zq, oracle, embed, ffn):
+    """Vectors that fill no warp of four-value lanes, that need a second pass of the exchange (8192 values each), that end between."""
+    cfg = dict(GEMMA_TINY, embed=embed, ffn=ffn, layer=2)
+    host = hostmodel.Gemma3Host.synthetic(cfg, qtype=ggml.Q8_0, seed=embed, std=0.05).randomize_small_params()
+    eng, steps, ref = zq.Gemma3(host), zq.Gemma3(host), oracle.Gemma3(host, 8)
+    assert eng.decode_mode == zq.DECODE_PERSISTENT
+    steps.set_decode_mode(zq.DECODE_LAUNCH_SEQUENCE)
+    prompt = np.random.default_rng(1).integers(0, cfg["vocab"], size=5)
+    got, other, want = eng.prefill(prompt), steps.prefill(prompt), ref.prefill(prompt)
+    for _ in range(3):
+        for g in (got, other):
+            assert np.array_equal(g.cpu().numpy().view(np.uint32), want.view(np.uint32))
+        t = int(np.argmax(want))
+        got, other, want = eng.decode_next(t), steps.decode_next(t), ref.decode_next(t)
+
+
 def test_persistent_decode_kernel_full_size_greedy_against_launch_sequence(zq):
     """Gemma-3-1B shape, Q8_0, 600-token context (beyond the window): 48 greedy tokens from the on-device loop
     of the persistent kernel equal those of the launch sequence, and so do the logits of the step after."""

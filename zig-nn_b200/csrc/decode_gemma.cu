@@ -122,6 +122,9 @@ __device__ __forceinline__ unsigned char* smem_base() {
     return zq_decode_smem;
 }
 __device__ __forceinline__ Shared& sh() { return *reinterpret_cast<Shared*>(smem_base()); }
+// A part of the dynamic shared memory by its offset. Functions that are not inlined take no pointers into it: through a parameter
+// its loads become generic ones, and a chain of ordered adds that feeds on them runs at 6.7 cycles an add instead of 4.8.
+__device__ __forceinline__ float* smem_floats(uint32_t off) { return reinterpret_cast<float*>(smem_base() + off); }
 
 // Per-thread view of the CTA's shared state; built (a few address computations) at the top of every device
 // function rather than passed by reference, which would put it into local memory.
@@ -341,10 +344,11 @@ __device__ __forceinline__ void image_padding(const Cta& c, const XImage& x, uin
 // quantise them, in a rolled loop: the kernel runs every phase once per layer, and code size, not arithmetic, is what
 // instruction fetch pays for.
 __device__ __noinline__ void quantise_exchanged(const unsigned long long* buf,
-                                                uint32_t dim, uint32_t epoch, float* stage) {
+                                                uint32_t dim, uint32_t epoch) {
     const Cta c = make_cta();
     const DParams& p = sh().p;
     const XImage x = ximage(c.smem + p.off_scratch, p.nbp_max);
+    float* stage = reinterpret_cast<float*>(x.xsum + p.nbp_max);
     for (uint32_t base = 0; base < dim; base += kConsumers * 16) {
         {
             float v[16];
@@ -364,14 +368,14 @@ __device__ __noinline__ void quantise_exchanged(const unsigned long long* buf,
 
 // xres (+)= rms_norm(src, w1) when src != nullptr; then h = rms_norm(xres, w2) quantised into the image
 // (gemma3.zig:662-666, 725-737, 768-773 followed by the row quantiser of the next linear). The norm weights
-// are requested (asynchronous copies into `wstage`, 2 * dim floats) together with the exchanged vector, so the
+// are requested (asynchronous copies behind the image, 2 * dim floats) together with the exchanged vector, so the
 // prologue pays one memory round trip.
 __device__ __noinline__ void norm_quant(const unsigned long long* src, uint32_t epoch,
-                                        const float* w1, const float* w2, float* xres, float* xs, uint32_t dim,
-                                        float eps, float* wstage) {
+                                        const float* w1, const float* w2, uint32_t dim, float eps) {
     const Cta c = make_cta();
     const DParams& p = sh().p;
     const XImage x = ximage(c.smem + p.off_scratch, p.nbp_max);
+    float *xres = smem_floats(p.off_xres), *xs = smem_floats(p.off_xs), *wstage = reinterpret_cast<float*>(x.xsum + p.nbp_max);
     float* w1s = wstage;
     float* w2s = wstage + dim;
     {
@@ -831,11 +835,9 @@ __device__ __noinline__ bool produce_phase(const DMat& m, uint32_t* unit_base,
 }
 
 // Embedding row of `tok`, dequantised and scaled (gemma3.zig:800-803, 855-871): q*d, then *scale.
-__device__ __noinline__ void embed_row(const DMat& m, uint32_t tok, float scale, float* xres,
-                                          uint32_t dim) {
+__device__ __noinline__ void embed_row(const DMat& m, uint32_t tok, float scale, uint32_t dim) {
     const Cta c = make_cta();
-    const DParams& p = sh().p;
-    (void)p;
+    float* xres = smem_floats(sh().p.off_xres);
     const unsigned char* qrow = m.qs + (size_t)tok * m.row_q_bytes;
     const unsigned char* srow = m.sc + (size_t)tok * m.row_s_bytes;
 #pragma unroll 1
@@ -867,12 +869,12 @@ __device__ __noinline__ void embed_row(const DMat& m, uint32_t tok, float scale,
 // spread over the CTAs in tiles of 32 (position, head) pairs and leave as exchange words.
 // Returns false (to every thread) when the CTA has to leave.
 __device__ __noinline__ bool scores_phase(const DLayer& L, uint32_t pos,
-                                             uint32_t kv_start, uint32_t kv_len, const float* rope, float* qn,
-                                             float* vnew, const unsigned long long* qkv_in, uint32_t ep_in,
+                                             uint32_t kv_start, uint32_t kv_len, const unsigned long long* qkv_in, uint32_t ep_in,
                                              unsigned long long* scores_out, uint32_t ep_out) {
     const Cta c = make_cta();
     const DParams& p = sh().p;
-    (void)p;
+    const float* rope = smem_floats(p.off_rope);
+    float *qn = smem_floats(p.off_scratch), *vnew = smem_floats(p.off_vnew);
     const uint32_t D = p.D, nh = p.n_head, nkv = p.n_kv, group = p.group, kv_dim = nkv * D;
     const uint32_t nvec = nh + nkv, nqk = nvec * D, nall = nqk + kv_dim;
     // The key rows of this CTA's first tile of (position, head) pairs are old cache rows: requested before the
@@ -1007,15 +1009,15 @@ __device__ __noinline__ bool scores_phase(const DLayer& L, uint32_t pos,
 // the cache, the current position's row from `vnew`) into prod[d][p], while eight threads of warp 0 add the
 // previous tile's products in order. Returns false when the CTA has to leave.
 __device__ __noinline__ bool softmax_v_phase(const DLayer& L, uint32_t kv_start,
-                                                uint32_t kv_len, unsigned char* scratch, const float* vnew,
-                                                const unsigned long long* scores_in, uint32_t ep_in,
+                                                uint32_t kv_len, const unsigned long long* scores_in, uint32_t ep_in,
                                                 unsigned long long* att_out, uint32_t ep_out) {
     const Cta c = make_cta();
     const DParams& p = sh().p;
     const uint32_t D = p.D, nh = p.n_head, nkv = p.n_kv, kv_dim = nkv * D;
     const uint32_t chunks = D / 8, jobs = nh * chunks;
     constexpr uint32_t PITCH = kVTile + 4;                             // 4 mod 32 banks: stores and chain loads conflict-free
-    float* w = reinterpret_cast<float*>(scratch);                      // [max_len]
+    const float* vnew = smem_floats(p.off_vnew);
+    float* w = smem_floats(p.off_scratch);                             // [max_len]
     float* prod = w + (((size_t)p.max_len + 3u) & ~(size_t)3u);        // [2][8][PITCH]
     bool ok = true;
 #pragma unroll 1
@@ -1183,12 +1185,7 @@ gemma3_decode_kernel(const __grid_constant__ DParams p_in, uint32_t n_steps, int
     }
 
     // -------------------------------------------------------------------- consumer warps
-    float* xres = reinterpret_cast<float*>(smem + p.off_xres);
-    float* xs = reinterpret_cast<float*>(smem + p.off_xs);
-    float* rope = reinterpret_cast<float*>(smem + p.off_rope);
-    float* vnew = reinterpret_cast<float*>(smem + p.off_vnew);
-    unsigned char* scratch = smem + p.off_scratch;
-    float* terms_all = reinterpret_cast<float*>(ximage(scratch, p.nbp_max).xsum + p.nbp_max);
+    float* rope = smem_floats(p.off_rope);
     const uint32_t E = p.E, D = p.D;
     const Exchange& ex = p.ex;
     uint32_t tok = __ldcg(p.state + 0), pos = __ldcg(p.state + 1), rec = __ldcg(p.state + 2);
@@ -1209,7 +1206,7 @@ gemma3_decode_kernel(const __grid_constant__ DParams p_in, uint32_t n_steps, int
     for (uint32_t step = 0; step < n_steps; ++step) {
         ZQ_STAMP();
         __threadfence();  // cache rows that the last CTA stored during earlier steps are read below
-        embed_row(p.head, tok, p.embed_scale, xres, E);
+        embed_row(p.head, tok, p.embed_scale, E);
         for (uint32_t j = c.tid; j < D / 2; j += kConsumers) {  // RoPE angles of this position, every layer
             const float theta = __fmul_rn((float)pos, __ldg(p.freqs + j));
             rope[2 * j] = (float)cos((double)theta);
@@ -1224,7 +1221,7 @@ gemma3_decode_kernel(const __grid_constant__ DParams p_in, uint32_t n_steps, int
             epoch += 6;
             // --- attention block
             norm_quant(l ? ex.ffn + (size_t)prev * ex.ffn_n : nullptr, e_ffn_prev,
-                       l ? layers[l - 1].post_ffw_norm_w : nullptr, L.attn_norm_w, xres, xs, E, p.eps, terms_all);
+                       l ? layers[l - 1].post_ffw_norm_w : nullptr, L.attn_norm_w, E, p.eps);
             if (l) {  // every CTA has finished the previous layer: its buffers of this parity may be rewritten
                 for (uint32_t base = 0; base < gridDim.x; base += kConsumers) {
                     float v[1];
@@ -1240,30 +1237,29 @@ gemma3_decode_kernel(const __grid_constant__ DParams p_in, uint32_t n_steps, int
             const uint32_t end = pos + 1;
             const uint32_t kv_len = (L.window && end > L.window) ? L.window : end;
             const uint32_t kv_start = end - kv_len;
-            if (!scores_phase(L, pos, kv_start, kv_len, rope, reinterpret_cast<float*>(scratch), vnew,
-                              ex.qkv + (size_t)par * ex.qkv_n, e_qkv, ex.scores + (size_t)par * ex.scores_n, e_scores))
+            if (!scores_phase(L, pos, kv_start, kv_len, ex.qkv + (size_t)par * ex.qkv_n, e_qkv, ex.scores + (size_t)par * ex.scores_n, e_scores))
                 return;
             ZQ_STAMP();
             cbar();  // qn is overwritten by the softmax weights
-            if (!softmax_v_phase(L, kv_start, kv_len, scratch, vnew, ex.scores + (size_t)par * ex.scores_n, e_scores,
+            if (!softmax_v_phase(L, kv_start, kv_len, ex.scores + (size_t)par * ex.scores_n, e_scores,
                                  ex.att + (size_t)par * ex.att_n, e_att))
                 return;
             ZQ_STAMP();
             cbar();
-            quantise_exchanged(ex.att + (size_t)par * ex.att_n, p.n_head * D, e_att, terms_all);
+            quantise_exchanged(ex.att + (size_t)par * ex.att_n, p.n_head * D, e_att);
             ZQ_CHECK_ABORT();
             ZQ_STAMP();
             unit_base = gemv_phase(L.o, unit_base, EP_VECTOR, ex.proj + (size_t)par * ex.proj_n, e_proj, nullptr, nullptr);
             ZQ_STAMP();
             cbar();
             // --- FFN block
-            norm_quant(ex.proj + (size_t)par * ex.proj_n, e_proj, L.post_attn_norm_w, L.ffn_norm_w, xres, xs, E, p.eps, terms_all);
+            norm_quant(ex.proj + (size_t)par * ex.proj_n, e_proj, L.post_attn_norm_w, L.ffn_norm_w, E, p.eps);
             ZQ_CHECK_ABORT();
             ZQ_STAMP();
             unit_base = gemv_phase(L.gate_up, unit_base, EP_GEGLU, ex.g + (size_t)par * ex.g_n, e_g, nullptr, nullptr);
             ZQ_STAMP();
             cbar();
-            quantise_exchanged(ex.g + (size_t)par * ex.g_n, p.F, e_g, terms_all);
+            quantise_exchanged(ex.g + (size_t)par * ex.g_n, p.F, e_g);
             ZQ_CHECK_ABORT();
             ZQ_STAMP();
             unit_base = gemv_phase(L.down, unit_base, EP_VECTOR, ex.ffn + (size_t)par * ex.ffn_n, e_ffn, nullptr, nullptr);
@@ -1274,7 +1270,7 @@ gemma3_decode_kernel(const __grid_constant__ DParams p_in, uint32_t n_steps, int
         if (want_logits) {
             const uint32_t last = (lc - 1) & 1u;
             norm_quant(ex.ffn + (size_t)last * ex.ffn_n, epoch - 1, layers[p.n_layer - 1].post_ffw_norm_w,
-                       p.output_norm_w, xres, xs, E, p.eps, terms_all);
+                       p.output_norm_w, E, p.eps);
             ZQ_CHECK_ABORT();
             ZQ_STAMP();
             Best best{-INFINITY, 0xFFFFFFFFu};
