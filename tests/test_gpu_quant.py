@@ -300,6 +300,17 @@ def test_quantize_rows_q8_bit_exact(zq, oracle):
 
 
 @pytest.mark.parametrize("qtype", TYPES)
+@pytest.mark.parametrize("n,k,m", [(700, 992, 47), (1000, 512, 33), (2290, 480, 47), (520, 96, 45), (9000, 96, 30), (9000, 224, 45), (11003, 96, 41)])
+def test_split_product_in_every_tile(zq, oracle, qtype, n, k, m):
+    """One call per tile of gemm_split.cu that a call of up to 48 rows takes, with rows, columns and blocks that fill none."""
+    raw = make_weight(oracle, qtype, n, k, seed=n)
+    x = make_x(m, k, seed=m)
+    got = zq.quant_matmul_no_grad(torch.from_numpy(x).cuda(), zq.QuantWeight(raw, qtype, n, k)).cpu().numpy()
+    want = oracle.linear(qtype, raw, x, n, k, act_mode=0, n_threads=8)
+    assert rel_l2(got, want) <= REL_L2_GUARD
+
+
+@pytest.mark.parametrize("qtype", TYPES)
 @pytest.mark.parametrize("n,k,m", [(2003, 96, 509), (1147, 160, 505), (1531, 64, 500), (5003, 64, 45), (700, 32, 30), (17, 480, 9)])
 def test_q8_product_in_every_cta_shape(zq, oracle, qtype, n, k, m):
     """One call per CTA shape of gemm_q8.cu (the last two take the smallest), with rows, columns and blocks that fill no tile."""

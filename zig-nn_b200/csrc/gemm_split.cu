@@ -10,8 +10,11 @@
 // core, whose accumulation is coarser than the f32 sum over blocks. The activations are split once per call into an image
 // in fragment order (split_rows_kernel), so the loop loads them with 128-bit accesses free of bank conflicts; a warp owns
 // 16 weight rows and unpacks a weight word once for all NT x 8 activation rows.
-// Measured (B200, graph-timed, split_rows included; passes of the decode kernel, this product tile by tile in its MMAs, as it
-// is): 3072 <- 768 at 48 rows 31, 15.2, 12.9 us and at 512 rows -, 79, 36.5; 1152 <- 6912 at 48 rows 137, 40, 31 us.
+// What a CTA's step costs besides is its instructions: the chain's first MMA takes its zeros from registers that stay, and a thread
+// finds its copies by one addition each (768 <- 3072 at 32 rows 12.8 -> 9.3 us, 1152 <- 6912 at 24 rows 24.2 -> 17.6; GPT-2 document of 900
+// tokens 7.33 -> 7.22 ms).
+// Measured (B200, graph-timed, split_rows included; passes of the decode kernel, this product): 3072 <- 768 at 48 rows 31, 7.3 us;
+// 1152 <- 6912 at 48 rows 137, 26 us.
 #include "zq_internal.h"
 
 namespace zq {
@@ -134,6 +137,12 @@ __device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], u
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
+// The first of a chain: zeros from registers of the caller's, so that none are cleared for it.
+__device__ __forceinline__ void mma_f16(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1, const float (&zero)[4]) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%10,%11,%12,%13};"
+        : "=f"(d[0]), "=f"(d[1]), "=f"(d[2]), "=f"(d[3])
+        : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(zero[0]), "f"(zero[1]), "f"(zero[2]), "f"(zero[3]));
+}
 __device__ __forceinline__ void rotate(uint4& v) {
     v.x = v.y;
     v.y = v.z;
@@ -207,6 +216,8 @@ gemm_split_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc
         ps[h] = sc + (size_t)row * scp * SB;
     }
     const uint32_t wslot = smem32 + S::kAct + warp * S::kWTile;
+    static_assert(THREADS == 256, "a thread copies 16 bytes of a tile's quad");
+    const uint4* px = im.frag + (size_t)tile0 * nbp * 64 + tid;
 
     auto issue_weights = [&](uint32_t stage, uint32_t step) {
         const uint32_t q = step * KS + ks;
@@ -228,10 +239,9 @@ gemm_split_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc
         for (int k = 0; k < KS; ++k) {
             const uint32_t q = step * KS + k;
             if (q >= nq) break;
-            for (uint32_t i = tid; i < nt * 256; i += THREADS) {
-                const uint32_t j = i >> 8, o = i & 255u;
-                cp_async16(base + (k * NT + j) * S::kTile + o * 16, im.frag + ((size_t)(tile0 + j) * nbp + q * 4) * 64 + o);
-            }
+#pragma unroll
+            for (int j = 0; j < NT; ++j)
+                if ((uint32_t)j < nt) cp_async16(base + (k * NT + j) * S::kTile + tid * 16, px + ((uint32_t)j * nbp + q * 4) * 64);
             if (Q41) {
                 for (uint32_t i = tid; i < nt * 8; i += THREADS) {
                     const uint32_t j = i >> 3, o = i & 7u;
@@ -245,7 +255,8 @@ gemm_split_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc
     // Sums in two levels, kFlush quads below and those above: the f32 chain over K stays as short as that of the
     // decode kernel, which cuts K into up to eight parts (in one level the error at 216 blocks was 1.6e-7 against 1.2e-7).
     constexpr uint32_t kFlush = 4;
-    float acc[NT][4], sum[NT][4];
+    float acc[NT][4], sum[NT][4], zero[4];
+    asm volatile("mov.b32 %0, 0; mov.b32 %1, 0; mov.b32 %2, 0; mov.b32 %3, 0;" : "=f"(zero[0]), "=f"(zero[1]), "=f"(zero[2]), "=f"(zero[3]));
 #pragma unroll
     for (int j = 0; j < NT; ++j)
 #pragma unroll
@@ -329,14 +340,14 @@ gemm_split_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc
                     const uint32_t at = act + j * S::kTile + b * 1024 + lane * 16;
                     lo[j] = lds128(at + 512);
                     hi[j] = lds128(at);
-                    p[j][0] = p[j][1] = p[j][2] = p[j][3] = 0.0f;
                 }
 #pragma unroll
                 for (int ph = 0; ph < 4; ++ph)
 #pragma unroll
                     for (int j = 0; j < NT; ++j) {
                         const uint4& v = ph < 2 ? lo[j] : hi[j];
-                        mma_f16(p[j], ph & 1 ? aH : aL, ph & 1 ? v.z : v.x, ph & 1 ? v.w : v.y);
+                        if (ph == 0) mma_f16(p[j], aL, v.x, v.y, zero);
+                        else mma_f16(p[j], ph & 1 ? aH : aL, ph & 1 ? v.z : v.x, ph & 1 ? v.w : v.y);
                     }
 #pragma unroll
                 for (int j = 0; j < NT; ++j) {
@@ -417,20 +428,42 @@ int launch_cfg(const zq_weight* w, const SplitImage& im, float* y, uint32_t M, c
     return ZQ_OK;
 }
 
+// The tile whose CTAs run all at once, one per SM, and whose chain of steps (KS quads of K each) is the shortest; `step` is what one
+// costs, in tenths of a microsecond: conversions and MMAs of NT tiles, and KS x NT x 4 KB of activations. With none that fits, three
+// small CTAs per SM take turns. (B200, us with the split, the seven tiles and the last in this order, the one taken in brackets:
+// 768 <- 3072 4_0 at 48 rows [9.9], 12.7, 13.5, 20.0, 25.1, 32.4, 54.0, 29.3; 1152 <- 6912 8_0 at 48 rows 28.2, [26.0], 28.3, 43.3, 50.3,
+// 61.7, 103, 67.7; 2304 <- 768 8_0 at 48 rows 11.6, 9.3, [7.0], 7.4, 8.9, 11.8, 16.3, 10.6; 5003 <- 1184 4_1 at 24 rows 20.8, 16.2, 13.7,
+// [10.9], 13.2, 16.8, 26.5, 16.1, at 32 rows 21.6, 16.8, 18.2, 17.9, [13.7], 16.9, 26.9, 16.8 and at 45 rows 29.2, 21.9, 19.5, 18.9, 23.4,
+// [17.8], 27.7, 17.2; 11000 <- 1152 8_0 at 33 rows 55.4, 37.0, 29.2, 25.7, 29.5, 27.2, [22.4], 25.4. A GPT-2 document of 900 tokens: 7.12 ms
+// with the last, 7.22 with tiles of 64 x 32, two per SM.)
 template <int TYPE>
 int launch_type(const zq_weight* w, const SplitImage& im, float* y, uint32_t M, const SplitEpilogue& ep, cudaStream_t st) {
-    const uint64_t sms = (uint64_t)sm_count();
-    auto ctas = [&](uint32_t rows, uint32_t cols) {
-        return (uint64_t)((w->out_dim + rows - 1) / rows) * ((M + cols - 1) / cols);
+    struct Tile {
+        uint32_t rows, cols, quads, step;
     };
-    // The smallest tile whose CTAs run all at once, its K cut over the warps; past that the tile that reads the least
-    // per MMA (us with the split, in the order of the lines, the tile taken in brackets: 768 <- 3072 at 32 rows [13.3], 15.9,
-    // 20.6, 31.2; 2304 <- 768 at 17 rows 9.8, [7.2], 9.0, 11.2; 2304 <- 768 at 48 rows 14.1, 11.5, [9.6], 13.1;
-    // 3072 <- 768 at 48 rows 18.0, 12.3, 15.2, [12.9] and at 512 rows 160, 105, 78, [36.5]).
-    if (ctas(16, 16) <= sms) return launch_cfg<TYPE, 1, 8, 2, 2>(w, im, y, M, ep, st);
-    if (ctas(32, 16) <= sms) return launch_cfg<TYPE, 2, 4, 2, 3>(w, im, y, M, ep, st);
-    if (ctas(32, 32) <= sms) return launch_cfg<TYPE, 2, 4, 4, 2>(w, im, y, M, ep, st);
-    return launch_cfg<TYPE, 4, 2, 4, 2>(w, im, y, M, ep, st);
+    constexpr Tile tiles[7] = {{16, 16, 8, 20}, {32, 16, 4, 16}, {32, 24, 4, 17}, {64, 24, 2, 14}, {64, 32, 2, 18}, {64, 48, 2, 23}, {128, 48, 1, 20}};
+    const uint32_t nq = w->nbp / 4;
+    int best = 7;
+    uint32_t least = ~0u;
+    for (int i = 0; i < 7; ++i) {
+        const Tile& t = tiles[i];
+        const uint64_t ctas = (uint64_t)((w->out_dim + t.rows - 1) / t.rows) * ((M + t.cols - 1) / t.cols);
+        const uint32_t cost = (nq + t.quads - 1) / t.quads * t.step;
+        if (ctas <= (uint64_t)sm_count() && cost < least) {
+            least = cost;
+            best = i;
+        }
+    }
+    switch (best) {
+        case 0: return launch_cfg<TYPE, 1, 8, 2, 2>(w, im, y, M, ep, st);
+        case 1: return launch_cfg<TYPE, 2, 4, 2, 3>(w, im, y, M, ep, st);
+        case 2: return launch_cfg<TYPE, 2, 4, 3, 3>(w, im, y, M, ep, st);
+        case 3: return launch_cfg<TYPE, 4, 2, 3, 4>(w, im, y, M, ep, st);
+        case 4: return launch_cfg<TYPE, 4, 2, 4, 4>(w, im, y, M, ep, st);
+        case 5: return launch_cfg<TYPE, 4, 2, 6, 3>(w, im, y, M, ep, st);
+        case 6: return launch_cfg<TYPE, 8, 1, 6, 2>(w, im, y, M, ep, st);
+        default: return launch_cfg<TYPE, 4, 2, 3, 2>(w, im, y, M, ep, st);
+    }
 }
 
 }  // namespace
