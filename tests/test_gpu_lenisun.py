@@ -77,6 +77,25 @@ def test_rows_do_not_depend_on_each_other(zq, f32, rows_k):
             assert torch.equal(call(x[:T]), alone[:T]), T
 
 
+@pytest.mark.parametrize("f32", PRECISIONS)
+@pytest.mark.parametrize("rows_k", [(301, 4200), (1000, 520), (2500, 1100), (5001, 1100), (2500, 1032)])
+def test_linear_of_one_to_eight_rows_in_deep_matrices(zq, f32, rows_k):
+    """Every count of rows that the streaming kernel has a form for, with more chunks of K than a lane holds ahead and a
+    ragged last one. A sum is at most k / 64 + 8 roundings deep (the lanes' even and odd columns, then a tree)."""
+    rng = np.random.default_rng(12)
+    k = rows_k[1]
+    W, bits = bf16(rng.standard_normal(rows_k))
+    w, bound = zq.DenseWeight(bits), (k / 64 + 8) * 2.0 ** -24
+    glu = zq.DenseWeight(bits, bits)
+    x = held(rng.standard_normal((8, k)) * 0.1, f32)
+    want, size = x @ W.T, np.abs(x) @ np.abs(W.T)
+    for T in range(1, 9):
+        xr = zq.dense_rows(torch.tensor(x[:T]), f32)
+        got = w.linear(xr).cpu().numpy().astype(np.float64)
+        assert (np.abs(got - want[:T]) <= bound * size[:T]).all(), T
+        close(glu.glu(xr, zq.GLU_SILU)[:, :rows_k[0]], plain.silu(want[:T]) * want[:T], 2e-5 if f32 else 5e-3, "T=%d" % T)
+
+
 def test_linear_many_tiles(zq):
     """More tiles than CTAs, so that the accumulators take turns, with ragged edges on both sides."""
     rng = np.random.default_rng(2)

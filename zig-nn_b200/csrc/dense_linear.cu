@@ -1,5 +1,5 @@
 // Linears over bf16 weights for few activation rows: one warp (or, for short deep matrices, the four warps of a
-// CTA) per few weight rows, 16-byte weight loads one step ahead of their use, the first of them ahead of the wait
+// CTA) per few weight rows, 16-byte weight loads one to four steps ahead of their use, the first of them ahead of the wait
 // for the producing kernel. f32 activations take this path for any number of rows; many bf16 rows go to the
 // tensor cores (gemm_bf16.cu).
 #include "dense.h"
@@ -32,12 +32,90 @@ struct GemvParams {
     GluSpec glu_shared;
 };
 
+// Sums and products of two neighbouring columns at once: half the instructions of scalar multiply-adds.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c) {
+    f32x2 d;
+    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+    return d;
+}
+__device__ __forceinline__ f32x2 pair_of(float lo, float hi) {
+    f32x2 d;
+    asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
+    return d;
+}
+__device__ __forceinline__ float pair_sum(f32x2 a) {
+    float lo, hi;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(lo), "=f"(hi) : "l"(a));
+    return lo + hi;
+}
+// Eight consecutive activations as they lie in memory, and as four pairs.
+template <typename TX>
+struct XChunk;
+template <>
+struct XChunk<bf16> {
+    uint4 v;
+};
+template <>
+struct XChunk<float> {
+    float4 a, b;
+};
+__device__ __forceinline__ void pairs(const uint4& u, f32x2 (&f)[4]) {
+    f[0] = pair_of(bf16_lo(u.x), bf16_hi(u.x));
+    f[1] = pair_of(bf16_lo(u.y), bf16_hi(u.y));
+    f[2] = pair_of(bf16_lo(u.z), bf16_hi(u.z));
+    f[3] = pair_of(bf16_lo(u.w), bf16_hi(u.w));
+}
+__device__ __forceinline__ void pairs(const XChunk<bf16>& x, f32x2 (&f)[4]) { pairs(x.v, f); }
+__device__ __forceinline__ void pairs(const XChunk<float>& x, f32x2 (&f)[4]) {
+    f[0] = pair_of(x.a.x, x.a.y);
+    f[1] = pair_of(x.a.z, x.a.w);
+    f[2] = pair_of(x.b.x, x.b.y);
+    f[3] = pair_of(x.b.z, x.b.w);
+}
+// Sums of N values over a warp. While the count is even a lane keeps half of its values and hands the other half on (16
+// values cost 16 exchanges in place of 80); it ends with the sums of the values from `result` on, as many as
+// N's odd part.
+template <int N, int OFF, int M>
+__device__ __forceinline__ uint32_t warp_sums(float (&v)[M], uint32_t lane) {
+    if constexpr (OFF == 0) {
+        return 0;
+    } else if constexpr (N % 2 == 0) {
+        const bool upper = lane & OFF;
+#pragma unroll
+        for (int i = 0; i < N / 2; ++i) {
+            const float give = upper ? v[i] : v[i + N / 2], keep = upper ? v[i + N / 2] : v[i];
+            v[i] = keep + __shfl_xor_sync(0xFFFFFFFFu, give, OFF);
+        }
+        return (upper ? N / 2 : 0) + warp_sums<N / 2, OFF / 2>(v, lane);
+    } else {
+#pragma unroll
+        for (int i = 0; i < N; ++i) v[i] += __shfl_xor_sync(0xFFFFFFFFu, v[i], OFF);
+        return warp_sums<N, OFF / 2>(v, lane);
+    }
+}
+
 // TR activation rows x RW weight rows per warp; SK: the four warps share the rows and split K.
+// Bound: for one row the latency of a step's chain of launches (a layer's matrices come from L2 ahead of their turn, the vocabulary's
+// at 5.3 TB/s); for several rows the instructions on the activations, which every warp unpacks for itself. Hence pairs of columns per
+// multiply-add, a reduction by halves, chunks requested again as soon as they are used, and a form for 3 and for 6 rows: at 6 rows of
+// 768 a layer's matrix takes 2.6 us of a step's chain in place of 4.7, the 50304-row vocabulary 32 us in place of 39 (77 MB, 12 us at
+// the memory's rate: short rows leave a warp three chunks and a reduction).
 // GLU: RW counts features, each one gate and one up row.
+// CTAs that an SM has to hold, of a kernel for TR activation rows and NR weight rows per warp. One row: the grids of a step (a CTA
+// per weight row with SK) run at once; with the 68 registers that the compiler takes of its own, 1152 rows are more than a wave and a
+// layer's output projection takes 3.3 us in place of 2.8. More rows: as many as cost no spills.
+template <typename TX, int TR, int RW, bool GLU, bool MOE>
+struct GemvShape {
+    static constexpr int NR = GLU ? 2 * RW : RW;
+    static constexpr int ctas = MOE ? 5 : TR == 1 ? (NR == 1 ? 9 : NR == 2 ? 6 : 4) : GLU ? 1 : sizeof(TX) == 4 ? 3 : RW == 2 && TR != 6 ? 4 : 5;
+    // chunks of a weight row that a lane holds ahead
+    static constexpr int ahead = TR == 1 ? (NR == 1 ? 4 : 2) : NR * TR > 16 ? 1 : NR * TR > 8 ? 2 : 4;
+};
 template <typename TX, int TR, int RW, bool SK, bool GLU, bool MOE>
-__global__ void __launch_bounds__(kGemvWarps * 32)
+__global__ void __launch_bounds__(kGemvWarps * 32, GemvShape<TX, TR, RW, GLU, MOE>::ctas)
 dense_gemv_kernel(const __grid_constant__ GemvParams p) {
-    constexpr int NR = GLU ? 2 * RW : RW;
+    constexpr int NR = GLU ? 2 * RW : RW, P = RW * TR;
     __shared__ float red[SK ? kGemvWarps * NR * TR : 1];
     pdl_launch_dependents();
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -96,95 +174,100 @@ dense_gemv_kernel(const __grid_constant__ GemvParams p) {
         const uint32_t j = min(j0 + (GLU ? lane / 2 : lane), rows - 1);
         prefetch_l2_bulk(w + (size_t)(w_row0 + (GLU ? glu_row(j, lane & 1) : j)) * kp, kp * 2);
     }
-    const TX* xr[TR];
+    const XChunk<TX>* xr[TR];
 #pragma unroll
-    for (int t = 0; t < TR; ++t) xr[t] = x + (size_t)(x_row0 + min((uint32_t)t, nt - 1)) * kp;
+    for (int t = 0; t < TR; ++t)
+        xr[t] = reinterpret_cast<const XChunk<TX>*>(x + (size_t)(x_row0 + min((uint32_t)t, nt - 1)) * kp);
 
     const uint32_t n_chunks = kp / 8;  // 16 bytes of a weight row each
-    const uint32_t step = SK ? kGemvWarps * 32 : 32;
+    constexpr uint32_t step = SK ? kGemvWarps * 32 : 32;
     uint32_t c = SK ? threadIdx.x : lane;
-    float acc[NR][TR];
+    f32x2 sums[NR][TR];  // of the even and of the odd columns
 #pragma unroll
     for (int r = 0; r < NR; ++r)
 #pragma unroll
-        for (int t = 0; t < TR; ++t) acc[r][t] = 0.0f;
+        for (int t = 0; t < TR; ++t) sums[r][t] = 0;
 
-    constexpr int U = NR >= 4 ? 1 : (NR == 2 ? 2 : 4);  // chunks held ahead
-    uint4 cur[U][NR];
+    // Chunks of a lane held ahead, of the weights and of the activations: a chunk's registers are loaded again as soon as it is used.
+    constexpr int U = GemvShape<TX, TR, RW, GLU, MOE>::ahead;
+    constexpr int V = TR * sizeof(TX) <= 2 ? U : TR * sizeof(TX) <= 8 && U > 1 ? 2 : 1;
+    uint4 wq[U][NR];
 #pragma unroll
     for (int u = 0; u < U; ++u)
 #pragma unroll
         for (int r = 0; r < NR; ++r)
-            cur[u][r] = c + u * step < n_chunks ? __ldg(wr[r] + c + u * step) : make_uint4(0, 0, 0, 0);
+            wq[u][r] = c + u * step < n_chunks ? __ldg(wr[r] + c + u * step) : make_uint4(0, 0, 0, 0);
     if (!waited) pdl_wait();
-    while (c < n_chunks) {
-        uint4 nxt[U][NR];
+    XChunk<TX> xq[V][TR];
 #pragma unroll
-        for (int u = 0; u < U; ++u) {
-            const uint32_t cn = c + (U + u) * step;
+    for (int v = 0; v < V; ++v)
+        if (c + v * step < n_chunks)
 #pragma unroll
-            for (int r = 0; r < NR; ++r) nxt[u][r] = cn < n_chunks ? __ldg(wr[r] + cn) : make_uint4(0, 0, 0, 0);
-        }
+            for (int t = 0; t < TR; ++t) xq[v][t] = xr[t][c + v * step];
+    for (; c < n_chunks; c += U * step) {
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const uint32_t cc = c + u * step;
-            if (cc < n_chunks) {
-                float wf[NR][8];
+            if (cc >= n_chunks) break;
+            f32x2 wf[NR][4];
 #pragma unroll
-                for (int r = 0; r < NR; ++r) unpack8(cur[u][r], wf[r]);
+            for (int r = 0; r < NR; ++r) pairs(wq[u][r], wf[r]);
+            if (cc + U * step < n_chunks)
 #pragma unroll
-                for (int t = 0; t < TR; ++t) {
-                    float xf[8];
-                    load8(xr[t] + (size_t)cc * 8, xf);
-#pragma unroll
-                    for (int r = 0; r < NR; ++r)
-#pragma unroll
-                        for (int e = 0; e < 8; ++e) acc[r][t] = fmaf(wf[r][e], xf[e], acc[r][t]);
-                }
-            }
-        }
-#pragma unroll
-        for (int u = 0; u < U; ++u)
-#pragma unroll
-            for (int r = 0; r < NR; ++r) cur[u][r] = nxt[u][r];
-        c += U * step;
-    }
-#pragma unroll
-    for (int r = 0; r < NR; ++r)
-#pragma unroll
-        for (int t = 0; t < TR; ++t) acc[r][t] = warp_sum_f(acc[r][t]);
-    if (SK) {
-        if (lane == 0) {
-#pragma unroll
-            for (int r = 0; r < NR; ++r)
-#pragma unroll
-                for (int t = 0; t < TR; ++t) red[(warp * NR + r) * TR + t] = acc[r][t];
-        }
-        __syncthreads();
-        if (warp != 0) return;
-#pragma unroll
-        for (int r = 0; r < NR; ++r)
+                for (int r = 0; r < NR; ++r) wq[u][r] = __ldg(wr[r] + cc + U * step);
+            const bool more = cc + V * step < n_chunks;
 #pragma unroll
             for (int t = 0; t < TR; ++t) {
-                float s = red[r * TR + t];
+                f32x2 xf[4];
+                pairs(xq[u % V][t], xf);
+                if (more) xq[u % V][t] = xr[t][cc + V * step];
 #pragma unroll
-                for (int q = 1; q < kGemvWarps; ++q) s += red[(q * NR + r) * TR + t];
-                acc[r][t] = s;
+                for (int r = 0; r < NR; ++r)
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) sums[r][t] = fma2(wf[r][e], xf[e], sums[r][t]);
             }
-    }
-    // the values of the warp are the same in every lane: lane i writes value i
-#pragma unroll
-    for (int f = 0; f < RW; ++f)
-#pragma unroll
-        for (int t = 0; t < TR; ++t) {
-            if (lane != (uint32_t)((f * TR + t) & 31) || j0 + f >= rows || (uint32_t)t >= nt) continue;
-            const size_t o = (size_t)(y_row0 + t) * y_stride + y_col + j0 + f;
-            if (GLU)
-                static_cast<TX*>(yv)[o] = to_act<TX>(
-                    glu_value(acc[2 * f][t] * in_scale, acc[(2 * f + 1) % NR][t] * in_scale, glu.kind, glu.limit));
-            else
-                static_cast<float*>(yv)[o] = acc[f][t];
         }
+    }
+    float val[P], up[GLU ? P : 1];
+#pragma unroll
+    for (int i = 0; i < P; ++i) {
+        val[i] = pair_sum(sums[GLU ? 2 * (i / TR) : i / TR][i % TR]);
+        if (GLU) up[i % (GLU ? P : 1)] = pair_sum(sums[(2 * (i / TR) + 1) % NR][i % TR]);
+    }
+    const uint32_t first = warp_sums<P, 16>(val, lane);
+    if (GLU) warp_sums<GLU ? P : 1, 16>(up, lane);
+    auto write = [&](uint32_t i, float v, float u) {
+        const uint32_t f = i / TR, t = i % TR;
+        if (j0 + f >= rows || t >= nt) return;
+        const size_t o = (size_t)(y_row0 + t) * y_stride + y_col + j0 + f;
+        if (GLU)
+            static_cast<TX*>(yv)[o] = to_act<TX>(glu_value(v * in_scale, u * in_scale, glu.kind, glu.limit));
+        else
+            static_cast<float*>(yv)[o] = v;
+    };
+    constexpr int KEPT = P / (P & -P), LANES = 32 / (P & -P);  // LANES neighbours have the same KEPT sums
+    if (!SK) {
+        if (lane % LANES == 0)
+#pragma unroll
+            for (int k = 0; k < KEPT; ++k) write(first + k, val[k], up[GLU ? k : 0]);
+        return;
+    }
+    if (lane % LANES == 0)
+#pragma unroll
+        for (int k = 0; k < KEPT; ++k) {
+            red[warp * NR * TR + first + k] = val[k];
+            if (GLU) red[warp * NR * TR + P + first + k] = up[GLU ? k : 0];
+        }
+    __syncthreads();
+    if (threadIdx.x >= P) return;
+    const float* part = red + threadIdx.x;
+    float v = part[0], u = GLU ? part[P] : 0.0f;
+#pragma unroll
+    for (int q = 1; q < kGemvWarps; ++q) {
+        v += part[q * NR * TR];
+        if (GLU) u += part[q * NR * TR + P];
+    }
+    write(threadIdx.x, v, u);
 }
 
 template <typename TX, int TR, bool GLU, bool MOE>
@@ -212,7 +295,9 @@ template <typename TX, bool GLU>
 int gemv_rows(const GemvParams& p, uint32_t rows, uint32_t n_groups, cudaStream_t st) {
     if (p.T == 1) return gemv_shape<TX, 1, GLU, false>(p, rows, p.kp, n_groups, 1, st);
     if (p.T == 2) return gemv_shape<TX, 2, GLU, false>(p, rows, p.kp, n_groups, 1, st);
-    if (p.T <= 4) return gemv_shape<TX, 4, GLU, false>(p, rows, p.kp, n_groups, 1, st);
+    if (p.T == 3) return gemv_shape<TX, 3, GLU, false>(p, rows, p.kp, n_groups, 1, st);
+    if (p.T == 4) return gemv_shape<TX, 4, GLU, false>(p, rows, p.kp, n_groups, 1, st);
+    if (p.T <= 6) return gemv_shape<TX, 6, GLU, false>(p, rows, p.kp, n_groups, 1, st);
     return gemv_shape<TX, 8, GLU, false>(p, rows, p.kp, n_groups, (p.T + 7) / 8, st);
 }
 
