@@ -193,6 +193,26 @@ def test_delta_portions_and_steps(zq, f32, shape):
         assert torch.equal(state[0], dev(start[0]))
 
 
+@pytest.mark.parametrize("taps,ranks", [(1, (64, 72)), (4, (3, 64)), (5, (130, 2)), (2, (27800, 3))])
+def test_delta_step_ahead_of_its_row(zq, taps, ranks):
+    """One token: taps and ranks that fit the registers loaded ahead of the row and that do not, positions before the ring is
+    full, and a rank whose staging leaves room for one sum at a time. Tolerance as for the steps above."""
+    (ra, rg), (H, d, e) = ranks, (1, 4, 4) if max(ranks) > 1000 else (2, 40, 72)
+    rng = np.random.default_rng(6)
+    x, conv, A, dt, a2, g2, low, n = delta_case(rng, 1, H, H, d, e, taps, ra, rg)
+    for pos in (0, 1, 3, 11):
+        before = rng.standard_normal((taps - 1, conv.shape[0])).astype(np.float32)
+        ring = dev(ring_of(before, pos, taps, 1, 0, rng))
+        before[:max(0, taps - 1 - pos)] = 0
+        start = rng.standard_normal((1, H, d, e)).astype(np.float32)
+        state = dev(start)
+        out = zq.delta(dev(x), H, H, d, e, taps, ra, rg, dev(conv), dev(A), dev(dt), zq.DenseWeight(low), dev(n), 1e-5, state, ring, [pos],
+                       [0], False, True)
+        want, S = delta_plain(x, H, H, d, e, taps, ra, conv, A, dt, a2, g2, n, 1e-5, start[0].astype(np.float64), before.astype(np.float64))
+        close(out[:, :H * e], want, 3e-5, "pos %d" % pos)
+        close(state[0], S, 2e-5)
+
+
 @pytest.mark.parametrize("f32", PRECISIONS)
 def test_delta_of_several_sequences_at_once(zq, f32):
     rng = np.random.default_rng(5)

@@ -380,6 +380,28 @@ __device__ __forceinline__ float conv_silu(const DeltaArgs& a, uint32_t channels
     return silu_f(fmaf(w[a.taps - 1], x[0], acc));
 }
 
+// The same for the next token of a sequence and up to kStepTaps taps: the places of the ring are requested together, and the
+// weights come from the caller, who has them before the token's row is there.
+constexpr uint32_t kStepTaps = 4;
+__device__ __forceinline__ void conv_weights(const DeltaArgs& a, uint32_t c, float (&w)[kStepTaps]) {
+#pragma unroll
+    for (uint32_t j = 0; j < kStepTaps; ++j) w[j] = j < a.taps ? a.conv[(size_t)c * a.taps + a.taps - 1 - j] : 0.0f;  // j tokens back
+}
+__device__ __forceinline__ float conv_silu_step(const DeltaArgs& a, uint32_t channels, float x, uint32_t pos, uint32_t slot, uint32_t c,
+                                                const float (&w)[kStepTaps]) {
+    const uint32_t here = pos % a.taps;
+    const float* ring = a.ring + (size_t)slot * a.taps * channels + c;
+    float v[kStepTaps];
+#pragma unroll
+    for (uint32_t j = 1; j < kStepTaps; ++j)
+        v[j] = j < a.taps && j <= pos ? ring[(size_t)(here >= j ? here - j : here + a.taps - j) * channels] : 0.0f;
+    float acc = 0.0f;
+#pragma unroll
+    for (uint32_t j = kStepTaps - 1; j > 0; --j)
+        if (j < a.taps) acc = fmaf(w[j], v[j], acc);
+    return silu_f(fmaf(w[0], x, acc));
+}
+
 __device__ __forceinline__ float channel_decay(float x, float A_log, float dt_bias) { return expf(-expf(A_log) * softplus_f(x + dt_bias)); }
 
 // Inputs of the low-rank products as activation rows.
@@ -707,11 +729,12 @@ memory_chunk_kernel(const __grid_constant__ MemoryArgs a, const __grid_constant_
 // Threads: CP of them side by side along a row of the state (VEC columns each), RG rows at a time.
 struct StepShape {
     uint32_t cp, rg;
+    bool both;  // shared memory holds the partial columns of two sums
 };
 inline StepShape step_shape(uint32_t vdim, uint32_t vec, uint32_t threads) {
     uint32_t cp = 1;
     while (cp < (vdim + vec - 1) / vec && cp < threads) cp <<= 1;
-    return StepShape{cp, threads / cp};
+    return StepShape{cp, threads / cp, false};
 }
 template <int VEC>
 struct Cols {
@@ -761,14 +784,52 @@ __device__ __forceinline__ void meet(float* red, const Cols<VEC>& mine, const St
     __syncthreads();
 }
 
-// Head norm and gate of the head's o in shared memory.
+// Two of them at once, red twice as long.
+template <int VEC>
+__device__ __forceinline__ void meet_two(float* red, const Cols<VEC>& a, const Cols<VEC>& b, const StepShape& s, float* out_a,
+                                         float* out_b, uint32_t limit) {
+    const uint32_t w = s.cp * VEC, cx = threadIdx.x % s.cp, rg = threadIdx.x / s.cp, second = s.rg * w;
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) {
+        red[rg * w + cx * VEC + e] = a.v[e];
+        red[second + rg * w + cx * VEC + e] = b.v[e];
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < 2 * w; i += blockDim.x) {
+        const uint32_t c = i < w ? i : i - w;
+        if (c >= limit) continue;
+        const float* p = red + (i < w ? 0 : second) + c;
+        float t = p[0];
+        for (uint32_t g = 1; g < s.rg; ++g) t += p[g * w];
+        (i < w ? out_a : out_b)[c] = t;
+    }
+    __syncthreads();
+}
+// Sums of two values over the block, as block_sum_f has them, behind one pair of barriers.
+__device__ __forceinline__ void block_sum_two(float& a, float& b, float* red_a, float* red_b) {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = (blockDim.x + 31) >> 5;
+    a = warp_sum_f(a);
+    b = warp_sum_f(b);
+    if (lane == 0) {
+        red_a[warp] = a;
+        red_b[warp] = b;
+    }
+    __syncthreads();
+    a = warp_sum_f(lane < nw ? red_a[lane] : 0.0f);
+    b = warp_sum_f(lane < nw ? red_b[lane] : 0.0f);
+    __syncthreads();
+}
+constexpr int kLowAhead = 2;  // chunks of eight that a thread holds of a row of the low-rank matrices (a rank of up to 64)
+
+// Head norm and gate of the head's o in shared memory; own: norm of the thread's first column, loaded early.
 template <typename TA>
-__device__ __forceinline__ void finish_head(const float* os, const float* gate, const float* norm, uint32_t E, float eps,
+__device__ __forceinline__ void finish_head(const float* os, const float* gate, const float* norm, float own, uint32_t E, float eps,
                                             TA* row, uint32_t h, uint32_t heads, uint32_t out_pitch, float* red) {
     float ss = 0.0f;
     for (uint32_t c = threadIdx.x; c < E; c += blockDim.x) ss = fmaf(os[c], os[c], ss);
     const float inv = 1.0f / sqrtf(block_sum_f(ss, red) / (float)E + eps);
-    for (uint32_t c = threadIdx.x; c < E; c += blockDim.x) row[h * E + c] = to_act<TA>(os[c] * inv * norm[c] * gate[c]);
+    for (uint32_t c = threadIdx.x; c < E; c += blockDim.x)
+        row[h * E + c] = to_act<TA>(os[c] * inv * (c == threadIdx.x ? own : norm[c]) * gate[c]);
     if (h + 1 == heads)
         for (uint32_t c = heads * E + threadIdx.x; c < out_pitch; c += blockDim.x) row[c] = to_act<TA>(0.0f);
 }
@@ -782,7 +843,7 @@ memory_step_kernel(const __grid_constant__ MemoryArgs a, StepShape sh) {
     const uint32_t D = a.dim, E = a.vdim, kd = a.heads * D, vd = a.heads * E, h = blockIdx.x, r = blockIdx.y, tid = threadIdx.x;
     float *qs = sm, *ks = qs + D, *vs = ks + D, *gate = vs + E, *os = gate + E, *red = os + E;
     const float* norm = a.norm + h * E;
-    const float ib = a.i_bias[h], fb = a.f_bias[h];
+    const float ib = a.i_bias[h], fb = a.f_bias[h], own_norm = tid < E ? norm[tid] : 0.0f;
     pdl_wait();
     const float* row = a.in + (size_t)r * a.ld;
     const size_t at = (size_t)(uint32_t)a.slots[r] * a.heads + h;
@@ -837,14 +898,17 @@ memory_step_kernel(const __grid_constant__ MemoryArgs a, StepShape sh) {
         meet<VEC>(red, o, sh, os + c0, E - c0);
     }
     for (uint32_t c = tid; c < E; c += blockDim.x) os[c] /= size;
-    finish_head<TA>(os, gate, norm, E, a.eps, static_cast<TA*>(a.out) + (size_t)r * a.out_pitch, h, a.heads, a.out_pitch, red33);
+    finish_head<TA>(os, gate, norm, own_norm, E, a.eps, static_cast<TA*>(a.out) + (size_t)r * a.out_pitch, h, a.heads, a.out_pitch, red33);
 }
 
+// Bound: the latency of a chain of dependent steps (row -> convolution -> norms -> decays -> state -> head norm), not its bytes
+// (0.4 MB of state for six sequences of twelve heads of 64 x 64). So what does not depend on the row is in registers before the row
+// is there, the taps are read together, and two sums share a pair of barriers (one sequence of nine heads of 128 x 128: a step of four such layers 15 us shorter).
 template <int VEC, typename TA>
 __global__ void __launch_bounds__(512)
 delta_step_kernel(const __grid_constant__ DeltaArgs a, StepShape sh) {
     extern __shared__ __align__(16) float sm[];
-    __shared__ float red33[33];
+    __shared__ float red33[33], red33b[33];
     pdl_launch_dependents();
     const uint32_t D = a.dim, E = a.vdim, h = blockIdx.x, r = blockIdx.y, tid = threadIdx.x, kp = a.low.kp;
     const uint32_t kd = a.kv_heads * D, vd = a.heads * E, channels = 2 * kd + vd, kv = h / (a.heads / a.kv_heads);
@@ -854,7 +918,25 @@ delta_step_kernel(const __grid_constant__ DeltaArgs a, StepShape sh) {
     const bf16* low_g = a.low.w + ((size_t)a.heads * D + (size_t)h * E) * kp;
     if (tid == 0) prefetch_l2_bulk(low_a, D * kp * 2);
     if (tid == 1) prefetch_l2_bulk(low_g, E * kp * 2);
-    const float decay = a.A_log[h];
+    // What does not depend on the token is loaded ahead of the wait: parameters of the thread's first channel, and of the low-rank
+    // matrices the first kLowAhead chunks of the thread's first two rows.
+    const float decay = a.A_log[h], own_norm = tid < E ? a.norm[tid] : 0.0f;
+    const bool short_conv = a.taps <= kStepTaps;
+    auto channel = [&](uint32_t i) { return i < D ? kv * D + i : i < 2 * D ? kd + kv * D + (i - D) : 2 * kd + h * E + (i - 2 * D); };
+    float cw[kStepTaps];
+    if (short_conv && tid < 2 * D + E) conv_weights(a, channel(tid), cw);
+    const uint32_t sub = tid & 3, low_step = blockDim.x / 4;
+    auto low_row = [&](uint32_t i) {
+        return reinterpret_cast<const uint4*>(i < D ? low_a + (size_t)i * kp : low_g + (size_t)(i - D) * kp);
+    };
+    uint4 low_w[2][kLowAhead];
+#pragma unroll
+    for (int n = 0; n < 2; ++n) {
+        const uint32_t i = n * low_step + (tid >> 2);
+#pragma unroll
+        for (int c = 0; c < kLowAhead; ++c)
+            if (i < D + E && sub + 4 * c < kp / 8) low_w[n][c] = __ldg(low_row(i) + sub + 4 * c);
+    }
     pdl_wait();
     const float* row = a.in + (size_t)r * a.ld;
     const uint32_t slot = (uint32_t)a.slots[r], pos = (uint32_t)a.pos[r];
@@ -870,8 +952,14 @@ delta_step_kernel(const __grid_constant__ DeltaArgs a, StepShape sh) {
     float qq = 0.0f, kk = 0.0f;
     float* ring = a.taps > 1 ? a.ring + ((size_t)slot * a.taps + pos % a.taps) * channels : nullptr;
     for (uint32_t i = tid; i < 2 * D + E; i += blockDim.x) {
-        const uint32_t c = i < D ? kv * D + i : i < 2 * D ? kd + kv * D + (i - D) : 2 * kd + h * E + (i - 2 * D);
-        const float x = conv_silu(a, channels, r, 0, pos, slot, c);
+        const uint32_t c = channel(i);
+        float x;
+        if (short_conv) {
+            if (i != tid) conv_weights(a, c, cw);
+            x = conv_silu_step(a, channels, row[c], pos, slot, c, cw);
+        } else {
+            x = conv_silu(a, channels, r, 0, pos, slot, c);
+        }
         if (ring) ring[c] = row[c];  // heads that share q and k write the same; nobody reads this place in this step
         if (i < D) {
             qs[i] = x;
@@ -883,24 +971,30 @@ delta_step_kernel(const __grid_constant__ DeltaArgs a, StepShape sh) {
             vs[i - 2 * D] = x;
         }
     }
-    const float fq = 1.0f / sqrtf(block_sum_f(qq, red33) + 1e-6f) / sqrtf((float)D), fk = 1.0f / sqrtf(block_sum_f(kk, red33) + 1e-6f);
+    block_sum_two(qq, kk, red33, red33b);
+    const float fq = 1.0f / sqrtf(qq + 1e-6f) / sqrtf((float)D), fk = 1.0f / sqrtf(kk + 1e-6f);
     const float beta = sigmoid_f(row[channels + h]);
     // decays and gates: four neighbouring threads share a row of the low-rank matrix
-    const uint32_t sub = tid & 3;
-    for (uint32_t base = 0; base < D + E; base += blockDim.x / 4) {
+    auto low = [&](uint32_t base, const uint4* held) {
         const uint32_t i = base + (tid >> 2);
         float acc = 0.0f;
         if (i < D + E) {
-            const uint4* w = reinterpret_cast<const uint4*>(i < D ? low_a + (size_t)i * kp : low_g + (size_t)(i - D) * kp);
+            const uint4* w = low_row(i);
             const float* x = i < D ? lo : lo + kp;
-#pragma unroll 4
-            for (uint32_t c = sub; c < kp / 8; c += 4) {
+            auto add = [&](const uint4& u, uint32_t c) {
                 float wf[8];
-                unpack8(__ldg(w + c), wf);
+                unpack8(u, wf);
                 const float4 p = reinterpret_cast<const float4*>(x + 8 * c)[0], q = reinterpret_cast<const float4*>(x + 8 * c)[1];
                 acc += (wf[0] * p.x + wf[1] * p.y) + (wf[2] * p.z + wf[3] * p.w) +
                        ((wf[4] * q.x + wf[5] * q.y) + (wf[6] * q.z + wf[7] * q.w));
-            }
+            };
+            uint32_t c = sub;
+            if (held)
+#pragma unroll
+                for (int k = 0; k < kLowAhead; ++k, c += 4)
+                    if (c < kp / 8) add(held[k], c);
+#pragma unroll 4
+            for (; c < kp / 8; c += 4) add(__ldg(w + c), c);
         }
         acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 1);
         acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 2);
@@ -910,7 +1004,10 @@ delta_step_kernel(const __grid_constant__ DeltaArgs a, StepShape sh) {
             else
                 gate[i - D] = sigmoid_f(acc);
         }
-    }
+    };
+    low(0, low_w[0]);
+    if (low_step < D + E) low(low_step, low_w[1]);
+    for (uint32_t base = 2 * low_step; base < D + E; base += low_step) low(base, nullptr);
     float kq = 0.0f;
     for (uint32_t i = tid; i < D; i += blockDim.x) {
         const float q = qs[i] * fq, k = ks[i] * fk;
@@ -941,8 +1038,12 @@ delta_step_kernel(const __grid_constant__ DeltaArgs a, StepShape sh) {
                 }
             }
         }
-        meet<VEC>(red, y, sh, ys + c0, E - c0);
-        meet<VEC>(red, o, sh, os + c0, E - c0);
+        if (sh.both) {
+            meet_two<VEC>(red, y, o, sh, ys + c0, os + c0, E - c0);
+        } else {
+            meet<VEC>(red, y, sh, ys + c0, E - c0);
+            meet<VEC>(red, o, sh, os + c0, E - c0);
+        }
         if (c < E) {
             float u[VEC];
 #pragma unroll
@@ -970,17 +1071,17 @@ delta_step_kernel(const __grid_constant__ DeltaArgs a, StepShape sh) {
         }
     }
     for (uint32_t c = tid; c < E; c += blockDim.x) os[c] = fmaf(beta * (vs[c] - ys[c]), kq, os[c]);
-    finish_head<TA>(os, gate, a.norm, E, a.eps, static_cast<TA*>(a.out) + (size_t)r * a.out_pitch, h, a.heads, a.out_pitch, red33);
+    finish_head<TA>(os, gate, a.norm, own_norm, E, a.eps, static_cast<TA*>(a.out) + (size_t)r * a.out_pitch, h, a.heads, a.out_pitch, red33);
 }
 
 // ---- launches ------------------------------------------------------------------------------------------------------
 int done(cudaError_t e) { return e == cudaSuccess ? ZQ_OK : cuda_fail(e); }
 
+constexpr size_t kMaxSmem = 220 * 1024;
 template <typename K>
 int allow_smem(K kern, size_t smem) {
-    constexpr size_t kMost = 220 * 1024;
-    if (smem > kMost) return ZQ_ERR_LIMIT;
-    if (smem > 48 * 1024) ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
+    if (smem > kMaxSmem) return ZQ_ERR_LIMIT;
+    if (smem > 48 * 1024) ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxSmem));
     return ZQ_OK;
 }
 
@@ -1021,11 +1122,14 @@ uint32_t step_threads(uint32_t dim, uint32_t vdim) {
     return n >= 16384 ? 512 : n >= 4096 ? 256 : 128;
 }
 template <typename Args, typename K>
-int step(const Args& a, K vec_f32, K vec_bf16, K one_f32, K one_bf16, size_t floats, uint32_t rows, bool f32, cudaStream_t st) {
+int step(const Args& a, K vec_f32, K vec_bf16, K one_f32, K one_bf16, size_t floats, bool two_sums, uint32_t rows, bool f32,
+         cudaStream_t st) {
     const bool v4 = a.vdim % 4 == 0;
     const uint32_t threads = step_threads(a.dim, a.vdim);
-    const StepShape sh = step_shape(a.vdim, v4 ? 4 : 1, threads);
-    const size_t smem = (floats + threads * (v4 ? 4 : 1)) * sizeof(float);
+    StepShape sh = step_shape(a.vdim, v4 ? 4 : 1, threads);
+    const size_t sum = threads * (v4 ? 4 : 1);
+    sh.both = two_sums && (floats + 2 * sum) * sizeof(float) <= kMaxSmem;
+    const size_t smem = (floats + (sh.both ? 2 : 1) * sum) * sizeof(float);
     K kern = v4 ? (f32 ? vec_f32 : vec_bf16) : (f32 ? one_f32 : one_bf16);
     const int rc = allow_smem(kern, smem);
     return rc != ZQ_OK ? rc : done(launch_pdl(kern, dim3(a.heads, rows), dim3(threads), smem, st, a, sh));
@@ -1076,7 +1180,7 @@ int launch_memory(const MemoryArgs& a, uint32_t rows, bool one_sequence, bool f3
     const uint32_t kd = a.heads * a.dim, vd = a.heads * a.vdim;
     if (!one_sequence || rows == 1)
         return step(a, memory_step_kernel<4, float>, memory_step_kernel<4, bf16>, memory_step_kernel<1, float>,
-                    memory_step_kernel<1, bf16>, 2 * (size_t)a.dim + 3 * (size_t)a.vdim, rows, f32, st);
+                    memory_step_kernel<1, bf16>, 2 * (size_t)a.dim + 3 * (size_t)a.vdim, false, rows, f32, st);
     FinishParams f{};
     f.heads = a.heads;
     f.vdim = a.vdim;
@@ -1154,7 +1258,7 @@ int launch_delta(const DeltaArgs& a, uint32_t rows, bool one_sequence, bool f32,
     if (a.dim == 0 || a.vdim == 0 || a.dim > kStateMaxDim || a.vdim > 4096) return ZQ_ERR_LIMIT;
     if (!one_sequence || rows == 1)
         return step(a, delta_step_kernel<4, float>, delta_step_kernel<4, bf16>, delta_step_kernel<1, float>, delta_step_kernel<1, bf16>,
-                    2 * (size_t)a.low.kp + 3 * (size_t)a.dim + 4 * (size_t)a.vdim, rows, f32, st);
+                    2 * (size_t)a.low.kp + 3 * (size_t)a.dim + 4 * (size_t)a.vdim, true, rows, f32, st);
     if (rows > a.max_rows) return ZQ_ERR_BAD_ARG;
     const uint32_t kd = a.kv_heads * a.dim, hd = a.heads * a.dim, vd = a.heads * a.vdim;
     const size_t R = a.max_rows;
