@@ -885,11 +885,10 @@ int zq_gemma3_decode_next_batch(zq_gemma3* m, const uint32_t* h_tokens, zq_strea
         if (m->seq_lens[r] >= m->c.ctx) return ZQ_ERR_SEQUENCE;
     }
     cudaStream_t st = as_stream(stream);
-    ZQ_CUDA(cudaMemcpyAsync(m->d_tokens, h_tokens, m->n_seq * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-    ZQ_CUDA(cudaMemcpyAsync(m->d_pos, m->seq_lens.data(), m->n_seq * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-    ZQ_CUDA(cudaStreamSynchronize(st));  // both sources are host memory that changes below / belongs to the caller
+    int rc = set_step_rows(nullptr, h_tokens, m->seq_lens.data(), m->n_seq, m->d_tokens, m->d_pos, nullptr, st);
+    if (rc != ZQ_OK) return rc;
     // tokens and positions live in device memory: the launch sequence is the same every step and is replayed
-    int rc = m->graphs.run(STEP_BATCH, st, [&](cudaStream_t s2) { return gemma3_forward(m, m->n_seq, STEP_LOGITS, s2, 0, true); });
+    rc = m->graphs.run(STEP_BATCH, st, [&](cudaStream_t s2) { return gemma3_forward(m, m->n_seq, STEP_LOGITS, s2, 0, true); });
     if (rc != ZQ_OK) return rc;
     for (uint32_t r = 0; r < m->n_seq; ++r) m->seq_lens[r] += 1;
     m->seq_len = m->seq_lens[0];

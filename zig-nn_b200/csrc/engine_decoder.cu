@@ -1017,24 +1017,19 @@ int zq_decoder_decode_next(zq_decoder* m, uint32_t seq, uint32_t token, zq_strea
 int zq_decoder_decode_next_batch(zq_decoder* m, const uint32_t* h_seqs, const uint32_t* h_tokens, uint32_t n,
                                  zq_stream stream, const float** d_logits) {
     if (!m || !h_seqs || !h_tokens || !d_logits || n == 0 || n > m->c.n_seq) return ZQ_ERR_BAD_ARG;
-    std::vector<uint32_t> pos(n);
     std::vector<bool> seen(m->c.n_seq, false);
     for (uint32_t r = 0; r < n; ++r) {
         const uint32_t s = h_seqs[r];
         if (s >= m->c.n_seq || seen[s] || h_tokens[r] >= m->c.vocab) return ZQ_ERR_BAD_ARG;
         if (m->seq_lens[s] >= m->c.ctx) return ZQ_ERR_SEQUENCE;
         seen[s] = true;
-        pos[r] = m->seq_lens[s];
     }
     cudaStream_t st = as_stream(stream);
-    ZQ_CUDA(cudaMemcpyAsync(m->d_tokens, h_tokens, n * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-    ZQ_CUDA(cudaMemcpyAsync(m->d_slots, h_seqs, n * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-    ZQ_CUDA(cudaMemcpyAsync(m->d_pos, pos.data(), n * sizeof(uint32_t), cudaMemcpyHostToDevice, st));
-    ZQ_CUDA(cudaStreamSynchronize(st));  // the sources are host memory of the caller
+    int rc = set_step_rows(h_seqs, h_tokens, m->seq_lens.data(), n, m->d_tokens, m->d_pos, m->d_slots, st);
+    if (rc != ZQ_OK) return rc;
     Pass P{n, false, 0, true, 0, nullptr, false, 0, 0};
     // every slot in one step is the recorded shape
-    const int rc = n == m->c.n_seq ? m->graphs.run(STEP_BATCH, st, [&](cudaStream_t s) { return forward(m, P, s); })
-                                   : forward(m, P, st);
+    rc = n == m->c.n_seq ? m->graphs.run(STEP_BATCH, st, [&](cudaStream_t s) { return forward(m, P, s); }) : forward(m, P, st);
     if (rc != ZQ_OK) return rc;
     for (uint32_t r = 0; r < n; ++r) m->seq_lens[h_seqs[r]] += 1;
     *d_logits = m->logits;
