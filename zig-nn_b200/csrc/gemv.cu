@@ -505,7 +505,7 @@ int zq_matmul(const zq_weight* w, const float* d_x, float* d_y, uint32_t m_rows,
             ((uintptr_t)d_workspace & 255) == 0 && workspace_bytes >= gemm_tc_workspace_bytes(w, m_rows))
             return launch_gemm_tc(w, d_x, d_y, m_rows, epilogue, d_workspace, st);
         // other calls of 17-48 rows: one f32-accurate product in place of two and more passes, where it is faster (3072 <- 768
-        // at 24 rows 17 us in passes, 8.6 split; 1152 <- 6912 at 48 rows 137 and 31; up to 16 rows one pass is faster)
+        // at 48 rows 31 us in passes, 7.4 split; up to 16 rows one pass is faster)
         if (gemm_split_takes(w, m_rows) && d_workspace && ((uintptr_t)d_workspace & 255) == 0 &&
             workspace_bytes >= gemm_split_workspace_bytes(w, m_rows))
             return launch_gemm_split(w, d_x, d_y, m_rows, epilogue, d_workspace, st);
