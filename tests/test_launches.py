@@ -1,0 +1,50 @@
+"""Which kernels a call launches, with which grid and in which order, by the library linked with a runtime that runs nothing."""
+import ctypes as C
+
+import numpy as np
+import pytest
+
+from host_runtime import Library, build
+from zignn_b200 import hostmodel
+
+
+@pytest.fixture(scope="module")
+def library(tmp_path_factory):
+    return Library(build(tmp_path_factory.mktemp("launches")))
+
+
+def u32(values):
+    return np.ascontiguousarray(values, np.uint32)
+
+
+def pointer(a):
+    return a.ctypes.data_as(C.c_void_p)
+
+
+LENISUN = dict(architecture="Lenisun", vocab=64, width=64, norm=dict(eps=1e-6), embedding=dict(scale=1.0), layers=[
+    dict(type="attention", mixer=dict(heads=2, kv_heads=1, dim=32, vdim=32, scale=0.2), mlp=dict(kind="dense", ff=64, limit=2.0))] * 2)
+
+
+def decoder(library, ctx=64, n_seq=3):
+    host = hostmodel.LenisunHost.synthetic(LENISUN, seed=1, std=0.2)
+    cfg, weights, engine = host.config_struct(ctx, n_seq, False), host.weights_struct(), C.c_void_p()
+    assert library.lib.zq_decoder_create(C.byref(cfg), C.byref(weights), None, C.byref(engine)) == 0
+    return engine
+
+
+def test_a_step_starts_when_its_rows_are_set(library):
+    """Kernels of a step read its positions and slots ahead of their wait, so its first kernel is no dependent launch; the others
+    are."""
+    engine, lg, lib = decoder(library), C.c_void_p(), library.lib
+    calls = [lambda: lib.zq_decoder_decode_next(engine, 0, 5, None, C.byref(lg)),
+             lambda: lib.zq_decoder_decode_next_batch(engine, pointer(u32([2, 0])), pointer(u32([1, 2])), 2, None, C.byref(lg)),
+             lambda: lib.zq_decoder_decode_next_batch(engine, pointer(u32([2, 0, 1])), pointer(u32([1, 2, 3])), 3, None, C.byref(lg)),
+             lambda: lib.zq_decoder_decode_greedy(engine, 1, 5, 1, None, pointer(u32([0]))),
+             lambda: lib.zq_decoder_extend(engine, 1, pointer(u32([7])), 1, None, 0, None, None)]
+    for call in calls:
+        seen, status = library.launches(call)
+        assert status == 0 and any("gqa_decode" in l.name for l in seen)
+        assert "set_row" in seen[0].name or "set_step_rows" in seen[0].name
+        assert not seen[0].dependent and not seen[1].dependent, [l.name for l in seen]
+        assert all(l.dependent for l in seen[2:] if "feed_row" not in l.name and "argmax" not in l.name), [(l.name, l.dependent) for l in seen]
+    lib.zq_decoder_free(engine)

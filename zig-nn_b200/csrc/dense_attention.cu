@@ -248,8 +248,9 @@ gqa_decode_kernel(const __grid_constant__ AttnArgs a) {
     extern __shared__ __align__(16) unsigned char sm[];
     pdl_launch_dependents();
     // With `pre`, the row's own key and value are made here, by the CTA whose range ends with them: its copies stop
-    // ahead of them. Its position and the keys and values ahead of its own are then those of earlier steps, which no kernel
-    // of this one writes, and are requested before the wait; without, the kernel ahead may have written any of them.
+    // ahead of them. Its position and slot are then set ahead of the step's first kernel, which waits for that as a whole (forward,
+    // engine_decoder.cu), and the keys and values ahead of its own are those of earlier steps: no kernel that may still be at work
+    // writes any of them, and they are requested before the wait. Without `pre` the kernel ahead may have written all of them.
     const bool fused = a.pre.qkv != nullptr;
     if (!fused) pdl_wait();
     const GqaShape& s = a.s;

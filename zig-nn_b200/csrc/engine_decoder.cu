@@ -826,7 +826,13 @@ int forward(zq_decoder* m, const Pass& P, cudaStream_t st) {
     a.embed_w = m->embed_norm;
     a.tokens = m->d_tokens;
     set_next(m, P, 0, a);
-    RUN(launch_add_norm(a, P.rows, m->f32, st));
+    // Starts when the kernel that set the rows is complete and its stores are visible, and so does every kernel behind it, whose part
+    // ahead of its own wait may then read them (gqa_decode_kernel: positions, slots and the cache of earlier steps). As a dependent
+    // launch it could start behind the setting kernel's last thread, which promises no visibility, and the next two behind it.
+    whole_dependency = true;
+    const int first = launch_add_norm(a, P.rows, m->f32, st);
+    whole_dependency = false;
+    RUN(first);
     for (uint32_t l = 0; l < m->layers.size(); ++l) {
         const Layer& d = m->layers[l];
         a = norm_args(m);

@@ -75,6 +75,9 @@ __host__ __device__ inline size_t qs_word_offset(uint32_t qb, uint32_t blk, uint
 // earlier kernel writes (weights), and must call pdl_wait() before it touches anything an earlier
 // kernel produces or still reads: pdl_wait() returns only when every earlier grid has completed and
 // its writes are visible. Without the launch attribute both calls do nothing.
+// What lies ahead of a launch without the attribute (a plain one, or one with whole_dependency) is complete and visible to
+// that kernel and to every one behind it, ahead of their waits too. A kernel ahead of a dependent launch is not, however it
+// was launched itself: a dependent kernel may start once its predecessor's threads have ended, before their stores are visible.
 #ifdef __CUDACC__
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
