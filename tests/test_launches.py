@@ -5,7 +5,9 @@ import numpy as np
 import pytest
 
 from host_runtime import Library, build
-from zignn_b200 import hostmodel
+from zignn_b200 import ggml, hostmodel
+
+ACT_Q8, ERR_LIMIT = 1, 5
 
 
 @pytest.fixture(scope="module")
@@ -48,3 +50,27 @@ def test_a_step_starts_when_its_rows_are_set(library):
         assert not seen[0].dependent and not seen[1].dependent, [l.name for l in seen]
         assert all(l.dependent for l in seen[2:] if "feed_row" not in l.name and "argmax" not in l.name), [(l.name, l.dependent) for l in seen]
     lib.zq_decoder_free(engine)
+
+
+def weight(library, qtype, n, k):
+    raw, w = np.zeros(ggml.tensor_bytes(qtype, n * k), np.uint8), C.c_void_p()
+    assert library.lib.zq_weight_upload(pointer(raw), qtype, n, k, None, C.byref(w)) == 0
+    return w
+
+
+def matmul(library, w, m, act):
+    """Launches and status of a product; nothing reads its operands."""
+    lib, somewhere = library.lib, C.c_void_p(1 << 20)
+    size = lib.zq_matmul_workspace_bytes(w, m, act)
+    return library.launches(lambda: lib.zq_matmul(w, somewhere, somewhere, m, act, None, somewhere, size, None))
+
+
+@pytest.mark.parametrize("n", [8, 64, 128, 160, 300])
+def test_q8_rows_up_to_the_limit_of_a_grid(library, n):
+    """65535 CTAs of 64 rows, whatever the count of weight rows; what goes beyond is refused."""
+    w = weight(library, ggml.Q8_0, n, 32)
+    for m in (2097120, 2097121, 4194240):
+        seen, status = matmul(library, w, m, ACT_Q8)
+        assert status == 0 and "gemm_q8_kernel" in seen[-1].name and seen[-1].grid[1] <= 65535, (m, status)
+    assert matmul(library, w, 4194241, ACT_Q8)[1] == ERR_LIMIT
+    library.lib.zq_weight_free(w)

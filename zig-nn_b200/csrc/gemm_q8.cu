@@ -526,6 +526,8 @@ uint32_t spread_smem(uint64_t ctas, uint32_t need, uint32_t most) {
     return spread < need ? need : spread > most ? most : (uint32_t)spread;
 }
 
+constexpr uint32_t kMostGridY = 65535;
+
 template <int TYPE, int NTL, bool WIDE>
 int launch_terms(const zq_weight* w, const int8_t* xq, const float* xs, const int32_t* xsum, float* y, uint32_t M,
                  QgEpilogue ep, bool split, cudaStream_t st) {
@@ -533,7 +535,7 @@ int launch_terms(const zq_weight* w, const int8_t* xq, const float* xs, const in
     constexpr uint32_t kMost = 112 * 1024 / kBlockBytes / 4 * 4;  // two CTAs share an SM
     const uint32_t rounds = (w->nb + kMost - 1) / kMost, per = ((w->nb + rounds - 1) / rounds + 3) / 4 * 4;
     const dim3 grid((w->out_dim + 8 * NTL - 1) / (8 * NTL), (M + 15) / 16);
-    if (grid.y > 65535u) return ZQ_ERR_LIMIT;
+    if (grid.y > kMostGridY) return ZQ_ERR_LIMIT;
     auto kern = gemm_q8_terms_kernel<TYPE, NTL, WIDE>;
     const uint32_t smem = spread_smem((uint64_t)grid.x * grid.y, per * kBlockBytes, kMost * kBlockBytes);
     // the most that any call asks for: the limit is the process's, and another thread may be about to launch a deeper matrix
@@ -547,7 +549,7 @@ template <int TYPE, int W, int MT, int NT, int D>
 int launch_cfg(const zq_weight* w, const int8_t* xq, const float* xs, const int32_t* xsum, float* y, uint32_t M,
                QgEpilogue ep, bool split, cudaStream_t st) {
     const dim3 grid((w->out_dim + W * MT * 16 - 1) / (W * MT * 16), (M + NT * 8 - 1) / (NT * 8));
-    if (grid.y > 65535u) return ZQ_ERR_LIMIT;
+    if (grid.y > kMostGridY) return ZQ_ERR_LIMIT;
     constexpr uint32_t kRing = D * QgStage<TYPE, W, MT, NT>::kBytes, kMost = 115 * 1024;
     static_assert(kRing <= kMost, "ring");
     const uint32_t smem = spread_smem((uint64_t)grid.x * grid.y, kRing, kMost);
@@ -564,7 +566,8 @@ int launch_cfg(const zq_weight* w, const int8_t* xq, const float* xs, const int3
 // tiles before `least`. Measured on a B200 with the quantiser, weights from HBM, us for shapes 0 to 4: 13824 <- 1152 8_0 at 24 rows 20.3,
 // 17.5, 15.0, 14.3, 20.7, at 88 rows 31.9, 30.0, 28.0, 32.0, 53, at 512 rows 89.7, 105, 105, 136, 264; 1152 <- 6912 8_0 at 512 rows
 // 103, 75, 72, 97, 127; 5003 <- 1184 4_0 at 45 rows 20.7, 17.6, 14.0, 10.8, 13.0. The count takes the best of the five or one within
-// 7 % of it for the three types, 1152 to 262144 weight rows and 2 to 512 activation rows.
+// 7 % of it for the three types, 1152 to 262144 weight rows and 2 to 512 activation rows. A shape whose rows of CTAs are more than a
+// grid has is left out; the first one, of the most columns, remains for the launch to refuse.
 int cheapest_shape(uint32_t n, uint32_t m, uint32_t sms) {
     struct Shape {
         uint32_t rows, cols, tiles, per_tile, least;  // per_tile in tenths of a cycle
@@ -574,7 +577,8 @@ int cheapest_shape(uint32_t n, uint32_t m, uint32_t sms) {
     uint64_t least = ~0ull;
     for (int i = 0; i < 5; ++i) {
         const Shape& s = shapes[i];
-        const uint64_t ctas = (uint64_t)((n + s.rows - 1) / s.rows) * ((m + s.cols - 1) / s.cols);
+        if (i && (m - 1) / s.cols >= kMostGridY) continue;
+        const uint64_t ctas = (uint64_t)((n + s.rows - 1) / s.rows) * ((m - 1) / s.cols + 1);
         uint64_t cost = (ctas + sms - 1) / sms * s.tiles * s.per_tile;
         if (cost < s.least * 10ull) cost = s.least * 10ull;
         if (cost < least) {
