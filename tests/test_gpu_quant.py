@@ -310,10 +310,14 @@ def test_split_product_in_every_tile(zq, oracle, qtype, n, k, m):
     assert rel_l2(got, want) <= REL_L2_GUARD
 
 
+# Sizes that take each of the CTA shapes of gemm_q8.cu (test_launches.py holds them to it), with rows, columns and blocks that fill no
+# tile; 5003 <- 96 takes two weight tiles per warp.
+Q8_SHAPES = [(2003, 96, 509), (1147, 160, 505), (1531, 64, 500), (5003, 64, 45), (700, 32, 30), (17, 480, 9), (5003, 96, 205)]
+
+
 @pytest.mark.parametrize("qtype", TYPES)
-@pytest.mark.parametrize("n,k,m", [(2003, 96, 509), (1147, 160, 505), (1531, 64, 500), (5003, 64, 45), (700, 32, 30), (17, 480, 9)])
+@pytest.mark.parametrize("n,k,m", Q8_SHAPES)
 def test_q8_product_in_every_cta_shape(zq, oracle, qtype, n, k, m):
-    """One call per CTA shape of gemm_q8.cu (the last two take the smallest), with rows, columns and blocks that fill no tile."""
     raw = make_weight(oracle, qtype, n, k, seed=n)
     x = make_x(m, k, seed=m)
     x[m // 2] = 0.0

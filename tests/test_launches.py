@@ -1,10 +1,12 @@
 """Which kernels a call launches, with which grid and in which order, by the library linked with a runtime that runs nothing."""
 import ctypes as C
+import re
 
 import numpy as np
 import pytest
 
 from host_runtime import Library, build
+from test_gpu_quant import Q8_SHAPES
 from zignn_b200 import ggml, hostmodel
 
 ACT_Q8, ERR_LIMIT = 1, 5
@@ -74,3 +76,15 @@ def test_q8_rows_up_to_the_limit_of_a_grid(library, n):
         assert status == 0 and "gemm_q8_kernel" in seen[-1].name and seen[-1].grid[1] <= 65535, (m, status)
     assert matmul(library, w, 4194241, ACT_Q8)[1] == ERR_LIMIT
     library.lib.zq_weight_free(w)
+
+
+@pytest.mark.parametrize("qtype", [ggml.Q4_0, ggml.Q4_1, ggml.Q8_0])
+def test_sizes_of_the_q8_product_test_take_every_shape(library, qtype):
+    """Of test_gpu_quant.py: (warps, weight tiles per warp, column tiles) of the kernel that each of its sizes launches on 148 SMs."""
+    taken = set()
+    for n, k, m in Q8_SHAPES:
+        w = weight(library, qtype, n, k)
+        name = matmul(library, w, m, ACT_Q8)[0][-1].name
+        taken.add(tuple(int(v) for v in re.search(r"gemm_q8_kernelILi\d+ELi(\d+)ELi(\d+)ELi(\d+)E", name).groups()))
+        library.lib.zq_weight_free(w)
+    assert taken == {(8, 1, 8), (4, 2, 4), (4, 1, 4), (4, 1, 2), (4, 1, 1)}
