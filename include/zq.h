@@ -539,7 +539,9 @@ int zq_gemma3_profile_step(zq_gemma3* m, uint32_t token, zq_stream stream, long 
 /* ---- mechanisms of bf16-weight decoders, one by one ----------------------------------------------------------
  * What the decoder engine below is made of, for hosts that assemble another layer stack. Activation rows ("act") are
  * bf16 or, with ZQ_PRECISION_F32, f32; rows that feed a linear have the pitch zq_dense_pitch(k) with zeros beyond
- * column k. Everything else is f32. Nothing synchronises except the uploads. */
+ * column k. Everything else is f32. Nothing synchronises except the uploads.
+ * A call may start before the kernel ahead of it on the stream has ended. It reads nothing that this one may write before
+ * then, but for matrices behind handles (zq_dense) and zq_wkv's d_w0, d_u and d_norm: these are constants while calls run. */
 #define ZQ_PRECISION_BF16 0 /* bf16 activations and cache, f32 accumulation, residual, norms, scores and states */
 #define ZQ_PRECISION_F32 1  /* everything f32 (the weights stay the bf16 values they are) */
 

@@ -9,7 +9,7 @@ import pytest
 import torch
 
 import vepinex as plain
-from zignn_b200 import hostmodel, safetensors
+from zignn_b200 import _lib, hostmodel, safetensors
 
 pytestmark = pytest.mark.gpu
 
@@ -211,6 +211,52 @@ def test_delta_step_ahead_of_its_row(zq, taps, ranks):
         want, S = delta_plain(x, H, H, d, e, taps, ra, conv, A, dt, a2, g2, n, 1e-5, start[0].astype(np.float64), before.astype(np.float64))
         close(out[:, :H * e], want, 3e-5, "pos %d" % pos)
         close(state[0], S, 2e-5)
+
+
+@pytest.mark.parametrize("which", ["conv", "A_log", "norm", "memory biases", "memory norm"])
+def test_state_steps_wait_for_parameters_that_the_call_ahead_writes(zq, which):
+    """A product directly ahead (one deep column per weight row, which triggers its dependents at once) writes a parameter of the step:
+    its new values count, not those that the buffer held before."""
+    rng = np.random.default_rng(8)
+    H, d, e, taps, k = 3, 16, 64, 4, 32768
+    channels = H * (2 * d + e)
+    sizes = {"conv": channels * taps, "A_log": H, "norm": e, "memory biases": H, "memory norm": H * e}
+    w = zq.DenseWeight(bf16(rng.standard_normal((sizes[which], k)) * k ** -0.5)[1])
+    row = zq.dense_rows(torch.tensor(rng.standard_normal((1, k)) * 0.3))
+    x, conv, A, dt, a2, g2, low, n = delta_case(rng, 1, H, H, d, e, taps, 8, 8)
+    low, slots, pos = zq.DenseWeight(low), torch.zeros(1, dtype=torch.int32, device="cuda"), torch.full((1,), 9, dtype=torch.int32, device="cuda")
+    x, conv, A, dt, n = dev(x), dev(conv), dev(A), dev(dt), dev(n)
+    S, ring = dev(rng.standard_normal((1, H, d, e))), dev(rng.standard_normal((1, taps, channels)))
+    mx, ib, mn = dev(rng.standard_normal((1, 2 * H * d + 2 * H * e + 2 * H))), dev(np.ones(H)), dev(np.ones(H * e))
+    mstate = [dev(s) for s in memory_state(rng, 1, H, d, e)]
+
+    y = torch.empty(sizes[which], device="cuda")
+    fill = lambda: y.fill_(-3.0)
+    produce = lambda: _lib.check(_lib.load().zq_dense_linear(w.handle, row.data_ptr(), 1, y.data_ptr(), 0, torch.cuda.current_stream().cuda_stream))
+
+    def step(*ahead):
+        s, r, state = S.clone(), ring.clone(), [t.clone() for t in mstate]
+        for call in ahead:
+            call()
+        if which.startswith("memory"):
+            b, m = (y, mn) if which == "memory biases" else (ib, y)
+            return zq.memory(mx, H, d, e, 4.0, b, b, m, 1e-6, state, slots, False, True)
+        own = dict(conv=conv, A_log=A, norm=n)
+        own[which] = y.view(channels, taps) if which == "conv" else y
+        return zq.delta(x, H, H, d, e, taps, 8, 8, own["conv"], own["A_log"], dt, low, own["norm"], 1e-6, s, r, pos, slots, False, True)
+
+    produce()
+    torch.cuda.synchronize()
+    want = step()
+    fill()
+    assert torch.isfinite(want).all() and not torch.equal(step(), want)
+    graph = torch.cuda.CUDAGraph()  # the launches follow each other without a gap
+    torch.cuda.synchronize()
+    with torch.cuda.graph(graph):
+        got = step(fill, produce)
+    for _ in range(5):
+        graph.replay()
+        assert torch.equal(got, want)
 
 
 @pytest.mark.parametrize("f32", PRECISIONS)

@@ -821,15 +821,15 @@ __device__ __forceinline__ void block_sum_two(float& a, float& b, float* red_a, 
 }
 constexpr int kLowAhead = 2;  // chunks of eight that a thread holds of a row of the low-rank matrices (a rank of up to 64)
 
-// Head norm and gate of the head's o in shared memory; own: norm of the thread's first column, loaded early.
-template <typename TA>
+// Head norm and gate of the head's o in shared memory; OWN: own is the norm of the thread's first column, loaded early.
+template <bool OWN, typename TA>
 __device__ __forceinline__ void finish_head(const float* os, const float* gate, const float* norm, float own, uint32_t E, float eps,
                                             TA* row, uint32_t h, uint32_t heads, uint32_t out_pitch, float* red) {
     float ss = 0.0f;
     for (uint32_t c = threadIdx.x; c < E; c += blockDim.x) ss = fmaf(os[c], os[c], ss);
     const float inv = 1.0f / sqrtf(block_sum_f(ss, red) / (float)E + eps);
     for (uint32_t c = threadIdx.x; c < E; c += blockDim.x)
-        row[h * E + c] = to_act<TA>(os[c] * inv * (c == threadIdx.x ? own : norm[c]) * gate[c]);
+        row[h * E + c] = to_act<TA>(os[c] * inv * (OWN && c == threadIdx.x ? own : norm[c]) * gate[c]);
     if (h + 1 == heads)
         for (uint32_t c = heads * E + threadIdx.x; c < out_pitch; c += blockDim.x) row[c] = to_act<TA>(0.0f);
 }
@@ -843,7 +843,6 @@ memory_step_kernel(const __grid_constant__ MemoryArgs a, StepShape sh) {
     const uint32_t D = a.dim, E = a.vdim, kd = a.heads * D, vd = a.heads * E, h = blockIdx.x, r = blockIdx.y, tid = threadIdx.x;
     float *qs = sm, *ks = qs + D, *vs = ks + D, *gate = vs + E, *os = gate + E, *red = os + E;
     const float* norm = a.norm + h * E;
-    const float ib = a.i_bias[h], fb = a.f_bias[h], own_norm = tid < E ? norm[tid] : 0.0f;
     pdl_wait();
     const float* row = a.in + (size_t)r * a.ld;
     const size_t at = (size_t)(uint32_t)a.slots[r] * a.heads + h;
@@ -851,8 +850,9 @@ memory_step_kernel(const __grid_constant__ MemoryArgs a, StepShape sh) {
     const uint32_t cx = tid % sh.cp, rg = tid / sh.cp;
     Cols<VEC> x[kStepBatch];  // the first rows of the state are requested ahead of everything else
     load_batch<VEC>(S, D, E, cx * VEC, rg, sh.rg, x);
-    const float in = soft_cap(row[2 * kd + 2 * vd + h] + ib, a.gate_cap);
-    const float f = log_sigmoid_f(soft_cap(row[2 * kd + 2 * vd + a.heads + h] + fb, a.gate_cap));
+    // biases behind the wait: in a caller's own call the kernel ahead may write them
+    const float in = soft_cap(row[2 * kd + 2 * vd + h] + a.i_bias[h], a.gate_cap);
+    const float f = log_sigmoid_f(soft_cap(row[2 * kd + 2 * vd + a.heads + h] + a.f_bias[h], a.gate_cap));
     const float m0 = a.m[at], m = fmaxf(f + m0, in), keep = expf(f + m0 - m), add = expf(in - m);
     const float scale = 1.0f / sqrtf((float)D);
     float nq = 0.0f;
@@ -898,7 +898,7 @@ memory_step_kernel(const __grid_constant__ MemoryArgs a, StepShape sh) {
         meet<VEC>(red, o, sh, os + c0, E - c0);
     }
     for (uint32_t c = tid; c < E; c += blockDim.x) os[c] /= size;
-    finish_head<TA>(os, gate, norm, own_norm, E, a.eps, static_cast<TA*>(a.out) + (size_t)r * a.out_pitch, h, a.heads, a.out_pitch, red33);
+    finish_head<false>(os, gate, norm, 0.0f, E, a.eps, static_cast<TA*>(a.out) + (size_t)r * a.out_pitch, h, a.heads, a.out_pitch, red33);
 }
 
 // Bound: the latency of a chain of dependent steps (row -> convolution -> norms -> decays -> state -> head norm), not its bytes
@@ -918,13 +918,18 @@ delta_step_kernel(const __grid_constant__ DeltaArgs a, StepShape sh) {
     const bf16* low_g = a.low.w + ((size_t)a.heads * D + (size_t)h * E) * kp;
     if (tid == 0) prefetch_l2_bulk(low_a, D * kp * 2);
     if (tid == 1) prefetch_l2_bulk(low_g, E * kp * 2);
-    // What does not depend on the token is loaded ahead of the wait: parameters of the thread's first channel, and of the low-rank
-    // matrices the first kLowAhead chunks of the thread's first two rows.
-    const float decay = a.A_log[h], own_norm = tid < E ? a.norm[tid] : 0.0f;
+    // What does not depend on the token is loaded ahead of the wait: parameters of the thread's first channel (in a caller's own call
+    // behind it: the kernel ahead may have written them), and of the low-rank matrices the first kLowAhead chunks of the thread's
+    // first two rows.
     const bool short_conv = a.taps <= kStepTaps;
     auto channel = [&](uint32_t i) { return i < D ? kv * D + i : i < 2 * D ? kd + kv * D + (i - D) : 2 * kd + h * E + (i - 2 * D); };
-    float cw[kStepTaps];
-    if (short_conv && tid < 2 * D + E) conv_weights(a, channel(tid), cw);
+    float decay = 0.0f, own_norm = 0.0f, cw[kStepTaps];
+    auto parameters = [&] {
+        decay = a.A_log[h];
+        if (tid < E) own_norm = a.norm[tid];
+        if (short_conv && tid < 2 * D + E) conv_weights(a, channel(tid), cw);
+    };
+    if (a.constant) parameters();
     const uint32_t sub = tid & 3, low_step = blockDim.x / 4;
     auto low_row = [&](uint32_t i) {
         return reinterpret_cast<const uint4*>(i < D ? low_a + (size_t)i * kp : low_g + (size_t)(i - D) * kp);
@@ -938,6 +943,7 @@ delta_step_kernel(const __grid_constant__ DeltaArgs a, StepShape sh) {
             if (i < D + E && sub + 4 * c < kp / 8) low_w[n][c] = __ldg(low_row(i) + sub + 4 * c);
     }
     pdl_wait();
+    if (!a.constant) parameters();
     const float* row = a.in + (size_t)r * a.ld;
     const uint32_t slot = (uint32_t)a.slots[r], pos = (uint32_t)a.pos[r];
     float* S = a.S + ((size_t)slot * a.heads + h) * D * E;
@@ -1071,7 +1077,7 @@ delta_step_kernel(const __grid_constant__ DeltaArgs a, StepShape sh) {
         }
     }
     for (uint32_t c = tid; c < E; c += blockDim.x) os[c] = fmaf(beta * (vs[c] - ys[c]), kq, os[c]);
-    finish_head<TA>(os, gate, a.norm, own_norm, E, a.eps, static_cast<TA*>(a.out) + (size_t)r * a.out_pitch, h, a.heads, a.out_pitch, red33);
+    finish_head<true>(os, gate, a.norm, own_norm, E, a.eps, static_cast<TA*>(a.out) + (size_t)r * a.out_pitch, h, a.heads, a.out_pitch, red33);
 }
 
 // ---- launches ------------------------------------------------------------------------------------------------------

@@ -712,6 +712,7 @@ int memory(zq_decoder* m, const MemoryLayer& w, const Pass& P, cudaStream_t st) 
 
 int delta(zq_decoder* m, const DeltaLayer& w, const Pass& P, cudaStream_t st) {
     DeltaArgs a = w.args;
+    a.constant = true;
     a.in = m->proj;
     a.pos = m->d_pos;
     a.slots = m->d_slots;
