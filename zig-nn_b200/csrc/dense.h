@@ -229,6 +229,7 @@ struct DeltaArgs {
     DenseWeight low;         // [heads * dim rows over the a1 output | heads * vdim rows over the g1 output]
     const float* norm;       // [vdim]
     bool constant;           // no kernel ahead writes conv, A_log or norm: they may be read ahead of the wait
+    bool both;               // launch_delta: shared memory holds the partial columns of two sums
     float eps;
     float* S;                // [slots][heads][dim][vdim]
     float* ring;             // [slots][taps][channels]: inputs of the convolution, token p at place p % taps (unused with 1 tap)

@@ -729,12 +729,11 @@ memory_chunk_kernel(const __grid_constant__ MemoryArgs a, const __grid_constant_
 // Threads: CP of them side by side along a row of the state (VEC columns each), RG rows at a time.
 struct StepShape {
     uint32_t cp, rg;
-    bool both;  // shared memory holds the partial columns of two sums
 };
 inline StepShape step_shape(uint32_t vdim, uint32_t vec, uint32_t threads) {
     uint32_t cp = 1;
     while (cp < (vdim + vec - 1) / vec && cp < threads) cp <<= 1;
-    return StepShape{cp, threads / cp, false};
+    return StepShape{cp, threads / cp};
 }
 template <int VEC>
 struct Cols {
@@ -934,13 +933,16 @@ delta_step_kernel(const __grid_constant__ DeltaArgs a, StepShape sh) {
     auto low_row = [&](uint32_t i) {
         return reinterpret_cast<const uint4*>(i < D ? low_a + (size_t)i * kp : low_g + (size_t)(i - D) * kp);
     };
+    // (Not where a thread holds single columns of the state: 16 more of its values live took 128 registers in place of 57 and one CTA of
+    // 512 threads per SM in place of two, 64 rows of six heads of 128 x 127 35 us in place of 31.)
+    constexpr bool kHeld = VEC == 4;
     uint4 low_w[2][kLowAhead];
 #pragma unroll
     for (int n = 0; n < 2; ++n) {
         const uint32_t i = n * low_step + (tid >> 2);
 #pragma unroll
         for (int c = 0; c < kLowAhead; ++c)
-            if (i < D + E && sub + 4 * c < kp / 8) low_w[n][c] = __ldg(low_row(i) + sub + 4 * c);
+            if (kHeld && i < D + E && sub + 4 * c < kp / 8) low_w[n][c] = __ldg(low_row(i) + sub + 4 * c);
     }
     pdl_wait();
     if (!a.constant) parameters();
@@ -1011,9 +1013,11 @@ delta_step_kernel(const __grid_constant__ DeltaArgs a, StepShape sh) {
                 gate[i - D] = sigmoid_f(acc);
         }
     };
-    low(0, low_w[0]);
-    if (low_step < D + E) low(low_step, low_w[1]);
-    for (uint32_t base = 2 * low_step; base < D + E; base += low_step) low(base, nullptr);
+    if (kHeld) {
+        low(0, low_w[0]);
+        if (low_step < D + E) low(low_step, low_w[1]);
+    }
+    for (uint32_t base = kHeld ? 2 * low_step : 0; base < D + E; base += low_step) low(base, nullptr);
     float kq = 0.0f;
     for (uint32_t i = tid; i < D; i += blockDim.x) {
         const float q = qs[i] * fq, k = ks[i] * fk;
@@ -1044,7 +1048,7 @@ delta_step_kernel(const __grid_constant__ DeltaArgs a, StepShape sh) {
                 }
             }
         }
-        if (sh.both) {
+        if (a.both) {
             meet_two<VEC>(red, y, o, sh, ys + c0, os + c0, E - c0);
         } else {
             meet<VEC>(red, y, sh, ys + c0, E - c0);
@@ -1127,15 +1131,14 @@ uint32_t step_threads(uint32_t dim, uint32_t vdim) {
     const uint32_t n = dim * vdim;
     return n >= 16384 ? 512 : n >= 4096 ? 256 : 128;
 }
+// Floats of shared memory that a sum over the rows of the state takes.
+uint32_t step_sum(uint32_t dim, uint32_t vdim) { return step_threads(dim, vdim) * (vdim % 4 == 0 ? 4 : 1); }
 template <typename Args, typename K>
-int step(const Args& a, K vec_f32, K vec_bf16, K one_f32, K one_bf16, size_t floats, bool two_sums, uint32_t rows, bool f32,
-         cudaStream_t st) {
+int step(const Args& a, K vec_f32, K vec_bf16, K one_f32, K one_bf16, size_t floats, uint32_t rows, bool f32, cudaStream_t st) {
     const bool v4 = a.vdim % 4 == 0;
     const uint32_t threads = step_threads(a.dim, a.vdim);
-    StepShape sh = step_shape(a.vdim, v4 ? 4 : 1, threads);
-    const size_t sum = threads * (v4 ? 4 : 1);
-    sh.both = two_sums && (floats + 2 * sum) * sizeof(float) <= kMaxSmem;
-    const size_t smem = (floats + (sh.both ? 2 : 1) * sum) * sizeof(float);
+    const StepShape sh = step_shape(a.vdim, v4 ? 4 : 1, threads);
+    const size_t smem = floats * sizeof(float);
     K kern = v4 ? (f32 ? vec_f32 : vec_bf16) : (f32 ? one_f32 : one_bf16);
     const int rc = allow_smem(kern, smem);
     return rc != ZQ_OK ? rc : done(launch_pdl(kern, dim3(a.heads, rows), dim3(threads), smem, st, a, sh));
@@ -1186,7 +1189,7 @@ int launch_memory(const MemoryArgs& a, uint32_t rows, bool one_sequence, bool f3
     const uint32_t kd = a.heads * a.dim, vd = a.heads * a.vdim;
     if (!one_sequence || rows == 1)
         return step(a, memory_step_kernel<4, float>, memory_step_kernel<4, bf16>, memory_step_kernel<1, float>,
-                    memory_step_kernel<1, bf16>, 2 * (size_t)a.dim + 3 * (size_t)a.vdim, false, rows, f32, st);
+                    memory_step_kernel<1, bf16>, 2 * (size_t)a.dim + 3 * (size_t)a.vdim + step_sum(a.dim, a.vdim), rows, f32, st);
     FinishParams f{};
     f.heads = a.heads;
     f.vdim = a.vdim;
@@ -1262,9 +1265,13 @@ size_t delta_work_floats(const DeltaArgs& a, uint32_t max_rows) {
 int launch_delta(const DeltaArgs& a, uint32_t rows, bool one_sequence, bool f32, cudaStream_t st) {
     if (rows == 0) return ZQ_OK;
     if (a.dim == 0 || a.vdim == 0 || a.dim > kStateMaxDim || a.vdim > 4096) return ZQ_ERR_LIMIT;
-    if (!one_sequence || rows == 1)
-        return step(a, delta_step_kernel<4, float>, delta_step_kernel<4, bf16>, delta_step_kernel<1, float>, delta_step_kernel<1, bf16>,
-                    2 * (size_t)a.low.kp + 3 * (size_t)a.dim + 4 * (size_t)a.vdim, true, rows, f32, st);
+    if (!one_sequence || rows == 1) {
+        const size_t floats = 2 * (size_t)a.low.kp + 3 * (size_t)a.dim + 4 * (size_t)a.vdim, sum = step_sum(a.dim, a.vdim);
+        DeltaArgs d = a;
+        d.both = (floats + 2 * sum) * sizeof(float) <= kMaxSmem;
+        return step(d, delta_step_kernel<4, float>, delta_step_kernel<4, bf16>, delta_step_kernel<1, float>, delta_step_kernel<1, bf16>,
+                    floats + (d.both ? 2 : 1) * sum, rows, f32, st);
+    }
     if (rows > a.max_rows) return ZQ_ERR_BAD_ARG;
     const uint32_t kd = a.kv_heads * a.dim, hd = a.heads * a.dim, vd = a.heads * a.vdim;
     const size_t R = a.max_rows;
