@@ -56,6 +56,16 @@ def test_gpt2_prompt_through_the_split_product(zq, oracle, tokens):
     assert max(errs) <= 1e-5, max(errs)
 
 
+@pytest.mark.parametrize("qtype", [ggml.Q4_0, ggml.Q8_0])
+def test_gpt2_prompt_whose_tiles_take_turns(zq, oracle, qtype):
+    """512 rows of the four matrices have more CTAs than run at once; the weight types that the test above leaves out."""
+    host = hostmodel.Gpt2Host.synthetic(dict(hostmodel.GPT2_SMALL, vocab=1000, layer=1), qtype=qtype, seed=42, device="cuda")
+    prompt = np.random.default_rng(47).integers(0, 1000, size=512)
+    gt, ct, errs = run_parity(zq.Gpt2(host.randomize_small_params()), oracle.Gpt2(host, 8), prompt, 1)
+    assert gt == ct
+    assert max(errs) <= 1e-5, max(errs)
+
+
 @pytest.mark.parametrize("qtypes", [(ggml.Q8_0, ggml.Q8_0, ggml.Q8_0), (ggml.Q4_0, ggml.Q8_0, ggml.Q4_1),
                                     (ggml.Q4_1, ggml.Q4_1, ggml.Q4_1)])
 def test_gemma3_tiny_parity(zq, oracle, qtypes):

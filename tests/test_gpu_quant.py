@@ -299,10 +299,14 @@ def test_quantize_rows_q8_bit_exact(zq, oracle):
     assert scale[0, 0].item() == 1.0 and q[1, 32].item() == -127 and q[1, 48].item() == 0
 
 
+# Sizes that take each of the tiles of gemm_split.cu (test_launches.py holds them to it), with rows, columns and blocks that fill none.
+SPLIT_SIZES = [(700, 992, 47), (1000, 512, 33), (2290, 480, 47), (520, 96, 45), (9000, 96, 30), (9000, 224, 45), (11003, 96, 41), (2381, 288, 27),
+               (4738, 288, 25), (4739, 1824, 41), (9487, 96, 27)]
+
+
 @pytest.mark.parametrize("qtype", TYPES)
-@pytest.mark.parametrize("n,k,m", [(700, 992, 47), (1000, 512, 33), (2290, 480, 47), (520, 96, 45), (9000, 96, 30), (9000, 224, 45), (11003, 96, 41)])
+@pytest.mark.parametrize("n,k,m", SPLIT_SIZES)
 def test_split_product_in_every_tile(zq, oracle, qtype, n, k, m):
-    """One call per tile of gemm_split.cu that a call of up to 48 rows takes, with rows, columns and blocks that fill none."""
     raw = make_weight(oracle, qtype, n, k, seed=n)
     x = make_x(m, k, seed=m)
     got = zq.quant_matmul_no_grad(torch.from_numpy(x).cuda(), zq.QuantWeight(raw, qtype, n, k)).cpu().numpy()

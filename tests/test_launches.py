@@ -6,10 +6,10 @@ import numpy as np
 import pytest
 
 from host_runtime import Library, build
-from test_gpu_quant import Q8_SHAPES
+from test_gpu_quant import Q8_SHAPES, SPLIT_SIZES
 from zignn_b200 import ggml, hostmodel
 
-ACT_Q8, ERR_LIMIT = 1, 5
+ACT_F32, ACT_Q8, ERR_LIMIT = 0, 1, 5
 
 
 @pytest.fixture(scope="module")
@@ -88,3 +88,27 @@ def test_sizes_of_the_q8_product_test_take_every_shape(library, qtype):
         taken.add(tuple(int(v) for v in re.search(r"gemm_q8_kernelILi\d+ELi(\d+)ELi(\d+)ELi(\d+)E", name).groups()))
         library.lib.zq_weight_free(w)
     assert taken == {(8, 1, 8), (4, 2, 4), (4, 1, 4), (4, 1, 2), (4, 1, 1)}
+
+
+def split_tile(library, qtype, n, k, m):
+    """(weight rows, activation rows, quads of K per step, stages) of the f32-accurate product that the call launches."""
+    w = weight(library, qtype, n, k)
+    name = matmul(library, w, m, ACT_F32)[0][-1].name
+    library.lib.zq_weight_free(w)
+    wr, ks, nt, d = (int(v) for v in re.search(r"gemm_split_kernelILi\d+ELi(\d+)ELi(\d+)ELi(\d+)ELi(\d+)E", name).groups())
+    return wr * 16, nt * 8, ks, d
+
+
+@pytest.mark.parametrize("qtype", [ggml.Q4_0, ggml.Q4_1, ggml.Q8_0])
+def test_sizes_of_the_split_product_test_take_every_tile(library, qtype):
+    assert {split_tile(library, qtype, n, k, m) for n, k, m in SPLIT_SIZES} == {
+        (16, 16, 8, 2), (32, 16, 4, 3), (32, 24, 4, 3), (32, 32, 4, 2), (64, 24, 2, 4), (64, 32, 2, 4), (64, 48, 2, 3), (128, 48, 1, 2),
+        (64, 24, 2, 2), (64, 32, 2, 2)}
+
+
+@pytest.mark.parametrize("n", [9473, 11000, 12160])
+def test_split_product_of_more_tiles_than_sms_takes_two_per_sm(library, n):
+    """21 to 32 rows: two CTAs per SM of a tile that holds the rows once, not one CTA of 48 columns (14.4 and 17.1 us against 23.0)."""
+    for m in (21, 24, 25, 32):
+        assert split_tile(library, ggml.Q4_0, n, 1152, m) == (64, 24 if m <= 24 else 32, 2, 2), m
+    assert split_tile(library, ggml.Q4_0, 4096, 6144, 32) == (32, 32, 4, 2)

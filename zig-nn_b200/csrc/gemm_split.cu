@@ -428,28 +428,33 @@ int launch_cfg(const zq_weight* w, const SplitImage& im, float* y, uint32_t M, c
     return ZQ_OK;
 }
 
-// The tile whose CTAs run all at once, one per SM, and whose chain of steps (KS quads of K each) is the shortest; `step` is what one
-// costs, in tenths of a microsecond: conversions and MMAs of NT tiles, and KS x NT x 4 KB of activations. With none that fits, three
-// small CTAs per SM take turns. (B200, us with the split, the seven tiles and the last in this order, the one taken in brackets:
-// 768 <- 3072 4_0 at 48 rows [9.9], 12.7, 13.5, 20.0, 25.1, 32.4, 54.0, 29.3; 1152 <- 6912 8_0 at 48 rows 28.2, [26.0], 28.3, 43.3, 50.3,
-// 61.7, 103, 67.7; 2304 <- 768 8_0 at 48 rows 11.6, 9.3, [7.0], 7.4, 8.9, 11.8, 16.3, 10.6; 5003 <- 1184 4_1 at 24 rows 20.8, 16.2, 13.7,
-// [10.9], 13.2, 16.8, 26.5, 16.1, at 32 rows 21.6, 16.8, 18.2, 17.9, [13.7], 16.9, 26.9, 16.8 and at 45 rows 29.2, 21.9, 19.5, 18.9, 23.4,
-// [17.8], 27.7, 17.2; 11000 <- 1152 8_0 at 33 rows 55.4, 37.0, 29.2, 25.7, 29.5, 27.2, [22.4], 25.4. A GPT-2 document of 900 tokens: 7.12 ms
-// with the last, 7.22 with tiles of 64 x 32, two per SM.)
+// The tile whose CTAs run all at once and whose chain of steps (KS quads of K each) is the shortest, `start` and `step` in tenths of a
+// microsecond: launch and sums of a CTA, conversions and MMAs of NT tiles and KS x NT x 4 KB of activations. Registers and rings
+// leave one CTA per SM to the first eight; the last two run two, whose steps (`pair`) then share the SM. With none that fits, CTAs of the
+// last but one take turns. (B200, us with the split, weights from HBM, the ten tiles in this order, the one taken in brackets:
+// 768 <- 3072 4_0 at 48 rows [10.0], 12.8, 13.5, 16.5, 20.0, 25.1, 32.4, 53.9, 27.4, 33.4; 1152 <- 6912 8_0 at 48 rows 27.8, [25.5], 27.1, 30.7, 43.8,
+// 50.7, 62.8, 107, 66.9, 75.9; 5003 <- 1184 4_1 at 24 rows 20.6, 16.3, 13.7, 16.6, [10.9], 13.1, 16.7, 26.6, 15.5, 18.4; 4096 <- 6144 4_0 at 32 rows
+// 47.7, 42.4, 42.7, [30.1], 39.5, 48.6, 60.0, 106, 63.3, 71.5; 12000 <- 1152 4_0 at 24 rows 42.3, 30.1, 18.3, 22.6, 17.4, 21.5, 27.9, 23.0, [14.4], 16.7
+// and at 32 rows 43.5, 30.8, 31.3, 23.5, 23.8, 22.0, 28.4, 23.3, 23.9, [17.1]. The tile taken is the best of the ten or within 17 % of it, 0.4 % in the mean,
+// for 17 to 48 rows of 16 matrices. A GPT-2 document of 900 tokens: 7.12 ms with CTAs of the last but one in turns, 7.22 with the last.)
 template <int TYPE>
 int launch_type(const zq_weight* w, const SplitImage& im, float* y, uint32_t M, const SplitEpilogue& ep, cudaStream_t st) {
     struct Tile {
-        uint32_t rows, cols, quads, step;
+        uint32_t rows, cols, quads, start, step, pair;
     };
-    constexpr Tile tiles[7] = {{16, 16, 8, 20}, {32, 16, 4, 16}, {32, 24, 4, 17}, {64, 24, 2, 14}, {64, 32, 2, 18}, {64, 48, 2, 23}, {128, 48, 1, 20}};
+    constexpr int kInTurns = 8;
+    constexpr Tile tiles[10] = {{16, 16, 8, 36, 20, 0}, {32, 16, 4, 33, 16, 0}, {32, 24, 4, 33, 17, 0}, {32, 32, 4, 40, 20, 0}, {64, 24, 2, 30, 15, 0},
+                                {64, 32, 2, 34, 18, 0}, {64, 48, 2, 49, 23, 0}, {128, 48, 1, 52, 20, 0}, {64, 24, 2, 22, 23, 27}, {64, 32, 2, 24, 26, 31}};
     const uint32_t nq = w->nbp / 4;
-    int best = 7;
+    const uint64_t sms = (uint64_t)sm_count();
+    int best = kInTurns;
     uint32_t least = ~0u;
-    for (int i = 0; i < 7; ++i) {
+    for (int i = 0; i < 10; ++i) {
         const Tile& t = tiles[i];
         const uint64_t ctas = (uint64_t)((w->out_dim + t.rows - 1) / t.rows) * ((M + t.cols - 1) / t.cols);
-        const uint32_t cost = (nq + t.quads - 1) / t.quads * t.step;
-        if (ctas <= (uint64_t)sm_count() && cost < least) {
+        if (ctas > (t.pair ? 2 : 1) * sms) continue;
+        const uint32_t cost = t.start + (nq + t.quads - 1) / t.quads * (ctas > sms ? t.pair : t.step);
+        if (cost < least) {
             least = cost;
             best = i;
         }
@@ -458,10 +463,12 @@ int launch_type(const zq_weight* w, const SplitImage& im, float* y, uint32_t M, 
         case 0: return launch_cfg<TYPE, 1, 8, 2, 2>(w, im, y, M, ep, st);
         case 1: return launch_cfg<TYPE, 2, 4, 2, 3>(w, im, y, M, ep, st);
         case 2: return launch_cfg<TYPE, 2, 4, 3, 3>(w, im, y, M, ep, st);
-        case 3: return launch_cfg<TYPE, 4, 2, 3, 4>(w, im, y, M, ep, st);
-        case 4: return launch_cfg<TYPE, 4, 2, 4, 4>(w, im, y, M, ep, st);
-        case 5: return launch_cfg<TYPE, 4, 2, 6, 3>(w, im, y, M, ep, st);
-        case 6: return launch_cfg<TYPE, 8, 1, 6, 2>(w, im, y, M, ep, st);
+        case 3: return launch_cfg<TYPE, 2, 4, 4, 2>(w, im, y, M, ep, st);
+        case 4: return launch_cfg<TYPE, 4, 2, 3, 4>(w, im, y, M, ep, st);
+        case 5: return launch_cfg<TYPE, 4, 2, 4, 4>(w, im, y, M, ep, st);
+        case 6: return launch_cfg<TYPE, 4, 2, 6, 3>(w, im, y, M, ep, st);
+        case 7: return launch_cfg<TYPE, 8, 1, 6, 2>(w, im, y, M, ep, st);
+        case 9: return launch_cfg<TYPE, 4, 2, 4, 2>(w, im, y, M, ep, st);
         default: return launch_cfg<TYPE, 4, 2, 3, 2>(w, im, y, M, ep, st);
     }
 }
