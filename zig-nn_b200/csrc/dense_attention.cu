@@ -15,12 +15,30 @@ namespace {
 
 constexpr uint32_t kTile = 64;  // keys per tile
 
-// Keys (or values) [k0, k0 + kTile) of one head -> shared memory rows of pitch (dp + 8) halves; zeros beyond k_end.
+// Keys (or values) [k0, k0 + kTile) of one head -> shared memory rows of pitch (dp + 8) halves; zeros beyond k_end. WALK: addresses
+// by steps of the loop, for the decode kernel, which requests its tiles one behind the other. In the prefill kernel the addresses
+// that live across the loop cost more than they save (255 registers and 44 spilled bytes at 256 dimensions; 8 tokens behind 2040: 161 us in
+// place of 155, behind none with heads of 64: 3.8 in place of 3.6).
+template <bool WALK>
 __device__ __forceinline__ void load_tile(uint32_t dst, const bf16* cache, uint32_t kv_heads, uint32_t g, uint32_t dp,
                                           uint32_t k0, uint32_t k_end) {
     const uint32_t cpr = dp / 8, pitch = (dp + 8) * 2;
     const uint32_t dr = blockDim.x / cpr, dc = blockDim.x % cpr;
     uint32_t row = threadIdx.x / cpr, c = threadIdx.x % cpr;
+    if constexpr (!WALK) {
+        while (row < kTile) {
+            const uint32_t key = k0 + row;
+            const bool ok = key < k_end;
+            copy16(dst + row * pitch + c * 16, cache + ((size_t)(ok ? key : k0) * kv_heads + g) * dp + c * 8, ok);
+            row += dr;
+            c += dc;
+            if (c >= cpr) {
+                c -= cpr;
+                ++row;
+            }
+        }
+        return;
+    }
     const size_t key_step = (size_t)kv_heads * dp;
     const bf16* first = cache + (size_t)k0 * key_step + (size_t)g * dp;  // what a copy of zeros names
     const bf16* from = first + row * key_step + c * 8;
@@ -180,8 +198,8 @@ gqa_prefill_kernel(const __grid_constant__ AttnArgs a) {
     const uint32_t last = min(m0 + 64, n_rows) - 1;
     const uint32_t k_end = a.pos0 + last / R + 1;
     const uint32_t n_tiles = (k_end + kTile - 1) / kTile;
-    load_tile(ktile(0), kc, s.kv_heads, g, s.dimp, 0, k_end);
-    load_tile(vtile(0), vc, s.kv_heads, g, s.vdimp, 0, k_end);
+    load_tile<false>(ktile(0), kc, s.kv_heads, g, s.dimp, 0, k_end);
+    load_tile<false>(vtile(0), vc, s.kv_heads, g, s.vdimp, 0, k_end);
     copy_commit();
 
     const uint32_t w0 = m0 + warp * 16;
@@ -200,8 +218,8 @@ gqa_prefill_kernel(const __grid_constant__ AttnArgs a) {
     const uint32_t see_all = a.pos0 + w0 / R + 1;  // keys that every row of the warp sees
     for (uint32_t t = 0; t < n_tiles; ++t) {
         if (t + 1 < n_tiles) {
-            load_tile(ktile((t + 1) & 1), kc, s.kv_heads, g, s.dimp, (t + 1) * kTile, k_end);
-            load_tile(vtile((t + 1) & 1), vc, s.kv_heads, g, s.vdimp, (t + 1) * kTile, k_end);
+            load_tile<false>(ktile((t + 1) & 1), kc, s.kv_heads, g, s.dimp, (t + 1) * kTile, k_end);
+            load_tile<false>(vtile((t + 1) & 1), vc, s.kv_heads, g, s.vdimp, (t + 1) * kTile, k_end);
         }
         copy_commit();
         copy_wait<1>();
@@ -284,8 +302,8 @@ gqa_decode_kernel(const __grid_constant__ AttnArgs a) {
     const uint32_t early = a.stages == 1 ? 1 : a.stages - 1;  // tiles requested here; one stage: the longest range is one tile
     for (uint32_t t = 0; t < early; ++t) {
         if (t < n_tiles) {
-            load_tile(ktile(t), kc, s.kv_heads, g, s.dimp, k_begin + t * kTile, c_end);
-            load_tile(vtile(t), vc, s.kv_heads, g, s.vdimp, k_begin + t * kTile, c_end);
+            load_tile<true>(ktile(t), kc, s.kv_heads, g, s.dimp, k_begin + t * kTile, c_end);
+            load_tile<true>(vtile(t), vc, s.kv_heads, g, s.vdimp, k_begin + t * kTile, c_end);
         }
         copy_commit();
     }
@@ -327,8 +345,8 @@ gqa_decode_kernel(const __grid_constant__ AttnArgs a) {
     for (uint32_t t = 0; t < n_tiles; ++t) {
         const uint32_t ahead = t + early;
         if (ahead < n_tiles) {
-            load_tile(ktile(ahead), kc, s.kv_heads, g, s.dimp, k_begin + ahead * kTile, c_end);
-            load_tile(vtile(ahead), vc, s.kv_heads, g, s.vdimp, k_begin + ahead * kTile, c_end);
+            load_tile<true>(ktile(ahead), kc, s.kv_heads, g, s.dimp, k_begin + ahead * kTile, c_end);
+            load_tile<true>(vtile(ahead), vc, s.kv_heads, g, s.vdimp, k_begin + ahead * kTile, c_end);
         }
         copy_commit();
         if (early == 2) copy_wait<2>();
