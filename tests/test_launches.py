@@ -7,7 +7,7 @@ import pytest
 
 from host_runtime import Library, build
 from test_gpu_quant import Q8_SHAPES, SPLIT_SIZES
-from zignn_b200 import ggml, hostmodel
+from zignn_b200 import ggml, hostmodel, structs
 
 ACT_F32, ACT_Q8, ERR_LIMIT = 0, 1, 5
 
@@ -112,3 +112,16 @@ def test_split_product_of_more_tiles_than_sms_takes_two_per_sm(library, n):
     for m in (21, 24, 25, 32):
         assert split_tile(library, ggml.Q4_0, n, 1152, m) == (64, 24 if m <= 24 else 32, 2, 2), m
     assert split_tile(library, ggml.Q4_0, 4096, 6144, 32) == (32, 32, 4, 2)
+
+
+@pytest.mark.parametrize("heads,kv_heads,dim,ctx,slots,ranges", [
+    (12, 4, 64, 2048, 1, 32), (12, 4, 64, 2048, 6, 16), (12, 4, 64, 2048, 16, 8), (12, 4, 64, 2048, 64, 8), (12, 4, 64, 256, 1, 1),
+    (8, 2, 128, 2048, 6, 32), (8, 2, 128, 2048, 8, 16), (8, 2, 128, 2048, 64, 8), (8, 2, 128, 256, 8, 4), (8, 2, 128, 256, 16, 1),
+    (4, 1, 256, 2048, 1, 32), (4, 1, 256, 2048, 64, 32), (4, 1, 256, 256, 64, 4), (12, 4, 64, 8192, 64, 32), (12, 4, 64, 1500, 1, 24)])
+def test_ranges_of_the_decode_attention(library, heads, kv_heads, dim, ctx, slots, ranges):
+    """By the cache alone: any count of rows of a step cuts a row's keys alike. No second kernel behind one range."""
+    g, somewhere, lib = structs.Gqa(heads, kv_heads, dim, dim, ctx, slots, 1.0, 1e-6, 0.0, 0.0), C.c_void_p(1 << 20), library.lib
+    for rows in (1, 2, slots):
+        seen, status = library.launches(lambda: lib.zq_gqa_attention(C.byref(g), *[somewhere] * 6, rows, 0, 0, somewhere, 0, None))
+        assert status == 0 and "gqa_decode" in seen[0].name and seen[0].grid == (ranges, kv_heads, rows)
+        assert len(seen) == (1 if ranges == 1 else 2)

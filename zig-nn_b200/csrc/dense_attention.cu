@@ -549,12 +549,29 @@ int plain_rows(const GqaShape& s, const void* q, const void* kc, const void* vc,
     return go(gqa_plain_kernel<TA, 32>, 32);
 }
 
-// Ranges of a row's keys, by the cache's capacity alone (a tile each when it is full, longer ones beyond 32 of them): a row's
-// ranges, and with them its bits, do not depend on the other rows of its step. (Prompts of 1500 tokens and 24 steps, Lenisun of width
-// 1152: 14.3 ms with ranges of 256 keys, 13.2 so; six of 200 tokens together 27.6 and 27.2.)
+// Ranges of a row's keys, by the cache alone (its capacity, key heads and slots), so that a row's ranges, and with them its bits, do
+// not depend on the other rows of its step: 256 keys each, or half or a quarter of that, the shortest whose CTAs run all at once when
+// every slot is full (by registers four per SM up to 64 dimensions, three up to 128); 32 of them at most. At 256 dimensions always
+// a tile: longer ranges want a ring that an SM gives to one CTA. A cache of one range needs no second kernel; it is cut only where its
+// four tiles take longer than that: beyond 128 dimensions, and beyond 64 for few CTAs. (B200, the whole call, us, 32, 16 and 8
+// ranges of 2048 keys, the choice in brackets: 12 heads over 4 of 64, 1 row [7.3], 6.9, 8.5, 6 rows 11.1, [9.0], 10.4, 64 rows 59.8, 43.8, [40.8]; 8 over 2
+// of 128, 6 rows [9.8], 10.6, 12.6, 16 rows 17.8, 16.2, [13.3]; 4 over 1 of 256, 1 row [9.2], 11.1, 16.0, 64 rows [53], 60, 57. 4 ranges and 1 of
+// 256 keys, at 64 keys and at 256: 12 over 4 of 64, 1 row 5.2 and 5.5, [3.5] and [6.2]; 8 over 2 of 128, 1 row [5.9] and [6.1], 4.2 and 9.1, 16 rows 7.2 and
+// 7.6, [4.4] and [9.5]; 4 over 1 of 256, 1 row [7.2] and [7.5], 5.8 and 14.3. Prompts of 1500 tokens and 24 steps, Lenisun of width 1152:
+// 14.3 ms with ranges of 256 keys, 13.2 so.)
 uint32_t decode_splits(const GqaShape& s) {
-    const uint32_t n = (s.ctx + kTile - 1) / kTile;
-    return n < 1 ? 1 : n > 32 ? 32 : n;
+    const uint32_t dim = s.dimp > s.vdimp ? s.dimp : s.vdimp, tiles = (s.ctx + kTile - 1) / kTile, whole = (s.ctx + 4 * kTile - 1) / (4 * kTile);
+    const uint64_t units = (uint64_t)s.kv_heads * ((s.heads / s.kv_heads + 15) / 16) * s.slots;  // CTAs per range
+    uint64_t n = tiles;
+    if (whole <= 1) {
+        if (dim <= 64 || (dim <= 128 && units > 16)) n = 1;
+    } else if (dim <= 128) {
+        const uint64_t fit = (uint64_t)sm_count() * (dim <= 64 ? 4 : 3);
+        n = whole;
+        while (n < tiles && n < 32 && 2 * n * units <= fit) n *= 2;
+        if (n > tiles) n = tiles;
+    }
+    return n < 1 ? 1 : n > 32 ? 32 : (uint32_t)n;
 }
 
 template <int D>
