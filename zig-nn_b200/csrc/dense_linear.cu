@@ -102,18 +102,54 @@ __device__ __forceinline__ uint32_t warp_sums(float (&v)[M], uint32_t lane) {
 // 768 a layer's matrix takes 2.6 us of a step's chain in place of 4.7, the 50304-row vocabulary 32 us in place of 39 (77 MB, 12 us at
 // the memory's rate: short rows leave a warp three chunks and a reduction).
 // GLU: RW counts features, each one gate and one up row.
-// CTAs that an SM has to hold, of a kernel for TR activation rows and NR weight rows per warp. One row: the grids of a step (a CTA
-// per weight row with SK) run at once; with the 68 registers that the compiler takes of its own, 1152 rows are more than a wave and a
-// layer's output projection takes 3.3 us in place of 2.8. More rows: as many as cost no spills.
-template <typename TX, int TR, int RW, bool GLU, bool MOE>
-struct GemvShape {
-    static constexpr int NR = GLU ? 2 * RW : RW;
-    static constexpr int ctas = MOE ? 5 : TR == 1 ? (NR == 1 ? 9 : NR == 2 ? 6 : 4) : GLU ? 1 : sizeof(TX) == 4 ? 3 : RW == 2 && TR != 6 ? 4 : 5;
-    // chunks of a weight row that a lane holds ahead
-    static constexpr int ahead = TR == 1 ? (NR == 1 ? 4 : 2) : NR * TR > 16 ? 1 : NR * TR > 8 ? 2 : 4;
+// Chunks of a weight row that a lane holds ahead, and the CTAs that an SM has to hold (a bound on the registers), of a kernel for TR
+// activation rows and NR weight rows per warp. More chunks hide the memory, more CTAs let a layer's grid run at once; past what the
+// registers hold either one spills. The general rule is for the forms without a line of their own: as many CTAs as cost no spills (five for
+// six rows of two weight rows, 28.8 and 43.9 us for 50304 <- 768 and <- 1152 against 30.1 and 45.2 with four; eight rows spill with five,
+// 42.0 and 65.9 against 33.8 and 52.5 with four). A line of its own has each form that the rule made slower than the kernel of
+// scalar multiply-adds ahead of it was, with the fastest choice of 1, 2, 4 chunks and 1, 3 to 6, 8, 9 CTAs that is not (B200, us, that kernel, the
+// rule, the line): gated bf16, 9000 <- 1152, one row 9.2, 9.4, 8.3, two rows 10.9, 11.7, 10.0; bf16 50304 <- 1152, one row 20.9,
+// 22.0, 20.6, two rows 25.4, 29.1, 23.8, eight rows 50.7, 52.5, 50.2; 1152 <- 6912, two rows 4.86, 5.54, 4.28; f32 2304 <- 768, one row
+// 2.32, 2.50, 1.90, six rows 5.1, 5.9, 4.0, eight rows 5.2, 7.2, 5.1; f32 768 <- 3072, one, two and four rows 2.33, 2.70, 2.31, 3.25, 3.58, 3.26 and
+// 4.75, 5.24, 4.80; f32 50304 <- 1152, one, two and four rows 21.1, 23.6, 20.9, 27.0, 30.5, 26.0 and 42.8, 44.9, 37.1. (One gated row with two
+// chunks and six CTAs is faster alone, 6.4 in place of 7.1 for 6912 <- 1152, and in a step of Lenisun, 146.6 us of 148.3 for four layers, but not in
+// one of Vepinex, 184.2 of 179.6 for six.)
+struct GemvChoice {
+    int ahead, ctas;
 };
 template <typename TX, int TR, int RW, bool SK, bool GLU, bool MOE>
-__global__ void __launch_bounds__(kGemvWarps * 32, GemvShape<TX, TR, RW, GLU, MOE>::ctas)
+constexpr GemvChoice gemv_choice() {
+    constexpr bool F32 = sizeof(TX) == 4;
+    constexpr int NR = GLU ? 2 * RW : RW;
+    constexpr int ahead = TR == 1 ? (NR == 1 ? 4 : 2) : NR * TR > 16 ? 1 : NR * TR > 8 ? 2 : 4;
+    if (MOE) return {ahead, 5};
+    if (GLU) {
+        if (TR == 1 && RW == 2) return F32 ? GemvChoice{4, 4} : GemvChoice{1, 8};
+        if (TR == 2 && RW == 2) return {2, 4};
+        if (TR == 2 && F32) return {2, 6};
+        return {ahead, TR == 1 ? 6 : 1};
+    }
+    if (TR == 1) {
+        if (RW == 2) return {2, 9};
+        return F32 ? (SK ? GemvChoice{1, 8} : GemvChoice{1, 3}) : GemvChoice{ahead, 9};
+    }
+    if (TR == 2 && SK) return F32 ? GemvChoice{1, 8} : GemvChoice{2, 8};
+    if (TR == 2 && RW == 2) return F32 ? GemvChoice{2, 6} : GemvChoice{1, 9};
+    if (F32) {
+        if (TR == 4 && RW == 2) return {2, 6};
+        if (TR == 4 && SK) return {1, 1};
+        if (TR >= 6 && RW == 1 && !SK) return {4, 4};
+        return {ahead, 3};
+    }
+    if (TR == 8 && RW == 2) return {4, 3};
+    return {ahead, RW == 2 && TR != 6 ? 4 : 5};
+}
+template <typename TX, int TR, int RW, bool SK, bool GLU, bool MOE>
+struct GemvShape {
+    static constexpr int ahead = gemv_choice<TX, TR, RW, SK, GLU, MOE>().ahead, ctas = gemv_choice<TX, TR, RW, SK, GLU, MOE>().ctas;
+};
+template <typename TX, int TR, int RW, bool SK, bool GLU, bool MOE>
+__global__ void __launch_bounds__(kGemvWarps * 32, GemvShape<TX, TR, RW, SK, GLU, MOE>::ctas)
 dense_gemv_kernel(const __grid_constant__ GemvParams p) {
     constexpr int NR = GLU ? 2 * RW : RW, P = RW * TR;
     __shared__ float red[SK ? kGemvWarps * NR * TR : 1];
@@ -189,7 +225,7 @@ dense_gemv_kernel(const __grid_constant__ GemvParams p) {
         for (int t = 0; t < TR; ++t) sums[r][t] = 0;
 
     // Chunks of a lane held ahead, of the weights and of the activations: a chunk's registers are loaded again as soon as it is used.
-    constexpr int U = GemvShape<TX, TR, RW, GLU, MOE>::ahead;
+    constexpr int U = GemvShape<TX, TR, RW, SK, GLU, MOE>::ahead;
     constexpr int V = TR * sizeof(TX) <= 2 ? U : TR * sizeof(TX) <= 8 && U > 1 ? 2 : 1;
     uint4 wq[U][NR];
 #pragma unroll
