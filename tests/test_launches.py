@@ -125,3 +125,12 @@ def test_ranges_of_the_decode_attention(library, heads, kv_heads, dim, ctx, slot
         seen, status = library.launches(lambda: lib.zq_gqa_attention(C.byref(g), *[somewhere] * 6, rows, 0, 0, somewhere, 0, None))
         assert status == 0 and "gqa_decode" in seen[0].name and seen[0].grid == (ranges, kv_heads, rows)
         assert len(seen) == (1 if ranges == 1 else 2)
+
+
+@pytest.mark.parametrize("rows,heads,alone", [(1, 4, True), (37, 4, True), (38, 4, False)])
+def test_plain_attention_has_an_sm_per_cta(library, rows, heads, alone):
+    """f32: as long as the CTAs are no more than the SMs, no two of them fit one."""
+    g, somewhere, lib = structs.Gqa(heads, 1, 64, 64, 256, rows, 1.0, 1e-6, 0.0, 0.0), C.c_void_p(1 << 20), library.lib
+    seen, status = library.launches(lambda: lib.zq_gqa_attention(C.byref(g), *[somewhere] * 6, rows, 0, 0, somewhere, 1, None))
+    assert status == 0 and "gqa_plain" in seen[0].name
+    assert (2 * (seen[0].smem + 1024) > 228 * 1024) == alone, seen[0].smem

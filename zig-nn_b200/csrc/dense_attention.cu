@@ -540,7 +540,13 @@ int plain_rows(const GqaShape& s, const void* q, const void* kc, const void* vc,
           const int32_t* pos, const int32_t* slots, uint32_t rows, cudaStream_t st) {
     const dim3 grid(rows, s.heads);
     auto go = [&](auto kern, uint32_t vr) {
-        const size_t smem = (s.dimp + 8 + 4 * 32 * vr) * sizeof(float);
+        // One CTA per SM as long as there are enough: launched while the kernels ahead still sit on the SMs, small CTAs are stacked on
+        // a few of them, the more so the more registers those kernels take (B200, a step of f32 Vepinex, width 768, six layers, us without
+        // and with it: one sequence 255 and 178, two 338 and 189, four 358 and 217, six 377 and 263).
+        size_t smem = (s.dimp + 8 + 4 * 32 * vr) * sizeof(float);
+        constexpr size_t kAlone = 115 * 1024;
+        if ((uint64_t)rows * s.heads <= (uint64_t)sm_count() && smem < kAlone) smem = kAlone;
+        ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAlone));
         return done(launch_pdl(kern, grid, dim3(128), smem, st, s, static_cast<const TA*>(q), static_cast<const TA*>(kc),
                                static_cast<const TA*>(vc), static_cast<TA*>(out), out_pitch, scale, pos, slots));
     };
