@@ -134,3 +134,12 @@ def test_plain_attention_has_an_sm_per_cta(library, rows, heads, alone):
     seen, status = library.launches(lambda: lib.zq_gqa_attention(C.byref(g), *[somewhere] * 6, rows, 0, 0, somewhere, 1, None))
     assert status == 0 and "gqa_plain" in seen[0].name
     assert (2 * (seen[0].smem + 1024) > 228 * 1024) == alone, seen[0].smem
+
+
+@pytest.mark.parametrize("n,k,m", [(1152, 6912, 2), (1152, 6912, 16), (1152, 6912, 17), (768, 768, 16), (1184, 1024, 8), (64, 64, 9)])
+def test_few_ctas_of_the_q8_product_have_an_sm_each(library, n, k, m):
+    """With K over the warps or not: no two CTAs of a grid of at most 148 fit one SM."""
+    w = weight(library, ggml.Q8_0, n, k)
+    product = matmul(library, w, m, ACT_Q8)[0][-1]
+    library.lib.zq_weight_free(w)
+    assert product.grid[0] * product.grid[1] <= 148 and 2 * (product.smem + 1024) > 228 * 1024, (product.name, product.grid, product.smem)

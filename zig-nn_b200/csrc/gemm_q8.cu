@@ -515,15 +515,16 @@ gemm_q8_terms_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__
     }
 }
 
-// Shared memory that a grid asks for: `need`, or as much as leaves no SM room for more than its share of the CTAs, up to `most`.
+// Shared memory that a grid asks for: `need`, or as much as leaves no SM room for more than its share of the CTAs.
 // Under programmatic launches the CTAs of a grid are placed while those of the kernels before it still sit on the SMs, and
 // small ones are then stacked on a few of them. (B200, prompts and steps of several sequences, ms without and with it, products
 // of this file only: eight sequences of 4_1 weights 33.4 and 31.4, six of 4_0 17.2 and 15.6, four of 8_0 21.7 and 20.6; a prompt of 600
-// tokens and 17 steps of 8_0 30.9 and 29.9.)
-uint32_t spread_smem(uint64_t ctas, uint32_t need, uint32_t most) {
+// tokens and 17 steps of 8_0 30.9 and 29.9. Alone: 1152 <- 6912 4_0 at 12 and 17 rows, 144 CTAs, 12.4 -> 11.7 and 16.7 -> 16.0 us.)
+constexpr uint32_t kAlone = 115 * 1024;  // no second CTA finds as much
+uint32_t spread_smem(uint64_t ctas, uint32_t need) {
     const uint64_t sms = (uint64_t)sm_count(), share = (ctas + sms - 1) / sms;
     const uint64_t spread = (227 * 1024 / (share + 1) + 128) & ~(uint64_t)127;
-    return spread < need ? need : spread > most ? most : (uint32_t)spread;
+    return spread < need ? need : spread > kAlone ? kAlone : (uint32_t)spread;
 }
 
 constexpr uint32_t kMostGridY = 65535;
@@ -537,9 +538,9 @@ int launch_terms(const zq_weight* w, const int8_t* xq, const float* xs, const in
     const dim3 grid((w->out_dim + 8 * NTL - 1) / (8 * NTL), (M + 15) / 16);
     if (grid.y > kMostGridY) return ZQ_ERR_LIMIT;
     auto kern = gemm_q8_terms_kernel<TYPE, NTL, WIDE>;
-    const uint32_t smem = spread_smem((uint64_t)grid.x * grid.y, per * kBlockBytes, kMost * kBlockBytes);
+    const uint32_t smem = spread_smem((uint64_t)grid.x * grid.y, per * kBlockBytes);
     // the most that any call asks for: the limit is the process's, and another thread may be about to launch a deeper matrix
-    ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kMost * kBlockBytes)));
+    ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAlone));
     ZQ_CUDA(launch_pdl_split(split, kern, grid, dim3(kTermWarps * 32), smem, st, w->qs,
                        static_cast<const uint8_t*>(w->sc), xq, xs, xsum, y, w->out_dim, w->in_dim, M, w->nb, w->scp, per, ep));
     return ZQ_OK;
@@ -550,12 +551,12 @@ int launch_cfg(const zq_weight* w, const int8_t* xq, const float* xs, const int3
                QgEpilogue ep, bool split, cudaStream_t st) {
     const dim3 grid((w->out_dim + W * MT * 16 - 1) / (W * MT * 16), (M + NT * 8 - 1) / (NT * 8));
     if (grid.y > kMostGridY) return ZQ_ERR_LIMIT;
-    constexpr uint32_t kRing = D * QgStage<TYPE, W, MT, NT>::kBytes, kMost = 115 * 1024;
-    static_assert(kRing <= kMost, "ring");
-    const uint32_t smem = spread_smem((uint64_t)grid.x * grid.y, kRing, kMost);
+    constexpr uint32_t kRing = D * QgStage<TYPE, W, MT, NT>::kBytes;
+    static_assert(kRing <= kAlone, "ring");
+    const uint32_t smem = spread_smem((uint64_t)grid.x * grid.y, kRing);
     auto kern = gemm_q8_kernel<TYPE, W, MT, NT, D>;
     // the most that any call asks for: the limit is the process's, and another thread may be about to launch a larger grid
-    ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMost));
+    ZQ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kAlone));
     ZQ_CUDA(launch_pdl_split(split, kern, grid, dim3(W * 32), smem, st, w->qs,
                        static_cast<const uint8_t*>(w->sc), xq, xs, xsum, y, w->out_dim, w->in_dim, M, w->nb, w->scp, 1.0f, ep));
     return ZQ_OK;
