@@ -24,6 +24,9 @@
 // only shape 1 gains. (The same on tcgen05.mma.kind::i8, a block per MMA of K = 32 and the scaling behind tcgen05.ld, came to 76 and 54
 // us for the two 512-row products, and was slower than this form at all smaller ones: about 8 cycles of an SM for a column of
 // 128 weight rows and a block, where its three f32 operations need 3.)
+// What a CTA takes besides its blocks counts for short rows: the copies' sources are 32-bit offsets from the CTA's first rows, and the
+// sums leave by rows without the epilogue's questions where it has none (30000 <- 320 8_0 at 64 and 512 rows 16.2 and 80.0 us with 64-bit
+// products per piece, 12.8 and 56.7 so).
 #include "zq_internal.h"
 
 namespace zq {
@@ -157,45 +160,49 @@ gemm_q8_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc, c
     const uint32_t n0 = blockIdx.x * QG_BN + warp * (MT * 16), m0 = blockIdx.y * QG_BM;
     const uint32_t wring = smem32 + S::kAct + warp * S::kWarp;  // this warp's part of stage 0
 
-    // Sources of this thread's copies of quad 0; a quad further they lie a constant number of bytes on.
+    // Sources of this thread's copies of quad 0, as offsets from the first of the CTA's rows; a quad further they lie a constant number
+    // of bytes on.
     // Weights: the words of its own rows g and g + 8 of each tile. 8_0: words 2t and 2t + 1 of the four blocks are 32 contiguous
     // bytes; 4-bit: word t, whose low nibbles are the block's word t and whose high ones its word 4 + t.
     // Scales: a lane per row of the warp. Activations: xq entries [blk][row][32 bytes], scales [blk][row], sums [blk][row]; rows
     // >= M and blocks >= nb are zero-filled (never used for output).
     uint32_t w_off[MT * 2];
 #pragma unroll
-    for (int r = 0; r < MT * 2; ++r) w_off[r] = min(n0 + r * 8 + g, N - 1) - min(n0, N - 1);
-    const uint8_t* w_base = qs + (size_t)min(n0, N - 1) * nbp * QB + 16 * t;
+    for (int r = 0; r < MT * 2; ++r) w_off[r] = (min(n0 + r * 8 + g, N - 1) - min(n0, N - 1)) * (nbp * QB);
+    const uint8_t* w_src = qs + (size_t)min(n0, N - 1) * nbp * QB + 16 * t;
     const uint8_t* s_src = sc + (size_t)min(n0 + (uint32_t)lane % (MT * 16), N - 1) * scp * (Q41 ? 4 : 2);
-    constexpr int XP = (8 * QG_BM + T - 1) / T, SP = (4 * QG_BM + T - 1) / T;  // pieces of a thread
+    constexpr int XP = (8 * QG_BM + T - 1) / T, SP = (4 * QG_BM + T - 1) / T;  // pieces of a thread, T / 8 and T / 4 rows apart
+    // a thread's pieces are of one block and half (T / 8 rows apart in the activations), of one block (T / 4 in the scales)
+    const uint32_t xr = tid >> 3, xb = (tid >> 1) & 3u, xh = tid & 1u, sr = tid >> 2, sb = tid & 3u;
+    const int8_t* x_src = xq + (size_t)m0 * K;
+    const float* sc_src = xscale + (size_t)m0 * nb;
+    const int32_t* qsum_src = xqsum + (size_t)m0 * nb;
+    const uint32_t x_off = xr * K + (tid & 7u) * 16, s_off = sr * nb + sb, rows = M - m0;
+    // 4-bit: the halves of rows with bit 2 set change places, or the fragment loads would meet in a bank
+    static_assert(T % 64 == 0, "pieces of a thread lie a multiple of eight rows apart");
+    const uint32_t x_to = ((xb * QG_BM + xr) * 2 + (Q8 ? xh : xh ^ ((xr >> 2) & 1u))) * 16, s_to = QG_XQ_BYTES + (sb * QG_BM + sr) * 4;
     auto issue = [&](uint32_t stage, uint32_t q) {
-        const uint32_t base = smem32 + stage * QG_STAGE;
+        const uint32_t base = smem32 + stage * QG_STAGE, left = nb - q * 4;  // blocks from this quad on
 #pragma unroll
-        for (int i = 0; i < XP; ++i) {  // (row, blk, half): a row's 128 bytes by eight neighbouring threads
-            const uint32_t idx = tid + i * T;
-            if (8 * QG_BM % T == 0 || idx < 8u * QG_BM) {
-                const uint32_t r = idx >> 3, b = (idx >> 1) & 3u, h = idx & 1u, m = m0 + r;
-                const bool ok = m < M && q * 4 + b < nb;
-                // 4-bit: the halves of rows with bit 2 set change places, or the fragment loads would meet in a bank
-                const uint32_t to = ((b * QG_BM + r) * 2 + (Q8 ? h : h ^ ((r >> 2) & 1u))) * 16;
-                cp_async16_zfill(base + to, xq + (ok ? (size_t)m * K + q * 128 + (idx & 7u) * 16 : 0), ok ? 16u : 0u);
+        for (int i = 0; i < XP; ++i) {
+            if (8 * QG_BM % T == 0 || tid + i * T < 8 * QG_BM) {
+                const bool ok = xr + i * (T / 8) < rows && xb < left;
+                cp_async16_zfill(base + x_to + i * (T / 8) * 32, x_src + (ok ? x_off + i * (T / 8) * K + q * 128 : 0), ok ? 16u : 0u);
             }
         }
 #pragma unroll
-        for (int i = 0; i < SP; ++i) {  // (row, blk)
-            const uint32_t idx = tid + i * T;
-            if (4 * QG_BM % T == 0 || idx < 4u * QG_BM) {
-                const uint32_t r = idx >> 2, b = idx & 3u, m = m0 + r;
-                const bool ok = m < M && q * 4 + b < nb;
-                const size_t o = ok ? (size_t)m * nb + q * 4 + b : 0;
-                cp_async4_zfill(base + QG_XQ_BYTES + (b * QG_BM + r) * 4, xscale + o, ok ? 4u : 0u);
-                if (Q41) cp_async4_zfill(base + QG_XQ_BYTES + QG_SC_BYTES + (b * QG_BM + r) * 4, xqsum + o, ok ? 4u : 0u);
+        for (int i = 0; i < SP; ++i) {
+            if (4 * QG_BM % T == 0 || tid + i * T < 4 * QG_BM) {
+                const bool ok = sr + i * (T / 4) < rows && sb < left;
+                const uint32_t o = ok ? s_off + i * (T / 4) * nb + q * 4 : 0;
+                cp_async4_zfill(base + s_to + i * (T / 4) * 4, sc_src + o, ok ? 4u : 0u);
+                if (Q41) cp_async4_zfill(base + s_to + QG_SC_BYTES + i * (T / 4) * 4, qsum_src + o, ok ? 4u : 0u);
             }
         }
         const uint32_t wb = wring + stage * QG_STAGE;
 #pragma unroll
         for (int r = 0; r < MT * 2; ++r) {
-            const uint8_t* from = w_base + (size_t)w_off[r] * nbp * QB + (size_t)q * QUAD;
+            const uint8_t* from = w_src + (w_off[r] + q * QUAD);
             if (Q8) {  // piece w of a row at w ^ (row & 1): the lanes of a fragment load meet in no bank
                 const uint32_t to = wb + (r * 8 + g) * 128 + ((t ^ (g & 1)) << 4);
                 cp_async16(to, from);
@@ -206,8 +213,8 @@ gemm_q8_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc, c
         }
         if (MT == 2 || lane < 16) {
             const uint32_t to = wb + S::kWq + lane * S::kRowScales;
-            if (Q41) cp_async16(to, s_src + (size_t)q * 16);
-            else cp_async8(to, s_src + (size_t)q * 8);
+            if (Q41) cp_async16(to, s_src + q * 16);
+            else cp_async8(to, s_src + q * 8);
         }
     };
 
@@ -320,24 +327,29 @@ gemm_q8_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__ sc, c
     }
     asm volatile("cp.async.wait_all;" ::: "memory");
 
+    const bool plain = !ep.bias && !ep.gelu && !ep.mul && !ep.residual;
 #pragma unroll
-    for (int i = 0; i < MT; ++i)
+    for (int j = 0; j < NT; ++j)
 #pragma unroll
-        for (int j = 0; j < NT; ++j)
+        for (int c = 0; c < 2; ++c) {
+            const uint32_t m = m0 + j * 8 + 2 * t + c;
+            if (m >= M) continue;
+            const size_t row = (size_t)m * N;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-                const uint32_t n = n0 + i * 16 + g + (e >> 1) * 8;
-                const uint32_t m = m0 + j * 8 + 2 * t + (e & 1);
-                if (n < N && m < M) {
-                    const size_t o = (size_t)m * N + n;
-                    float v = __uint_as_float((uint32_t)(e & 1 ? run[i][j][e >> 1] >> 32 : run[i][j][e >> 1]));
+            for (int r = 0; r < MT * 2; ++r) {
+                const uint32_t n = n0 + r * 8 + g;
+                if (n >= N) continue;
+                const f32x2 pair = run[r >> 1][j][r & 1];
+                float v = __uint_as_float((uint32_t)(c ? pair >> 32 : pair));
+                if (!plain) {
                     if (ep.bias) v = __fadd_rn(v, ep.bias[n]);
                     if (ep.gelu) v = gelu_tanh(v);
-                    if (ep.mul) v = __fmul_rn(v, ep.mul[o]);
-                    if (ep.residual) v = __fadd_rn(ep.residual[o], v);
-                    y[o] = v;
+                    if (ep.mul) v = __fmul_rn(v, ep.mul[row + n]);
+                    if (ep.residual) v = __fadd_rn(ep.residual[row + n], v);
                 }
+                y[row + n] = v;
             }
+        }
 }
 
 // ---- the same for products that leave the GPU idle: K split over the warps of a CTA -------------------
