@@ -315,12 +315,14 @@ def test_split_product_in_every_tile(zq, oracle, qtype, n, k, m):
 
 
 # Sizes that take each of the CTA shapes of gemm_q8.cu (test_launches.py holds them to it), with rows, columns and blocks that fill no
-# tile; 5003 <- 96 takes two weight tiles per warp.
-Q8_SHAPES = [(2003, 96, 509), (1147, 160, 505), (1531, 64, 500), (5003, 64, 45), (700, 32, 30), (17, 480, 9), (5003, 96, 205)]
+# tile; 4_1 takes the largest only where the others have more rows of CTAs than a grid.
+Q8_SHAPES = {t: [(2003, 96, 509), (1147, 160, 505), (1531, 64, 500), (5003, 64, 45), (700, 32, 30), (17, 480, 9), (5003, 96, 205)] for t in TYPES}
+Q8_SHAPES[ggml.Q4_0] += [(18538, 288, 35)]
+Q8_SHAPES[ggml.Q4_1] += [(258, 32, 485), (9, 32, 2097121)]
+Q8_SHAPES[ggml.Q8_0] += [(4763, 32, 23)]
 
 
-@pytest.mark.parametrize("qtype", TYPES)
-@pytest.mark.parametrize("n,k,m", Q8_SHAPES)
+@pytest.mark.parametrize("qtype,n,k,m", [(t, *s) for t in TYPES for s in Q8_SHAPES[t]])
 def test_q8_product_in_every_cta_shape(zq, oracle, qtype, n, k, m):
     raw = make_weight(oracle, qtype, n, k, seed=n)
     x = make_x(m, k, seed=m)

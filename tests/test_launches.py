@@ -82,7 +82,7 @@ def test_q8_rows_up_to_the_limit_of_a_grid(library, n):
 def test_sizes_of_the_q8_product_test_take_every_shape(library, qtype):
     """Of test_gpu_quant.py: (warps, weight tiles per warp, column tiles) of the kernel that each of its sizes launches on 148 SMs."""
     taken = set()
-    for n, k, m in Q8_SHAPES:
+    for n, k, m in Q8_SHAPES[qtype]:
         w = weight(library, qtype, n, k)
         name = matmul(library, w, m, ACT_Q8)[0][-1].name
         taken.add(tuple(int(v) for v in re.search(r"gemm_q8_kernelILi\d+ELi(\d+)ELi(\d+)ELi(\d+)E", name).groups()))

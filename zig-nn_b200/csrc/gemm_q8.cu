@@ -18,10 +18,10 @@
 // What bounds it: issue slots and their latencies around the scaling. Per MMA tile of 16 x 8 that is four conversions and, two
 // columns at a time (f32x2), two multiplies and an add for each of its pairs; 4_0 weights are centred before the product, so
 // that no sum of activations is needed. Against one column at a time and sums subtracted behind the product (B200, us with the
-// quantiser and weights from HBM, before and after): 14336 <- 4096 4_0 at 8, 64 and 140 rows 27.4, 91.8, 180 and 22.3, 56.2, 101; 262144 <-
-// 1152 4_1 at 8 rows 86.3 and 58.4; 13824 <- 1152 8_0 at 16, 88 and 512 rows 15.5, 32.4, 91.2 and 11.8, 26.2, 89.2; 1152 <- 6912 8_0 at 512
-// rows 112 and 70.6 (its shape, cheapest_shape). Two weight tiles per warp (MT) share the activation fragments, which costs registers:
-// only shape 1 gains. (The same on tcgen05.mma.kind::i8, a block per MMA of K = 32 and the scaling behind tcgen05.ld, came to 76 and 54
+// quantiser and weights from HBM, before and now): 14336 <- 4096 4_0 at 8, 64 and 140 rows 27.3, 92.2, 181 and 22.0, 50.3, 94.5; 262144 <-
+// 1152 4_1 at 8 rows 87.0 and 65.1; 13824 <- 1152 8_0 at 16, 100 and 512 rows 14.2, 32.5, 91.1 and 9.5, 24.7, 84.8; 1152 <- 6912 8_0 at 512
+// rows 112 and 67.6 (its shape, cheapest_shape). Two weight tiles per warp (MT) share the activation fragments, which costs registers:
+// only shape 1 has them. (The same on tcgen05.mma.kind::i8, a block per MMA of K = 32 and the scaling behind tcgen05.ld, came to 76 and 54
 // us for the two 512-row products, and was slower than this form at all smaller ones: about 8 cycles of an SM for a column of
 // 128 weight rows and a block, where its three f32 operations need 3.)
 // What a CTA takes besides its blocks counts for short rows: the copies' sources are 32-bit offsets from the CTA's first rows, and the
@@ -574,26 +574,36 @@ int launch_cfg(const zq_weight* w, const int8_t* xq, const float* xs, const int3
     return ZQ_OK;
 }
 
-// CTA shape: the one whose busiest SM is through a block of K first, by a count of cycles. A CTA holds W * MT * NT MMA tiles; an SM
-// that is full takes `per_tile` cycles for one (more tiles per warp share the fragments of a block), and no warp is through its own
-// tiles before `least`. Measured on a B200 with the quantiser, weights from HBM, us for shapes 0 to 4: 13824 <- 1152 8_0 at 24 rows 20.3,
-// 17.5, 15.0, 14.3, 20.7, at 88 rows 31.9, 30.0, 28.0, 32.0, 53, at 512 rows 89.7, 105, 105, 136, 264; 1152 <- 6912 8_0 at 512 rows
-// 103, 75, 72, 97, 127; 5003 <- 1184 4_0 at 45 rows 20.7, 17.6, 14.0, 10.8, 13.0. The count takes the best of the five or one within
-// 7 % of it for the three types, 1152 to 262144 weight rows and 2 to 512 activation rows. A shape whose rows of CTAs are more than a
+// CTA shape: the one whose busiest SM is through first, by a count of nanoseconds. A CTA holds W * MT * NT MMA tiles. An SM that is full
+// takes `tile` for one of them and a block of K, and `tile_start` for the start and the sums of each; no warp is through its own tiles
+// before `block` for a block and `start`; of the two a geometric sum. The constants are a fit to 671 calls of 17 matrices (96 to 6912
+// columns) at 2 to 1000 rows, in all five shapes, nudged where the choice was not the fastest: it is within 11 % of the fastest for each
+// type, 0.3 to 0.7 % in the mean (the count of blocks alone, the same for all types, within 34 %, 1.5 to 5.1 % in the mean).
+// Measured on a B200 with the quantiser, weights from HBM, us for shapes 0 to 4, the one taken in brackets: 30000 <- 320 8_0 at 333 rows 43.6, [41.9],
+// 47.3, 55.8, 101; 30000 <- 640 4_1 at 333 rows 97.3, [74.1], 90.5, 93.6, 126; 3000 <- 512 4_0 at 24 rows 8.8, 6.8, 6.2, 4.9, [4.3]; 8000 <- 1152 4_1 at
+// 200 rows 38.7, [28.0], 31.8, 31.4, 40.4; 1152 <- 6912 8_0 at 140 rows 94.5, 57.8, 43.3, [39.0], 41.9. A shape whose rows of CTAs are more than a
 // grid has is left out; the first one, of the most columns, remains for the launch to refuse.
-int cheapest_shape(uint32_t n, uint32_t m, uint32_t sms) {
+template <int TYPE>
+int cheapest_shape(uint32_t n, uint32_t m, uint32_t nb, uint32_t sms) {
     struct Shape {
-        uint32_t rows, cols, tiles, per_tile, least;  // per_tile in tenths of a cycle
+        uint32_t rows, cols, tiles;
+        float tile, tile_start, block, start;
     };
-    constexpr Shape shapes[5] = {{128, 64, 64, 113, 740}, {128, 32, 32, 130, 560}, {64, 32, 16, 135, 370}, {64, 16, 8, 175, 255}, {64, 8, 4, 340, 215}};
+    constexpr bool Q41 = TYPE == ZQ_TYPE_Q4_1, Q8 = TYPE == ZQ_TYPE_Q8_0;
+    constexpr Shape shapes[5] = {
+        Q41 ? Shape{128, 64, 64, 6.9f, 8, 222, 290} : Q8 ? Shape{128, 64, 64, 5.2f, 10, 263, 0} : Shape{128, 64, 64, 4.5f, 11, 154, 22},
+        Q41 ? Shape{128, 32, 32, 6.1f, 6, 170, 65} : Q8 ? Shape{128, 32, 32, 5.5f, 13, 179, 0} : Shape{128, 32, 32, 4.8f, 9, 148, 0},
+        Q41 ? Shape{64, 32, 16, 7.3f, 12, 161, 96} : Q8 ? Shape{64, 32, 16, 6.2f, 16, 146, 150} : Shape{64, 32, 16, 5.7f, 12, 144, 170},
+        Q41 ? Shape{64, 16, 8, 7.5f, 20, 101, 78} : Q8 ? Shape{64, 16, 8, 7.7f, 27, 93, 190} : Shape{64, 16, 8, 7.3f, 19, 92, 122},
+        Q41 ? Shape{64, 8, 4, 10.8f, 35, 86, 0} : Q8 ? Shape{64, 8, 4, 14.9f, 60, 77, 1} : Shape{64, 8, 4, 11.3f, 35, 90, 0}};
     int best = 0;
-    uint64_t least = ~0ull;
+    float least = INFINITY;
     for (int i = 0; i < 5; ++i) {
         const Shape& s = shapes[i];
         if (i && (m - 1) / s.cols >= kMostGridY) continue;
         const uint64_t ctas = (uint64_t)((n + s.rows - 1) / s.rows) * ((m - 1) / s.cols + 1);
-        uint64_t cost = (ctas + sms - 1) / sms * s.tiles * s.per_tile;
-        if (cost < s.least * 10ull) cost = s.least * 10ull;
+        const float full = (float)((ctas + sms - 1) / sms * s.tiles) * (s.tile * nb + s.tile_start), warp = s.block * nb + s.start;
+        const float cost = full * full + warp * warp;
         if (cost < least) {
             least = cost;
             best = i;
@@ -625,7 +635,7 @@ int launch_one(const zq_weight* w, const int8_t* xq, const float* xs, const int3
     if (M > 8 && (tiles <= sms ? nb >= 16 : tiles <= most && nb >= 24))
         return tiles <= 192 ? launch_terms<TYPE, 1, true>(w, xq, xs, xsum, y, M, ep, split, st)
                             : launch_terms<TYPE, 2, true>(w, xq, xs, xsum, y, M, ep, split, st);
-    switch (cheapest_shape(w->out_dim, M, (uint32_t)sms)) {
+    switch (cheapest_shape<TYPE>(w->out_dim, M, nb, (uint32_t)sms)) {
         case 0: return launch_cfg<TYPE, 8, 1, 8, 3>(w, xq, xs, xsum, y, M, ep, split, st);
         case 1: return launch_cfg<TYPE, 4, 2, 4, 3>(w, xq, xs, xsum, y, M, ep, split, st);
         case 2: return launch_cfg<TYPE, 4, 1, 4, 3>(w, xq, xs, xsum, y, M, ep, split, st);
