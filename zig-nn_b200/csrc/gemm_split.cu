@@ -475,11 +475,11 @@ int launch_type(const zq_weight* w, const SplitImage& im, float* y, uint32_t M, 
 
 }  // namespace
 
-// Up to 20 rows the last pass has at most four and costs the least, while the product pads to 24 rows or 32. On matrices whose
-// tiles of 32 x 32 do not run all at once the passes stay ahead, unless K is so deep that a pass holds two rows or the
-// matrix so large that its passes take the ring (B200, us in passes and split, 17 rows: 5760 <- 6144 8_0 62.8 and 78.9, 9472 <-
-// 5120 4_1 57.1 and 69.4; 4096 <- 6144 8_0 as 0.65; 6912 <- 14336 4_0 as 0.63; 8192 <- 8192 8_0 as 0.42; 24 rows of 5760 <- 6144
-// 8_0 level, 25 as 0.88).
+// Up to 20 rows the calls of more weight rows than 32 per SM stay with the passes (unless K is so deep that a pass holds two rows, or
+// the matrix so large that its passes take the ring): where a call needs a workspace is a line that callers have sized theirs by, and
+// it was drawn when these calls took tiles of 32 x 32 in turns. With the tiles of now the product is ahead there too (B200, us in passes and
+// split at 17 rows: 5760 <- 6144 4_0 84.5 and 39.2, 9472 <- 5120 4_1 60.5 and 40.3, 12000 <- 512 4_0 13.2 and 7.8), and closer to 64 bits with 4-bit
+// weights (4_0 8.2e-7 in passes, 1.1e-7 split), though not with 8_0 of few columns (11000 <- 1152 0.95e-7 and 1.06e-7).
 bool gemm_split_takes(const zq_weight* w, uint32_t m_rows) {
     if (m_rows < 17) return false;
     const bool ring = w->type != ZQ_TYPE_Q4_1 && (size_t)w->out_dim * w->nbp * w->qb >= ((size_t)64 << 20);

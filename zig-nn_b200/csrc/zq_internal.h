@@ -208,7 +208,7 @@ int launch_gemm_trans_pair(const zq_weight* w, const float* grad_out, float* gra
 int launch_gemm_split(const zq_weight* w, const float* x, float* y, uint32_t m_rows, const zq_epilogue* ep, void* workspace,
                       cudaStream_t st);
 size_t gemm_split_workspace_bytes(const zq_weight* w, uint32_t m_rows);
-// Whether it is faster than passes of up to 16 rows (gemm_split.cu); from 17 rows on.
+// Whether it takes the call from the passes of up to 16 rows (gemm_split.cu); from 17 rows on.
 bool gemm_split_takes(const zq_weight* w, uint32_t m_rows);
 constexpr uint32_t kStreamMinRowsF32 = 17;  // f32-activation calls from this many rows on take it when they bring a workspace
 
