@@ -494,6 +494,7 @@ int zq_gemma3_decode_greedy(zq_gemma3* m, uint32_t first_token, uint32_t n_steps
  *   zq_gemma3_create_batch      n_seq cache slots (1 <= n_seq <= 1024); n_seq == 1 is zq_gemma3_create
  *   zq_gemma3_prefill_seq       prefill of sequence `seq`; *d_logits = its last token's logits [vocab]
  *   zq_gemma3_decode_next_batch h_tokens[n_seq] = next token of every sequence; *d_logits = [n_seq][vocab]
+ *                               (a stream that is capturing is refused, ZQ_ERR_CUDA: the call advances the host's lengths)
  *   zq_gemma3_seq_len_of        tokens held by sequence `seq`
  * zq_gemma3_decode_next / _decode_greedy need n_seq == 1. */
 int zq_gemma3_create_batch(const zq_gemma3_config* cfg, const zq_gemma3_weights* w, uint32_t n_seq,
@@ -732,7 +733,8 @@ int zq_decoder_prefill_seq(zq_decoder* m, uint32_t seq, const uint32_t* h_tokens
                            const float** d_logits);
 /* The next token of one sequence. */
 int zq_decoder_decode_next(zq_decoder* m, uint32_t seq, uint32_t token, zq_stream stream, const float** d_logits);
-/* The next token of n different sequences h_seqs[n] at once; *d_logits = [n][vocab]. */
+/* The next token of n different sequences h_seqs[n] at once; *d_logits = [n][vocab]. The arrays may change when the call is
+ * back. A stream that is capturing is refused (ZQ_ERR_CUDA): the call advances the host's lengths. */
 int zq_decoder_decode_next_batch(zq_decoder* m, const uint32_t* h_seqs, const uint32_t* h_tokens, uint32_t n,
                                  zq_stream stream, const float** d_logits);
 /* n_steps greedy steps of one sequence, the arg-max feeding the next step on the device. */

@@ -569,6 +569,29 @@ def test_batched_sequences_equal_each_alone(zq, dtype):
             assert eng.seq_len_of(i) == lens[i] + at[i]
     eng.check()
 
+def test_step_of_more_sequences_than_one_kernel_sets(zq):
+    """300 sequences, rows in any order of slots: tokens, positions and slots go to the device 256 rows at a time. All of them (the
+    recorded step), then a few less; rows at the borders against each sequence alone."""
+    cfg = dict(MODELS["attention_only"], layers=MODELS["attention_only"]["layers"][2:])
+    host = hostmodel.LenisunHost.synthetic(cfg, seed=3, std=0.25)
+    n, rng = 300, np.random.default_rng(7)
+    eng, alone = zq.Lenisun(host, ctx=16, n_seq=n, dtype="float32"), zq.Lenisun(host, ctx=16, dtype="float32")
+    fed = [[] for _ in range(n)]
+    for count in (n, n, n, 290, 257, n):
+        slots = list(rng.permutation(n)[:count])
+        tokens = [int(t) for t in rng.integers(0, cfg["vocab"], count)]
+        logits = eng.decode_next_batch(slots, tokens)
+        for s, t in zip(slots, tokens):
+            fed[s].append(t)
+        for r in (0, 1, 255, 256, count - 1):
+            s = slots[r]
+            alone.reset()
+            want = alone.extend(fed[s], [len(fed[s]) - 1])
+            assert row_err(logits[r:r + 1], want.cpu().numpy()).max() <= TOL["float32"], (count, r)
+            assert eng.seq_len_of(s) == len(fed[s])
+    eng.check()
+
+
 
 @pytest.mark.parametrize("dtype", ["float32", "bfloat16"])
 @pytest.mark.parametrize("name", ["mixed", "recurrence_only"])

@@ -106,6 +106,25 @@ def test_gemma3_batched_sequences_bit_exact(zq, oracle):
             toks[i] = int(np.argmax(lc))
     assert [eng.seq_len(i) for i in range(n_seq)] == [len(p) + steps for p in prompts]
 
+def test_gemma3_step_of_more_sequences_than_one_kernel_sets(zq):
+    """300 sequences: tokens and positions go to the device 256 rows at a time; the bits of each sequence alone."""
+    cfg = dict(GEMMA_TINY, layer=2, vocab=256, ctx=16)
+    host = hostmodel.Gemma3Host.synthetic(cfg, qtype=ggml.Q8_0, seed=9, std=0.08).randomize_small_params()
+    n, rng = 300, np.random.default_rng(8)
+    eng, alone = zq.Gemma3Batch(host, n), zq.Gemma3(host)
+    fed = [[int(t) for t in rng.integers(0, 256, size=1 + s % 3)] for s in range(n)]
+    for s in range(n):
+        eng.prefill(s, fed[s])
+    for _ in range(4):
+        tokens = rng.integers(0, 256, size=n)
+        logits = eng.decode_next(tokens)
+        for s in range(n):
+            fed[s].append(int(tokens[s]))
+        for s in (0, 1, 255, 256, 299):
+            assert torch.equal(logits[s], alone.prefill(fed[s])), s
+            assert eng.seq_len(s) == len(fed[s])
+
+
 
 def test_device_greedy_loop_matches_stepwise(zq):
     host = hostmodel.Gemma3Host.synthetic(GEMMA_TINY, qtype=ggml.Q8_0, seed=3, std=0.08)

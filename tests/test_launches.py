@@ -9,7 +9,7 @@ from host_runtime import Library, build
 from test_gpu_quant import Q8_SHAPES, SPLIT_SIZES
 from zignn_b200 import ggml, hostmodel, structs
 
-ACT_F32, ACT_Q8, ERR_LIMIT = 0, 1, 5
+ACT_F32, ACT_Q8, ERR_CUDA, ERR_LIMIT = 0, 1, 3, 5
 
 
 @pytest.fixture(scope="module")
@@ -143,3 +143,26 @@ def test_few_ctas_of_the_q8_product_have_an_sm_each(library, n, k, m):
     product = matmul(library, w, m, ACT_Q8)[0][-1]
     library.lib.zq_weight_free(w)
     assert product.grid[0] * product.grid[1] <= 148 and 2 * (product.smem + 1024) > 228 * 1024, (product.name, product.grid, product.smem)
+
+
+def test_a_step_of_several_sequences_is_refused_while_its_stream_captures(library):
+    """It advances the host's lengths, so a recording could not be replayed: nothing is launched and no length changes."""
+    engine, lg, lib, n = decoder(library), C.c_void_p(), library.lib, C.c_uint32()
+    step = lambda: lib.zq_decoder_decode_next_batch(engine, pointer(u32([2, 0])), pointer(u32([1, 2])), 2, None, C.byref(lg))
+    lib.set_capturing(1)
+    seen, status = library.launches(step)
+    lib.set_capturing(0)
+    assert status == ERR_CUDA and not seen
+    assert lib.zq_decoder_seq_len_of(engine, 2, C.byref(n)) == 0 and n.value == 0
+    assert step() == 0 and lib.zq_decoder_seq_len_of(engine, 2, C.byref(n)) == 0 and n.value == 1
+    lib.zq_decoder_free(engine)
+
+
+@pytest.mark.parametrize("rows,kernels", [(256, 1), (257, 2), (300, 2), (600, 3)])
+def test_rows_of_a_step_in_portions(library, rows, kernels):
+    engine, lg, lib = decoder(library, n_seq=rows), C.c_void_p(), library.lib
+    seen, status = library.launches(lambda: lib.zq_decoder_decode_next_batch(
+        engine, pointer(u32(range(rows))), pointer(u32([1] * rows)), rows, None, C.byref(lg)))
+    assert status == 0 and ["set_step_rows" in l.name for l in seen[:kernels + 1]] == [True] * kernels + [False]
+    assert not seen[kernels].dependent
+    lib.zq_decoder_free(engine)
