@@ -4,8 +4,8 @@
 // (ThreadPool.matmul, src/gguf/thread_pool.zig:96-181 -> src/gguf/simd_dot.zig:71-152): per 32-block an
 // exact int8 x int8 -> int32 dot, turned into the f32 term (d * s) * float(idot) [+ (m * s) * float(qsum)],
 // and the terms of a row added in block order. Here the block dots of 16 weight rows x 8 activation rows
-// come from one mma.sync.m16n8k32 (s8 x s8 -> s32, exact), the weights are read once per 64 activation
-// rows instead of once per row, and each (weight row, activation row) pair keeps its running f32 sum in
+// come from one mma.sync.m16n8k32 (s8 x s8 -> s32, exact), the weights are read once per CTA's 8 to
+// 64 activation rows instead of once per row, and each (weight row, activation row) pair keeps its running f32 sum in
 // a register, so the result is bit-identical to running the decode kernel row by row.
 //
 // Tile: W warps x MT x 16 weight rows, NT x 8 activation rows per CTA; K advances by one quad of blocks
@@ -397,7 +397,8 @@ gemm_q8_terms_kernel(const uint8_t* __restrict__ qs, const uint8_t* __restrict__
     }
     const uint32_t row_a = min(m0 + g, M - 1), row_b = min(m0 + g + 8, M - 1);
     pdl_launch_dependents();
-    // the weight rows on their way into L2 while the kernel before this one still runs
+    // the weight rows on their way into L2 while the kernel before this one still runs (the engines' quantisers, which let this one
+    // start early; behind the quantiser of a single call, a plain launch, this begins when that has ended)
     if (tid < 8 * NTL && n0 + tid < N) {
         const uint8_t* row = qs + (size_t)(n0 + tid) * nbp * QB;
         for (uint32_t o = 0; o < nbp * QB; o += 16384) prefetch_l2_bulk(row + o, min(nbp * QB - o, 16384u));
